@@ -4,44 +4,16 @@
 // (three passes: row maximum, sum of exponentials, normalise), attention-output.glsl / attention-output-gpt.glsl
 // (weights . V, the GPT form summing only over k <= q) and attention-backward.glsl (grad_V = A^T gO; grad_A = gO V^T;
 // softmax backward; grad_Q, grad_K).  The fused kernels are the fast path; these exist so that code written against
-// the separate shaders keeps working, and so that training code has a backward.  Every product is one strided,
-// batched, shared-memory tiled float32 GEMM with the sum over the inner index in ascending order, as the
-// shaders' loops run.
+// the separate shaders keeps working, and so that training code has a backward.  Every product is a batched float32
+// product of sgemm.cuh with the sum over the inner index in ascending order, as the shaders' loops run.
 #include "common.cuh"
+#include "sgemm.cuh"
 
 namespace grl {
 
-struct GemmView {          // element (r, c) of batch (b, h) lives at base[b*sb + h*sh + r*sr + c*sc]
-    const float* base;
-    long long sb, sh, sr, sc;
-};
-struct GemmOut {
-    float* base;
-    long long sb, sh, sr, sc;
-};
-
-// C(m,n) = alpha * sum_k A(m,k) B(k,n), k ascending; causal_k != 0 limits the sum to k <= m (attention-output-gpt).
-__global__ void __launch_bounds__(256) bgemm_kernel(GemmView A, GemmView B, GemmOut C, int M, int N, int K, int H,
-                                                     float alpha, int causal_k) {
-    __shared__ float As[16][17], Bs[16][17];
-    const int lx = threadIdx.x & 15, ly = threadIdx.x >> 4;
-    const int bh = blockIdx.z, b = bh / H, h = bh % H;
-    const int m = blockIdx.y * 16 + ly, n = blockIdx.x * 16 + lx;
-    const float* a = A.base + b * A.sb + h * A.sh;
-    const float* bb = B.base + b * B.sb + h * B.sh;
-    const int k_end = causal_k ? min(K, blockIdx.y * 16 + 16) : K;      // rows of this tile see k <= m only
-    float acc = 0.f;
-    for (int k0 = 0; k0 < k_end; k0 += 16) {
-        As[ly][lx] = (m < M && k0 + lx < K) ? a[m * A.sr + (k0 + lx) * A.sc] : 0.f;
-        Bs[ly][lx] = (n < N && k0 + ly < K) ? bb[(k0 + ly) * B.sr + n * B.sc] : 0.f;
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < 16; ++kk)
-            if (!causal_k || k0 + kk <= m) acc = fmaf(As[ly][kk], Bs[kk][lx], acc);
-        __syncthreads();
-    }
-    if (m < M && n < N) C.base[b * C.sb + h * C.sh + m * C.sr + n * C.sc] = acc * alpha;
-}
+using sgemm::Operand;
+using sgemm::Output;
+using sgemm::operand;
 
 // Row-wise softmax of (rows, features): max from -1e10 as activation-softmax.glsl:34-84 starts it, exp(x - max) / sum.
 __global__ void __launch_bounds__(256) softmax_rows_kernel(const float* __restrict__ in, float* __restrict__ out,
@@ -93,11 +65,98 @@ __global__ void __launch_bounds__(256) softmax_backward_rows_kernel(const float*
     for (int f = tid; f < features; f += 256) g[f] = a[f] * (g[f] - dot);
 }
 
-static int launch_bgemm(grl_device* dev, GemmView A, GemmView B, GemmOut C, int M, int N, int K, int batch, int H,
-                        float alpha, int causal_k) {
-    dim3 grid((N + 15) / 16, (M + 15) / 16, batch * H);
-    bgemm_kernel<<<grid, 256, 0, dev->stream>>>(A, B, C, M, N, K, H, alpha, causal_k);
-    GRL_LAUNCHED("bgemm_kernel");
+// ---- the backward pass in three launches.  The softmax backward, gS = attn * (gA - dot) with
+// dot[i] = sum_j attn[i][j] gA[i][j], is not a pass of its own: the gA product leaves, next to gA, the partial row sums
+// of its tiles, and the two products that read gS form it while they stage their tiles.  The partial sums of row i wait
+// in grad_v[i][0 .. tiles), which is written last.
+// Measured (B4 x 12 heads x 512 tokens x 64, 6.4 GFLOP): 1244 us with 16 x 16 tiles and five launches before.
+constexpr int kMaxDotRows = 8192;       // row sums of one head that fit in shared memory beside the tiles
+
+template <typename SH>
+__global__ void __launch_bounds__(SH::THREADS, SH::MIN_CTAS) grad_attn_kernel(Operand GO, Operand V, Output G, const float* attn, float* parts,
+                                                                int S, int D, int H) {
+    __shared__ __align__(16) float smem[2 * SH::TILE];
+    const int z = blockIdx.z, b = z / H, h = z % H;
+    const int m0 = blockIdx.y * SH::BM, n0 = blockIdx.x * SH::BN;
+    float2 acc[8][4];
+    sgemm::mainloop<SH, true, true, false, false>(acc, smem, GO.base + b * GO.sb + h * GO.sh, GO, V.base + b * V.sb + h * V.sh, V, m0, n0, S,
+                                           S, D, nullptr, nullptr);
+    sgemm::store_tile<SH>(acc, G.base + b * G.sb + h * G.sh, G.ld, m0, n0, S, S, 1.f, nullptr);
+    const sgemm::Place<SH> at(threadIdx.x);
+    const float* arow = attn + (size_t)z * S * S;
+    const bool vec = ((uintptr_t)attn % 16 == 0) && S % 4 == 0;
+    float* red = smem;                  // [WARPS_N][BM]; every warp has passed the main loop's last barrier
+    const int lane = threadIdx.x & 31, wn = (threadIdx.x >> 5) % SH::WARPS_N;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int m = m0 + at.row(i);
+        float dot = 0.f;
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) {
+            const int n = n0 + at.col(4 * hh);
+            const float4 a = m < S ? sgemm::load4(arow + (size_t)m * S, n, S, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+            dot = fmaf(a.x, acc[i][2 * hh].x, dot); dot = fmaf(a.y, acc[i][2 * hh].y, dot);
+            dot = fmaf(a.z, acc[i][2 * hh + 1].x, dot); dot = fmaf(a.w, acc[i][2 * hh + 1].y, dot);
+        }
+#pragma unroll
+        for (int o = SH::LANES_N / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+        if (lane % SH::LANES_N == 0) red[wn * SH::BM + at.row(i)] = dot;
+    }
+    __syncthreads();
+    for (int r = threadIdx.x; r < SH::BM; r += SH::THREADS) {
+        if (m0 + r >= S) break;
+        float dot = red[r];
+        for (int w = 1; w < SH::WARPS_N; ++w) dot += red[w * SH::BM + r];
+        parts[((size_t)z * S + m0 + r) * D + blockIdx.x] = dot;
+    }
+}
+
+// blockIdx.z < batch * H: grad_Q[i][d] = scale sum_j gS[i][j] K[j][d]; the other half: grad_K[j][d] = scale sum_i gS[i][j] Q[i][d].
+template <typename SH>
+__global__ void __launch_bounds__(SH::THREADS, SH::MIN_CTAS) grad_qk_kernel(const float* __restrict__ attn, const float* __restrict__ ga,
+                                                              const float* __restrict__ q, const float* __restrict__ k,
+                                                              const float* __restrict__ parts, int n_parts, float* gq, float* gk, int S,
+                                                              int D, int n_bh, int vec_s, int vec_d, float scale) {
+    extern __shared__ __align__(16) float dyn[];      // two tile stages, then the row sums of this head
+    float* dots = dyn + 2 * SH::TILE;
+    const bool is_q = (int)blockIdx.z < n_bh;
+    const int z = is_q ? blockIdx.z : blockIdx.z - n_bh;
+    const int m0 = blockIdx.y * SH::BM, n0 = blockIdx.x * SH::BN;
+    const int d0 = is_q ? m0 : 0, d1 = is_q ? min(S, m0 + SH::BM) : S;          // rows whose sums this CTA needs
+    for (int i = d0 + threadIdx.x; i < d1; i += SH::THREADS) {
+        const float* p = parts + ((size_t)z * S + i) * D;
+        float dot = 0.f;
+        for (int j = 0; j < n_parts; ++j) dot += __ldg(p + j);
+        dots[i - d0] = dot;
+    }
+    __syncthreads();
+    const size_t so = (size_t)z * S * S, to = (size_t)z * S * D;
+    const Operand A{ga + so, 0, 0, S, vec_s}, B{(is_q ? k : q) + to, 0, 0, D, vec_d};
+    float2 acc[8][4];
+    if (is_q) sgemm::mainloop<SH, true, false, false, true>(acc, dyn, A.base, A, B.base, B, m0, n0, S, D, S, attn + so, dots - m0);
+    else sgemm::mainloop<SH, false, false, false, true>(acc, dyn, A.base, A, B.base, B, m0, n0, S, D, S, attn + so, dots);
+    sgemm::store_tile<SH>(acc, (is_q ? gq : gk) + to, D, m0, n0, S, D, scale, nullptr);
+}
+
+template <typename SH>
+static int launch_grad_attn(grl_device* dev, const Operand& go, const Operand& v, const Output& g, const float* attn, float* parts, int S,
+                            int D, int batch, int H) {
+    dim3 grid((S + SH::BN - 1) / SH::BN, (S + SH::BM - 1) / SH::BM, batch * H);
+    grad_attn_kernel<SH><<<grid, SH::THREADS, 0, dev->stream>>>(go, v, g, attn, parts, S, D, H);
+    GRL_LAUNCHED("grad_attn_kernel");
+    return GRL_OK;
+}
+
+template <typename SH>
+static int launch_grad_qk(grl_device* dev, const float* attn, const float* ga, const float* q, const float* k, const float* parts,
+                          int n_parts, float* gq, float* gk, int S, int D, int n_bh, float scale) {
+    const size_t smem = (2 * SH::TILE + (size_t)S) * sizeof(float);
+    GRL_CUDA(cudaFuncSetAttribute(grad_qk_kernel<SH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * SH::TILE + kMaxDotRows) * 4));
+    const int vec_s = S % 4 == 0 && (uintptr_t)attn % 16 == 0 && (uintptr_t)ga % 16 == 0;
+    const int vec_d = D % 4 == 0 && (uintptr_t)q % 16 == 0 && (uintptr_t)k % 16 == 0;
+    dim3 grid((D + SH::BN - 1) / SH::BN, (S + SH::BM - 1) / SH::BM, 2 * n_bh);
+    grad_qk_kernel<SH><<<grid, SH::THREADS, smem, dev->stream>>>(attn, ga, q, k, parts, n_parts, gq, gk, S, D, n_bh, vec_s, vec_d, scale);
+    GRL_LAUNCHED("grad_qk_kernel");
     return GRL_OK;
 }
 
@@ -115,9 +174,9 @@ int grl_attention_scores(grl_device* dev, const float* q, const float* k, float*
     const long long S = seq_len, H = heads, D = head_dim;
     if (scale == 0.f) scale = 1.f / sqrtf((float)head_dim);
     // Q, K: (B,S,H,D); scores (B,H,S,S)
-    GemmView A{q, S * H * D, D, H * D, 1}, B{k, S * H * D, D, 1, H * D};
-    GemmOut C{scores, H * S * S, S * S, S, 1};
-    return launch_bgemm(dev, A, B, C, seq_len, seq_len, head_dim, batch, heads, scale, 0);
+    return sgemm::launch<true, true>(dev, operand(q, S * H * D, D, H * D), operand(k, S * H * D, D, H * D),
+                                     Output{scores, H * S * S, S * S, S}, nullptr, seq_len, seq_len, head_dim, batch, heads, scale,
+                                     "attention_scores");
 }
 
 int grl_softmax(grl_device* dev, const float* in, float* out, size_t rows, int features) {
@@ -137,9 +196,11 @@ int grl_attention_output(grl_device* dev, const float* weights, const float* v, 
     DeviceGuard g(dev->ordinal);
     const long long S = seq_len, H = heads, D = head_dim;
     // weights (B,H,S,S); V, out (B,S,H,D)
-    GemmView A{weights, H * S * S, S * S, S, 1}, B{v, S * H * D, D, H * D, 1};
-    GemmOut C{out, S * H * D, D, H * D, 1};
-    return launch_bgemm(dev, A, B, C, seq_len, head_dim, seq_len, batch, heads, 1.f, causal ? 1 : 0);
+    const Operand A = operand(weights, H * S * S, S * S, S), B = operand(v, S * H * D, D, H * D);
+    const Output C{out, S * H * D, D, H * D};
+    if (causal)
+        return sgemm::launch<true, false, true>(dev, A, B, C, nullptr, seq_len, head_dim, seq_len, batch, heads, 1.f, "attention_output");
+    return sgemm::launch<true, false>(dev, A, B, C, nullptr, seq_len, head_dim, seq_len, batch, heads, 1.f, "attention_output");
 }
 
 int grl_attention_backward(grl_device* dev, const float* grad_out, const float* q, const float* k, const float* v,
@@ -152,24 +213,42 @@ int grl_attention_backward(grl_device* dev, const float* grad_out, const float* 
     if (scale == 0.f) scale = 1.f / sqrtf((float)head_dim);
     // all of Q, K, V, grad_out and the three gradients: (B,H,S,D); attn, scratch: (B,H,S,S)
     const long long qb = H * S * D, qh = S * D, ab = H * S * S, ah = S * S;
-    // pass 0: grad_V[j][d] = sum_i attn[i][j] grad_out[i][d]
-    int rc = launch_bgemm(dev, GemmView{attn, ab, ah, 1, S}, GemmView{grad_out, qb, qh, D, 1}, GemmOut{grad_v, qb, qh, D, 1},
-                          seq_len, head_dim, seq_len, batch, heads, 1.f, 0);
-    // pass 1: grad_attn[i][j] = sum_d grad_out[i][d] V[j][d]  -> scratch
-    if (!rc) rc = launch_bgemm(dev, GemmView{grad_out, qb, qh, D, 1}, GemmView{v, qb, qh, 1, D}, GemmOut{scratch, ab, ah, S, 1},
-                               seq_len, seq_len, head_dim, batch, heads, 1.f, 0);
-    if (rc) return rc;
-    // softmax backward, row by row, in place over scratch
     const size_t rows = (size_t)batch * heads * seq_len;
     GRL_REQUIRE(rows <= 0x7fffffffull, "too many rows");
-    softmax_backward_rows_kernel<<<(unsigned)rows, 256, 0, dev->stream>>>(attn, scratch, rows, seq_len);
-    GRL_LAUNCHED("softmax_backward_rows_kernel");
-    // pass 2: grad_Q[i][d] = scale * sum_j gS[i][j] K[j][d];  grad_K[j][d] = scale * sum_i gS[i][j] Q[i][d]
-    rc = launch_bgemm(dev, GemmView{scratch, ab, ah, S, 1}, GemmView{k, qb, qh, D, 1}, GemmOut{grad_q, qb, qh, D, 1}, seq_len,
-                      head_dim, seq_len, batch, heads, scale, 0);
-    if (!rc) rc = launch_bgemm(dev, GemmView{scratch, ab, ah, 1, S}, GemmView{q, qb, qh, D, 1}, GemmOut{grad_k, qb, qh, D, 1},
-                               seq_len, head_dim, seq_len, batch, heads, scale, 0);
-    return rc;
+    const Operand go_rows = operand(grad_out, qb, qh, D), v_rows = operand(v, qb, qh, D);
+    const Output g_attn{scratch, ab, ah, S};
+    // gA[i][j] = sum_d gO[i][d] V[j][d] -> scratch, with the row sums of attn * gA on the side when grad_v has room for
+    // them (a column per tile) and both products that read them can hold a head's sums in shared memory
+    const int sms = dev->prop.multiProcessorCount, n_bh = batch * heads;
+    const bool wide = sgemm::tile_rows(seq_len, seq_len, n_bh, 128, sms) == 128;
+    const int n_parts = (seq_len + (wide ? 127 : 63)) / (wide ? 128 : 64);
+    int rc;
+    if (n_parts <= head_dim && seq_len <= kMaxDotRows && 2LL * n_bh <= 65535) {
+        rc = wide ? launch_grad_attn<sgemm::Shape<128, 128>>(dev, go_rows, v_rows, g_attn, attn, grad_v, seq_len, head_dim, batch, heads)
+                  : launch_grad_attn<sgemm::Shape<64, 64>>(dev, go_rows, v_rows, g_attn, attn, grad_v, seq_len, head_dim, batch, heads);
+        if (rc) return rc;
+        auto qk = [&](auto shape) {
+            return launch_grad_qk<decltype(shape)>(dev, attn, scratch, q, k, grad_v, n_parts, grad_q, grad_k, seq_len, head_dim, n_bh, scale);
+        };
+        if (head_dim <= 32) rc = qk(sgemm::Shape<64, 32>());
+        else if (sgemm::tile_rows(seq_len, head_dim, 2 * n_bh, 64, sms) == 128) rc = qk(sgemm::Shape<128, 64>());
+        else rc = qk(sgemm::Shape<64, 64>());
+        if (rc) return rc;
+    } else {
+        rc = sgemm::launch<true, true>(dev, go_rows, v_rows, g_attn, nullptr, seq_len, seq_len, head_dim, batch, heads, 1.f, "grad_attn");
+        if (rc) return rc;
+        softmax_backward_rows_kernel<<<(unsigned)rows, 256, 0, dev->stream>>>(attn, scratch, rows, seq_len);
+        GRL_LAUNCHED("softmax_backward_rows_kernel");
+        rc = sgemm::launch<true, false>(dev, operand(scratch, ab, ah, S), operand(k, qb, qh, D), Output{grad_q, qb, qh, D}, nullptr, seq_len,
+                                        head_dim, seq_len, batch, heads, scale, "grad_q");
+        if (!rc)
+            rc = sgemm::launch<false, false>(dev, operand(scratch, ab, ah, S), operand(q, qb, qh, D), Output{grad_k, qb, qh, D}, nullptr,
+                                             seq_len, head_dim, seq_len, batch, heads, scale, "grad_k");
+        if (rc) return rc;
+    }
+    // grad_V[j][d] = sum_i attn[i][j] gO[i][d]
+    return sgemm::launch<false, false>(dev, operand(attn, ab, ah, S), go_rows, Output{grad_v, qb, qh, D}, nullptr, seq_len, head_dim,
+                                       seq_len, batch, heads, 1.f, "grad_v");
 }
 
 }  // extern "C"

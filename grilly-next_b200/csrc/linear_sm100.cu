@@ -12,6 +12,7 @@
 // and warps 4-7 read the accumulator back, add the bias and write rows through a shared-memory transpose so
 // that every warp store covers contiguous bytes of one row.  Every mbarrier wait is bounded.
 #include "common.cuh"
+#include "sgemm.cuh"
 #include "sm100_ptx.cuh"
 #include "tmem_ops.cuh"
 
@@ -177,25 +178,52 @@ linear_sm100_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_consta
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(128) : "memory");
 }
 
-// Exact fp32 form: the arithmetic of fnn-linear / fused-qkv-projection (one dot product per output, k ascending),
-// 16 x 16 tiles in shared memory.
-__global__ void __launch_bounds__(256) linear_f32_kernel(const float* __restrict__ x, const float* __restrict__ w,
-                                                          const float* __restrict__ bias, float* __restrict__ y, int M,
-                                                          int K, int N) {
-    __shared__ float xs[16][17], ws[16][17];
-    const int lx = threadIdx.x & 15, ly = threadIdx.x >> 4;
-    const int m = blockIdx.y * 16 + ly, n = blockIdx.x * 16 + lx;
-    float acc = 0.f;
-    for (int k0 = 0; k0 < K; k0 += 16) {
-        xs[ly][lx] = (m < M && k0 + lx < K) ? x[(size_t)m * K + k0 + lx] : 0.f;
-        const int wn = blockIdx.x * 16 + ly;
-        ws[ly][lx] = (wn < N && k0 + lx < K) ? w[(size_t)wn * K + k0 + lx] : 0.f;
-        __syncthreads();
+// Exact fp32 form for a handful of rows: bound by the one pass over W, so a warp takes one row of W (one output column),
+// reads it once in 16-byte pieces and multiplies it with every row of x (which stays in L1).  Above kGemvRows the
+// tiled product of sgemm.cuh, whose 64-row tiles would be mostly padding here, is the faster one.
+constexpr int kGemvRows = 8;
+template <int MR>
+__global__ void __launch_bounds__(256) linear_f32_rows_kernel(const float* __restrict__ x, const float* __restrict__ w,
+                                                              const float* __restrict__ bias, float* __restrict__ y, int M, int K, int N,
+                                                              int vec) {
+    const int n = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (n >= N) return;
+    const float* wr = w + (size_t)n * K;
+    float acc[MR];
 #pragma unroll
-        for (int kk = 0; kk < 16; ++kk) acc = fmaf(xs[ly][kk], ws[lx][kk], acc);
-        __syncthreads();
+    for (int m = 0; m < MR; ++m) acc[m] = 0.f;
+#pragma unroll 4
+    for (int k = lane * 4; k < K; k += 128) {
+        const float4 a = sgemm::load4(wr, k, K, vec);
+#pragma unroll
+        for (int m = 0; m < MR; ++m) {
+            if (m >= M) break;
+            const float4 b = sgemm::load4(x + (size_t)m * K, k, K, vec);
+            acc[m] = fmaf(a.x, b.x, acc[m]); acc[m] = fmaf(a.y, b.y, acc[m]);
+            acc[m] = fmaf(a.z, b.z, acc[m]); acc[m] = fmaf(a.w, b.w, acc[m]);
+        }
     }
-    if (m < M && n < N) y[(size_t)m * N + n] = acc + (bias ? bias[n] : 0.f);
+    const float bn = bias ? bias[n] : 0.f;
+#pragma unroll
+    for (int m = 0; m < MR; ++m) {
+        if (m >= M) break;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc[m] += __shfl_xor_sync(0xffffffffu, acc[m], o);
+        if (lane == 0) y[(size_t)m * N + n] = acc[m] + bn;
+    }
+}
+
+static int linear_f32(grl_device* dev, const float* x, const float* w, const float* bias, float* y, int M, int K, int N) {
+    if (M > kGemvRows)
+        return sgemm::launch<true, true>(dev, sgemm::operand(x, 0, 0, K), sgemm::operand(w, 0, 0, K), sgemm::Output{y, 0, 0, N}, bias, M,
+                                         N, K, 1, 1, 1.f, "linear_f32");
+    const int vec = K % 4 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)w % 16 == 0;
+    const unsigned grid = (unsigned)((N + 7) / 8);
+    if (M == 1) linear_f32_rows_kernel<1><<<grid, 256, 0, dev->stream>>>(x, w, bias, y, M, K, N, vec);
+    else if (M <= 4) linear_f32_rows_kernel<4><<<grid, 256, 0, dev->stream>>>(x, w, bias, y, M, K, N, vec);
+    else linear_f32_rows_kernel<8><<<grid, 256, 0, dev->stream>>>(x, w, bias, y, M, K, N, vec);
+    GRL_LAUNCHED("linear_f32_rows_kernel");
+    return GRL_OK;
 }
 
 }  // namespace lin
@@ -209,12 +237,8 @@ extern "C" int grl_linear(grl_device* dev, const void* x, const void* w, const f
     GRL_REQUIRE(m > 0 && k > 0 && n > 0, "bad shape (%d,%d,%d)", m, k, n);
     GRL_REQUIRE(in_dtype == GRL_F32 || in_dtype == GRL_BF16, "unknown in_dtype");
     DeviceGuard g(dev->ordinal);
-    if (in_dtype == GRL_F32) {
-        lin::linear_f32_kernel<<<dim3((n + 15) / 16, (m + 15) / 16), 256, 0, dev->stream>>>(
-            static_cast<const float*>(x), static_cast<const float*>(w), bias, y, m, k, n);
-        GRL_LAUNCHED("linear_f32_kernel");
-        return GRL_OK;
-    }
+    if (in_dtype == GRL_F32)
+        return lin::linear_f32(dev, static_cast<const float*>(x), static_cast<const float*>(w), bias, y, m, k, n);
     GRL_REQUIRE(k % 8 == 0, "the tensor-core projection needs the inner dimension to be a multiple of 8 (got %d): rows must "
                             "start on 16-byte boundaries for TMA", k);
     GRL_REQUIRE(((uintptr_t)x % 16 == 0) && ((uintptr_t)w % 16 == 0) && ((uintptr_t)y % 8 == 0), "x, w must be 16-byte aligned");

@@ -1,0 +1,242 @@
+// Batched float32 matrix products on the FMA pipe, shared by the exact linear projection and the unfused attention
+// pieces with their backward pass: C(m,n) = alpha * sum_k A(m,k) B(k,n), every output one chain of fused multiply-adds
+// in ascending k.
+//
+// Bound: the FP32 pipe (128 FMA per clock per SM: 74 TFLOP/s).  A thread owns 8 x 8 outputs as 8 x 4 packed pairs
+// (fma.rn.f32x2 halves the issue slots, which leaves room for the shared-memory loads and the tile traffic); a warp
+// 32 x 64 (or 64 x 32 where the product has only 32 columns).  Tiles of A and B cross shared memory as [k][m] and [k][n],
+// double-buffered through registers: the global loads of slice i+1 are in flight under the products of slice i.
+#pragma once
+#include "common.cuh"
+
+namespace grl {
+namespace sgemm {
+
+constexpr int BK = 16;
+
+// One operand.  Element (outer, inner) of batch (b, h) lives at base[b*sb + h*sh + outer*ld + inner]; which of its two
+// indices is the contiguous one is a template parameter of the kernel.  vec: rows start on 16-byte boundaries.
+struct Operand {
+    const float* base;
+    long long sb, sh, ld;
+    int vec;
+};
+struct Output {
+    float* base;
+    long long sb, sh, ld;
+};
+inline Operand operand(const float* base, long long sb, long long sh, long long ld) {
+    const bool vec = ((uintptr_t)base % 16 == 0) && sb % 4 == 0 && sh % 4 == 0 && ld % 4 == 0;
+    return Operand{base, sb, sh, ld, vec ? 1 : 0};
+}
+
+template <int BM_, int BN_>
+struct Shape {
+    static constexpr int BM = BM_, BN = BN_;
+    static constexpr int WM = BN >= 64 ? 32 : 64, WN = BN >= 64 ? 64 : 32;      // outputs of a warp
+    static constexpr int WARPS_N = BN / WN, WARPS = (BM / WM) * WARPS_N, THREADS = WARPS * 32;
+    static constexpr int LANES_N = WN / 8;
+    static constexpr int LDA = BM + 4, LDB = BN + 4;                            // floats per k row of a tile
+    static constexpr int TILE = BK * (LDA + LDB);                               // floats per stage
+    static constexpr int MIN_CTAS = THREADS == 256 ? 2 : 1;                     // 128 registers there: two CTAs hide each other's barriers
+};
+
+__device__ __forceinline__ float4 load4(const float* row, int i, int n, bool vec) {
+    if (vec && i + 3 < n) return __ldg(reinterpret_cast<const float4*>(row + i));
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i < n) v.x = __ldg(row + i);
+    if (i + 1 < n) v.y = __ldg(row + i + 1);
+    if (i + 2 < n) v.z = __ldg(row + i + 2);
+    if (i + 3 < n) v.w = __ldg(row + i + 3);
+    return v;
+}
+
+// One k slice of an operand on its way from global to shared memory: EXT rows (m or n) x BK.  KC: the k index is the
+// contiguous one (a thread's float4 is four k of one row and is stored transposed); otherwise the row index is.
+// PAIR: a second tensor w of the same shape is read along, and what is stored is w * (v - dot) with one `dot` per row
+// (KC) or per k -- the softmax backward, formed on the way to shared memory.
+template <int EXT, int THREADS, bool KC, bool PAIR = false>
+struct Fetch {
+    static constexpr int VECS = EXT * BK / 4 / THREADS;
+    static_assert(EXT * BK / 4 % THREADS == 0, "slice must divide over the threads");
+    float4 v[VECS], w[PAIR ? VECS : 1];
+    __device__ __forceinline__ void load(const float* base, const float* pair, long long ld, bool vec, int row0, int rows, int k0, int K,
+                                         int tid) {
+#pragma unroll
+        for (int i = 0; i < VECS; ++i) {
+            const int q = tid + i * THREADS;
+            const int outer = KC ? row0 + q / (BK / 4) : k0 + q / (EXT / 4), inner = KC ? k0 + (q % (BK / 4)) * 4 : row0 + (q % (EXT / 4)) * 4;
+            const bool in = outer < (KC ? rows : K);
+            const long long off = (long long)outer * ld;
+            v[i] = in ? load4(base + off, inner, KC ? K : rows, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+            if constexpr (PAIR) w[i] = in ? load4(pair + off, inner, KC ? K : rows, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
+    __device__ __forceinline__ void store(float* tile, int LD, int tid, const float* dots, int row0, int rows, int k0, int K) const {
+#pragma unroll
+        for (int i = 0; i < VECS; ++i) {
+            const int q = tid + i * THREADS;
+            float4 x = v[i];
+            if constexpr (PAIR) {
+                const int outer = KC ? row0 + q / (BK / 4) : k0 + q / (EXT / 4);
+                const float d = outer < (KC ? rows : K) ? dots[outer] : 0.f;
+                x = make_float4(w[i].x * (x.x - d), w[i].y * (x.y - d), w[i].z * (x.z - d), w[i].w * (x.w - d));
+            }
+            if constexpr (KC) {
+                float* p = tile + (q % (BK / 4)) * 4 * LD + q / (BK / 4);
+                p[0] = x.x; p[LD] = x.y; p[2 * LD] = x.z; p[3 * LD] = x.w;
+            } else {
+                *reinterpret_cast<float4*>(tile + (q / (EXT / 4)) * LD + (q % (EXT / 4)) * 4) = x;
+            }
+        }
+    }
+};
+
+// The 8 x 8 outputs of a thread: rows row(i), columns col(j).
+template <typename SH>
+struct Place {
+    int m0, n0;         // first row / column of this thread inside the CTA's tile
+    __device__ __forceinline__ Place(int tid) {
+        const int warp = tid >> 5, lane = tid & 31;
+        m0 = (warp / SH::WARPS_N) * SH::WM + (lane / SH::LANES_N) * 4;
+        n0 = (warp % SH::WARPS_N) * SH::WN + (lane % SH::LANES_N) * 4;
+    }
+    __device__ __forceinline__ int row(int i) const { return m0 + (i & 3) + (i >> 2) * (SH::WM / 2); }
+    __device__ __forceinline__ int col(int j) const { return n0 + (j & 3) + (j >> 2) * (SH::WN / 2); }
+};
+
+// acc[i][j/2] over k in [0, K): the main loop.  CAUSAL: rows of the product only see k <= m (slices that straddle the
+// diagonal test every term; the caller passes the tile's own upper limit as K).  With `pair` A is pair * (a - dots).
+template <typename SH, bool AKC, bool BKC, bool CAUSAL, bool PAIR>
+__device__ __forceinline__ void mainloop(float2 (&acc)[8][4], float* smem, const float* a, const Operand& A, const float* b,
+                                         const Operand& B, int m0, int n0, int M, int N, int K, const float* pair, const float* dots) {
+    const int tid = threadIdx.x;
+    const Place<SH> at(tid);
+    Fetch<SH::BM, SH::THREADS, AKC, PAIR> fa;
+    Fetch<SH::BN, SH::THREADS, BKC> fb;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = make_float2(0.f, 0.f);
+    fa.load(a, pair, A.ld, A.vec, m0, M, 0, K, tid);
+    fb.load(b, nullptr, B.ld, B.vec, n0, N, 0, K, tid);
+    fa.store(smem, SH::LDA, tid, dots, m0, M, 0, K);
+    fb.store(smem + BK * SH::LDA, SH::LDB, tid, nullptr, n0, N, 0, K);
+    __syncthreads();
+    const int slices = (K + BK - 1) / BK;
+    for (int s = 0; s < slices; ++s) {
+        const float* as = smem + (s & 1) * SH::TILE;
+        const float* bs = as + BK * SH::LDA;
+        if (s + 1 < slices) {
+            fa.load(a, pair, A.ld, A.vec, m0, M, (s + 1) * BK, K, tid);
+            fb.load(b, nullptr, B.ld, B.vec, n0, N, (s + 1) * BK, K, tid);
+        }
+        const bool diagonal = CAUSAL && (s + 1) * BK > m0;
+        if (!diagonal) {
+#pragma unroll
+            for (int k = 0; k < BK; ++k) {
+                float av[8];
+                float2 bv[4];
+                *reinterpret_cast<float4*>(av) = *reinterpret_cast<const float4*>(as + k * SH::LDA + at.m0);
+                *reinterpret_cast<float4*>(av + 4) = *reinterpret_cast<const float4*>(as + k * SH::LDA + at.m0 + SH::WM / 2);
+                *reinterpret_cast<float4*>(bv) = *reinterpret_cast<const float4*>(bs + k * SH::LDB + at.n0);
+                *reinterpret_cast<float4*>(bv + 2) = *reinterpret_cast<const float4*>(bs + k * SH::LDB + at.n0 + SH::WN / 2);
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) acc[i][j] = __ffma2_rn(make_float2(av[i], av[i]), bv[j], acc[i][j]);
+            }
+        } else {
+            for (int k = 0; k < BK; ++k) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float av = as[k * SH::LDA + at.row(i)];
+                    if (s * BK + k <= m0 + at.row(i)) {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+                            acc[i][j] = __ffma2_rn(make_float2(av, av), *reinterpret_cast<const float2*>(bs + k * SH::LDB + at.col(2 * j)), acc[i][j]);
+                    }
+                }
+            }
+        }
+        if (s + 1 < slices) {
+            float* ns = smem + ((s + 1) & 1) * SH::TILE;
+            fa.store(ns, SH::LDA, tid, dots, m0, M, (s + 1) * BK, K);
+            fb.store(ns + BK * SH::LDA, SH::LDB, tid, nullptr, n0, N, (s + 1) * BK, K);
+        }
+        __syncthreads();
+    }
+}
+
+// Write alpha * acc (+ bias) to C, rows < M and columns < N only.
+template <typename SH>
+__device__ __forceinline__ void store_tile(const float2 (&acc)[8][4], float* c, long long ld, int m0, int n0, int M, int N, float alpha,
+                                           const float* bias) {
+    const Place<SH> at(threadIdx.x);
+    const bool vec = ((uintptr_t)c % 16 == 0) && ld % 4 == 0;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int n = n0 + at.col(4 * h);
+        if (n >= N) continue;
+        const float4 bv = bias ? load4(bias, n, N, (uintptr_t)bias % 16 == 0) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int m = m0 + at.row(i);
+            if (m >= M) continue;
+            const float2 x = acc[i][2 * h], y = acc[i][2 * h + 1];
+            const float4 v = make_float4(x.x * alpha + bv.x, x.y * alpha + bv.y, y.x * alpha + bv.z, y.y * alpha + bv.w);
+            float* dst = c + (long long)m * ld + n;
+            if (vec && n + 3 < N) *reinterpret_cast<float4*>(dst) = v;
+            else {
+                dst[0] = v.x;
+                if (n + 1 < N) dst[1] = v.y;
+                if (n + 2 < N) dst[2] = v.z;
+                if (n + 3 < N) dst[3] = v.w;
+            }
+        }
+    }
+}
+
+template <typename SH, bool AKC, bool BKC, bool CAUSAL>
+__global__ void __launch_bounds__(SH::THREADS, SH::MIN_CTAS) kernel(Operand A, Operand B, Output C, const float* bias, int M, int N, int K, int H,
+                                                      float alpha) {
+    __shared__ __align__(16) float smem[2 * SH::TILE];
+    const int z = blockIdx.z, b = z / H, h = z % H;
+    const int m0 = blockIdx.y * SH::BM, n0 = blockIdx.x * SH::BN;
+    float2 acc[8][4];
+    mainloop<SH, AKC, BKC, CAUSAL, false>(acc, smem, A.base + b * A.sb + h * A.sh, A, B.base + b * B.sb + h * B.sh, B, m0, n0, M, N,
+                                   CAUSAL ? min(K, m0 + SH::BM) : K, nullptr, nullptr);
+    store_tile<SH>(acc, C.base + b * C.sb + h * C.sh, C.ld, m0, n0, M, N, alpha, bias);
+}
+
+// Which tile: the widest one whose grid still gives every SM two CTAs; 64 rows otherwise, so that a small product
+// spreads over more SMs.  32 columns only where the product has no more (half of a 64-column tile would be padding).
+inline int tile_rows(int M, int N, int batch, int bn, int sms) {
+    const long long big = (long long)((M + 127) / 128) * ((N + bn - 1) / bn) * batch;
+    return big >= 2LL * sms ? 128 : 64;
+}
+
+template <bool AKC, bool BKC, bool CAUSAL = false>
+int launch(grl_device* dev, const Operand& A, const Operand& B, const Output& C, const float* bias, int M, int N, int K, int batch,
+           int H, float alpha, const char* name) {
+    auto go = [&](auto shape) {
+        using SH = decltype(shape);
+        dim3 grid((N + SH::BN - 1) / SH::BN, (M + SH::BM - 1) / SH::BM, batch * H);
+        kernel<SH, AKC, BKC, CAUSAL><<<grid, SH::THREADS, 0, dev->stream>>>(A, B, C, bias, M, N, K, H, alpha);
+    };
+    const int sms = dev->prop.multiProcessorCount;
+    if (N <= 32) {
+        go(Shape<64, 32>());
+    } else if (N > 64 && tile_rows(M, N, batch * H, 128, sms) == 128) {
+        go(Shape<128, 128>());
+    } else if (tile_rows(M, N, batch * H, 64, sms) == 128) {
+        go(Shape<128, 64>());
+    } else {
+        go(Shape<64, 64>());
+    }
+    GRL_LAUNCHED(name);
+    return GRL_OK;
+}
+
+}  // namespace sgemm
+}  // namespace grl

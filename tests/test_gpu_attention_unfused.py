@@ -105,3 +105,18 @@ def test_argument_errors(gpu):
         gpu.attention_backward(z, z, z[:, :3], z, np.zeros((1, 4, 2, 2), np.float32))
     with pytest.raises(RuntimeError, match="attn_weights"):
         gpu.attention_backward(z, z, z, z, np.zeros((1, 4, 2, 3), np.float32))
+
+
+@pytest.mark.parametrize("B,H,S,D", [
+    (1, 1, 1, 8), (1, 2, 65, 32), (3, 8, 129, 64),      # one row; 64-row tiles and their remainders
+    (1, 3, 70, 33), (1, 1, 600, 8),                     # rows off 16-byte boundaries; more tiles a row than head_dim
+    (8, 40, 130, 64), (4, 40, 256, 96)])                # 128-row tiles, two tiles of columns
+def test_backward_tile_edges(gpu, B, H, S, D):
+    from oracle import attention_unfused_oracle as uo
+    rng = np.random.default_rng(S + D)
+    q, k, v, go = (rng.standard_normal((B, H, S, D), dtype=np.float32) for _ in range(4))
+    attn = uo.softmax(np.einsum("bhid,bhjd->bhij", q, k) / np.sqrt(D)).astype(np.float32)
+    got = gpu.attention_backward(go, q, k, v, attn)
+    pick = slice(0, 1) if B * H > 24 else slice(0, B)    # the oracle is slow: one sequence of the large ones
+    for g, w in zip(got, uo.attention_backward(go[pick], q[pick], k[pick], v[pick], attn[pick])):
+        assert np.abs(g[pick] - w).max() <= 2e-4

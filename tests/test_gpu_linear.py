@@ -74,3 +74,12 @@ def test_fused_qkv_projection_feeds_attention(gpu):
     assert out.shape == (B, S, hidden) and np.abs(out - ref).max() <= 2e-4
     qkv16 = gpu.fused_qkv_projection(x, w, b, num_heads=H, head_dim=D, dtype="bf16")
     assert np.abs(qkv16.reshape(-1, 3 * H * D) - want).max() <= 0.05
+
+
+@pytest.mark.parametrize("M,K,N", [(1, 4, 1), (2, 131, 9), (8, 132, 300), (9, 17, 65), (64, 33, 32), (130, 40, 2500), (2100, 70, 1025)])
+def test_linear_fp32_tile_edges(gpu, M, K, N):
+    rng = np.random.default_rng(M + K + N)
+    x, w = rng.standard_normal((M, K), dtype=np.float32), rng.standard_normal((N, K), dtype=np.float32)
+    b = rng.standard_normal(N, dtype=np.float32)
+    want = x.astype(np.float64) @ w.astype(np.float64).T + b
+    assert np.abs(gpu.linear(x, w, b) - want).max() <= 1e-4
