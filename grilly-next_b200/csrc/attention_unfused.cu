@@ -72,29 +72,47 @@ __global__ void __launch_bounds__(256) softmax_backward_rows_kernel(const float*
 // Measured (B4 x 12 heads x 512 tokens x 64, 6.4 GFLOP): 1244 us with 16 x 16 tiles and five launches before.
 constexpr int kMaxDotRows = 8192;       // row sums of one head that fit in shared memory beside the tiles
 
+// The attn tile of a CTA is fetched into shared memory under its products (cp.async): read in the epilogue it was
+// eight dependent trips to L2 or DRAM per thread, two thirds of this kernel's time (75 us; 22 us of FMA work).
+template <typename SH> struct GradAttn {
+    static constexpr int LDS = SH::BN + 4;
+    static constexpr size_t SMEM = (2 * SH::TILE + SH::BM * LDS) * sizeof(float);
+    static constexpr int MIN_CTAS = SH::THREADS == 256 ? 2 : 6;
+};
 template <typename SH>
-__global__ void __launch_bounds__(SH::THREADS, SH::MIN_CTAS) grad_attn_kernel(Operand GO, Operand V, Output G, const float* attn, float* parts,
-                                                                int S, int D, int H) {
-    __shared__ __align__(16) float smem[2 * SH::TILE];
+__global__ void __launch_bounds__(SH::THREADS, GradAttn<SH>::MIN_CTAS) grad_attn_kernel(Operand GO, Operand V, Output G, const float* attn,
+                                                                                        float* parts, int S, int D, int H) {
+    extern __shared__ __align__(16) float dyn[];
+    constexpr int LDS = GradAttn<SH>::LDS;
+    float* tile = dyn + 2 * SH::TILE;   // [BM][LDS] of attn; zeros outside the tensor
     const int z = blockIdx.z, b = z / H, h = z % H;
     const int m0 = blockIdx.y * SH::BM, n0 = blockIdx.x * SH::BN;
-    float2 acc[8][4];
-    sgemm::mainloop<SH, true, true, false, false>(acc, smem, GO.base + b * GO.sb + h * GO.sh, GO, V.base + b * V.sb + h * V.sh, V, m0, n0, S,
-                                           S, D, nullptr, nullptr);
-    sgemm::store_tile<SH>(acc, G.base + b * G.sb + h * G.sh, G.ld, m0, n0, S, S, 1.f, nullptr);
-    const sgemm::Place<SH> at(threadIdx.x);
-    const float* arow = attn + (size_t)z * S * S;
+    const float* ahead = attn + (size_t)z * S * S;
     const bool vec = ((uintptr_t)attn % 16 == 0) && S % 4 == 0;
-    float* red = smem;                  // [WARPS_N][BM]; every warp has passed the main loop's last barrier
+    for (int q = threadIdx.x; q < SH::BM * SH::BN / 4; q += SH::THREADS) {
+        const int r = q / (SH::BN / 4), c = (q % (SH::BN / 4)) * 4;
+        float* dst = tile + r * LDS + c;
+        if (vec && m0 + r < S && n0 + c < S)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                         "l"(ahead + (size_t)(m0 + r) * S + n0 + c) : "memory");
+        else
+            *reinterpret_cast<float4*>(dst) = m0 + r < S ? sgemm::load4(ahead + (size_t)(m0 + r) * S, n0 + c, S, false) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    float2 acc[8][4];
+    sgemm::mainloop<SH, true, true, false, false>(acc, dyn, GO.base + b * GO.sb + h * GO.sh, GO, V.base + b * V.sb + h * V.sh, V, m0, n0, S,
+                                                  S, D, nullptr, nullptr);
+    sgemm::store_tile<SH>(acc, G.base + b * G.sb + h * G.sh, G.ld, m0, n0, S, S, 1.f, nullptr);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    const sgemm::Place<SH> at(threadIdx.x);
+    float* red = dyn;                   // [WARPS_N][BM]
     const int lane = threadIdx.x & 31, wn = (threadIdx.x >> 5) % SH::WARPS_N;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        const int m = m0 + at.row(i);
         float dot = 0.f;
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {
-            const int n = n0 + at.col(4 * hh);
-            const float4 a = m < S ? sgemm::load4(arow + (size_t)m * S, n, S, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float4 a = *reinterpret_cast<const float4*>(tile + at.row(i) * LDS + at.col(4 * hh));
             dot = fmaf(a.x, acc[i][2 * hh].x, dot); dot = fmaf(a.y, acc[i][2 * hh].y, dot);
             dot = fmaf(a.z, acc[i][2 * hh + 1].x, dot); dot = fmaf(a.w, acc[i][2 * hh + 1].y, dot);
         }
@@ -130,6 +148,7 @@ __global__ void __launch_bounds__(SH::THREADS, SH::MIN_CTAS) grad_qk_kernel(cons
         dots[i - d0] = dot;
     }
     __syncthreads();
+    pdl_trigger();      // the row sums are read: the grad_V product, which overwrites them, may take the idle SMs
     const size_t so = (size_t)z * S * S, to = (size_t)z * S * D;
     const Operand A{ga + so, 0, 0, S, vec_s}, B{(is_q ? k : q) + to, 0, 0, D, vec_d};
     float2 acc[8][4];
@@ -142,7 +161,8 @@ template <typename SH>
 static int launch_grad_attn(grl_device* dev, const Operand& go, const Operand& v, const Output& g, const float* attn, float* parts, int S,
                             int D, int batch, int H) {
     dim3 grid((S + SH::BN - 1) / SH::BN, (S + SH::BM - 1) / SH::BM, batch * H);
-    grad_attn_kernel<SH><<<grid, SH::THREADS, 0, dev->stream>>>(go, v, g, attn, parts, S, D, H);
+    GRL_CUDA(cudaFuncSetAttribute(grad_attn_kernel<SH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GradAttn<SH>::SMEM));
+    grad_attn_kernel<SH><<<grid, SH::THREADS, GradAttn<SH>::SMEM, dev->stream>>>(go, v, g, attn, parts, S, D, H);
     GRL_LAUNCHED("grad_attn_kernel");
     return GRL_OK;
 }
@@ -230,10 +250,14 @@ int grl_attention_backward(grl_device* dev, const float* grad_out, const float* 
         auto qk = [&](auto shape) {
             return launch_grad_qk<decltype(shape)>(dev, attn, scratch, q, k, grad_v, n_parts, grad_q, grad_k, seq_len, head_dim, n_bh, scale);
         };
+        const int tile = sgemm::tile_rows(seq_len, head_dim, 3 * n_bh, 64, sms);    // the grad_V product runs beside these two
         if (head_dim <= 32) rc = qk(sgemm::Shape<64, 32>());
-        else if (sgemm::tile_rows(seq_len, head_dim, 2 * n_bh, 64, sms) == 128) rc = qk(sgemm::Shape<128, 64>());
+        else if (tile == 128) rc = qk(sgemm::Shape<128, 64>());
         else rc = qk(sgemm::Shape<64, 64>());
         if (rc) return rc;
+        // grad_V[j][d] = sum_i attn[i][j] gO[i][d]
+        return sgemm::launch<false, false, false, true>(dev, operand(attn, ab, ah, S), go_rows, Output{grad_v, qb, qh, D}, nullptr, seq_len,
+                                                        head_dim, seq_len, batch, heads, 1.f, "grad_v", tile);
     } else {
         rc = sgemm::launch<true, true>(dev, go_rows, v_rows, g_attn, nullptr, seq_len, seq_len, head_dim, batch, heads, 1.f, "grad_attn");
         if (rc) return rc;
@@ -246,7 +270,6 @@ int grl_attention_backward(grl_device* dev, const float* grad_out, const float* 
                                              seq_len, head_dim, seq_len, batch, heads, scale, "grad_k");
         if (rc) return rc;
     }
-    // grad_V[j][d] = sum_i attn[i][j] gO[i][d]
     return sgemm::launch<false, false>(dev, operand(attn, ab, ah, S), go_rows, Output{grad_v, qb, qh, D}, nullptr, seq_len, head_dim,
                                        seq_len, batch, heads, 1.f, "grad_v");
 }

@@ -135,6 +135,24 @@ extern std::atomic<long long> g_launches;
                                   cudaGetErrorString(_e));                                    \
     } while (0)
 
+#ifdef __CUDACC__
+// Launch that may begin while the kernel before it on the stream is still running (programmatic dependent launch): its
+// CTAs take the SMs that the earlier kernel leaves idle.  The kernel must call pdl_wait() before it touches anything the
+// earlier kernel writes or still reads, and in any case before it ends, so that stream order holds for what follows.
+template <typename... P, typename... A>
+inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr; cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+#endif
+
 struct DeviceGuard {
     int prev = -1;
     explicit DeviceGuard(int ordinal) {

@@ -38,7 +38,7 @@ struct Shape {
     static constexpr int LANES_N = WN / 8;
     static constexpr int LDA = BM + 4, LDB = BN + 4;                            // floats per k row of a tile
     static constexpr int TILE = BK * (LDA + LDB);                               // floats per stage
-    static constexpr int MIN_CTAS = THREADS == 256 ? 2 : 1;                     // 128 registers there: two CTAs hide each other's barriers
+    static constexpr int MIN_CTAS = 384 / THREADS > 8 ? 8 : THREADS == 256 ? 2 : 384 / THREADS;   // at least 12 warps an SM (<= 168 registers)
 };
 
 __device__ __forceinline__ float4 load4(const float* row, int i, int n, bool vec) {
@@ -197,7 +197,7 @@ __device__ __forceinline__ void store_tile(const float2 (&acc)[8][4], float* c, 
     }
 }
 
-template <typename SH, bool AKC, bool BKC, bool CAUSAL>
+template <typename SH, bool AKC, bool BKC, bool CAUSAL, bool EARLY>
 __global__ void __launch_bounds__(SH::THREADS, SH::MIN_CTAS) kernel(Operand A, Operand B, Output C, const float* bias, int M, int N, int K, int H,
                                                       float alpha) {
     __shared__ __align__(16) float smem[2 * SH::TILE];
@@ -207,6 +207,7 @@ __global__ void __launch_bounds__(SH::THREADS, SH::MIN_CTAS) kernel(Operand A, O
     mainloop<SH, AKC, BKC, CAUSAL, false>(acc, smem, A.base + b * A.sb + h * A.sh, A, B.base + b * B.sb + h * B.sh, B, m0, n0, M, N,
                                    CAUSAL ? min(K, m0 + SH::BM) : K, nullptr, nullptr);
     store_tile<SH>(acc, C.base + b * C.sb + h * C.sh, C.ld, m0, n0, M, N, alpha, bias);
+    if constexpr (EARLY) pdl_wait();
 }
 
 // Which tile: the widest one whose grid still gives every SM two CTAs; 64 rows otherwise, so that a small product
@@ -216,20 +217,22 @@ inline int tile_rows(int M, int N, int batch, int bn, int sms) {
     return big >= 2LL * sms ? 128 : 64;
 }
 
-template <bool AKC, bool BKC, bool CAUSAL = false>
+// EARLY: the launch starts under the kernel before it on the stream, of which it needs nothing but the end (see launch_pdl).
+template <bool AKC, bool BKC, bool CAUSAL = false, bool EARLY = false>
 int launch(grl_device* dev, const Operand& A, const Operand& B, const Output& C, const float* bias, int M, int N, int K, int batch,
-           int H, float alpha, const char* name) {
+           int H, float alpha, const char* name, int rows_hint = 0) {
     auto go = [&](auto shape) {
         using SH = decltype(shape);
         dim3 grid((N + SH::BN - 1) / SH::BN, (M + SH::BM - 1) / SH::BM, batch * H);
-        kernel<SH, AKC, BKC, CAUSAL><<<grid, SH::THREADS, 0, dev->stream>>>(A, B, C, bias, M, N, K, H, alpha);
+        if constexpr (EARLY) launch_pdl(kernel<SH, AKC, BKC, CAUSAL, true>, grid, SH::THREADS, 0, dev->stream, A, B, C, bias, M, N, K, H, alpha);
+        else kernel<SH, AKC, BKC, CAUSAL, false><<<grid, SH::THREADS, 0, dev->stream>>>(A, B, C, bias, M, N, K, H, alpha);
     };
     const int sms = dev->prop.multiProcessorCount;
     if (N <= 32) {
         go(Shape<64, 32>());
-    } else if (N > 64 && tile_rows(M, N, batch * H, 128, sms) == 128) {
+    } else if (N > 64 && !rows_hint && tile_rows(M, N, batch * H, 128, sms) == 128) {
         go(Shape<128, 128>());
-    } else if (tile_rows(M, N, batch * H, 64, sms) == 128) {
+    } else if ((rows_hint ? rows_hint : tile_rows(M, N, batch * H, 64, sms)) == 128) {
         go(Shape<128, 64>());
     } else {
         go(Shape<64, 64>());
