@@ -21,6 +21,7 @@ struct AppendArgs {
     int32_t* status;     // device status word: GRL_ERR_INVALID when a sequence has no room for the new tokens
     uint16_t* scales;    // quantised cache only
     int skip_kv;         // rotate the queries only (the quantised append stores K and V with its own kernel)
+    int heads_per_item;  // quantised append: kv heads that one warp walks for the same token and group
     RopeFreq freq;
 };
 
@@ -92,6 +93,130 @@ __global__ void __launch_bounds__(1024) kv_append_kernel(AppendArgs a) {
     }
 }
 
+// Append, head_dim a multiple of 8 and rows on 16-byte boundaries.  Bound by HBM (float32 in, cache elements out), so a
+// thread moves 8 elements of a row (two 16-byte loads, one 16-byte store of bf16), two heads of keys and values in flight.
+// It owns four rotation pairs of ONE token and walks that token's heads: the double-precision angle reduction, once per
+// (token, head, pair) in the element-wise kernel above and most of its time, runs once per (token, pair).  Measured (4 x 2048
+// tokens x 8 kv heads x 128, bf16, RoPE; 100 MB): 61 us before.
+constexpr int kAppendHeads = 2;
+template <typename T>
+__device__ __forceinline__ void store8(T* row, int o0, int o1, const float (&y)[8]);
+template <>
+__device__ __forceinline__ void store8<float>(float* row, int o0, int o1, const float (&y)[8]) {
+    *reinterpret_cast<float4*>(row + o0) = make_float4(y[0], y[1], y[2], y[3]);
+    *reinterpret_cast<float4*>(row + o1) = make_float4(y[4], y[5], y[6], y[7]);
+}
+template <>
+__device__ __forceinline__ void store8<__nv_bfloat16>(__nv_bfloat16* row, int o0, int o1, const float (&y)[8]) {
+    uint32_t w[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const __nv_bfloat162 v = __floats2bfloat162_rn(y[2 * e], y[2 * e + 1]);
+        w[e] = *reinterpret_cast<const uint32_t*>(&v);
+    }
+    if (o1 == o0 + 4) *reinterpret_cast<uint4*>(row + o0) = make_uint4(w[0], w[1], w[2], w[3]);
+    else {
+        *reinterpret_cast<uint2*>(row + o0) = make_uint2(w[0], w[1]);
+        *reinterpret_cast<uint2*>(row + o1) = make_uint2(w[2], w[3]);
+    }
+}
+// y = the eight elements x[0..3] at o0, x[4..7] at o1, rotated: neighbours (interleaved) or x[e] with x[e + 4] (half)
+__device__ __forceinline__ void rotate8(const float4 lo, const float4 hi, int mode, const float (&c)[4], const float (&s)[4], float (&y)[8]) {
+    const float x[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        if (mode == GRL_ROPE_INTERLEAVED) {
+            y[2 * e] = x[2 * e] * c[e] - x[2 * e + 1] * s[e];
+            y[2 * e + 1] = x[2 * e] * s[e] + x[2 * e + 1] * c[e];
+        } else if (mode == GRL_ROPE_HALF) {
+            y[e] = x[e] * c[e] - x[e + 4] * s[e];
+            y[e + 4] = x[e] * s[e] + x[e + 4] * c[e];
+        } else {
+            y[2 * e] = x[2 * e];
+            y[2 * e + 1] = x[2 * e + 1];
+        }
+    }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256, 3) kv_append_rows_kernel(const __grid_constant__ AppendArgs a) {
+    __shared__ double freq[128];        // lanes index the frequencies apart, which the constant bank would serialise
+    const int b = blockIdx.y, lanes = a.D / 8, groups = 256 / lanes;
+    const int group = threadIdx.x / lanes, l = threadIdx.x % lanes;
+    const int len0 = a.seq_lens[b];
+    if (len0 < 0 || len0 + a.n_new > a.max_pages * a.P) {      // no room: nothing is stored (see kv_append_kernel)
+        if (threadIdx.x == 0 && blockIdx.x == 0 && a.status && atomicCAS(a.status, 0, GRL_ERR_INVALID) == 0) {
+            a.status[1] = 4 << 28;
+            a.status[2] = b;
+            a.status[3] = len0;
+        }
+        return;
+    }
+    if (a.rope_mode != GRL_ROPE_NONE) {
+        if (threadIdx.x < a.D / 2) freq[threadIdx.x] = a.freq.inv_freq[threadIdx.x];
+        __syncthreads();
+    }
+    const int pos0 = a.pos_base + (a.pos_offsets ? a.pos_offsets[b] : 0) + len0;
+    T* kp = reinterpret_cast<T*>(a.k_pages);
+    T* vp = reinterpret_cast<T*>(a.v_pages);
+    // A token's runs: pairs of kv heads, then pairs of query heads.  Every thread group takes an equal, contiguous share of
+    // all (token, run): the CTAs that fit the SMs at once are busy to the end, and the angles change only with the token.
+    const int kv_runs = a.skip_kv ? 0 : (a.Hkv + kAppendHeads - 1) / kAppendHeads;
+    const int runs = kv_runs + (a.q_in ? (a.Hq + kAppendHeads - 1) / kAppendHeads : 0);
+    const int o0 = a.rope_mode == GRL_ROPE_HALF ? 4 * l : 8 * l, o1 = a.rope_mode == GRL_ROPE_HALF ? o0 + a.D / 2 : o0 + 4;
+    if (group < groups) {
+        const long long total = (long long)a.n_new * runs, all = (long long)gridDim.x * groups, mine = (long long)blockIdx.x * groups + group;
+        const long long lo = mine * total / all, hi = (mine + 1) * total / all;
+        float c[4] = {1.f, 1.f, 1.f, 1.f}, s[4] = {0.f, 0.f, 0.f, 0.f};
+        int i = (int)(lo / runs), r = (int)(lo % runs), angles_of = -1, page = 0;
+        for (long long item = lo; item < hi; ++item, ++r) {
+            if (r == runs) { r = 0; ++i; }
+            const int slot = len0 + i;
+            const bool is_kv = r < kv_runs;
+            const int h0 = (is_kv ? r : r - kv_runs) * kAppendHeads, heads = is_kv ? a.Hkv : a.Hq;
+            const size_t src = (((size_t)b * a.n_new + i) * heads + h0) * a.D;
+            const float* in = (is_kv ? a.k_new : a.q_in) + src;
+            float4 k[kAppendHeads][2], v[kAppendHeads][2];
+#pragma unroll
+            for (int h = 0; h < kAppendHeads; ++h)
+                if (h0 + h < heads) {
+                    k[h][0] = __ldcs(reinterpret_cast<const float4*>(in + h * a.D + o0));
+                    k[h][1] = __ldcs(reinterpret_cast<const float4*>(in + h * a.D + o1));
+                    if (is_kv) {
+                        v[h][0] = __ldcs(reinterpret_cast<const float4*>(a.v_new + src + h * a.D + o0));
+                        v[h][1] = __ldcs(reinterpret_cast<const float4*>(a.v_new + src + h * a.D + o1));
+                    }
+                }
+            if (angles_of != i) {       // under the first run's loads
+                page = a.block_table[(size_t)b * a.max_pages + slot / a.P];
+                if (a.rope_mode != GRL_ROPE_NONE) {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) rope_sincos(pos0 + i, freq[4 * l + e], &c[e], &s[e]);
+                }
+                angles_of = i;
+            }
+            float y[8];
+#pragma unroll
+            for (int h = 0; h < kAppendHeads; ++h)
+                if (h0 + h < heads) {
+                    rotate8(k[h][0], k[h][1], a.rope_mode, c, s, y);
+                    if (is_kv) {
+                        const size_t dst = (((size_t)page * a.Hkv + h0 + h) * a.P + slot % a.P) * a.D;
+                        store8<T>(kp + dst, o0, o1, y);
+                        rotate8(v[h][0], v[h][1], GRL_ROPE_NONE, c, s, y);
+                        store8<T>(vp + dst, o0, o1, y);
+                    } else {
+                        store8<float>(a.q_out + src + h * a.D, o0, o1, y);
+                    }
+                }
+        }
+    }
+    if (a.update_lens) {    // gridDim.x == 1 here: every thread has read len0
+        __syncthreads();
+        if (threadIdx.x == 0) a.seq_lens[b] = len0 + a.n_new;
+    }
+}
+
 __global__ void advance_lens_kernel(int32_t* seq_lens, int B, int n, int capacity) {
     int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b < B && seq_lens[b] >= 0 && seq_lens[b] + n <= capacity) seq_lens[b] += n;   // a full sequence was skipped
@@ -151,14 +276,24 @@ __device__ __forceinline__ float half_bits_to_scale(uint16_t h) {           // k
     if (e == 0) return (float)m * 5.9604644775390625e-08f;                  // ldexp(m, -24), exact
     return __uint_as_float((sign << 31) | ((e + 112u) << 23) | (m << 13));
 }
-// int(log2f(a)) of the reference (kv_cache.cpp:318): the float32 logarithm, truncated toward zero.  The
-// logarithm is taken in double and rounded to float, which is what a correctly rounded log2f returns.
+// int(log2f(a)) of the reference (kv_cache.cpp:318): the float32 logarithm, truncated toward zero.  Away from the powers of
+// two that is the exponent field (plus one below 1, where truncation rounds up).  Within 64 ulps of a power of two the float32
+// logarithm may round to the integer: there it is taken in double and rounded to float, which is what a correctly rounded
+// log2f returns (the double logarithm for every element was most of a bulk append's time).
+__device__ __forceinline__ int trunc_log2f(float a) {                       // a >= 2^-9, a normal number
+    const uint32_t bits = __float_as_uint(a), m = bits & 0x7fffffu;
+    if (m - 64u < 0x7fffffu - 128u) {
+        const int e = (int)(bits >> 23) - 127;
+        return e < 0 ? e + 1 : e;
+    }
+    return (int)(float)log2((double)a);
+}
 __device__ __forceinline__ uint8_t fp8_encode(float scaled) {               // kv_cache.cpp:306-327
     scaled = fmaxf(-448.0f, fminf(448.0f, scaled));
     const int sign = scaled < 0.f ? 1 : 0;
     const float a = fabsf(scaled);
     if (a < 1.0f / 512.0f) return 0;
-    int e = (int)(float)log2((double)a);
+    int e = trunc_log2f(a);
     e = max(0, min(15, e + 7));
     const float mantissa = __fsub_rn(__fdiv_rn(a, __uint_as_float((uint32_t)(e - 7 + 127) << 23)), 1.0f);
     // a negative fraction (magnitudes below 1, whose exponent came out one too high) wraps like the reference's
@@ -188,45 +323,51 @@ __global__ void __launch_bounds__(1024) kv_append_quant_kernel(AppendArgs a) {
         return;
     }
     const int pos_off = a.pos_offsets ? a.pos_offsets[b] : 0;
-    const int items = a.n_new * a.Hkv * G;
-    const int half = a.D / 2;
+    // an item is one group of one token for a run of heads: the angles of its elements are the same for all of them
+    const int half = a.D / 2, per = a.heads_per_item, runs = (a.Hkv + per - 1) / per;
+    const int items = a.n_new * runs * G;
     uint8_t* kp = reinterpret_cast<uint8_t*>(a.k_pages);
     uint8_t* vp = reinterpret_cast<uint8_t*>(a.v_pages);
     for (int item = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); item < items; item += gridDim.x * (blockDim.x >> 5)) {
-        const int g = item % G, h = (item / G) % a.Hkv, i = item / (G * a.Hkv);
+        const int g = item % G, h0 = ((item / G) % runs) * per, i = item / (G * runs);
         const int d = g * 32 + lane;
         const int slot_pos = len0 + i;
-        const size_t src = (((size_t)b * a.n_new + i) * a.Hkv + h) * a.D;
-        float kx = a.k_new[src + d];
+        const int page = a.block_table[(size_t)b * a.max_pages + slot_pos / a.P];
+        float c = 1.f, s = 0.f;
+        int d_other = d;
+        bool first = true;
         if (a.rope_mode != GRL_ROPE_NONE) {
-            int j, d_other;
-            bool first;
+            int j;
             if (a.rope_mode == GRL_ROPE_INTERLEAVED) { j = d >> 1; first = (d & 1) == 0; d_other = d ^ 1; }
             else { j = d % half; first = d < half; d_other = first ? d + half : d - half; }
-            float c, s;
             rope_sincos(a.pos_base + pos_off + slot_pos, a.freq.inv_freq[j], &c, &s);
-            const float other = a.k_new[src + d_other];
-            kx = first ? kx * c - other * s : other * s + kx * c;
         }
-        const float vx = a.v_new[src + d];
-        float kmax = fabsf(kx), vmax = fabsf(vx);
+        for (int h = h0; h < min(h0 + per, a.Hkv); ++h) {
+            const size_t src = (((size_t)b * a.n_new + i) * a.Hkv + h) * a.D;
+            float kx = a.k_new[src + d];
+            if (a.rope_mode != GRL_ROPE_NONE) {
+                const float other = a.k_new[src + d_other];
+                kx = first ? kx * c - other * s : other * s + kx * c;
+            }
+            const float vx = a.v_new[src + d];
+            float kmax = fabsf(kx), vmax = fabsf(vx);
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            kmax = fmaxf(kmax, __shfl_xor_sync(0xffffffffu, kmax, o));
-            vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
+            for (int o = 16; o > 0; o >>= 1) {
+                kmax = fmaxf(kmax, __shfl_xor_sync(0xffffffffu, kmax, o));
+                vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
+            }
+            const float kscale = kmax > 0.f ? __fdiv_rn(448.0f, kmax) : 1.0f;
+            const float vscale = vmax > 0.f ? __fdiv_rn(7.0f, vmax) : 1.0f;
+            const size_t row = ((size_t)page * a.Hkv + h) * a.P + slot_pos % a.P;
+            kp[row * a.D + d] = fp8_encode(__fmul_rn(kx, kscale));
+            int q = (int)roundf(__fmul_rn(vx, vscale)) + 8;                       // kv_cache.cpp:363-366
+            q = max(0, min(15, q));
+            const int q_hi = __shfl_down_sync(0xffffffffu, q, 1);
+            if ((lane & 1) == 0)
+                vp[((size_t)page * a.Hkv + h) * a.P * half + quant_v_off(slot_pos % a.P, d >> 1, a.D)] =
+                    (uint8_t)((q & 0x0F) | ((q_hi & 0x0F) << 4));
+            if (lane == 0) a.scales[row * G + g] = scale_to_half_bits(kscale);   // the value scale is dropped (:393-398)
         }
-        const float kscale = kmax > 0.f ? __fdiv_rn(448.0f, kmax) : 1.0f;
-        const float vscale = vmax > 0.f ? __fdiv_rn(7.0f, vmax) : 1.0f;
-        const int page = a.block_table[(size_t)b * a.max_pages + slot_pos / a.P];
-        const size_t row = ((size_t)page * a.Hkv + h) * a.P + slot_pos % a.P;
-        kp[row * a.D + d] = fp8_encode(__fmul_rn(kx, kscale));
-        int q = (int)roundf(__fmul_rn(vx, vscale)) + 8;                       // kv_cache.cpp:363-366
-        q = max(0, min(15, q));
-        const int q_hi = __shfl_down_sync(0xffffffffu, q, 1);
-        if ((lane & 1) == 0)
-            vp[((size_t)page * a.Hkv + h) * a.P * half + quant_v_off(slot_pos % a.P, d >> 1, a.D)] =
-                (uint8_t)((q & 0x0F) | ((q_hi & 0x0F) << 4));
-        if (lane == 0) a.scales[row * G + g] = scale_to_half_bits(kscale);   // the value scale is dropped (:393-398)
     }
     if (a.q_in) {           // the queries of the new positions, rotated like the keys (float32 in, float32 out)
         const int qitems = a.n_new * a.Hq * half;
@@ -311,6 +452,19 @@ __global__ void mla_split_kernel(const float* __restrict__ in, float* __restrict
     }
 }
 
+// kv_append_rows_kernel: rows of whole 8-element pieces, everything on 16-byte boundaries
+static bool append_rows_fit(const AppendArgs& a) {
+    const uintptr_t all = (uintptr_t)a.k_new | (uintptr_t)a.v_new | (uintptr_t)a.q_in | (uintptr_t)a.q_out | (uintptr_t)a.k_pages | (uintptr_t)a.v_pages;
+    return a.D % 8 == 0 && all % 16 == 0;
+}
+// One (token, run of heads) a thread group while that leaves SMs idle, the CTAs that are resident at once beyond.
+static dim3 append_rows_grid(grl_device* dev, const AppendArgs& a) {
+    const int runs = (a.skip_kv ? 0 : (a.Hkv + kAppendHeads - 1) / kAppendHeads) + (a.q_in ? (a.Hq + kAppendHeads - 1) / kAppendHeads : 0);
+    const int groups = 256 / (a.D / 8);
+    const long long ctas = ((long long)a.n_new * runs + groups - 1) / groups, resident = (3LL * dev->prop.multiProcessorCount + a.B - 1) / a.B;
+    return dim3((unsigned)(ctas < resident ? ctas : resident), a.B);
+}
+
 static int check_layout(const grl_kv_layout& kv) {
     GRL_REQUIRE(kv.k_pages && kv.v_pages && kv.block_table && kv.seq_lens, "NULL cache pointer");
     GRL_REQUIRE(kv.batch > 0 && kv.num_kv_heads > 0 && kv.page_tokens > 0 && kv.max_pages > 0, "bad cache shape");
@@ -356,11 +510,14 @@ int grl_kv_append(grl_device* dev, const grl_append_params* p) {
         const long long warps = (long long)p->n_new * kv.num_kv_heads * (kv.head_dim / 32);
         if (warps <= 32) {      // a decode step: one wide CTA per sequence does keys, values, queries and the length
             a.update_lens = p->update_lens ? 1 : 0;
+            a.heads_per_item = 1;
             kv_append_quant_kernel<<<dim3(1, kv.batch), 1024, 0, dev->stream>>>(a);
             GRL_LAUNCHED("kv_append_quant_kernel");
             return GRL_OK;
         }
-        int ctas = (int)((warps + 7) / 8);
+        // eight heads a warp once there are enough tokens to fill the SMs (64 warps each) all the same
+        a.heads_per_item = warps * kv.batch / 8 >= 64LL * dev->prop.multiProcessorCount ? 8 : 1;
+        int ctas = (int)((warps / a.heads_per_item + 7) / 8);
         if (ctas > 1024) ctas = 1024;
         a.q_in = nullptr;       // bulk append: the queries go through the plain kernel below
         a.update_lens = 0;
@@ -370,10 +527,13 @@ int grl_kv_append(grl_device* dev, const grl_append_params* p) {
         if (p->q_in) {
             a.skip_kv = 1;
             a.update_lens = 0;
-            const long long qitems = (long long)p->n_new * (kv.num_kv_heads + p->num_q_heads) * (kv.head_dim / 2);
-            int qchunks = (int)((qitems + 4095) / 4096);
-            if (qchunks > 128) qchunks = 128;
-            kv_append_kernel<float><<<dim3(qchunks, kv.batch), 256, 0, dev->stream>>>(a);
+            if (append_rows_fit(a)) {
+                kv_append_rows_kernel<float><<<append_rows_grid(dev, a), 256, 0, dev->stream>>>(a);
+            } else {
+                const long long qitems = (long long)p->n_new * (kv.num_kv_heads + p->num_q_heads) * (kv.head_dim / 2);
+                const int qchunks = (int)((qitems + 4095) / 4096);
+                kv_append_kernel<float><<<dim3(qchunks < 128 ? qchunks : 128, kv.batch), 256, 0, dev->stream>>>(a);
+            }
             GRL_LAUNCHED("kv_append_kernel");
         }
         if (p->update_lens) {
@@ -383,17 +543,28 @@ int grl_kv_append(grl_device* dev, const grl_append_params* p) {
         }
         return GRL_OK;
     }
-    const long long items = (long long)p->n_new * (kv.num_kv_heads + (p->q_in ? p->num_q_heads : 0)) * (kv.head_dim / 2);
-    // one CTA per sequence while a CTA has at most 16 items per thread (a decode step), more for bulk appends
-    int chunks = (int)((items + 4095) / 4096);
-    if (chunks > 128) chunks = 128;
-    const bool fused_update = p->update_lens && chunks == 1;
-    a.update_lens = fused_update ? 1 : 0;
-    dim3 grid(chunks, kv.batch);
-    // one chunk (the decode step): a wide CTA, so that every thread has only a few dependent load chains
-    const int threads = chunks == 1 ? (items > 512 ? 1024 : 512) : 256;
-    if (kv.cache_dtype == GRL_BF16) kv_append_kernel<__nv_bfloat16><<<grid, threads, 0, dev->stream>>>(a);
-    else kv_append_kernel<float><<<grid, threads, 0, dev->stream>>>(a);
+    bool fused_update;
+    if (append_rows_fit(a)) {
+        dim3 grid = append_rows_grid(dev, a);
+        // a decode step (or a few tokens): one CTA per sequence also advances the length, which saves a launch
+        if (p->update_lens && grid.x <= 4) grid.x = 1;
+        fused_update = p->update_lens && grid.x == 1;
+        a.update_lens = fused_update ? 1 : 0;
+        if (kv.cache_dtype == GRL_BF16) kv_append_rows_kernel<__nv_bfloat16><<<grid, 256, 0, dev->stream>>>(a);
+        else kv_append_rows_kernel<float><<<grid, 256, 0, dev->stream>>>(a);
+    } else {
+        const long long items = (long long)p->n_new * (kv.num_kv_heads + (p->q_in ? p->num_q_heads : 0)) * (kv.head_dim / 2);
+        // one CTA per sequence while a CTA has at most 16 items per thread (a decode step), more for bulk appends
+        int chunks = (int)((items + 4095) / 4096);
+        if (chunks > 128) chunks = 128;
+        fused_update = p->update_lens && chunks == 1;
+        a.update_lens = fused_update ? 1 : 0;
+        dim3 grid(chunks, kv.batch);
+        // one chunk (the decode step): a wide CTA, so that every thread has only a few dependent load chains
+        const int threads = chunks == 1 ? (items > 512 ? 1024 : 512) : 256;
+        if (kv.cache_dtype == GRL_BF16) kv_append_kernel<__nv_bfloat16><<<grid, threads, 0, dev->stream>>>(a);
+        else kv_append_kernel<float><<<grid, threads, 0, dev->stream>>>(a);
+    }
     GRL_LAUNCHED("kv_append_kernel");
     if (p->update_lens && !fused_update) {
         advance_lens_kernel<<<(kv.batch + 127) / 128, 128, 0, dev->stream>>>(kv.seq_lens, kv.batch, p->n_new,

@@ -325,3 +325,40 @@ def test_attention_mask_op(gpu):
     assert np.array_equal(gpu.attention_mask(s, mask=km, mask_value=-7.5), orc.attention_mask(s, mask=km, mask_value=-7.5))
     with pytest.raises(RuntimeError):
         gpu.attention_mask(s)
+
+
+@pytest.mark.parametrize("D,Hkv,Hq,n,P,mode,dtype", [
+    (128, 8, 0, 700, 64, "interleaved", "bf16"),    # a prompt: many CTAs, several heads a thread group
+    (64, 3, 9, 130, 16, "half", "bf16"),            # an odd head left over, queries, small pages
+    (32, 1, 2, 65, 32, "interleaved", "fp32"),
+    (40, 5, 5, 33, 16, "half", "fp32"),             # thread groups that do not divide the CTA
+    (128, 8, 32, 1, 64, "none", "bf16"),            # a decode step
+    (12, 2, 4, 9, 16, "half", "fp32")])             # not a multiple of 8: the element-wise kernel
+def test_append_vector_rows(dev, D, Hkv, Hq, n, P, mode, dtype):
+    from gpu_helpers import PagedCache
+    from grilly_next import cabi
+    rng = np.random.default_rng(D + n)
+    k, v = (rng.standard_normal((2, n, Hkv, D), dtype=np.float32) for _ in range(2))
+    q = rng.standard_normal((2, n, Hq, D), dtype=np.float32) if Hq else None
+    pc = PagedCache(dev, 2, Hkv, D, n + 7, page_tokens=P, dtype=cabi.BF16 if dtype == "bf16" else cabi.F32, shuffle_pages=True, seed=1)
+    code = {"none": cabi.ROPE_NONE, "interleaved": cabi.ROPE_INTERLEAVED, "half": cabi.ROPE_HALF}[mode]
+    qo = pc.append(k, v, q, rope_mode=code, pos_base=5)
+    half = D // 2
+    ang = (5 + np.arange(n))[:, None] * (10000.0 ** (-2.0 * np.arange(half) / D))[None, :]
+    c, s = np.cos(ang)[None, :, None, :], np.sin(ang)[None, :, None, :]
+
+    def rotated(x):
+        if mode == "none":
+            return x
+        a, b = (x[..., 0::2], x[..., 1::2]) if mode == "interleaved" else (x[..., :half], x[..., half:])
+        y = np.empty_like(x)
+        ya, yb = (y[..., 0::2], y[..., 1::2]) if mode == "interleaved" else (y[..., :half], y[..., half:])
+        ya[...], yb[...] = a * c - b * s, a * s + b * c
+        return y
+
+    for b in range(2):
+        gk, gv = pc.gather(b)
+        assert np.array_equal(gv, orc.round_bf16(v[b]) if dtype == "bf16" else v[b])
+        assert np.abs(gk - rotated(k)[b]).max() <= (2e-2 if dtype == "bf16" else 1e-5)
+    if q is not None:
+        assert np.abs(qo - rotated(q)).max() <= 1e-5
