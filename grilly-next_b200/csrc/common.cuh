@@ -24,7 +24,7 @@ struct TmapKey {
     uint64_t dims[3];
     uint64_t strides[2];       // bytes, dimensions 1..rank-1
     uint32_t box[3];
-    uint32_t bytes;            // 1: uint8 elements; 0: bf16 (two bytes)
+    uint32_t bytes;            // 1: uint8 elements; 4: float32; 0: bf16 (two bytes)
 };
 constexpr long long kDefaultWaitLimitCycles = 2000000000LL;       // ~1 s at 2 GHz: mbarrier waits inside a kernel
 constexpr long long kDefaultPeerWaitLimitCycles = 1000000000LL;   // ~0.5 s: a peer GPU that never posts
@@ -147,6 +147,19 @@ inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &attr; cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+// The same with clusters of `size` CTAs along x.
+template <typename... P, typename... A>
+inline cudaError_t launch_pdl_cluster(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, int size, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+    cudaLaunchAttribute attr[2] = {};
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)size; attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -6,11 +6,12 @@
 // i.e. the steps on either side of attention.  x is (M, K) row-major, W (N, K) row-major -- both K-major,
 // which is what tcgen05.mma wants from shared memory -- and y (M, N).
 //
-// One CTA computes a 128 x 128 tile of y: warp 0 streams 128 x 64 boxes of x and W through a four-stage
-// shared-memory ring with TMA (128-byte swizzle; rows and columns past the edge arrive as zeros), one thread of
-// warp 1 issues four 128x128x16 tcgen05.mma per stage into a TMEM accumulator (128 lanes x 128 fp32 columns),
-// and warps 4-7 read the accumulator back, add the bias and write rows through a shared-memory transpose so
-// that every warp store covers contiguous bytes of one row.  Every mbarrier wait is bounded.
+// Two kernels:
+//  linear_pair_kernel   products that fill the GPU: two SMs share one 256 x BN tile of y (cta_group::2), persistent.
+//  linear_split_kernel  everything smaller, above all the few rows of a decode step, where the one pass over W bounds the
+//                       time: W rows are the 128 rows of the product, x rows its columns, and the K range is cut over the
+//                       CTAs of a cluster, which add their partial tiles through distributed shared memory.
+// Every mbarrier wait is bounded.
 #include "common.cuh"
 #include "sgemm.cuh"
 #include "sm100_ptx.cuh"
@@ -21,19 +22,18 @@ namespace lin {
 
 using namespace sm100;
 
-constexpr int BM = 128, BN = 128, BK = 64;
-constexpr int NST = 3;             // 96 KiB of ring: two CTAs per SM, so one CTA's epilogue overlaps the other's products
-constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2, STAGE = A_BYTES + B_BYTES;   // 16 + 16 KiB
-constexpr int SMEM_BAR = NST * STAGE;
-constexpr int SMEM_TOTAL = SMEM_BAR + 128 + 1024;
-constexpr int kThreads = 256;      // warp 0 TMA, warp 1 MMA, warps 2-3 idle, warps 4-7 epilogue (TMEM lanes 0..127)
-constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+constexpr int BK = 64;             // one 128-byte swizzle row of bf16
+constexpr int kThreads = 256;      // warp 0 TMA, warp 1 MMA, warp 2 TMEM, warp 3 idle, warps 4-7 epilogue (TMEM lanes 0..127)
+constexpr int kSmemMax = 227 * 1024;
 
 struct Args {
     const float* bias;     // (N) or NULL
     float* y;              // (M, N)
     int32_t* status;
     int M, N, K;
+    int tile_rows;         // split kernel: x rows per tile (a multiple of 16, at most 256)
+    int stages, splits;    // split kernel: ring stages, CTAs of a cluster along K
+    int tma_store;         // pair kernel: rows of y start on 16-byte boundaries
     long long wait_limit;
 };
 
@@ -55,22 +55,207 @@ __device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity, volatile int
     }
 }
 
-__global__ void __launch_bounds__(kThreads, 2)
-linear_sm100_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const Args a) {
+__device__ __forceinline__ uint32_t instr_desc(int m, int n) {   // D f32, A and B bf16, both K-major
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+}
+
+// ---- the pair kernel.  A 128 x 128 tile per SM reads its operands from shared memory as fast as the tensor core eats them
+// (64 cycles of reads and 64 of TMA writes per 64 cycles of products), which held a one-SM kernel at 1.0 PFLOP/s; a pair
+// reads each half of W's tile once for both SMs.  A CTA stages its 128 rows of x and BN/2 rows of W; the even CTA's thread
+// issues the products for both; the accumulator (128 lanes x BN columns in each SM) is double-buffered, so that one tile's
+// epilogue runs under the next tile's products.
+template <int BN_>
+struct Pair {
+    static constexpr int BN = BN_, A_BYTES = 128 * BK * 2, B_BYTES = BN / 2 * BK * 2, STAGE = A_BYTES + B_BYTES;
+    static constexpr int OUT_BYTES = 4 * 2 * 4096;                  // a warp's two 32 x 32 float boxes on their way out
+    static constexpr int NST = (kSmemMax - 2048 - OUT_BYTES) / STAGE;      // 6 or 8
+    static constexpr int SMEM_OUT = NST * STAGE, SMEM_BAR = SMEM_OUT + OUT_BYTES, SMEM = SMEM_BAR + 256 + 1024;
+};
+
+template <int BN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+linear_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmY,
+                   const Args a) {
+    using P = Pair<BN>;
+    constexpr int NST = P::NST;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
     uint8_t* smem = smem_raw + (base - raw);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    const uint32_t rank = cluster_ctarank();
+    const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+    const int tiles_m = (a.M + 255) / 256, tiles_n = (a.N + BN - 1) / BN, tiles = tiles_m * tiles_n;
     const int n_k = (a.K + BK - 1) / BK;
 
-    const uint32_t bars = base + SMEM_BAR;
+    const uint32_t bars = base + P::SMEM_BAR;
+    auto full = [&](int s) { return bars + (uint32_t)s * 8u; };
+    auto empty = [&](int s) { return bars + (uint32_t)(NST + s) * 8u; };
+    auto acc_full = [&](int i) { return bars + (uint32_t)(2 * NST + i) * 8u; };
+    auto acc_empty = [&](int i) { return bars + (uint32_t)(2 * NST + 2 + i) * 8u; };
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + P::SMEM_BAR + (2 * NST + 4) * 8);
+    volatile int* abort = reinterpret_cast<volatile int*>(smem + P::SMEM_BAR + (2 * NST + 4) * 8 + 4);
+
+    if (tid == 0) {
+        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmX)) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmW)) : "memory");
+        for (int s = 0; s < NST; ++s) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
+        for (int i = 0; i < 2; ++i) { mbar_init(acc_full(i), 1); mbar_init(acc_empty(i), 8); }     // 4 epilogue warps of 2 CTAs
+        *abort = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        fence_async_smem();
+    }
+    if (warp == 2) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();                    // the peer's barriers exist
+    tc_fence_after();
+    const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
+    pdl_wait();
+
+    // Tiles in groups of eight rows of tiles, walked column by column: the pairs at work at one time share both operands' tiles
+    // in L2.
+    auto place = [&](int t, int& tm, int& tn) {
+        const int g = t / (8 * tiles_n), rows = min(8, tiles_m - 8 * g), r = t - g * 8 * tiles_n;
+        tm = 8 * g + r % rows;
+        tn = r / rows;
+    };
+
+    if (warp == 0) {
+        if (lane == 0) {
+            int it = 0;
+            bool ok = true;
+            for (int t = pair; t < tiles && ok; t += pairs) {
+                int tm, tn;
+                place(t, tm, tn);
+                const int m0 = tm * 256 + (int)rank * 128, n0 = tn * BN + (int)rank * (BN / 2);
+                for (int k = 0; k < n_k; ++k, ++it) {
+                    const int s = it % NST, ph = it / NST;
+                    if (ph > 0 && !wait(empty(s), (ph - 1) & 1, abort, a, NST + s)) { ok = false; break; }
+                    const uint32_t dst = base + (uint32_t)s * P::STAGE, bar = cluster_map(full(s), 0);
+                    if (rank == 0) mbar_expect_tx(full(s), 2 * P::STAGE);        // both CTAs' copies signal the even CTA
+                    tma_load_2d_pair(dst, &tmX, k * BK, m0, bar);
+                    tma_load_2d_pair(dst + P::A_BYTES, &tmW, k * BK, n0, bar);
+                }
+            }
+            if (*abort && rank == 0) {     // copies already issued must land before the shared memory is released
+                const long long t0 = clock64();
+                for (int i = max(0, it - NST); i < it; ++i)
+                    while (!mbar_try_wait(full(i % NST), (i / NST) & 1) && clock64() - t0 < a.wait_limit) {}
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0 && rank == 0) {
+            const uint32_t idesc = instr_desc(256, BN);
+            int it = 0, n = 0;
+            bool ok = true;
+            for (int t = pair; t < tiles && ok; t += pairs, ++n) {
+                const int acc = n & 1;
+                if (n >= 2 && !wait(acc_empty(acc), ((n >> 1) - 1) & 1, abort, a, 2 * NST + 2 + acc)) break;
+                tc_fence_after();
+                const uint32_t d = tmem + (uint32_t)acc * 256u;
+                for (int k = 0; k < n_k; ++k, ++it) {
+                    const int s = it % NST, ph = it / NST;
+                    ok = wait(full(s), ph & 1, abort, a, s);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint32_t a_lo = desc_lo(base + (uint32_t)s * P::STAGE, 16), b_lo = desc_lo(base + (uint32_t)s * P::STAGE + P::A_BYTES, 16);
+#pragma unroll
+                    for (int ks = 0; ks < BK / 16; ++ks)
+                        mma_ss_pair(d, a_lo + (uint32_t)(ks * 32 >> 4), b_lo + (uint32_t)(ks * 32 >> 4), idesc, (k | ks) != 0);
+                    mma_commit_pair(empty(s));       // in both CTAs: the stage is free once these products have read it
+                }
+                if (ok) mma_commit_pair(acc_full(acc));
+            }
+        }
+    } else if (warp >= 4) {
+        // ------------------------------------------------------------------ epilogue: TMEM -> (+ bias) -> global
+        const int w = warp & 3;
+        const uint32_t stage = base + P::SMEM_OUT + (uint32_t)w * 8192u;
+        int n = 0;
+        for (int t = pair; t < tiles; t += pairs, ++n) {
+            const int acc = n & 1;
+            int tm, tn;
+            place(t, tm, tn);
+            if (!__all_sync(0xffffffffu, wait(acc_full(acc), (n >> 1) & 1, abort, a, 2 * NST + acc))) break;
+            tc_fence_after();
+            const int row0 = tm * 256 + (int)rank * 128 + w * 32;
+            const uint32_t t_addr = tmem + (uint32_t)acc * 256u + ((uint32_t)(w * 32) << 16);
+#pragma unroll 1
+            for (int c = 0; c < BN / 32; ++c) {
+                uint32_t r[32];
+                tmem_ld_x32_sync(t_addr + c * 32, r);
+                const int col = tn * BN + c * 32;
+                if (c == BN / 32 - 1) {        // the last read of this accumulator: the next tile's products may overwrite it
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_cluster(cluster_map(acc_empty(acc), 0));
+                }
+                if (row0 >= a.M || col >= a.N) continue;
+                if (a.bias) {
+                    const float bl = col + lane < a.N ? __ldg(a.bias + col + lane) : 0.f;
+#pragma unroll
+                    for (int e = 0; e < 32; ++e) r[e] = __float_as_uint(__uint_as_float(r[e]) + __shfl_sync(0xffffffffu, bl, e));
+                }
+                if (a.tma_store) {
+                    // 32 rows x 128 bytes under the 128-byte swizzle, two boxes in turn
+                    const uint32_t box = stage + (uint32_t)(c & 1) * 4096u;
+                    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+                    __syncwarp();
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        sts128(box + lane * 128 + ((q ^ (lane & 7)) << 4), make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]));
+                    fence_async_smem();
+                    __syncwarp();
+                    if (lane == 0) {
+                        tma_store_2d(&tmY, box, col, row0);
+                        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                    }
+                } else if (row0 + lane < a.M) {
+                    float* dst = a.y + (size_t)(row0 + lane) * a.N + col;
+#pragma unroll
+                    for (int e = 0; e < 32; ++e)
+                        if (col + e < a.N) dst[e] = __uint_as_float(r[e]);
+                }
+            }
+        }
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    __syncwarp();
+    cluster_sync();                    // neither CTA leaves while the other may still signal or read it
+    tc_fence_after();
+    if (warp == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+}
+
+// ---- the split kernel.  Tile: 128 rows of W x tile_rows rows of x, y^T of it in TMEM (lane = column n of y, TMEM column = row m),
+// so that few rows of x waste no product rows and a warp's store of one m is 32 consecutive floats of y.  Bound by the pass
+// over W: two CTAs an SM keep about 200 KB in flight.
+__global__ void __launch_bounds__(kThreads, 2)
+linear_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const Args a) {
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t raw = smem_u32(smem_raw);
+    const uint32_t base = (raw + 1023u) & ~1023u;
+    uint8_t* smem = smem_raw + (base - raw);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int NST = a.stages, NT = a.tile_rows;
+    const int w_bytes = 128 * BK * 2, stage_bytes = w_bytes + NT * BK * 2;
+    const int part = a.splits > 1 ? (int)cluster_ctarank() : 0;
+    const int n0 = (int)(blockIdx.x / a.splits) * 128, m0 = blockIdx.y * NT;
+    const int n_k = (a.K + BK - 1) / BK, k0 = part * n_k / a.splits, k1 = (part + 1) * n_k / a.splits;
+    const int tmem_cols = NT <= 32 ? 32 : NT <= 64 ? 64 : NT <= 128 ? 128 : 256;
+
+    const uint32_t bars = base;        // barriers first (1 KiB), then the ring
+    const uint32_t ring = base + 1024;
     auto full = [&](int s) { return bars + (uint32_t)s * 8u; };
     auto empty = [&](int s) { return bars + (uint32_t)(NST + s) * 8u; };
     const uint32_t acc_full = bars + 2 * NST * 8;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + SMEM_BAR + (2 * NST + 1) * 8);
-    volatile int* abort = reinterpret_cast<volatile int*>(smem + SMEM_BAR + (2 * NST + 1) * 8 + 4);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + (2 * NST + 1) * 8);
+    volatile int* abort = reinterpret_cast<volatile int*>(smem + (2 * NST + 1) * 8 + 4);
 
     if (tid == 0) {
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmX)) : "memory");
@@ -82,100 +267,99 @@ linear_sm100_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_consta
         fence_async_smem();
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(128) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(tmem_cols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
+    pdl_wait();
 
+    bool good = true;
     if (warp == 0) {
         if (lane == 0) {
             int issued = 0;
-            for (int k = 0; k < n_k; ++k) {
-                const int s = k % NST, it = k / NST;
-                if (it > 0 && !wait(empty(s), (it - 1) & 1, abort, a, NST + s)) break;
-                const uint32_t dst = base + (uint32_t)s * STAGE;
-                mbar_expect_tx(full(s), STAGE);
-                tma_load_2d(dst, &tmX, k * BK, m0, full(s));
-                tma_load_2d(dst + A_BYTES, &tmW, k * BK, n0, full(s));
-                issued = k + 1;
+            for (int k = k0; k < k1; ++k) {
+                const int i = k - k0, s = i % NST, ph = i / NST;
+                if (ph > 0 && !wait(empty(s), (ph - 1) & 1, abort, a, NST + s)) break;
+                const uint32_t dst = ring + (uint32_t)(s * stage_bytes);
+                mbar_expect_tx(full(s), stage_bytes);
+                tma_load_2d(dst, &tmW, k * BK, n0, full(s));
+                tma_load_2d(dst + w_bytes, &tmX, k * BK, m0, full(s));
+                issued = i + 1;
             }
             if (*abort) {     // copies already issued must land before the shared memory is released
                 const long long t0 = clock64();
-                for (int k = max(0, issued - NST); k < issued; ++k)
-                    while (!mbar_try_wait(full(k % NST), (k / NST) & 1) && clock64() - t0 < a.wait_limit) {}
+                for (int i = max(0, issued - NST); i < issued; ++i)
+                    while (!mbar_try_wait(full(i % NST), (i / NST) & 1) && clock64() - t0 < a.wait_limit) {}
             }
         }
     } else if (warp == 1) {
         if (lane == 0) {
+            const uint32_t idesc = instr_desc(128, NT);
             bool ok = true;
-            for (int k = 0; k < n_k && ok; ++k) {
-                const int s = k % NST, it = k / NST;
-                ok = wait(full(s), it & 1, abort, a, s);
+            for (int k = k0; k < k1 && ok; ++k) {
+                const int i = k - k0, s = i % NST, ph = i / NST;
+                ok = wait(full(s), ph & 1, abort, a, s);
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t a_lo = desc_lo(base + (uint32_t)s * STAGE, 16), b_lo = desc_lo(base + (uint32_t)s * STAGE + A_BYTES, 16);
-                if (k == 0) mma_ss2<false>(tmem, a_lo, b_lo, IDESC);
-                else mma_ss2<true>(tmem, a_lo, b_lo, IDESC);
+                const uint32_t w_lo = desc_lo(ring + (uint32_t)(s * stage_bytes), 16), x_lo = desc_lo(ring + (uint32_t)(s * stage_bytes + w_bytes), 16);
 #pragma unroll
-                for (int ks = 1; ks < BK / 16; ++ks) mma_ss2<true>(tmem, a_lo + (uint32_t)(ks * 32 >> 4), b_lo + (uint32_t)(ks * 32 >> 4), IDESC);
-                mma_commit(empty(s));                 // the stage is free once these MMAs have read it
+                for (int ks = 0; ks < BK / 16; ++ks)
+                    mma_ss3(tmem, w_lo + (uint32_t)(ks * 32 >> 4), x_lo + (uint32_t)(ks * 32 >> 4), idesc, (i | ks) != 0);
+                mma_commit(empty(s));                 // the stage is free once these products have read it
             }
             if (ok) mma_commit(acc_full);
         }
     } else if (warp >= 4) {
-        // ------------------------------------------------------------------ epilogue: TMEM -> (+ bias) -> global
-        const bool ok = __all_sync(0xffffffffu, wait(acc_full, 0, abort, a, 2 * NST));
-        if (ok) {
-            tc_fence_after();
-            const int w = warp & 3;
-            const uint32_t t_addr = tmem + ((uint32_t)(w * 32) << 16);
-            // the ring is idle now (every MMA has completed): 8 KiB of it per warp stage 32 rows x 64 columns
-            const uint32_t stage = base + (uint32_t)w * 8192;
-            const int row_w0 = m0 + w * 32;
-            const bool vec2 = (a.N % 2) == 0;
+        good = __all_sync(0xffffffffu, wait(acc_full, 0, abort, a, 2 * NST));
+        tc_fence_after();
+        const int w = warp & 3, n = n0 + w * 32 + lane;
+        const uint32_t t_addr = tmem + ((uint32_t)(w * 32) << 16);
+        const float b = a.bias && n < a.N ? __ldg(a.bias + n) : 0.f;
+        float* part_tile = reinterpret_cast<float*>(smem + 1024) + w * 32 + lane;     // [m][128]; the ring is idle by now
+        const int rows = min(NT, a.M - m0);
+        if (good) {
+            for (int c = 0; c < rows; c += 32) {
+                uint32_t r[32];
+                tmem_ld_x32_sync(t_addr + c, r);
 #pragma unroll
-            for (int pass = 0; pass < 2; ++pass) {
-#pragma unroll
-                for (int ch = 0; ch < 2; ++ch) {
-                    uint32_t r[32];
-                    tmem_ld_x32_sync(t_addr + pass * 64 + ch * 32, r);
-#pragma unroll
-                    for (int c = 0; c < 8; ++c) {
-                        const int chunk = ch * 8 + c;
-                        sts128(stage + lane * 256 + ((chunk ^ (lane & 15)) << 4), make_uint4(r[4 * c], r[4 * c + 1], r[4 * c + 2], r[4 * c + 3]));
-                    }
+                for (int e = 0; e < 32; ++e) {
+                    if (c + e >= rows) break;
+                    if (a.splits > 1) part_tile[(c + e) * 128] = __uint_as_float(r[e]);
+                    else if (n < a.N) a.y[(size_t)(m0 + c + e) * a.N + n] = __uint_as_float(r[e]) + b;
                 }
-                __syncwarp();
-                const int col = n0 + pass * 64 + 2 * lane;
-                float b0 = 0.f, b1 = 0.f;
-                if (a.bias) {
-                    if (col < a.N) b0 = __ldg(a.bias + col);
-                    if (col + 1 < a.N) b1 = __ldg(a.bias + col + 1);
-                }
-#pragma unroll 8
-                for (int rr = 0; rr < 32; ++rr) {
-                    const float2 v = lds64f(stage + rr * 256 + (((lane >> 1) ^ (rr & 15)) << 4) + (lane & 1) * 8);
-                    const int row = row_w0 + rr;
-                    if (row < a.M) {
-                        float* dst = a.y + (size_t)row * a.N + col;
-                        if (vec2 && col + 1 < a.N) *reinterpret_cast<float2*>(dst) = make_float2(v.x + b0, v.y + b1);
-                        else {
-                            if (col < a.N) dst[0] = v.x + b0;
-                            if (col + 1 < a.N) dst[1] = v.y + b1;
-                        }
-                    }
-                }
-                __syncwarp();
             }
         }
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(128) : "memory");
+    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols) : "memory");
+    if (a.splits > 1) {
+        __syncwarp();
+        // every CTA of the cluster adds up its share of the rows, parts in ascending k
+        cluster_sync();
+        const int rows = min(NT, a.M - m0), lo = part * rows / a.splits, hi = (part + 1) * rows / a.splits;
+        const int c = tid & 127, n = n0 + c;
+        if (n < a.N && !*abort) {
+            const float b = a.bias ? __ldg(a.bias + n) : 0.f;
+            for (int m = lo + (tid >> 7); m < hi; m += 2) {
+                float v[8];
+#pragma unroll
+                for (int p = 0; p < 8; ++p)
+                    if (p < a.splits) v[p] = ld_cluster_f32(cluster_map(base + 1024u + (uint32_t)(m * 128 + c) * 4u, (uint32_t)p));
+                float sum = v[0];
+#pragma unroll
+                for (int p = 1; p < 8; ++p)
+                    if (p < a.splits) sum += v[p];
+                a.y[(size_t)(m0 + m) * a.N + n] = sum + b;
+            }
+        }
+        __syncwarp();
+        cluster_sync();        // a CTA leaves only when nobody reads its part any more
+    }
 }
 
 // Exact fp32 form for a handful of rows: bound by the one pass over W, so a warp takes one row of W (one output column),
@@ -226,6 +410,66 @@ static int linear_f32(grl_device* dev, const float* x, const float* w, const flo
     return GRL_OK;
 }
 
+static int make_map(grl_device* dev, CUtensorMap* tm, const void* ptr, int rows, int cols, int box_rows, int box_cols, int elem_bytes) {
+    TmapKey k{};
+    k.ptr = ptr; k.rank = 2; k.swizzle_128b = 1; k.bytes = elem_bytes == 4 ? 4 : 0;
+    k.dims[0] = (uint64_t)cols; k.dims[1] = (uint64_t)rows; k.strides[0] = (uint64_t)cols * elem_bytes;
+    k.box[0] = (uint32_t)box_cols; k.box[1] = (uint32_t)box_rows;
+    return get_tensor_map(dev, k, tm);
+}
+
+template <int BN>
+static int launch_pair(grl_device* dev, const void* x, const void* w, Args a) {
+    using P = Pair<BN>;
+    CUtensorMap tx, tw, ty;
+    int rc = make_map(dev, &tx, x, a.M, a.K, 128, BK, 2);
+    if (!rc) rc = make_map(dev, &tw, w, a.N, a.K, BN / 2, BK, 2);
+    a.tma_store = a.N % 4 == 0 && (uintptr_t)a.y % 16 == 0;
+    ty = tx;
+    if (!rc && a.tma_store) rc = make_map(dev, &ty, a.y, a.M, a.N, 32, 32, 4);
+    if (rc) return rc;
+    static bool attr_set[64] = {};
+    if (!attr_set[dev->ordinal & 63]) {
+        GRL_CUDA(cudaFuncSetAttribute(linear_pair_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, P::SMEM));
+        attr_set[dev->ordinal & 63] = true;
+    }
+    const int tiles = (a.M + 255) / 256 * ((a.N + BN - 1) / BN), pairs = dev->prop.multiProcessorCount / 2;
+    GRL_CUDA(launch_pdl(linear_pair_kernel<BN>, 2 * (tiles < pairs ? tiles : pairs), kThreads, P::SMEM, dev->stream, tx, tw, ty, a));
+    GRL_LAUNCHED("linear_pair_kernel");
+    return GRL_OK;
+}
+
+static int launch_split(grl_device* dev, const void* x, const void* w, Args a) {
+    // x rows per tile: all of them up to 256 (W is then read once), else tiles of 128
+    a.tile_rows = a.M <= 256 ? (a.M + 15) / 16 * 16 : 128;
+    const int n_k = (a.K + BK - 1) / BK, sms = dev->prop.multiProcessorCount;
+    const int tiles = (a.N + 127) / 128 * ((a.M + a.tile_rows - 1) / a.tile_rows);
+    // K cut so that the CTAs come to two an SM; at least four slices each, at most a portable cluster
+    a.splits = 2 * sms / tiles;
+    if (a.splits > n_k / 4) a.splits = n_k / 4;
+    if (a.splits > 8) a.splits = 8;
+    if (a.splits < 1) a.splits = 1;
+    const int stage = (128 + a.tile_rows) * BK * 2, half = kSmemMax / 2 - 3072, whole = kSmemMax - 3072;
+    a.stages = (half / stage >= 3 ? half : whole) / stage;
+    if (a.stages > 8) a.stages = 8;
+    int smem = a.stages * stage;
+    if (a.splits > 1 && smem < a.tile_rows * 512) smem = a.tile_rows * 512;      // the partial tile
+    smem += 2048;
+    CUtensorMap tx, tw;
+    int rc = make_map(dev, &tx, x, a.M, a.K, a.tile_rows, BK, 2);
+    if (!rc) rc = make_map(dev, &tw, w, a.N, a.K, 128, BK, 2);
+    if (rc) return rc;
+    static bool attr_set[64] = {};
+    if (!attr_set[dev->ordinal & 63]) {
+        GRL_CUDA(cudaFuncSetAttribute(linear_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
+        attr_set[dev->ordinal & 63] = true;
+    }
+    dim3 grid((a.N + 127) / 128 * a.splits, (a.M + a.tile_rows - 1) / a.tile_rows);
+    GRL_CUDA(launch_pdl_cluster(linear_split_kernel, grid, kThreads, smem, dev->stream, a.splits, tx, tw, a));
+    GRL_LAUNCHED("linear_split_kernel");
+    return GRL_OK;
+}
+
 }  // namespace lin
 }  // namespace grl
 
@@ -242,24 +486,15 @@ extern "C" int grl_linear(grl_device* dev, const void* x, const void* w, const f
     GRL_REQUIRE(k % 8 == 0, "the tensor-core projection needs the inner dimension to be a multiple of 8 (got %d): rows must "
                             "start on 16-byte boundaries for TMA", k);
     GRL_REQUIRE(((uintptr_t)x % 16 == 0) && ((uintptr_t)w % 16 == 0) && ((uintptr_t)y % 8 == 0), "x, w must be 16-byte aligned");
-    CUtensorMap tx, tw;
-    TmapKey kx{}, kw{};
-    kx.ptr = x; kx.rank = 2; kx.swizzle_128b = 1; kx.dims[0] = (uint64_t)k; kx.dims[1] = (uint64_t)m; kx.strides[0] = (uint64_t)k * 2;
-    kx.box[0] = lin::BK; kx.box[1] = lin::BM;
-    kw = kx; kw.ptr = w; kw.dims[1] = (uint64_t)n; kw.box[1] = lin::BN;
-    int rc = get_tensor_map(dev, kx, &tx);
-    if (!rc) rc = get_tensor_map(dev, kw, &tw);
-    if (rc) return rc;
     lin::Args a{};
     a.bias = bias; a.y = y; a.status = dev->d_status; a.M = m; a.N = n; a.K = k; a.wait_limit = dev->wait_limit_cycles;
     dev->status_dirty = true;
-    static bool attr_set[64] = {};
-    if (!attr_set[dev->ordinal & 63]) {
-        GRL_CUDA(cudaFuncSetAttribute(lin::linear_sm100_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, lin::SMEM_TOTAL));
-        attr_set[dev->ordinal & 63] = true;
-    }
-    dim3 grid((n + lin::BN - 1) / lin::BN, (m + lin::BM - 1) / lin::BM);
-    lin::linear_sm100_kernel<<<grid, lin::kThreads, lin::SMEM_TOTAL, dev->stream>>>(tx, tw, a);
-    GRL_LAUNCHED("linear_sm100_kernel");
-    return GRL_OK;
+    // The pair kernel wants whole 256-row tiles and at least as many tiles as half the pairs; below that the split kernel has
+    // more SMs at work.
+    const int pairs = dev->prop.multiProcessorCount / 2;
+    const long long t128 = (long long)((m + 255) / 256) * ((n + 127) / 128), t256 = (long long)((m + 255) / 256) * ((n + 255) / 256);
+    if (m <= 256 || t128 < pairs / 2) return lin::launch_split(dev, x, w, a);
+    // the tile whose last wave wastes least (a 128-column tile costs a quarter more per column)
+    const long long c256 = (t256 + pairs - 1) / pairs * 4, c128 = ((t128 + pairs - 1) / pairs * 5 + 1) / 2;
+    return c256 <= c128 ? lin::launch_pair<256>(dev, x, w, a) : lin::launch_pair<128>(dev, x, w, a);
 }

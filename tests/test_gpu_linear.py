@@ -83,3 +83,18 @@ def test_linear_fp32_tile_edges(gpu, M, K, N):
     b = rng.standard_normal(N, dtype=np.float32)
     want = x.astype(np.float64) @ w.astype(np.float64).T + b
     assert np.abs(gpu.linear(x, w, b) - want).max() <= 1e-4
+
+
+@pytest.mark.parametrize("M,K,N", [
+    (1, 8, 1), (3, 4096, 300), (17, 520, 128), (250, 1032, 129),     # split over a cluster, and too short to split
+    (300, 72, 4000), (512, 2048, 520),                                # several tiles of rows
+    (2100, 72, 1025), (4097, 64, 640), (2500, 136, 516),              # pairs of SMs: odd rows, 256 and 128 columns a tile
+    (9000, 80, 260)])                                                 # more tiles than pairs
+def test_linear_bf16_tiles(gpu, M, K, N):
+    from oracle import attention_oracle as orc
+    rng = np.random.default_rng(M + K + N)
+    x, w = rng.standard_normal((M, K), dtype=np.float32), rng.standard_normal((N, K), dtype=np.float32)
+    b = rng.standard_normal(N, dtype=np.float32)
+    want = orc.round_bf16(x).astype(np.float64) @ orc.round_bf16(w).astype(np.float64).T
+    assert np.abs(gpu.linear(x, w, b, dtype="bf16") - (want + b)).max() <= 2e-5 * max(K, 64)
+    assert np.abs(gpu.linear(x, w, dtype="bf16") - want).max() <= 2e-5 * max(K, 64)
