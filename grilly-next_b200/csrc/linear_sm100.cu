@@ -114,6 +114,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     cluster_sync();                    // the peer's barriers exist
     tc_fence_after();
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
+    pdl_trigger();
     pdl_wait();
 
     // Tiles in groups of eight rows of tiles, walked column by column: the pairs at work at one time share both operands' tiles
@@ -274,6 +275,7 @@ linear_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_consta
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
+    pdl_trigger();
     pdl_wait();
 
     bool good = true;
@@ -342,19 +344,30 @@ linear_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_consta
         // every CTA of the cluster adds up its share of the rows, parts in ascending k
         cluster_sync();
         const int rows = min(NT, a.M - m0), lo = part * rows / a.splits, hi = (part + 1) * rows / a.splits;
-        const int c = tid & 127, n = n0 + c;
-        if (n < a.N && !*abort) {
-            const float b = a.bias ? __ldg(a.bias + n) : 0.f;
-            for (int m = lo + (tid >> 7); m < hi; m += 2) {
-                float v[8];
+        const bool vec = a.N % 4 == 0 && (uintptr_t)a.y % 16 == 0;
+        if (!*abort) {
+            for (int q = lo * 32 + tid; q < hi * 32; q += kThreads) {        // four columns of one row, all parts in flight
+                float4 v[8];
 #pragma unroll
                 for (int p = 0; p < 8; ++p)
-                    if (p < a.splits) v[p] = ld_cluster_f32(cluster_map(base + 1024u + (uint32_t)(m * 128 + c) * 4u, (uint32_t)p));
-                float sum = v[0];
+                    if (p < a.splits) v[p] = ld_cluster_f32x4(cluster_map(base + 1024u + (uint32_t)q * 16u, (uint32_t)p));
+                float4 t = v[0];
 #pragma unroll
                 for (int p = 1; p < 8; ++p)
-                    if (p < a.splits) sum += v[p];
-                a.y[(size_t)(m0 + m) * a.N + n] = sum + b;
+                    if (p < a.splits) { t.x += v[p].x; t.y += v[p].y; t.z += v[p].z; t.w += v[p].w; }
+                const int n = n0 + (q & 31) * 4;
+                if (a.bias) {
+                    const float4 b = sgemm::load4(a.bias, n, a.N, (uintptr_t)a.bias % 16 == 0);
+                    t.x += b.x; t.y += b.y; t.z += b.z; t.w += b.w;
+                }
+                float* dst = a.y + (size_t)(m0 + (q >> 5)) * a.N + n;
+                if (vec && n + 3 < a.N) *reinterpret_cast<float4*>(dst) = t;
+                else {
+                    if (n < a.N) dst[0] = t.x;
+                    if (n + 1 < a.N) dst[1] = t.y;
+                    if (n + 2 < a.N) dst[2] = t.z;
+                    if (n + 3 < a.N) dst[3] = t.w;
+                }
             }
         }
         __syncwarp();
@@ -439,31 +452,62 @@ static int launch_pair(grl_device* dev, const void* x, const void* w, Args a) {
     return GRL_OK;
 }
 
+// Stands in for linear_split_kernel in the question below: the occupancy of a kernel that allocates TMEM is given as one CTA
+// an SM whatever it allocates.
+__global__ void __launch_bounds__(kThreads, 2) placement_probe() {}
+
+// Clusters of `splits` CTAs with this much shared memory that the device holds at once (it packs them by GPC, so fewer than
+// the SM count suggests; a cluster too many is a second wave: 32 x 4096 x 12288 in clusters of 3 at two CTAs an SM took 31 us
+// for 22).  Asked once per size.
+static int clusters_resident(grl_device* dev, int smem, int splits) {
+    static std::mutex mu;
+    static std::map<std::tuple<int, int, int>, int> known;
+    std::lock_guard<std::mutex> lock(mu);
+    const auto key = std::make_tuple(dev->ordinal, smem, splits);
+    const auto it = known.find(key);
+    if (it != known.end()) return it->second;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)splits * 1024u); cfg.blockDim = dim3(kThreads); cfg.dynamicSmemBytes = (size_t)smem;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)splits; attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr; cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaFuncSetAttribute(placement_probe, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, placement_probe, &cfg) != cudaSuccess) {
+        (void)cudaGetLastError();
+        n = 0;
+    }
+    known[key] = n;
+    return n;
+}
+
 static int launch_split(grl_device* dev, const void* x, const void* w, Args a) {
-    // x rows per tile: all of them up to 256 (W is then read once), else tiles of 128
-    a.tile_rows = a.M <= 256 ? (a.M + 15) / 16 * 16 : 128;
-    const int n_k = (a.K + BK - 1) / BK, sms = dev->prop.multiProcessorCount;
+    // x rows per tile: all of them up to 128 (W is then read once), tiles of 128 beyond
+    a.tile_rows = a.M <= 128 ? (a.M + 15) / 16 * 16 : 128;
+    const int n_k = (a.K + BK - 1) / BK;
     const int tiles = (a.N + 127) / 128 * ((a.M + a.tile_rows - 1) / a.tile_rows);
-    // K cut so that the CTAs come to two an SM; at least four slices each, at most a portable cluster
-    a.splits = 2 * sms / tiles;
-    if (a.splits > n_k / 4) a.splits = n_k / 4;
-    if (a.splits > 8) a.splits = 8;
-    if (a.splits < 1) a.splits = 1;
-    const int stage = (128 + a.tile_rows) * BK * 2, half = kSmemMax / 2 - 3072, whole = kSmemMax - 3072;
-    a.stages = (half / stage >= 3 ? half : whole) / stage;
-    if (a.stages > 8) a.stages = 8;
+    const int stage = (128 + a.tile_rows) * BK * 2;
+    // three CTAs an SM while each still has three stages (two beyond 64 rows): one's start and end run under the others' copies
+    const int per_sm = a.tile_rows <= 64 ? 3 : 2;
+    a.stages = (kSmemMax / per_sm - 3072) / stage;
+    if (a.stages > n_k) a.stages = n_k;
     int smem = a.stages * stage;
-    if (a.splits > 1 && smem < a.tile_rows * 512) smem = a.tile_rows * 512;      // the partial tile
+    if (smem < a.tile_rows * 512) smem = a.tile_rows * 512;      // the partial tile of a split
     smem += 2048;
-    CUtensorMap tx, tw;
-    int rc = make_map(dev, &tx, x, a.M, a.K, a.tile_rows, BK, 2);
-    if (!rc) rc = make_map(dev, &tw, w, a.N, a.K, 128, BK, 2);
-    if (rc) return rc;
     static bool attr_set[64] = {};
     if (!attr_set[dev->ordinal & 63]) {
         GRL_CUDA(cudaFuncSetAttribute(linear_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
         attr_set[dev->ordinal & 63] = true;
     }
+    // K cut as far as one wave of clusters goes, at least four slices a CTA (measured, us at 1 / 2 / 4 / 8 parts: 32 x 4096 x 4096
+    // 28 / 18.6 / 13.1 / 11.2, 32 x 4096 x 12288 32 / 22.9 / 21.5 / 26.8, 128 x 4096 x 4096 33 / 23.5 / 17.5 / 16.5)
+    a.splits = 8;
+    while (a.splits > 1 && (n_k < 4 * a.splits || tiles > clusters_resident(dev, smem, a.splits))) a.splits /= 2;
+    CUtensorMap tx, tw;
+    int rc = make_map(dev, &tx, x, a.M, a.K, a.tile_rows, BK, 2);
+    if (!rc) rc = make_map(dev, &tw, w, a.N, a.K, 128, BK, 2);
+    if (rc) return rc;
     dim3 grid((a.N + 127) / 128 * a.splits, (a.M + a.tile_rows - 1) / a.tile_rows);
     GRL_CUDA(launch_pdl_cluster(linear_split_kernel, grid, kThreads, smem, dev->stream, a.splits, tx, tw, a));
     GRL_LAUNCHED("linear_split_kernel");
@@ -489,12 +533,14 @@ extern "C" int grl_linear(grl_device* dev, const void* x, const void* w, const f
     lin::Args a{};
     a.bias = bias; a.y = y; a.status = dev->d_status; a.M = m; a.N = n; a.K = k; a.wait_limit = dev->wait_limit_cycles;
     dev->status_dirty = true;
-    // The pair kernel wants whole 256-row tiles and at least as many tiles as half the pairs; below that the split kernel has
-    // more SMs at work.
+    // The pair kernel wants more than one of its two 128-row halves and tiles for half the pairs; below that the split kernel
+    // has more SMs at work.
     const int pairs = dev->prop.multiProcessorCount / 2;
-    const long long t128 = (long long)((m + 255) / 256) * ((n + 127) / 128), t256 = (long long)((m + 255) / 256) * ((n + 255) / 256);
-    if (m <= 256 || t128 < pairs / 2) return lin::launch_split(dev, x, w, a);
-    // the tile whose last wave wastes least (a 128-column tile costs a quarter more per column)
-    const long long c256 = (t256 + pairs - 1) / pairs * 4, c128 = ((t128 + pairs - 1) / pairs * 5 + 1) / 2;
-    return c256 <= c128 ? lin::launch_pair<256>(dev, x, w, a) : lin::launch_pair<128>(dev, x, w, a);
+    auto waves = [&](int bn) { return ((long long)((m + 255) / 256) * ((n + bn - 1) / bn) + pairs - 1) / pairs; };
+    if (m <= 128 || (long long)((m + 255) / 256) * ((n + 127) / 128) < pairs / 2) return lin::launch_split(dev, x, w, a);
+    // the tile whose waves cost least: a wave of 256 / 192 / 128 columns took 29.7 / 26.3 / 22.7 us at K = 4096 (narrower tiles are
+    // bound by shared memory)
+    const long long c256 = waves(256) * 297, c192 = waves(192) * 263, c128 = waves(128) * 227;
+    if (c256 <= c192 && c256 <= c128) return lin::launch_pair<256>(dev, x, w, a);
+    return c192 <= c128 ? lin::launch_pair<192>(dev, x, w, a) : lin::launch_pair<128>(dev, x, w, a);
 }
