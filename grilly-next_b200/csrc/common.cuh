@@ -30,6 +30,13 @@ constexpr long long kDefaultWaitLimitCycles = 2000000000LL;       // ~1 s at 2 G
 constexpr long long kDefaultPeerWaitLimitCycles = 1000000000LL;   // ~0.5 s: a peer GPU that never posts
 }  // namespace grl
 
+namespace grl {
+// inv_freq[i] = theta^(-2i/D) / scaling in double, for i < D/2 <= 128.
+struct RopeFreq {
+    double inv_freq[128];
+};
+}  // namespace grl
+
 struct grl_device {
     int ordinal = 0;
     cudaStream_t own_stream = nullptr;
@@ -39,6 +46,8 @@ struct grl_device {
     // RoPE cos/sin tables, float2 (cos, sin) per (position, pair), one per (head_dim, theta bits,
     // scaling bits); a table covers `first` positions and is replaced by a longer one on demand.
     std::map<std::tuple<int, uint32_t, uint32_t>, std::pair<int, float2*>> rope_tables;
+    std::tuple<int, uint32_t, uint32_t> freq_key{0, 0, 0};   // of `freq`, the inverse frequencies of the last append or rope call
+    grl::RopeFreq freq;
     std::vector<float2*> retired_tables;   // replaced tables: kernels in flight may still read them; freed at close
     // Tensor maps already encoded for this device (the descriptor-set cache of the reference's
     // PipelineCache, cpp/src/pipeline_cache.cpp:217-305): a launch looks its maps up by
@@ -162,6 +171,9 @@ inline cudaError_t launch_pdl_cluster(void (*kernel)(P...), dim3 grid, dim3 bloc
     cfg.attrs = attr; cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
+// Clusters of `size` CTAs (threads, dynamic shared memory as given) of `kernel` that the device holds at once; asked once per
+// combination.  Clusters are packed by GPC, so they are fewer than the SM count suggests.
+int max_active_clusters(grl_device* dev, const void* kernel, int threads, int smem, int size);
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 #endif
@@ -178,11 +190,9 @@ struct DeviceGuard {
     }
 };
 
-// inv_freq[i] = theta^(-2i/D) / scaling in double, for i < D/2 <= 128.
-struct RopeFreq {
-    double inv_freq[128];
-};
 RopeFreq make_rope_freq(int head_dim, float theta, float scaling);
+// The same, remembered from the device's last call: 64 powers took longer than the launch they were for.
+RopeFreq cached_rope_freq(grl_device* dev, int head_dim, float theta, float scaling);
 
 // Device table of (cos, sin) for positions [0, >= n_pos) x pairs [0, D/2); cached per device.  Creating or
 // growing a table allocates and launches, which a capturing stream does not allow: the call then fails and

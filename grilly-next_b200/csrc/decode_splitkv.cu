@@ -345,14 +345,32 @@ int grl_decode_pick_splits(grl_device* dev, const grl_decode_params* p, int* n_s
     const int unit = generic ? kv.page_tokens : 64;
     const int pages = (max_len + unit - 1) / unit;
     const int base_ctas = kv.batch * kv.num_kv_heads;
-    // At most one CTA per SM: that already keeps HBM saturated (three 32 KB stages in flight each), and one
-    // CTA more than there are SMs makes a pair share an SM and finish last.  Measured on B200, B1 x 8 KV
-    // heads x 131072 tokens: 87 us with 18 splits (144 CTAs), 94 us with 19 (152), 100 us with 64; B32 x 8
-    // heads x 4096 tokens is fastest unsplit.
     const int sms = dev->prop.multiProcessorCount;
     // The generic kernel (128-thread CTAs, no shared-memory ring) wants several CTAs per SM to hide its loads and,
     // over a quantised cache, its dequantising arithmetic: aim at eight per SM.
     int s = generic ? (8 * sms + base_ctas - 1) / base_ctas : sms / base_ctas;
+    if (!generic && !p->exchange) {
+        // Two CTAs an SM (twice the bytes in flight, or twice the warps that dequantise) while the splits of a head are one
+        // cluster: a power of two up to 16, which packs into the GPCs (16 sequences x 8 heads x 4096 tokens: 63 us unsplit, 51 us
+        // in 2 splits; 4 x 8 x 2048: 15.0 us in 8 splits, 19.1 in 9).  Few heads: one CTA an SM over the bf16 cache (131072 tokens
+        // x 8 heads: 98 us with 18 splits, 98 with 36), two over the quantised one (105 us with 18, 79 with 37), in whole
+        // clusters of 16 of at least 8 stages a split while splits are short enough to merge in clusters (see launch_instance).
+        // More heads than SMs: unsplit.
+        const int twice = 2 * sms / base_ctas;
+        if (base_ctas > sms) s = 1;
+        else if (twice < 32) {
+            s = 1;
+            while (2 * s <= twice) s *= 2;
+            const int wide = kv.cache_dtype == GRL_FP8_INT4 ? twice : sms / base_ctas;
+            if (s == 16 && pages > 32 * wide) s = wide;
+        } else {
+            s = kv.cache_dtype == GRL_FP8_INT4 ? twice : sms / base_ctas;
+            if (pages <= 32 * s) {
+                if (s > pages / 8) s = pages / 8;
+                s = s < 32 ? 16 : s / 16 * 16;
+            }
+        }
+    }
     if (s > pages / 2) s = pages / 2;          // every split keeps at least 2 pages
     if (s > 256) s = 256;
     if (s < 1) s = 1;

@@ -30,6 +30,19 @@ RopeFreq make_rope_freq(int head_dim, float theta, float scaling) {
     return f;
 }
 
+RopeFreq cached_rope_freq(grl_device* dev, int head_dim, float theta, float scaling) {
+    uint32_t tb, sb;
+    memcpy(&tb, &theta, 4);
+    memcpy(&sb, &scaling, 4);
+    const auto key = std::make_tuple(head_dim, tb, sb);
+    std::lock_guard<std::mutex> lock(dev->mu);
+    if (dev->freq_key != key) {
+        dev->freq = make_rope_freq(head_dim, theta, scaling);
+        dev->freq_key = key;
+    }
+    return dev->freq;
+}
+
 __global__ void rope_table_kernel(float2* table, int n_pos, int half, RopeFreq f) {
     int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= n_pos * half) return;
@@ -119,6 +132,28 @@ int get_tensor_map(grl_device* dev, const TmapKey& key, CUtensorMap* out) {
         dev->tmap_next = (dev->tmap_next + 1) % kMaxCached;
     }
     return GRL_OK;
+}
+
+int max_active_clusters(grl_device* dev, const void* kernel, int threads, int smem, int size) {
+    static std::mutex mu;
+    static std::map<std::tuple<int, const void*, int, int>, int> known;
+    std::lock_guard<std::mutex> lock(mu);
+    const auto key = std::make_tuple(dev->ordinal, kernel, smem, size);
+    const auto it = known.find(key);
+    if (it != known.end()) return it->second;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)size * 1024u); cfg.blockDim = dim3((unsigned)threads); cfg.dynamicSmemBytes = (size_t)smem;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)size; attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr; cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+        (void)cudaGetLastError();
+        n = 0;
+    }
+    known[key] = n;
+    return n;
 }
 
 template <typename S, typename D>

@@ -143,7 +143,37 @@ __global__ void __launch_bounds__(256, 3) kv_append_rows_kernel(const __grid_con
     __shared__ double freq[128];        // lanes index the frequencies apart, which the constant bank would serialise
     const int b = blockIdx.y, lanes = a.D / 8, groups = 256 / lanes;
     const int group = threadIdx.x / lanes, l = threadIdx.x % lanes;
+    if (a.rope_mode != GRL_ROPE_NONE && threadIdx.x < a.D / 2) freq[threadIdx.x] = a.freq.inv_freq[threadIdx.x];
+    pdl_wait();
+    pdl_trigger();      // the decode that follows sets itself up meanwhile
     const int len0 = a.seq_lens[b];
+    const int pos0 = a.pos_base + (a.pos_offsets ? a.pos_offsets[b] : 0) + len0;
+    // A token's runs: pairs of kv heads, then pairs of query heads.  Every thread group takes an equal, contiguous share of
+    // all (token, run): the CTAs that fit the SMs at once are busy to the end, and the angles change only with the token.
+    const int kv_runs = a.skip_kv ? 0 : (a.Hkv + kAppendHeads - 1) / kAppendHeads;
+    const int runs = kv_runs + (a.q_in ? (a.Hq + kAppendHeads - 1) / kAppendHeads : 0);
+    const int o0 = a.rope_mode == GRL_ROPE_HALF ? 4 * l : 8 * l, o1 = a.rope_mode == GRL_ROPE_HALF ? o0 + a.D / 2 : o0 + 4;
+    const long long total = (long long)a.n_new * runs, all = (long long)gridDim.x * groups, mine = (long long)blockIdx.x * groups + group;
+    const long long lo = group < groups ? mine * total / all : 0, hi = group < groups ? (mine + 1) * total / all : 0;
+    float4 k[kAppendHeads][2], v[kAppendHeads][2];
+    auto fetch = [&](int i, int r) {
+        const bool is_kv = r < kv_runs;
+        const int h0 = (is_kv ? r : r - kv_runs) * kAppendHeads, heads = is_kv ? a.Hkv : a.Hq;
+        const size_t src = (((size_t)b * a.n_new + i) * heads + h0) * a.D;
+        const float* in = (is_kv ? a.k_new : a.q_in) + src;
+#pragma unroll
+        for (int h = 0; h < kAppendHeads; ++h)
+            if (h0 + h < heads) {
+                k[h][0] = __ldcs(reinterpret_cast<const float4*>(in + h * a.D + o0));
+                k[h][1] = __ldcs(reinterpret_cast<const float4*>(in + h * a.D + o1));
+                if (is_kv) {
+                    v[h][0] = __ldcs(reinterpret_cast<const float4*>(a.v_new + src + h * a.D + o0));
+                    v[h][1] = __ldcs(reinterpret_cast<const float4*>(a.v_new + src + h * a.D + o1));
+                }
+            }
+    };
+    int i = (int)(lo / runs), r = (int)(lo % runs);
+    if (lo < hi) fetch(i, r);           // beside the length: in a decode step the trips to memory are the time
     if (len0 < 0 || len0 + a.n_new > a.max_pages * a.P) {      // no room: nothing is stored (see kv_append_kernel)
         if (threadIdx.x == 0 && blockIdx.x == 0 && a.status && atomicCAS(a.status, 0, GRL_ERR_INVALID) == 0) {
             a.status[1] = 4 << 28;
@@ -152,41 +182,19 @@ __global__ void __launch_bounds__(256, 3) kv_append_rows_kernel(const __grid_con
         }
         return;
     }
-    if (a.rope_mode != GRL_ROPE_NONE) {
-        if (threadIdx.x < a.D / 2) freq[threadIdx.x] = a.freq.inv_freq[threadIdx.x];
-        __syncthreads();
-    }
-    const int pos0 = a.pos_base + (a.pos_offsets ? a.pos_offsets[b] : 0) + len0;
+    __syncthreads();                    // freq
     T* kp = reinterpret_cast<T*>(a.k_pages);
     T* vp = reinterpret_cast<T*>(a.v_pages);
-    // A token's runs: pairs of kv heads, then pairs of query heads.  Every thread group takes an equal, contiguous share of
-    // all (token, run): the CTAs that fit the SMs at once are busy to the end, and the angles change only with the token.
-    const int kv_runs = a.skip_kv ? 0 : (a.Hkv + kAppendHeads - 1) / kAppendHeads;
-    const int runs = kv_runs + (a.q_in ? (a.Hq + kAppendHeads - 1) / kAppendHeads : 0);
-    const int o0 = a.rope_mode == GRL_ROPE_HALF ? 4 * l : 8 * l, o1 = a.rope_mode == GRL_ROPE_HALF ? o0 + a.D / 2 : o0 + 4;
-    if (group < groups) {
-        const long long total = (long long)a.n_new * runs, all = (long long)gridDim.x * groups, mine = (long long)blockIdx.x * groups + group;
-        const long long lo = mine * total / all, hi = (mine + 1) * total / all;
+    {
         float c[4] = {1.f, 1.f, 1.f, 1.f}, s[4] = {0.f, 0.f, 0.f, 0.f};
-        int i = (int)(lo / runs), r = (int)(lo % runs), angles_of = -1, page = 0;
+        int angles_of = -1, page = 0;
         for (long long item = lo; item < hi; ++item, ++r) {
             if (r == runs) { r = 0; ++i; }
+            if (item > lo) fetch(i, r);
             const int slot = len0 + i;
             const bool is_kv = r < kv_runs;
             const int h0 = (is_kv ? r : r - kv_runs) * kAppendHeads, heads = is_kv ? a.Hkv : a.Hq;
             const size_t src = (((size_t)b * a.n_new + i) * heads + h0) * a.D;
-            const float* in = (is_kv ? a.k_new : a.q_in) + src;
-            float4 k[kAppendHeads][2], v[kAppendHeads][2];
-#pragma unroll
-            for (int h = 0; h < kAppendHeads; ++h)
-                if (h0 + h < heads) {
-                    k[h][0] = __ldcs(reinterpret_cast<const float4*>(in + h * a.D + o0));
-                    k[h][1] = __ldcs(reinterpret_cast<const float4*>(in + h * a.D + o1));
-                    if (is_kv) {
-                        v[h][0] = __ldcs(reinterpret_cast<const float4*>(a.v_new + src + h * a.D + o0));
-                        v[h][1] = __ldcs(reinterpret_cast<const float4*>(a.v_new + src + h * a.D + o1));
-                    }
-                }
             if (angles_of != i) {       // under the first run's loads
                 page = a.block_table[(size_t)b * a.max_pages + slot / a.P];
                 if (a.rope_mode != GRL_ROPE_NONE) {
@@ -310,9 +318,11 @@ __device__ __forceinline__ float fp8_decode(uint8_t c) {                    // k
 
 // grid (ceil(n_new*Hkv*G / warps per CTA), B), G = D/32 groups per head.  With one CTA per sequence (a decode step) the
 // kernel also rotates the step's queries (q_in != NULL) and advances the length (update_lens): one launch per step.
-__global__ void __launch_bounds__(1024) kv_append_quant_kernel(AppendArgs a) {
+__global__ void __launch_bounds__(1024) kv_append_quant_kernel(const __grid_constant__ AppendArgs a) {
     const int b = blockIdx.y, lane = threadIdx.x & 31;
     const int G = a.D / 32;
+    pdl_wait();
+    pdl_trigger();      // the decode that follows sets itself up meanwhile
     const int len0 = a.seq_lens[b];
     if (len0 < 0 || len0 + a.n_new > a.max_pages * a.P) {
         if (threadIdx.x == 0 && blockIdx.x == 0 && a.status && atomicCAS(a.status, 0, GRL_ERR_INVALID) == 0) {
@@ -504,14 +514,14 @@ int grl_kv_append(grl_device* dev, const grl_append_params* p) {
     a.status = dev->d_status;
     a.scales = static_cast<uint16_t*>(kv.scales);
     dev->status_dirty = true;
-    if (p->rope_mode != GRL_ROPE_NONE) a.freq = make_rope_freq(kv.head_dim, p->rope_theta, p->rope_scaling);
+    if (p->rope_mode != GRL_ROPE_NONE) a.freq = cached_rope_freq(dev, kv.head_dim, p->rope_theta, p->rope_scaling);
     if (kv.cache_dtype == GRL_FP8_INT4) {
         // K and V: one warp per (token, kv head, group of 32); the queries, if any, through the plain kernel
         const long long warps = (long long)p->n_new * kv.num_kv_heads * (kv.head_dim / 32);
         if (warps <= 32) {      // a decode step: one wide CTA per sequence does keys, values, queries and the length
             a.update_lens = p->update_lens ? 1 : 0;
             a.heads_per_item = 1;
-            kv_append_quant_kernel<<<dim3(1, kv.batch), 1024, 0, dev->stream>>>(a);
+            GRL_CUDA(launch_pdl(kv_append_quant_kernel, dim3(1, kv.batch), 1024, 0, dev->stream, a));
             GRL_LAUNCHED("kv_append_quant_kernel");
             return GRL_OK;
         }
@@ -521,14 +531,14 @@ int grl_kv_append(grl_device* dev, const grl_append_params* p) {
         if (ctas > 1024) ctas = 1024;
         a.q_in = nullptr;       // bulk append: the queries go through the plain kernel below
         a.update_lens = 0;
-        kv_append_quant_kernel<<<dim3(ctas, kv.batch), 256, 0, dev->stream>>>(a);
+        GRL_CUDA(launch_pdl(kv_append_quant_kernel, dim3(ctas, kv.batch), 256, 0, dev->stream, a));
         GRL_LAUNCHED("kv_append_quant_kernel");
         a.q_in = p->q_in;
         if (p->q_in) {
             a.skip_kv = 1;
             a.update_lens = 0;
             if (append_rows_fit(a)) {
-                kv_append_rows_kernel<float><<<append_rows_grid(dev, a), 256, 0, dev->stream>>>(a);
+                GRL_CUDA(launch_pdl(kv_append_rows_kernel<float>, append_rows_grid(dev, a), 256, 0, dev->stream, a));
             } else {
                 const long long qitems = (long long)p->n_new * (kv.num_kv_heads + p->num_q_heads) * (kv.head_dim / 2);
                 const int qchunks = (int)((qitems + 4095) / 4096);
@@ -550,8 +560,8 @@ int grl_kv_append(grl_device* dev, const grl_append_params* p) {
         if (p->update_lens && grid.x <= 4) grid.x = 1;
         fused_update = p->update_lens && grid.x == 1;
         a.update_lens = fused_update ? 1 : 0;
-        if (kv.cache_dtype == GRL_BF16) kv_append_rows_kernel<__nv_bfloat16><<<grid, 256, 0, dev->stream>>>(a);
-        else kv_append_rows_kernel<float><<<grid, 256, 0, dev->stream>>>(a);
+        GRL_CUDA(launch_pdl(kv.cache_dtype == GRL_BF16 ? kv_append_rows_kernel<__nv_bfloat16> : kv_append_rows_kernel<float>, grid, 256, 0,
+                            dev->stream, a));
     } else {
         const long long items = (long long)p->n_new * (kv.num_kv_heads + (p->q_in ? p->num_q_heads : 0)) * (kv.head_dim / 2);
         // one CTA per sequence while a CTA has at most 16 items per thread (a decode step), more for bulk appends

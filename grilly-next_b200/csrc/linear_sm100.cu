@@ -114,7 +114,6 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     cluster_sync();                    // the peer's barriers exist
     tc_fence_after();
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
-    pdl_trigger();
     pdl_wait();
 
     // Tiles in groups of eight rows of tiles, walked column by column: the pairs at work at one time share both operands' tiles
@@ -182,6 +181,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
             int tm, tn;
             place(t, tm, tn);
             if (!__all_sync(0xffffffffu, wait(acc_full(acc), (n >> 1) & 1, abort, a, 2 * NST + acc))) break;
+            if (t + pairs >= tiles) pdl_trigger();        // the next kernel may launch under the last epilogues
             tc_fence_after();
             const int row0 = tm * 256 + (int)rank * 128 + w * 32;
             const uint32_t t_addr = tmem + (uint32_t)acc * 256u + ((uint32_t)(w * 32) << 16);
@@ -275,7 +275,6 @@ linear_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_consta
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
-    pdl_trigger();
     pdl_wait();
 
     bool good = true;
@@ -316,6 +315,7 @@ linear_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_consta
         }
     } else if (warp >= 4) {
         good = __all_sync(0xffffffffu, wait(acc_full, 0, abort, a, 2 * NST));
+        pdl_trigger();        // the next kernel may launch under the epilogues; earlier it would take slots and sit unevenly
         tc_fence_after();
         const int w = warp & 3, n = n0 + w * 32 + lane;
         const uint32_t t_addr = tmem + ((uint32_t)(w * 32) << 16);
@@ -452,35 +452,9 @@ static int launch_pair(grl_device* dev, const void* x, const void* w, Args a) {
     return GRL_OK;
 }
 
-// Stands in for linear_split_kernel in the question below: the occupancy of a kernel that allocates TMEM is given as one CTA
-// an SM whatever it allocates.
+// Stands in for linear_split_kernel when max_active_clusters is asked: the occupancy of a kernel that allocates TMEM is given
+// as one CTA an SM whatever it allocates.
 __global__ void __launch_bounds__(kThreads, 2) placement_probe() {}
-
-// Clusters of `splits` CTAs with this much shared memory that the device holds at once (it packs them by GPC, so fewer than
-// the SM count suggests; a cluster too many is a second wave: 32 x 4096 x 12288 in clusters of 3 at two CTAs an SM took 31 us
-// for 22).  Asked once per size.
-static int clusters_resident(grl_device* dev, int smem, int splits) {
-    static std::mutex mu;
-    static std::map<std::tuple<int, int, int>, int> known;
-    std::lock_guard<std::mutex> lock(mu);
-    const auto key = std::make_tuple(dev->ordinal, smem, splits);
-    const auto it = known.find(key);
-    if (it != known.end()) return it->second;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)splits * 1024u); cfg.blockDim = dim3(kThreads); cfg.dynamicSmemBytes = (size_t)smem;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = (unsigned)splits; attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr; cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaFuncSetAttribute(placement_probe, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&n, placement_probe, &cfg) != cudaSuccess) {
-        (void)cudaGetLastError();
-        n = 0;
-    }
-    known[key] = n;
-    return n;
-}
 
 static int launch_split(grl_device* dev, const void* x, const void* w, Args a) {
     // x rows per tile: all of them up to 128 (W is then read once), tiles of 128 beyond
@@ -498,12 +472,14 @@ static int launch_split(grl_device* dev, const void* x, const void* w, Args a) {
     static bool attr_set[64] = {};
     if (!attr_set[dev->ordinal & 63]) {
         GRL_CUDA(cudaFuncSetAttribute(linear_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
+        GRL_CUDA(cudaFuncSetAttribute(placement_probe, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax));
         attr_set[dev->ordinal & 63] = true;
     }
-    // K cut as far as one wave of clusters goes, at least four slices a CTA (measured, us at 1 / 2 / 4 / 8 parts: 32 x 4096 x 4096
+    // K cut as far as one wave of clusters goes (a cluster too many is a second wave: 32 x 4096 x 12288 in clusters of 3 at two
+    // CTAs an SM took 31 us for 22), at least four slices a CTA (measured, us at 1 / 2 / 4 / 8 parts: 32 x 4096 x 4096
     // 28 / 18.6 / 13.1 / 11.2, 32 x 4096 x 12288 32 / 22.9 / 21.5 / 26.8, 128 x 4096 x 4096 33 / 23.5 / 17.5 / 16.5)
     a.splits = 8;
-    while (a.splits > 1 && (n_k < 4 * a.splits || tiles > clusters_resident(dev, smem, a.splits))) a.splits /= 2;
+    while (a.splits > 1 && (n_k < 4 * a.splits || tiles > max_active_clusters(dev, (const void*)placement_probe, kThreads, smem, a.splits))) a.splits /= 2;
     CUtensorMap tx, tw;
     int rc = make_map(dev, &tx, x, a.M, a.K, a.tile_rows, BK, 2);
     if (!rc) rc = make_map(dev, &tw, w, a.N, a.K, 128, BK, 2);

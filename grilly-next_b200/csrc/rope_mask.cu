@@ -63,7 +63,7 @@ int grl_rope(grl_device* dev, const float* x, float* y, int batch, int seq_len, 
                            ? (n_pairs + 255) / 256
                            : (size_t)dev->prop.multiProcessorCount * 32);
     rope_kernel<<<blocks, 256, 0, dev->stream>>>(x, y, n_pairs, seq_len, heads, head_dim, mode, cos_table,
-                                                 sin_table, make_rope_freq(head_dim, base, scaling));
+                                                 sin_table, cached_rope_freq(dev, head_dim, base, scaling));
     GRL_LAUNCHED("rope_kernel");
     return GRL_OK;
 }

@@ -362,3 +362,26 @@ def test_append_vector_rows(dev, D, Hkv, Hq, n, P, mode, dtype):
         assert np.abs(gk - rotated(k)[b]).max() <= (2e-2 if dtype == "bf16" else 1e-5)
     if q is not None:
         assert np.abs(qo - rotated(q)).max() <= 1e-5
+
+
+@pytest.mark.parametrize("dtype,D", [("bf16", 128), ("bf16", 64), ("quant", 128)])
+@pytest.mark.parametrize("Hq,Hkv,lens", [(8, 2, (3001, 1)), (6, 1, (70,)), (8, 8, (640, 2500, 63))])
+def test_every_split_form_agrees(dev, dtype, D, Hq, Hkv, lens):
+    """Unsplit, one cluster per head, several clusters per head, splits without a common cluster, more splits than stages."""
+    from gpu_helpers import PagedCache
+    from grilly_next import cabi
+    rng = np.random.default_rng(sum(lens) + D)
+    B, T = len(lens), max(lens)
+    k, v = (rng.standard_normal((B, T, Hkv, D), dtype=np.float32) for _ in range(2))
+    q = rng.standard_normal((B, 1, Hq, D), dtype=np.float32)
+    pc = PagedCache(dev, B, Hkv, D, T, dtype=cabi.BF16 if dtype == "bf16" else cabi.FP8_INT4, shuffle_pages=True, seed=5)
+    pc.append(k, v)
+    dev.L.grl_memcpy_h2d(dev.h, pc.seq_lens, np.asarray(lens, np.int32).ctypes.data, 4 * B)
+    dev.sync()
+    want = pc.decode(q, n_splits=1)
+    scale = np.abs(want).max()
+    for ns in (2, 5, 8, 16, 18, 23, 32, 48):
+        assert np.abs(pc.decode(q, n_splits=ns) - want).max() <= 2e-3 * scale, ns
+        part = pc.decode(q, n_splits=ns, partial=True)
+        o, l = part[:B * Hq * D].reshape(B, 1, Hq, D), part[B * Hq * (D + 1):].reshape(B, 1, Hq, 1)
+        assert np.abs(o / l - want).max() <= 2e-3 * scale, ns
