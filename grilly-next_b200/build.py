@@ -24,9 +24,9 @@ HOST_CXX = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++"
 CUDA_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-ccbin", HOST_CXX, "-I", os.path.join(ROOT, "include"), "-I", CSRC]
 
-CU_SOURCES = ["device.cu", "flash.cu", "prefill_fp32.cu", "prefill_sm100.cu", "decode_splitkv.cu", "decode_mma.cu", "p2p_merge.cu", "kv_evict.cu",
+CU_SOURCES = ["device.cu", "host_copy.cu", "flash.cu", "prefill_fp32.cu", "prefill_sm100.cu", "decode_splitkv.cu", "decode_mma.cu", "p2p_merge.cu", "kv_evict.cu",
               "kv_cache.cu", "rope_mask.cu", "nccl_group.cu", "linear_sm100.cu", "attention_unfused.cu"]
-HEADERS = ["common.cuh", "sgemm.cuh", "tmem_ops.cuh", "sm100_ptx.cuh", os.path.join(ROOT, "include", "grilly_cuda.h")]
+HEADERS = ["common.cuh", "host_copy.cuh", "sgemm.cuh", "tmem_ops.cuh", "sm100_ptx.cuh", os.path.join(ROOT, "include", "grilly_cuda.h")]
 
 
 def _newer(target, deps):
@@ -62,7 +62,7 @@ def build_cuda(force=False, verbose=False):
             raise RuntimeError(f"nvcc failed on {src}")
     lib = os.path.join(LIBDIR, "libgrilly_cuda.so")
     if force or procs or _newer(lib, objs):
-        _run([NVCC, "-shared", "-ccbin", HOST_CXX, "-o", lib] + objs + ["-lcudart", "-ldl"], verbose)
+        _run([NVCC, "-shared", "-ccbin", HOST_CXX, "-o", lib] + objs + ["-lcudart", "-ldl", "-lpthread"], verbose)
     return lib
 
 

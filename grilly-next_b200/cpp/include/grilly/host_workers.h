@@ -26,7 +26,7 @@ private:
     HostWorkers();
     void loop(int id);
     std::vector<std::thread> workers_;
-    std::mutex mu_;
+    std::mutex callMu_, mu_;
     std::condition_variable start_, done_;
     const std::function<void(int, int)>* job_ = nullptr;
     uint64_t generation_ = 0;

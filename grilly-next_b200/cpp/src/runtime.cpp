@@ -112,6 +112,7 @@ void HostWorkers::loop(int id) {
 }
 
 void HostWorkers::parallel(const std::function<void(int, int)>& fn) {
+    std::lock_guard<std::mutex> call(callMu_);      // one job at a time (DeviceGroup calls from a thread per GPU)
     {
         std::lock_guard<std::mutex> lock(mu_);
         job_ = &fn;

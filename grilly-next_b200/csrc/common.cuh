@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "grilly_cuda.h"
+#include "host_copy.cuh"
 
 namespace grl {
 // Key of a cached tiled tensor map (bf16 elements): everything cuTensorMapEncodeTiled is given.
@@ -61,6 +62,8 @@ struct grl_device {
     // Status word written by kernels with bounded waits; read back by grl_sync when dirty.
     int32_t* d_status = nullptr;   // device int32[4], followed by the arrival counters below
     bool status_dirty = false;
+    bool status_queued = false;    // a copy to h_status is on the stream and has not been reported yet
+    grl::HostStage stage;          // page-locked staging of pageable copies
     int32_t* h_status = nullptr;   // pinned host int32[4]: the status word is copied here ahead of a wait
     // Arrival counters of the split-KV decode (one per (sequence, kv head), zero between launches: the
     // CTA that brings a counter to its final value resets it) and, last, the count of finished heads.
@@ -93,6 +96,9 @@ struct PeerExchange {
     int rank, world, flag_slots;
     long long wait_cycles;               // a missing peer ends in an error code after this many cycles, not in a hang
 };
+// A kernel with bounded waits leaves its failure in the device status word, which is copied to pinned host memory by the same
+// stream AHEAD of the wait, so that one wait serves both.
+bool queue_status_copy(grl_device* dev);
 int fill_peer_exchange(grl_device* dev, const grl_exchange_params* p, PeerExchange* x);
 
 // Cached cuTensorMapEncodeTiled for bf16 tensors (zero fill out of bounds, 256-byte L2 promotion).

@@ -156,6 +156,15 @@ int max_active_clusters(grl_device* dev, const void* kernel, int threads, int sm
     return n;
 }
 
+bool queue_status_copy(grl_device* dev) {
+    if (dev->status_dirty) {
+        dev->status_dirty = false;
+        dev->status_queued = cudaMemcpyAsync(dev->h_status, dev->d_status, 4 * sizeof(int32_t), cudaMemcpyDeviceToHost, dev->stream) ==
+                             cudaSuccess;
+    }
+    return dev->status_queued;
+}
+
 template <typename S, typename D>
 __global__ void cast_kernel(const S* __restrict__ src, D* __restrict__ dst, size_t n) {
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -334,9 +343,27 @@ int grl_host_free(void* ptr) {
     return GRL_OK;
 }
 
+// Whether a copy from or to this host memory goes through the staging ring (host_copy.cuh): from the size at which the driver's
+// own path is slower, and outside a stream capture, whose copies run at replay.
+static bool pageable(grl_device* dev, const void* host, size_t bytes, size_t least) {
+    if (bytes < least) return false;
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, host) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    if (at.type != cudaMemoryTypeUnregistered) return false;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(dev->stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+}
+
 int grl_memcpy_h2d(grl_device* dev, void* dst, const void* src_host, size_t bytes) {
     GRL_REQUIRE(dev && (bytes == 0 || (dst && src_host)), "NULL argument");
     DeviceGuard g(dev->ordinal);
+    if (pageable(dev, src_host, bytes, 512u << 10)) {
+        GRL_CUDA(staged_upload(dev, dst, src_host, bytes));
+        return GRL_OK;
+    }
     GRL_CUDA(cudaMemcpyAsync(dst, src_host, bytes, cudaMemcpyHostToDevice, dev->stream));
     return GRL_OK;
 }
@@ -344,6 +371,10 @@ int grl_memcpy_h2d(grl_device* dev, void* dst, const void* src_host, size_t byte
 int grl_memcpy_d2h(grl_device* dev, void* dst_host, const void* src, size_t bytes) {
     GRL_REQUIRE(dev && (bytes == 0 || (dst_host && src)), "NULL argument");
     DeviceGuard g(dev->ordinal);
+    if (pageable(dev, dst_host, bytes, 16u << 10)) {
+        GRL_CUDA(staged_download(dev, dst_host, src, bytes));
+        return GRL_OK;
+    }
     GRL_CUDA(cudaMemcpyAsync(dst_host, src, bytes, cudaMemcpyDeviceToHost, dev->stream));
     return GRL_OK;
 }
@@ -362,17 +393,9 @@ int grl_memset(grl_device* dev, void* dst, int value, size_t bytes) {
     return GRL_OK;
 }
 
-// A kernel with bounded waits leaves its failure in the device status word.  The word is copied to
-// pinned host memory by the same stream AHEAD of the wait, so that one wait serves both.
-static bool queue_status_copy(grl_device* dev) {
-    if (!dev->status_dirty) return false;
-    dev->status_dirty = false;
-    return cudaMemcpyAsync(dev->h_status, dev->d_status, 4 * sizeof(int32_t), cudaMemcpyDeviceToHost, dev->stream) ==
-           cudaSuccess;
-}
-
 static int report_kernel_status(grl_device* dev, bool copied) {
     if (!copied) return GRL_OK;
+    dev->status_queued = false;
     const int32_t* st = dev->h_status;
     if (st[0] == 0) return GRL_OK;
     // a kernel that gave up may have left arrival counters half-way: clear them with the status

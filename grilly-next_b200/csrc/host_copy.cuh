@@ -1,0 +1,64 @@
+// Copies between pageable host memory and the device through page-locked staging.
+//
+// cudaMemcpyAsync on pageable memory copies on the calling thread alone: measured (16-core host, PCIe 5) 1 MiB up 82 us and down
+// 92 us, 9 MiB 0.5 ms either way, where the link needs 20 and 172 us and a host memcpy of 9 MiB takes 546 us on one thread and 60
+// on eight.  So pageable copies go through a ring of page-locked pieces: large pieces are copied by a few threads, and the copy
+// of one piece runs beside the transfer of the one before.  Uploads below 512 KiB stay with the driver, which is as fast there.
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include <atomic>
+#include <condition_variable>
+#include <mutex>
+#include <thread>
+#include <vector>
+
+struct grl_device;
+
+namespace grl {
+
+// Threads that copy a piece together.  One caller at a time; another one meanwhile copies on its own thread.
+class CopyPool {
+public:
+    static CopyPool& instance();
+    void copy(void* dst, const void* src, size_t bytes);
+
+private:
+    CopyPool();
+    ~CopyPool();
+    void loop(int id);
+    void share(int id) const;
+    std::vector<std::thread> threads_;
+    std::mutex caller_, mu_;
+    std::condition_variable wake_;
+    std::atomic<uint32_t> generation_{0};
+    std::atomic<int> pending_{0}, sleeping_{0};
+    std::atomic<bool> stop_{false};
+    int parts_ = 1;
+    char* dst_ = nullptr;
+    const char* src_ = nullptr;
+    size_t bytes_ = 0;
+};
+
+// The page-locked rings of one device handle: allocated on first use, given back when the handle is closed.
+struct HostStage {
+    static constexpr size_t kPiece = 2u << 20, kShort = 512u << 10;    // the end of a copy that no transfer hides is short
+    static constexpr int kSlots = 4;
+    struct Ring {
+        char* mem = nullptr;
+        cudaEvent_t ev[kSlots] = {};
+        bool busy[kSlots] = {};
+        int next = 0;
+    };
+    std::mutex mu;
+    Ring up, down;
+    ~HostStage();
+};
+
+// Stream-ordered copies with the semantics of cudaMemcpyAsync on pageable memory: `src` may be reused when the upload returns,
+// `dst` is complete when the download returns.
+cudaError_t staged_upload(grl_device* dev, void* dst, const void* src, size_t bytes);
+cudaError_t staged_download(grl_device* dev, void* dst, const void* src, size_t bytes);
+
+}  // namespace grl
