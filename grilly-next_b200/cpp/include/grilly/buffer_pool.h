@@ -48,4 +48,27 @@ private:
     PoolStats stats_;
 };
 
+/// Host arrays of one small call in ONE transfer each way.  A transfer costs some 10 us of driver and link latency whatever its
+/// size, which is most of a small call's time: the inputs are packed into one page-locked block, and the result leaves through
+/// another.  Reused by the next call on the device, so a call waits for its work (CommandBatch::submit) before it ends.
+class SmallCall {
+public:
+    static constexpr size_t kMaxBytes = 1u << 20;      // inputs together, and the result
+    static constexpr int kInSlot = 6, kOutSlot = 7;    // GrillyDevice::pinnedStaging
+    static bool fits(size_t inputBytes, size_t outputBytes) { return inputBytes <= kMaxBytes && outputBytes <= kMaxBytes; }
+    explicit SmallCall(BufferPool& pool);
+    ~SmallCall();
+    SmallCall(const SmallCall&) = delete;
+    /// Packs `bytes` from `host`; returns where they will be on the device.  Every input adds up to 256 bytes of alignment.
+    void* input(const void* host, size_t bytes);
+    void send();                                       // after the last input
+    void fetch(const void* device, size_t bytes);      // queue the result's transfer
+    void deliver(void* host, size_t bytes) const;      // after CommandBatch::submit
+
+private:
+    BufferPool& pool_;
+    GrillyBuffer in_;
+    size_t used_ = 0;
+};
+
 }  // namespace grilly

@@ -38,8 +38,9 @@ public:
     /// to its compute queue.  Order between queues is set with grl_event_record / grl_event_wait.
     grl_device* uploadQueue();
     grl_device* downloadQueue();
-    /// Pinned host scratch kept for the life of the device (slot 0..5): staging for converted uploads.
-    static constexpr int kStagingSlots = 6;
+    /// Pinned host scratch kept for the life of the device: staging for converted uploads (slots 0..5), for the inputs and the
+    /// result of small calls (6, 7: SmallCall).
+    static constexpr int kStagingSlots = 8;
     void* pinnedStaging(int slot, size_t bytes);
     /// Waits (without limit, ignoring errors) for everything queued on the main, upload and download queues.
     /// Error paths call it before they hand buffers back to the pool: a buffer that a kernel or a copy in

@@ -6,6 +6,7 @@
 #include <mutex>
 #include <cstdlib>
 #include <exception>
+#include <optional>
 #include <string>
 #include <vector>
 
@@ -85,6 +86,10 @@ void flashAttention2Ex(CommandBatch& batch, BufferPool& pool, PipelineCache& cac
     Scoped scope(pool);
     const size_t slice = size_t(S) * D;                       // elements of one (b, h) slice
     const bool pipelined = n * 4 >= kPipelineMinBytes && (!mask || opt.maskRank == 2) && size_t(B) * H > 1;
+    size_t mElems = 0;          // of the mask array
+    if (mask)
+        mElems = opt.maskRank == 2 ? size_t(B) * S : (opt.maskRank == 3 || opt.maskBroadcastHeads) ? size_t(B) * S * S : size_t(B) * H * S * S;
+    const bool small = SmallCall::fits((3 * n + mElems + B) * 4, n * 4);
     GrillyBuffer q32, k32, v32, out = pool.acquire(n * 4);
     // share of a chunk that the host threads round to bf16 themselves (the rest is cast on the device)
     size_t hostPct = kPipelineHostCastPct;
@@ -106,7 +111,7 @@ void flashAttention2Ex(CommandBatch& batch, BufferPool& pool, PipelineCache& cac
         else if (rh > 0.0 && rl > 0.0) hostPct = size_t(std::min(100.0, std::max(0.0, 100.0 * 2.0 * rh / (2.0 * rl + rh))));
     }
     if (const char* e = std::getenv("GRILLY_PIPELINE_HOST_CAST_PCT")) hostPct = size_t(std::min(100, std::max(0, std::atoi(e))));
-    if (!(pipelined && bf16 && hostPct == 100)) {
+    if (!small && !(pipelined && bf16 && hostPct == 100)) {
         q32 = pool.acquire(n * 4); k32 = pool.acquire(n * 4); v32 = pool.acquire(n * 4);
     }
     scope.add(q32); scope.add(k32); scope.add(v32); scope.add(out);
@@ -246,7 +251,7 @@ void flashAttention2Ex(CommandBatch& batch, BufferPool& pool, PipelineCache& cac
                     p.in_dtype = GRL_BF16; p.kernel = GRL_KERNEL_TCGEN05;
                 } else {
                     p.q = at(q32, pe * 4); p.k = at(k32, pe * 4); p.v = at(v32, pe * 4);
-                    p.in_dtype = GRL_F32; p.kernel = GRL_KERNEL_AUTO;
+                    p.in_dtype = GRL_F32; p.kernel = GRL_KERNEL_SIMT_F32_WIDE;
                 }
                 p.out_dtype = GRL_F32;
                 p.batch = 1; p.heads = int(p1 - p0); p.seq_len = int(S); p.head_dim = int(D);
@@ -296,12 +301,18 @@ void flashAttention2Ex(CommandBatch& batch, BufferPool& pool, PipelineCache& cac
     }
 
     Recording rec(batch);
-    pool.upload(q32, Q, n * 4);
-    pool.upload(k32, K, n * 4);
-    pool.upload(v32, V, n * 4);
-
+    std::optional<SmallCall> block;
+    if (small) block.emplace(pool);
+    // an input array on the device: packed with the others, or in a buffer of its own
+    auto place = [&](GrillyBuffer& buf, const void* host, size_t bytes) -> const void* {
+        if (small) return block->input(host, bytes);
+        if (!buf.valid()) buf = pool.acquire(bytes);
+        pool.upload(buf, host, bytes);
+        return buf.dptr;
+    };
     grl_flash_params p{};
-    p.q = q32.dptr; p.k = k32.dptr; p.v = v32.dptr; p.o = out.dptr;
+    p.q = place(q32, Q, n * 4); p.k = place(k32, K, n * 4); p.v = place(v32, V, n * 4);
+    p.o = out.dptr;
     p.in_dtype = GRL_F32; p.out_dtype = GRL_F32;
     p.batch = int(B); p.heads = int(H); p.seq_len = int(S); p.head_dim = int(D);
     p.scale = scale;
@@ -309,31 +320,25 @@ void flashAttention2Ex(CommandBatch& batch, BufferPool& pool, PipelineCache& cac
     p.rope_mode = int(opt.ropeMode); p.rope_theta = opt.ropeTheta; p.rope_scaling = opt.ropeScaling;
     p.kernel = GRL_KERNEL_AUTO;
     if (mask) {
-        size_t mElems;
-        if (opt.maskRank == 2) { mElems = size_t(B) * S; p.mask_kind = GRL_MASK_KEY; }
-        else if (opt.maskRank == 3 || opt.maskBroadcastHeads) { mElems = size_t(B) * S * S; p.mask_kind = GRL_MASK_BSS; }
-        else { mElems = size_t(B) * H * S * S; p.mask_kind = GRL_MASK_BHSS; }
-        maskBuf = pool.acquire(mElems * 4);
-        pool.upload(maskBuf, mask, mElems * 4);
-        p.mask = static_cast<const float*>(maskBuf.dptr);
+        p.mask_kind = opt.maskRank == 2 ? GRL_MASK_KEY : (opt.maskRank == 3 || opt.maskBroadcastHeads) ? GRL_MASK_BSS : GRL_MASK_BHSS;
+        p.mask = static_cast<const float*>(place(maskBuf, mask, mElems * 4));
     }
-    if (opt.seqLens) {
-        lensBuf = pool.acquire(size_t(B) * 4);
-        pool.upload(lensBuf, opt.seqLens, size_t(B) * 4);
-        p.seq_lens = static_cast<const int32_t*>(lensBuf.dptr);
-    }
+    if (opt.seqLens) p.seq_lens = static_cast<const int32_t*>(place(lensBuf, opt.seqLens, size_t(B) * 4));
+    if (small) block->send();
     if (bf16) {
         q16 = pool.acquire(n * 2); k16 = pool.acquire(n * 2); v16 = pool.acquire(n * 2);
-        check(grl_cast(dev, q32.dptr, GRL_F32, q16.dptr, GRL_BF16, n), "flashAttention2: cast");
-        check(grl_cast(dev, k32.dptr, GRL_F32, k16.dptr, GRL_BF16, n), "flashAttention2: cast");
-        check(grl_cast(dev, v32.dptr, GRL_F32, v16.dptr, GRL_BF16, n), "flashAttention2: cast");
+        check(grl_cast(dev, p.q, GRL_F32, q16.dptr, GRL_BF16, n), "flashAttention2: cast");
+        check(grl_cast(dev, p.k, GRL_F32, k16.dptr, GRL_BF16, n), "flashAttention2: cast");
+        check(grl_cast(dev, p.v, GRL_F32, v16.dptr, GRL_BF16, n), "flashAttention2: cast");
         p.q = q16.dptr; p.k = k16.dptr; p.v = v16.dptr;
         p.in_dtype = GRL_BF16;
         p.kernel = GRL_KERNEL_TCGEN05;
     }
     check(grl_flash_fwd(dev, &p), "flashAttention2");
-    check(grl_memcpy_d2h(dev, output, out.dptr, n * 4), "flashAttention2: download");
+    if (small) block->fetch(out.dptr, n * 4);
+    else check(grl_memcpy_d2h(dev, output, out.dptr, n * 4), "flashAttention2: download");
     batch.submit();
+    if (small) block->deliver(output, n * 4);
 }
 
 void flashAttention2Device(CommandBatch& /*batch*/, PipelineCache& cache, const GrillyBuffer& q, const GrillyBuffer& k,

@@ -1,11 +1,18 @@
 // Host side of the linear projection: upload -> (cast) -> one kernel -> download.
+#include <algorithm>
+#include <optional>
 #include <stdexcept>
 #include <string>
+#include <vector>
 
 #include "grilly/ops/linear.h"
 
 namespace grilly {
 namespace ops {
+
+namespace {
+constexpr size_t kPieceBytes = 2u << 20, kPieceRows = 64;     // results from 2 MiB up, in pieces of whole 64-row tiles
+}
 
 void linearEx(CommandBatch& batch, BufferPool& pool, PipelineCache& cache, const float* x, const float* weights,
               const float* bias, float* output, const LinearParams& p, Precision precision) {
@@ -16,33 +23,71 @@ void linearEx(CommandBatch& batch, BufferPool& pool, PipelineCache& cache, const
     grl_device* dev = pool.device().handle();
     cache.getOrCreate(std::string(bf16 ? "fnn-linear-tcgen05/" : "fnn-linear/") + std::to_string(p.inputDim));
     const size_t nx = size_t(p.batchSeq) * p.inputDim, nw = size_t(p.outputDim) * p.inputDim, ny = size_t(p.batchSeq) * p.outputDim;
-    GrillyBuffer xb = pool.acquire(nx * 4), wb = pool.acquire(nw * 4), yb = pool.acquire(ny * 4), bb, x16, w16;
+    const bool small = SmallCall::fits((nx + nw + p.outputDim) * 4, ny * 4);
+    GrillyBuffer xb, wb, yb = pool.acquire(ny * 4), bb, x16, w16;
+    std::vector<grl_event*> events;
     auto releaseAll = [&]() {
         pool.release(xb); pool.release(wb); pool.release(yb); pool.release(bb); pool.release(x16); pool.release(w16);
+        for (auto* e : events) grl_event_destroy(e);
     };
     try {
         batch.begin();
-        pool.upload(xb, x, nx * 4);
-        pool.upload(wb, weights, nw * 4);
-        const float* biasDev = nullptr;
-        if (p.hasBias && bias) {
-            bb = pool.acquire(size_t(p.outputDim) * 4);
-            pool.upload(bb, bias, size_t(p.outputDim) * 4);
-            biasDev = static_cast<const float*>(bb.dptr);
-        }
+        std::optional<SmallCall> block;
+        if (small) block.emplace(pool);
+        // an input array on the device: packed with the others, or in a buffer of its own
+        auto place = [&](GrillyBuffer& buf, const float* host, size_t n) -> const void* {
+            if (small) return block->input(host, n * 4);
+            buf = pool.acquire(n * 4);
+            pool.upload(buf, host, n * 4);
+            return buf.dptr;
+        };
+        const void* xd = place(xb, x, nx);
+        const void* wd = place(wb, weights, nw);
+        const float* biasDev = p.hasBias && bias ? static_cast<const float*>(place(bb, bias, p.outputDim)) : nullptr;
+        if (small) block->send();
         if (bf16) {
             x16 = pool.acquire(nx * 2);
             w16 = pool.acquire(nw * 2);
-            check(grl_cast(dev, xb.dptr, GRL_F32, x16.dptr, GRL_BF16, nx), "linear: cast");
-            check(grl_cast(dev, wb.dptr, GRL_F32, w16.dptr, GRL_BF16, nw), "linear: cast");
-            check(grl_linear(dev, x16.dptr, w16.dptr, biasDev, static_cast<float*>(yb.dptr), int(p.batchSeq), int(p.inputDim),
-                             int(p.outputDim), GRL_BF16), "linear");
-        } else {
-            check(grl_linear(dev, xb.dptr, wb.dptr, biasDev, static_cast<float*>(yb.dptr), int(p.batchSeq), int(p.inputDim),
-                             int(p.outputDim), GRL_F32), "linear");
+            check(grl_cast(dev, xd, GRL_F32, x16.dptr, GRL_BF16, nx), "linear: cast");
+            check(grl_cast(dev, wd, GRL_F32, w16.dptr, GRL_BF16, nw), "linear: cast");
+            xd = x16.dptr;
+            wd = w16.dptr;
         }
-        check(grl_memcpy_d2h(dev, output, yb.dptr, ny * 4), "linear: download");
+        // A large result leaves in pieces of rows: the transfer of one piece, which bounds the time, runs beside the product of
+        // the next ones.
+        const size_t pieces = ny * 4 >= kPieceBytes && p.batchSeq >= 4 * kPieceRows ? 4 : 1;
+        const size_t per = (p.batchSeq / pieces + kPieceRows - 1) / kPieceRows * kPieceRows;
+        const size_t esz = bf16 ? 2 : 4;
+        for (size_t r = 0; r < p.batchSeq; r += per) {
+            const size_t rows = std::min(per, size_t(p.batchSeq) - r);
+            check(grl_linear(dev, static_cast<const char*>(xd) + r * p.inputDim * esz, wd, biasDev,
+                             static_cast<float*>(yb.dptr) + r * p.outputDim, int(rows), int(p.inputDim), int(p.outputDim),
+                             bf16 ? GRL_BF16 : GRL_F32), "linear");
+            if (pieces > 1) {
+                events.push_back(nullptr);
+                check(grl_event_create_untimed(&events.back()), "linear: event");
+                check(grl_event_record(dev, events.back()), "linear: event");
+            }
+        }
+        if (small) {
+            block->fetch(yb.dptr, ny * 4);
+        } else if (pieces > 1) {
+            grl_device* down = pool.device().downloadQueue();
+            size_t i = 0;
+            for (size_t r = 0; r < p.batchSeq; r += per, ++i) {
+                const size_t rows = std::min(per, size_t(p.batchSeq) - r), off = r * p.outputDim;
+                check(grl_event_wait(down, events[i]), "linear: event");
+                check(grl_memcpy_d2h(down, output + off, static_cast<const float*>(yb.dptr) + off, rows * p.outputDim * 4), "linear: download");
+            }
+            events.push_back(nullptr);          // a page-locked output array is still being written: the wait below is for it too
+            check(grl_event_create_untimed(&events.back()), "linear: event");
+            check(grl_event_record(down, events.back()), "linear: event");
+            check(grl_event_wait(dev, events.back()), "linear: event");
+        } else {
+            check(grl_memcpy_d2h(dev, output, yb.dptr, ny * 4), "linear: download");
+        }
         batch.submit();
+        if (small) block->deliver(output, ny * 4);
     } catch (...) {
         if (batch.recording()) batch.submitNoWait();
         pool.device().quiesce();   // nothing in flight may still touch the buffers released below

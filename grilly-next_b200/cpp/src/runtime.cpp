@@ -3,6 +3,7 @@
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
+#include <exception>
 
 #if defined(__AVX2__)
 #include <immintrin.h>
@@ -251,6 +252,38 @@ void BufferPool::download(const GrillyBuffer& buf, void* host, size_t bytes) {
 PoolStats BufferPool::stats() const {
     std::lock_guard<std::mutex> lock(mu_);
     return stats_;
+}
+
+// ---------------------------------------------------------------- SmallCall
+static constexpr size_t kSmallBlock = SmallCall::kMaxBytes + 4096;   // + alignment of a handful of inputs
+
+SmallCall::SmallCall(BufferPool& pool) : pool_(pool), in_(pool.acquire(kSmallBlock)) {}
+
+SmallCall::~SmallCall() {
+    if (std::uncaught_exceptions() > 0) pool_.device().quiesce();     // the transfer may still read the block
+    pool_.release(in_);
+}
+
+void* SmallCall::input(const void* host, size_t bytes) {
+    if (used_ + bytes > kSmallBlock) throw std::runtime_error("SmallCall: inputs exceed the block");
+    char* block = static_cast<char*>(pool_.device().pinnedStaging(kInSlot, kSmallBlock));
+    std::memcpy(block + used_, host, bytes);
+    void* at = static_cast<char*>(in_.dptr) + used_;
+    used_ += (bytes + 255) & ~size_t(255);
+    return at;
+}
+
+void SmallCall::send() {
+    check(grl_memcpy_h2d(pool_.device().handle(), in_.dptr, pool_.device().pinnedStaging(kInSlot, kSmallBlock), std::min(used_, kSmallBlock)),
+          "SmallCall: upload");
+}
+
+void SmallCall::fetch(const void* device, size_t bytes) {
+    check(grl_memcpy_d2h(pool_.device().handle(), pool_.device().pinnedStaging(kOutSlot, kMaxBytes), device, bytes), "SmallCall: download");
+}
+
+void SmallCall::deliver(void* host, size_t bytes) const {
+    std::memcpy(host, pool_.device().pinnedStaging(kOutSlot, kMaxBytes), bytes);
 }
 
 // ---------------------------------------------------------------- PipelineCache

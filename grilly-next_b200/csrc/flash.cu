@@ -2,7 +2,7 @@
 #include "common.cuh"
 
 namespace grl {
-int flash_fwd_simt(grl_device* dev, const grl_flash_params* p, float scale, const float2* rope);
+int flash_fwd_simt(grl_device* dev, const grl_flash_params* p, float scale, const float2* rope, bool wide);
 int flash_fwd_sm100(grl_device* dev, const grl_flash_params* p, float scale, const float2* rope, int32_t* status);
 }  // namespace grl
 
@@ -33,7 +33,8 @@ extern "C" int grl_flash_fwd(grl_device* dev, const grl_flash_params* p) {
     if (kernel == GRL_KERNEL_AUTO)
         kernel = (p->in_dtype == GRL_BF16 && (p->head_dim == 128 || p->head_dim == 64) && !p->mask && scale > 0.f) ? GRL_KERNEL_TCGEN05
                                                                                             : GRL_KERNEL_SIMT_F32;
-    if (kernel == GRL_KERNEL_SIMT_F32) return flash_fwd_simt(dev, p, scale, rope);
+    if (kernel == GRL_KERNEL_SIMT_F32 || kernel == GRL_KERNEL_SIMT_F32_WIDE)
+        return flash_fwd_simt(dev, p, scale, rope, kernel == GRL_KERNEL_SIMT_F32_WIDE);
     if (kernel == GRL_KERNEL_TCGEN05) {
         int32_t* status = p->status ? p->status : dev->d_status;
         if (!p->status) dev->status_dirty = true;

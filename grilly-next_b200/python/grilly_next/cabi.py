@@ -12,7 +12,7 @@ LIB_PATH = os.path.normpath(os.path.join(_HERE, "..", "..", "lib", "libgrilly_cu
 F32, BF16, FP8_INT4 = 0, 1, 2
 ROPE_NONE, ROPE_INTERLEAVED, ROPE_HALF = 0, 1, 2
 MASK_NONE, MASK_KEY, MASK_BSS, MASK_BHSS = 0, 1, 2, 3
-KERNEL_AUTO, KERNEL_SIMT_F32, KERNEL_TCGEN05 = 0, 1, 2
+KERNEL_AUTO, KERNEL_SIMT_F32, KERNEL_TCGEN05, KERNEL_SIMT_F32_WIDE = 0, 1, 2, 3
 ERR_TIMEOUT = -4
 
 # every symbol that include/grilly_cuda.h declares

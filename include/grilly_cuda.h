@@ -52,7 +52,9 @@ enum {
     GRL_MASK_BSS = 2,  /* (B,S,S): the size cpp/src/ops/attention.cpp:63-66 uploads; also (B,1,S,S) */
     GRL_MASK_BHSS = 3  /* (B,H,S,S): tests/test_attention.py:29-30 */
 };
-enum { GRL_KERNEL_AUTO = 0, GRL_KERNEL_SIMT_F32 = 1, GRL_KERNEL_TCGEN05 = 2 };
+enum { GRL_KERNEL_AUTO = 0, GRL_KERNEL_SIMT_F32 = 1, GRL_KERNEL_TCGEN05 = 2,
+       GRL_KERNEL_SIMT_F32_WIDE = 3 /* the float32 kernel in its form for large calls whatever the size: the pieces of one large
+                                     * call then add up exactly as one launch would */ };
 
 const char* grl_last_error(void);
 

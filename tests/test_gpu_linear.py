@@ -98,3 +98,14 @@ def test_linear_bf16_tiles(gpu, M, K, N):
     want = orc.round_bf16(x).astype(np.float64) @ orc.round_bf16(w).astype(np.float64).T
     assert np.abs(gpu.linear(x, w, b, dtype="bf16") - (want + b)).max() <= 2e-5 * max(K, 64)
     assert np.abs(gpu.linear(x, w, dtype="bf16") - want).max() <= 2e-5 * max(K, 64)
+
+
+@pytest.mark.parametrize("M,K,N,dtype", [(300, 64, 2048, "fp32"), (1000, 136, 700, "bf16"), (700, 1300, 1024, "fp32")])
+def test_linear_in_pieces(gpu, M, K, N, dtype):
+    # a result of several transfers: row pieces, more than one staging piece each way
+    from oracle import attention_oracle as orc
+    rng = np.random.default_rng(M)
+    x, w = rng.standard_normal((M, K), dtype=np.float32), rng.standard_normal((N, K), dtype=np.float32)
+    r = orc.round_bf16 if dtype == "bf16" else (lambda t: t)
+    want = r(x).astype(np.float64) @ r(w).astype(np.float64).T
+    assert np.abs(gpu.linear(x, w, dtype=dtype) - want).max() <= 2e-5 * K + 1e-4

@@ -303,3 +303,30 @@ def test_python_op_chunked_pipeline_is_bit_identical(dev, gpu):
     got = gpu.flash_attention2(Q, K, V, mask=mask)
     want = flash_cabi(dev, Q, K, V, mask=mask, mask_kind=cabi.MASK_KEY)
     assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("B,H,S,D,causal,rope,lens,kind", [
+    (1, 1, 1, 32, True, "none", None, None), (1, 3, 17, 64, True, "half", None, "key"),      # 16-row CTAs and their remainders
+    (2, 2, 129, 128, False, "interleaved", (129, 40), None), (1, 5, 200, 32, True, "half", None, "full"),
+    (2, 80, 70, 64, True, "interleaved", (70, 3), None), (1, 50, 190, 128, False, "half", None, "key"),   # 64-row CTAs
+    (2, 100, 65, 32, False, "none", None, "full")])
+def test_fp32_kernel_tile_edges(gpu, B, H, S, D, causal, rope, lens, kind):
+    rng = np.random.default_rng(S + D)
+    Q, K, V = (rng.standard_normal((B, H, S, D), dtype=np.float32) for _ in range(3))
+    keep = orc.causal_length_mask(B, H, S, lens, causal)
+    kw = {"causal": causal, "seq_lens": None if lens is None else np.array(lens, np.int32)}
+    if kind:
+        kw["mask"] = (rng.random((B, S) if kind == "key" else (B, H, S, S)) > 0.3).astype(np.float32)
+        kw["mask"][..., 0] = 1.0
+        keep = keep * orc.expand_mask(kw["mask"], B, H, S)
+    q, k = Q, K
+    if rope == "interleaved":
+        q, k = (orc.rope_interleaved(t, np.arange(S)) for t in (Q, K))
+    elif rope == "half":
+        q, k = (orc.rope_half(t.transpose(0, 2, 1, 3)).transpose(0, 2, 1, 3) for t in (Q, K))
+    if rope != "none":
+        kw.update(rope_theta=10000.0, rope_mode=rope)
+    want = orc.attention_4d(q, k, V, mask=keep)
+    for b in range(B if lens else 0):
+        want[b, :, lens[b]:] = 0.0
+    assert np.abs(gpu.flash_attention2(Q, K, V, **kw) - want).max() <= TOL_F32
