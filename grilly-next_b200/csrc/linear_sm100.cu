@@ -375,16 +375,21 @@ linear_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_consta
     }
 }
 
-// Exact fp32 form for a handful of rows: bound by the one pass over W, so a warp takes one row of W (one output column),
-// reads it once in 16-byte pieces and multiplies it with every row of x (which stays in L1).  Above kGemvRows the
-// tiled product of sgemm.cuh, whose 64-row tiles would be mostly padding here, is the faster one.
+// Exact fp32 form for small products: a warp takes one row of W (one output column) and multiplies it with up to eight rows of
+// x, all in 16-byte pieces (x stays in L1).  As long as its warps are one wave on the GPU this beats the 64 x 64 tiles of
+// sgemm.cuh, of which there are too few then: 9 x 768 x 3000 14.4 us (tiles 26.7), 64 x 256 x 1024 12.3 (12.3), 48 x 700 x 700
+// 14.4 (24.6); past the wave 32 x 768 x 3000 34.9 (26.7).
 constexpr int kGemvRows = 8;
+constexpr int kGemvWarps = 56;     // per SM, of the 64 it holds
 template <int MR>
 __global__ void __launch_bounds__(256) linear_f32_rows_kernel(const float* __restrict__ x, const float* __restrict__ w,
                                                               const float* __restrict__ bias, float* __restrict__ y, int M, int K, int N,
                                                               int vec) {
     const int n = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (n >= N) return;
+    x += (size_t)blockIdx.y * MR * K;
+    y += (size_t)blockIdx.y * MR * N;
+    M -= blockIdx.y * MR;
     const float* wr = w + (size_t)n * K;
     float acc[MR];
 #pragma unroll
@@ -411,14 +416,15 @@ __global__ void __launch_bounds__(256) linear_f32_rows_kernel(const float* __res
 }
 
 static int linear_f32(grl_device* dev, const float* x, const float* w, const float* bias, float* y, int M, int K, int N) {
-    if (M > kGemvRows)
+    const long long warps = (long long)((M + kGemvRows - 1) / kGemvRows) * ((N + 7) / 8) * 8;
+    if (M > kGemvRows && warps > (long long)kGemvWarps * dev->prop.multiProcessorCount)
         return sgemm::launch<true, true>(dev, sgemm::operand(x, 0, 0, K), sgemm::operand(w, 0, 0, K), sgemm::Output{y, 0, 0, N}, bias, M,
                                          N, K, 1, 1, 1.f, "linear_f32");
     const int vec = K % 4 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)w % 16 == 0;
-    const unsigned grid = (unsigned)((N + 7) / 8);
+    const dim3 grid((unsigned)((N + 7) / 8), (unsigned)((M + kGemvRows - 1) / kGemvRows));
     if (M == 1) linear_f32_rows_kernel<1><<<grid, 256, 0, dev->stream>>>(x, w, bias, y, M, K, N, vec);
     else if (M <= 4) linear_f32_rows_kernel<4><<<grid, 256, 0, dev->stream>>>(x, w, bias, y, M, K, N, vec);
-    else linear_f32_rows_kernel<8><<<grid, 256, 0, dev->stream>>>(x, w, bias, y, M, K, N, vec);
+    else linear_f32_rows_kernel<kGemvRows><<<grid, 256, 0, dev->stream>>>(x, w, bias, y, M, K, N, vec);
     GRL_LAUNCHED("linear_f32_rows_kernel");
     return GRL_OK;
 }

@@ -1,6 +1,6 @@
 // Batched float32 matrix products on the FMA pipe, shared by the exact linear projection and the unfused attention
 // pieces with their backward pass: C(m,n) = alpha * sum_k A(m,k) B(k,n), every output one chain of fused multiply-adds
-// in ascending k.
+// in ascending k (four chains, one per quarter of the k range, where split_kernel takes it).
 //
 // Bound: the FP32 pipe (128 FMA per clock per SM: 74 TFLOP/s).  A thread owns 8 x 8 outputs as 8 x 4 packed pairs
 // (fma.rn.f32x2 halves the issue slots, which leaves room for the shared-memory loads and the tile traffic); a warp
@@ -49,6 +49,17 @@ __device__ __forceinline__ float4 load4(const float* row, int i, int n, bool vec
     if (i + 2 < n) v.z = __ldg(row + i + 2);
     if (i + 3 < n) v.w = __ldg(row + i + 3);
     return v;
+}
+
+__device__ __forceinline__ void store4(float* dst, float4 v, int left, bool vec) {     // left: values that are inside the row
+    if (vec && left > 3) {
+        *reinterpret_cast<float4*>(dst) = v;
+        return;
+    }
+    if (left > 0) dst[0] = v.x;
+    if (left > 1) dst[1] = v.y;
+    if (left > 2) dst[2] = v.z;
+    if (left > 3) dst[3] = v.w;
 }
 
 // One k slice of an operand on its way from global to shared memory: EXT rows (m or n) x BK.  KC: the k index is the
@@ -107,10 +118,15 @@ struct Place {
 
 // acc[i][j/2] over k in [0, K): the main loop.  CAUSAL: rows of the product only see k <= m (slices that straddle the
 // diagonal test every term; the caller passes the tile's own upper limit as K).  With `pair` A is pair * (a - dots).
-template <typename SH, bool AKC, bool BKC, bool CAUSAL, bool PAIR>
+// GROUPS > 1: the threads are one of several groups with a product of their own (group `g`, barrier g + 1).
+template <typename SH, bool AKC, bool BKC, bool CAUSAL, bool PAIR, int GROUPS = 1>
 __device__ __forceinline__ void mainloop(float2 (&acc)[8][4], float* smem, const float* a, const Operand& A, const float* b,
                                          const Operand& B, int m0, int n0, int M, int N, int K, const float* pair, const float* dots) {
-    const int tid = threadIdx.x;
+    const int tid = GROUPS == 1 ? threadIdx.x : threadIdx.x % SH::THREADS;
+    auto sync = [&]() {
+        if constexpr (GROUPS == 1) __syncthreads();
+        else asm volatile("bar.sync %0, %1;" ::"r"((int)threadIdx.x / SH::THREADS + 1), "n"(SH::THREADS) : "memory");
+    };
     const Place<SH> at(tid);
     Fetch<SH::BM, SH::THREADS, AKC, PAIR> fa;
     Fetch<SH::BN, SH::THREADS, BKC> fb;
@@ -122,7 +138,7 @@ __device__ __forceinline__ void mainloop(float2 (&acc)[8][4], float* smem, const
     fb.load(b, nullptr, B.ld, B.vec, n0, N, 0, K, tid);
     fa.store(smem, SH::LDA, tid, dots, m0, M, 0, K);
     fb.store(smem + BK * SH::LDA, SH::LDB, tid, nullptr, n0, N, 0, K);
-    __syncthreads();
+    sync();
     const int slices = (K + BK - 1) / BK;
     for (int s = 0; s < slices; ++s) {
         const float* as = smem + (s & 1) * SH::TILE;
@@ -164,7 +180,7 @@ __device__ __forceinline__ void mainloop(float2 (&acc)[8][4], float* smem, const
             fa.store(ns, SH::LDA, tid, dots, m0, M, (s + 1) * BK, K);
             fb.store(ns + BK * SH::LDA, SH::LDB, tid, nullptr, n0, N, (s + 1) * BK, K);
         }
-        __syncthreads();
+        sync();
     }
 }
 
@@ -185,14 +201,7 @@ __device__ __forceinline__ void store_tile(const float2 (&acc)[8][4], float* c, 
             if (m >= M) continue;
             const float2 x = acc[i][2 * h], y = acc[i][2 * h + 1];
             const float4 v = make_float4(x.x * alpha + bv.x, x.y * alpha + bv.y, y.x * alpha + bv.z, y.y * alpha + bv.w);
-            float* dst = c + (long long)m * ld + n;
-            if (vec && n + 3 < N) *reinterpret_cast<float4*>(dst) = v;
-            else {
-                dst[0] = v.x;
-                if (n + 1 < N) dst[1] = v.y;
-                if (n + 2 < N) dst[2] = v.z;
-                if (n + 3 < N) dst[3] = v.w;
-            }
+            store4(c + (long long)m * ld + n, v, N - n, vec);
         }
     }
 }
@@ -208,6 +217,53 @@ __global__ void __launch_bounds__(SH::THREADS, SH::MIN_CTAS) kernel(Operand A, O
                                    CAUSAL ? min(K, m0 + SH::BM) : K, nullptr, nullptr);
     store_tile<SH>(acc, C.base + b * C.sb + h * C.sh, C.ld, m0, n0, M, N, alpha, bias);
     if constexpr (EARLY) pdl_wait();
+}
+
+// 64 x 64 tiles with the K range cut over four groups of threads, whose partial tiles are added in ascending order.  One group
+// alone is two warps an SM where there is one tile for each: the chain of load, barrier and products of a slice is the time
+// then (128 x 768 x 3072: 64 us), and it is four times shorter this way.
+constexpr int kSplit = 4;
+template <typename SH, bool AKC, bool BKC>
+__global__ void __launch_bounds__(SH::THREADS * kSplit) split_kernel(Operand A, Operand B, Output C, const float* bias, int M, int N, int K,
+                                                                     int H, float alpha) {
+    extern __shared__ __align__(16) float dyn[];
+    constexpr int REGION = 2 * SH::TILE;
+    static_assert(REGION >= SH::THREADS * 64, "a partial tile reuses its group's stages");
+    const int z = blockIdx.z, b = z / H, h = z % H, g = threadIdx.x / SH::THREADS, tid = threadIdx.x % SH::THREADS;
+    const int m0 = blockIdx.y * SH::BM, n0 = blockIdx.x * SH::BN;
+    const int slices = (K + BK - 1) / BK, k0 = g * slices / kSplit * BK, k1 = min(K, (g + 1) * slices / kSplit * BK);
+    const float* a = A.base + b * A.sb + h * A.sh + (AKC ? k0 : k0 * A.ld);
+    const float* bb = B.base + b * B.sb + h * B.sh + (BKC ? k0 : k0 * B.ld);
+    float2 acc[8][4];
+    mainloop<SH, AKC, BKC, false, false, kSplit>(acc, dyn + g * REGION, a, A, bb, B, m0, n0, M, N, k1 - k0, nullptr, nullptr);
+    float2* mine = reinterpret_cast<float2*>(dyn + g * REGION) + tid;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) mine[(i * 4 + j) * SH::THREADS] = acc[i][j];
+    __syncthreads();
+    // group g finishes rows 2g and 2g + 1 of every thread's eight
+    const Place<SH> at(tid);
+    float* c = C.base + b * C.sb + h * C.sh;
+    const bool vec = ((uintptr_t)c % 16 == 0) && C.ld % 4 == 0;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const int i = 2 * g + q, m = m0 + at.row(i);
+        if (m >= M) continue;
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) {
+            const int n = n0 + at.col(4 * hh);
+            float2 x = make_float2(0.f, 0.f), y = x;
+#pragma unroll
+            for (int p = 0; p < kSplit; ++p) {
+                const float2* part = reinterpret_cast<const float2*>(dyn + p * REGION) + tid;
+                x = __fadd2_rn(x, part[(i * 4 + 2 * hh) * SH::THREADS]);
+                y = __fadd2_rn(y, part[(i * 4 + 2 * hh + 1) * SH::THREADS]);
+            }
+            const float4 bv = bias ? load4(bias, n, N, (uintptr_t)bias % 16 == 0) : make_float4(0.f, 0.f, 0.f, 0.f);
+            store4(c + (long long)m * C.ld + n, make_float4(x.x * alpha + bv.x, x.y * alpha + bv.y, y.x * alpha + bv.z, y.y * alpha + bv.w), N - n, vec);
+        }
+    }
 }
 
 // Which tile: the widest one whose grid still gives every SM two CTAs; 64 rows otherwise, so that a small product
@@ -234,6 +290,12 @@ int launch(grl_device* dev, const Operand& A, const Operand& B, const Output& C,
         go(Shape<128, 128>());
     } else if ((rows_hint ? rows_hint : tile_rows(M, N, batch * H, 64, sms)) == 128) {
         go(Shape<128, 64>());
+    } else if (!CAUSAL && !EARLY && K >= 16 * BK) {
+        using SH = Shape<64, 64>;
+        constexpr int smem = kSplit * 2 * SH::TILE * (int)sizeof(float);
+        GRL_CUDA(cudaFuncSetAttribute(split_kernel<SH, AKC, BKC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        dim3 grid((N + SH::BN - 1) / SH::BN, (M + SH::BM - 1) / SH::BM, batch * H);
+        split_kernel<SH, AKC, BKC><<<grid, SH::THREADS * kSplit, smem, dev->stream>>>(A, B, C, bias, M, N, K, H, alpha);
     } else {
         go(Shape<64, 64>());
     }
