@@ -73,12 +73,8 @@ void linearEx(CommandBatch& batch, BufferPool& pool, PipelineCache& cache, const
             block->fetch(yb.dptr, ny * 4);
         } else if (pieces > 1) {
             grl_device* down = pool.device().downloadQueue();
-            size_t i = 0;
-            for (size_t r = 0; r < p.batchSeq; r += per, ++i) {
-                const size_t rows = std::min(per, size_t(p.batchSeq) - r), off = r * p.outputDim;
-                check(grl_event_wait(down, events[i]), "linear: event");
-                check(grl_memcpy_d2h(down, output + off, static_cast<const float*>(yb.dptr) + off, rows * p.outputDim * 4), "linear: download");
-            }
+            check(grl_memcpy_d2h_parts(down, output, yb.dptr, ny * 4, events.data(), int(events.size()), per * p.outputDim * 4),
+                  "linear: download");
             events.push_back(nullptr);          // a page-locked output array is still being written: the wait below is for it too
             check(grl_event_create_untimed(&events.back()), "linear: event");
             check(grl_event_record(down, events.back()), "linear: event");

@@ -379,6 +379,28 @@ int grl_memcpy_d2h(grl_device* dev, void* dst_host, const void* src, size_t byte
     return GRL_OK;
 }
 
+int grl_memcpy_d2h_parts(grl_device* dev, void* dst_host, const void* src, size_t bytes, grl_event* const* parts, int n_parts,
+                         size_t part_bytes) {
+    GRL_REQUIRE(dev && (bytes == 0 || (dst_host && src)) && parts && n_parts > 0 && n_parts <= 64, "NULL argument, or not 1 to 64 parts");
+    GRL_REQUIRE(part_bytes > 0 && (size_t)n_parts * part_bytes >= bytes, "the parts do not cover the %zu bytes", bytes);
+    DeviceGuard g(dev->ordinal);
+    cudaEvent_t ev[64];
+    for (int i = 0; i < n_parts; ++i) {
+        GRL_REQUIRE(parts[i], "NULL event");
+        ev[i] = parts[i]->ev;
+    }
+    if (pageable(dev, dst_host, bytes, 16u << 10)) {
+        GRL_CUDA(staged_download(dev, dst_host, src, bytes, ev, n_parts, part_bytes));
+        return GRL_OK;
+    }
+    for (int i = 0; i < n_parts && (size_t)i * part_bytes < bytes; ++i) {
+        const size_t off = (size_t)i * part_bytes, n = bytes - off < part_bytes ? bytes - off : part_bytes;
+        GRL_CUDA(cudaStreamWaitEvent(dev->stream, ev[i], 0));
+        GRL_CUDA(cudaMemcpyAsync((char*)dst_host + off, (const char*)src + off, n, cudaMemcpyDeviceToHost, dev->stream));
+    }
+    return GRL_OK;
+}
+
 int grl_memcpy_d2d(grl_device* dev, void* dst, const void* src, size_t bytes) {
     GRL_REQUIRE(dev && (bytes == 0 || (dst && src)), "NULL argument");
     DeviceGuard g(dev->ordinal);

@@ -91,6 +91,10 @@ int grl_host_alloc(size_t bytes, void** out); /* pinned host memory for staging 
 int grl_host_free(void* ptr);
 int grl_memcpy_h2d(grl_device* dev, void* dst, const void* src_host, size_t bytes);
 int grl_memcpy_d2h(grl_device* dev, void* dst_host, const void* src, size_t bytes);
+/* The same in up to 64 parts: bytes [i*part_bytes, (i+1)*part_bytes) are copied once parts[i] has completed, so that the copy of
+ * one part of a result runs beside the kernel that makes the next. */
+int grl_memcpy_d2h_parts(grl_device* dev, void* dst_host, const void* src, size_t bytes, grl_event* const* parts, int n_parts,
+                         size_t part_bytes);
 int grl_memcpy_d2d(grl_device* dev, void* dst, const void* src, size_t bytes);
 int grl_memset(grl_device* dev, void* dst, int value, size_t bytes);
 /* Wait for the stream.  timeout_ns == 0 waits without limit; otherwise polls and returns
