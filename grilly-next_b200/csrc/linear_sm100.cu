@@ -55,6 +55,10 @@ __device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity, volatile int
     }
 }
 
+__device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity, volatile int* abort, const Args& a, int which) {
+    return __all_sync(0xffffffffu, wait(bar, parity, abort, a, which));
+}
+
 __device__ __forceinline__ uint32_t instr_desc(int m, int n) {   // D f32, A and B bf16, both K-major
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
@@ -148,18 +152,18 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
             const uint32_t idesc = instr_desc(256, BN);
             int it = 0, n = 0;
             bool ok = true;
             for (int t = pair; t < tiles && ok; t += pairs, ++n) {
                 const int acc = n & 1;
-                if (n >= 2 && !wait(acc_empty(acc), ((n >> 1) - 1) & 1, abort, a, 2 * NST + 2 + acc)) break;
+                if (n >= 2 && !wait_warp(acc_empty(acc), ((n >> 1) - 1) & 1, abort, a, 2 * NST + 2 + acc)) break;
                 tc_fence_after();
                 const uint32_t d = tmem + (uint32_t)acc * 256u;
                 for (int k = 0; k < n_k; ++k, ++it) {
                     const int s = it % NST, ph = it / NST;
-                    ok = wait(full(s), ph & 1, abort, a, s);
+                    ok = wait_warp(full(s), ph & 1, abort, a, s);
                     if (!ok) break;
                     tc_fence_after();
                     const uint32_t a_lo = desc_lo(base + (uint32_t)s * P::STAGE, 16), b_lo = desc_lo(base + (uint32_t)s * P::STAGE + P::A_BYTES, 16);
@@ -180,7 +184,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
             const int acc = n & 1;
             int tm, tn;
             place(t, tm, tn);
-            if (!__all_sync(0xffffffffu, wait(acc_full(acc), (n >> 1) & 1, abort, a, 2 * NST + acc))) break;
+            if (!wait_warp(acc_full(acc), (n >> 1) & 1, abort, a, 2 * NST + acc)) break;
             if (t + pairs >= tiles) pdl_trigger();        // the next kernel may launch under the last epilogues
             tc_fence_after();
             const int row0 = tm * 256 + (int)rank * 128 + w * 32;
@@ -297,24 +301,24 @@ linear_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_consta
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
             const uint32_t idesc = instr_desc(128, NT);
             bool ok = true;
             for (int k = k0; k < k1 && ok; ++k) {
                 const int i = k - k0, s = i % NST, ph = i / NST;
-                ok = wait(full(s), ph & 1, abort, a, s);
+                ok = wait_warp(full(s), ph & 1, abort, a, s);
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t w_lo = desc_lo(ring + (uint32_t)(s * stage_bytes), 16), x_lo = desc_lo(ring + (uint32_t)(s * stage_bytes + w_bytes), 16);
 #pragma unroll
                 for (int ks = 0; ks < BK / 16; ++ks)
-                    mma_ss3(tmem, w_lo + (uint32_t)(ks * 32 >> 4), x_lo + (uint32_t)(ks * 32 >> 4), idesc, (i | ks) != 0);
+                    mma_ss2(tmem, w_lo + (uint32_t)(ks * 32 >> 4), x_lo + (uint32_t)(ks * 32 >> 4), idesc, (i | ks) != 0);
                 mma_commit(empty(s));                 // the stage is free once these products have read it
             }
             if (ok) mma_commit(acc_full);
         }
     } else if (warp >= 4) {
-        good = __all_sync(0xffffffffu, wait(acc_full, 0, abort, a, 2 * NST));
+        good = wait_warp(acc_full, 0, abort, a, 2 * NST);
         pdl_trigger();        // the next kernel may launch under the epilogues; earlier it would take slots and sit unevenly
         tc_fence_after();
         const int w = warp & 3, n = n0 + w * 32 + lane;

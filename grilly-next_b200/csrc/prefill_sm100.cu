@@ -9,7 +9,7 @@
 //                64-column boxes, 128-byte swizzle) into a 2-stage shared-memory ring.
 //   warps 12-15  RoPE: rotate each K tile in place in shared memory, fence.proxy.async, hand the
 //                tile to the MMA warp.  (Each softmax warpgroup rotates its own Q tile once.)
-//   warps 0, 2   one thread per query tile issues tcgen05.mma: S_t = Q_t K^T (A,B from shared memory, K-major)
+//   warps 0, 2   one warp per query tile issues tcgen05.mma: S_t = Q_t K^T (A,B from shared memory, K-major)
 //                into TMEM, then O_t += P_t V with P_t read from TMEM and V as an MN-major
 //                shared-memory operand; per 64-key step i the issue order is PV0_i, QK0_i+2, PV1_i, QK1_i+2.
 //   warps 4-7 / 8-11  softmax warpgroup of query tile 0 / 1, one thread per query row:
@@ -290,6 +290,38 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     uint8_t* smem = smem_raw + (base_addr - raw_addr);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + SMEM_BAR + NUM_BARS * 8);
+    int* abort_flag = reinterpret_cast<int*>(smem + SMEM_BAR + NUM_BARS * 8 + 4);
+    Ctx ctx{base_addr + SMEM_BAR, abort_flag, a.status, a.wait_limit};
+    auto bar = [&](int i) { return ctx.bars + (uint32_t)i * 8u; };
+    if (warp == WARP_TMA && lane == 0) {
+        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmQ)) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmK)) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmV)) : "memory");
+        for (int t = 0; t < NQ; ++t) {
+            mbar_init(bar(Q_FULL + t), 1);
+            mbar_init(bar(Q_READY + t), 128);
+            for (int bf = 0; bf < 2; ++bf) {
+                mbar_init(bar(S_FULL + 2 * t + bf), 1);
+                mbar_init(bar(P_READY + 2 * t + bf), 128);
+            }
+            mbar_init(bar(O_DONE + t), 1);
+            mbar_init(bar(EXP_TURN + t), 128);
+        }
+        for (int s = 0; s < NSTAGE; ++s) {
+            mbar_init(bar(K_FULL + s), 1);
+            mbar_init(bar(K_READY + s), 128);
+            mbar_init(bar(K_EMPTY + s), 2);   // one arrival per reading query tile (twice from a lone reader)
+            mbar_init(bar(V_FULL + s), 1);
+            mbar_init(bar(V_EMPTY + s), 2);
+        }
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        fence_async_smem();
+    }
+    // all of the above beside the tail of the kernel before this one on the stream, nothing below
+    pdl_wait();
+
     // 1-D grid over (batch*heads) x (query tile pairs).  Causal: the work of a tile pair grows with its index,
     // so within a group of kHeadGroup heads CTAs are handed out longest pair first and the shortest ones form
     // the tail; groups follow one another so that the K/V of the heads in flight (1 MiB per head at S=2048) stay
@@ -342,40 +374,12 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     const int n_total = max(n_kt[0], n_kt[1]);
     const bool use_rope = a.rope_mode != GRL_ROPE_NONE;
 
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + SMEM_BAR + NUM_BARS * 8);
-    int* abort_flag = reinterpret_cast<int*>(smem + SMEM_BAR + NUM_BARS * 8 + 4);
-    Ctx ctx{base_addr + SMEM_BAR, abort_flag, a.status, a.wait_limit};
-    auto bar = [&](int i) { return ctx.bars + (uint32_t)i * 8u; };
-
     auto load_tile = [&](uint32_t dst, const CUtensorMap* tm, int row, int full_bar) {
         mbar_expect_tx(bar(full_bar), (HD / 64) * HALF_BYTES);
         tma_load_3d(dst, tm, 0, row, bh, bar(full_bar));
         if (HD == 128) tma_load_3d(dst + HALF_BYTES, tm, 64, row, bh, bar(full_bar));
     };
     if (warp == WARP_TMA && lane == 0) {
-        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmQ)) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmK)) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmV)) : "memory");
-        for (int t = 0; t < NQ; ++t) {
-            mbar_init(bar(Q_FULL + t), 1);
-            mbar_init(bar(Q_READY + t), 128);
-            for (int bf = 0; bf < 2; ++bf) {
-                mbar_init(bar(S_FULL + 2 * t + bf), 1);
-                mbar_init(bar(P_READY + 2 * t + bf), 128);
-            }
-            mbar_init(bar(O_DONE + t), 1);
-            mbar_init(bar(EXP_TURN + t), 128);
-        }
-        for (int s = 0; s < NSTAGE; ++s) {
-            mbar_init(bar(K_FULL + s), 1);
-            mbar_init(bar(K_READY + s), 128);
-            mbar_init(bar(K_EMPTY + s), 2);   // one arrival per reading query tile (twice from a lone reader)
-            mbar_init(bar(V_FULL + s), 1);
-            mbar_init(bar(V_EMPTY + s), 2);
-        }
-        *abort_flag = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        fence_async_smem();
         // The first loads need no "empty" wait: put them in flight now, behind nothing but the barrier
         // initialisation, while the other warps are still setting up.  QK(0,0) needs Q0 and K0 first.
         load_tile(base_addr + SMEM_Q, &tmQ, q0, Q_FULL);
@@ -429,16 +433,16 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
             }
         }
       } else if (warp == WARP_MMA || warp == WARP_MMA1) {
-        // ------------------------------------------------------------------ MMA issuers: one thread per query tile
-        // Each tile has its own in-order chain  wait P -> P.V(i) -> Q.K^T(i+2)  issued by its own thread, so that
+        // ------------------------------------------------------------------ MMA issuers: one warp per query tile
+        // Each tile has its own in-order chain  wait P -> P.V(i) -> Q.K^T(i+2)  issued by its own warp, so that
         // one tile's softmax never holds up the other tile's tensor work; the tensor pipe interleaves the two.
-        const int t = (warp == WARP_MMA) ? 0 : 1;
-        if (lane == 0 && n_half[t] > 0) {
+        const int t = uniform(warp) == WARP_MMA ? 0 : 1;
+        if ((t ? n_half[1] : n_half[0]) > 0) {
             bool ok = true;
             const uint32_t qa = desc_lo(base_addr + SMEM_Q + t * TILE_BYTES, 16);
             const uint32_t k_lo = desc_lo(base_addr + SMEM_K, 16), v_lo = desc_lo(base_addr + SMEM_V, HALF_BYTES);
-            const int nh = n_half[t], other_tiles = n_kt[t ^ 1];
-            const uint32_t s_tmem = tmem_base + (uint32_t)t * TMEM_TILE, o_tmem = s_tmem + TMEM_O;
+            const int nh = uniform(t ? n_half[1] : n_half[0]), other_tiles = uniform(t ? n_kt[0] : n_kt[1]);
+            const uint32_t s_tmem = (uint32_t)uniform((int)tmem_base) + (uint32_t)t * TMEM_TILE, o_tmem = s_tmem + TMEM_O;
             // A K or V tile (two 64-key steps) is released once per reading tile: the K_EMPTY / V_EMPTY barriers
             // count two arrivals, and a tile that reads a K/V tile alone arrives twice.
             auto release = [&](int bar_id, int j) {
@@ -448,26 +452,25 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
             // S_t[i & 1] = Q_t K[64 keys of step i]^T
             auto issue_qk = [&](int i) -> bool {
                 const int j = i >> 1, s = j % NSTAGE, it = j / NSTAGE;
-                if (!wait_bar(ctx, (use_rope ? K_READY : K_FULL) + s, it & 1)) return false;
+                if (!wait_bar_warp(ctx, (use_rope ? K_READY : K_FULL) + s, it & 1)) return false;
                 tc_fence_after();
                 const uint32_t d_tmem = s_tmem + (uint32_t)(i & 1) * BH;
                 const uint32_t kb = k_lo + (uint32_t)s * (TILE_BYTES >> 4) + (uint32_t)(i & 1) * ((BH * 128) >> 4);  // rows 64.. of each box
-                mma_ss2<false>(d_tmem, qa, kb, IDESC_QK);
 #pragma unroll
-                for (int ks = 1; ks < HD / 16; ++ks) {
+                for (int ks = 0; ks < HD / 16; ++ks) {
                     const uint32_t off = (uint32_t)(((ks >> 2) * HALF_BYTES + (ks & 3) * 32) >> 4);
-                    mma_ss2<true>(d_tmem, qa + off, kb + off, IDESC_QK);
+                    mma_ss2(d_tmem, qa + off, kb + off, IDESC_QK, ks != 0);
                 }
                 mma_commit(bar(S_FULL + 2 * t + (i & 1)));
                 if ((i & 1) || i + 1 >= nh) release(K_EMPTY + s, j);   // last step of this tile on K tile j
                 return true;
             };
-            ok = wait_bar(ctx, (use_rope ? Q_READY : Q_FULL) + t, 0);
+            ok = wait_bar_warp(ctx, (use_rope ? Q_READY : Q_FULL) + t, 0);
             for (int i = 0; i < 2 && i < nh && ok; ++i) ok = issue_qk(i);   // two steps of S ahead of the softmax
             for (int i = 0; i < nh && ok; ++i) {
                 const int j = i >> 1, s = j % NSTAGE, it = j / NSTAGE;
-                ok = wait_bar(ctx, P_READY + 2 * t + (i & 1), (i >> 1) & 1);
-                if (ok) ok = wait_bar(ctx, V_FULL + s, it & 1);
+                ok = wait_bar_warp(ctx, P_READY + 2 * t + (i & 1), (i >> 1) & 1);
+                if (ok) ok = wait_bar_warp(ctx, V_FULL + s, it & 1);
                 if (!ok) break;
                 tc_fence_after();
                 // O_t += P_t[step i] V[64 keys]: A = P in TMEM (16 keys = 8 packed columns per k-step), B = 16 key
@@ -676,6 +679,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         }
     }
 
+    pdl_trigger();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -729,13 +733,9 @@ int flash_fwd_sm100(grl_device* dev, const grl_flash_params* p, float scale, con
         attr_set[dev->ordinal & 63] = true;
     }
     const bool f32 = p->out_dtype == GRL_F32;
-    if (HD == 128) {
-        if (f32) flash_fwd_sm100_kernel<float, 128><<<grid, kThreads, SMEM_TOTAL, dev->stream>>>(tq, tk, tv, a);
-        else flash_fwd_sm100_kernel<__nv_bfloat16, 128><<<grid, kThreads, SMEM_TOTAL, dev->stream>>>(tq, tk, tv, a);
-    } else {
-        if (f32) flash_fwd_sm100_kernel<float, 64><<<grid, kThreads, SMEM_TOTAL, dev->stream>>>(tq, tk, tv, a);
-        else flash_fwd_sm100_kernel<__nv_bfloat16, 64><<<grid, kThreads, SMEM_TOTAL, dev->stream>>>(tq, tk, tv, a);
-    }
+    auto kernel = HD == 128 ? (f32 ? flash_fwd_sm100_kernel<float, 128> : flash_fwd_sm100_kernel<__nv_bfloat16, 128>)
+                            : (f32 ? flash_fwd_sm100_kernel<float, 64> : flash_fwd_sm100_kernel<__nv_bfloat16, 64>);
+    GRL_CUDA(launch_pdl(kernel, grid, kThreads, SMEM_TOTAL, dev->stream, tq, tk, tv, a));
     GRL_LAUNCHED("flash_fwd_sm100_kernel");
     return GRL_OK;
 }
