@@ -11,6 +11,11 @@
 // multiply-adds, 16-byte shared-memory loads).  FM = 16: four groups of 64 threads take every fourth 32-key tile each, with
 // a softmax state of their own, and merge at the end: a call too small to give every SM a 64-row tile is bound by the chain of
 // its tiles (load, products, softmax, products), which is four times shorter this way and on four times as many SMs.
+// Tiles that need no rotation are copied asynchronously, Q with the first K and V: a small CTA has few tiles, so its round trips
+// to memory are much of its time.
+// Measured as a host call (float32 in and out, 4 heads x 256 x 64): 138 us with 64-row CTAs alone, 130 us with both shapes and
+// 110 us with the asynchronous tiles and the inputs streamed to the transfer block; 8 heads x 512 x 64: 404 and 182 us, 2 x 8
+// heads x 512 x 128: 1188 and 510 us.
 #include "common.cuh"
 
 namespace grl {
@@ -86,6 +91,21 @@ __device__ __forceinline__ void load_tile(float* dst, const TIn* src, int row0, 
     }
 }
 
+// The same by asynchronous copies, for float32 tiles that need no rotation: all of a tile's loads are in flight at once and none
+// waits in a register.  tile_wait() before the barrier that hands the tile over.
+template <int D, int ROWS, int NT>
+__device__ __forceinline__ void load_tile_async(float* dst, const float* src, int row0, int n_valid, int tid) {
+    constexpr int LD = D + 4;
+#pragma unroll
+    for (int q = tid; q < ROWS * D / 4; q += NT) {
+        const int r = q / (D / 4), d = (q % (D / 4)) * 4;
+        const float* from = src + (size_t)(row0 + min(r, n_valid - 1)) * D + d;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + r * LD + d)), "l"(from),
+                     "r"(r < n_valid ? 16 : 0) : "memory");
+    }
+}
+__device__ __forceinline__ void tile_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 template <int D, int FM>
 struct FlashF32Shape {
     static constexpr int G = 64 / FM;                  // groups of threads
@@ -137,7 +157,16 @@ __global__ void __launch_bounds__(256) flash_fwd_f32_kernel(FlashF32Args a) {
     const TIn* K = reinterpret_cast<const TIn*>(a.k) + base;
     const TIn* V = reinterpret_cast<const TIn*>(a.v) + base;
 
-    load_tile<TIn, D, FM, 256>(Qs, Q, q0, min(FM, S - q0), a.rope_mode, a.rope, a.vec, threadIdx.x);
+    const bool async = sizeof(TIn) == 4 && a.vec;
+    if (async && a.rope_mode == GRL_ROPE_NONE) load_tile_async<D, FM, 256>(Qs, reinterpret_cast<const float*>(Q), q0, min(FM, S - q0), threadIdx.x);
+    else load_tile<TIn, D, FM, 256>(Qs, Q, q0, min(FM, S - q0), a.rope_mode, a.rope, a.vec, threadIdx.x);
+    auto load_kv = [&](int kt) {
+        const int k0 = kt * FN, rows = min(FN, S - k0);
+        if (async) load_tile_async<D, FN, GT>(Vs, reinterpret_cast<const float*>(V), k0, rows, tid);
+        if (async && a.rope_mode == GRL_ROPE_NONE) load_tile_async<D, FN, GT>(Ks, reinterpret_cast<const float*>(K), k0, rows, tid);
+        else load_tile<TIn, D, FN, GT>(Ks, K, k0, rows, a.rope_mode, a.rope, a.vec, tid);
+        if (!async) load_tile<TIn, D, FN, GT>(Vs, V, k0, rows, GRL_ROPE_NONE, nullptr, a.vec, tid);
+    };
 
     float m[4], l[4];
     float2 acc[4][DPT / 2];
@@ -152,14 +181,18 @@ __global__ void __launch_bounds__(256) flash_fwd_f32_kernel(FlashF32Args a) {
     int k_end = len;
     if (a.causal) k_end = min(k_end, q0 + FM);
     const int n_kt = (k_end + FN - 1) / FN;
-    if (G > 1) __syncthreads();      // Q is the whole CTA's
+    if (group < n_kt) load_kv(group);
+    tile_wait();
+    __syncthreads();      // Q is the whole CTA's
 
     for (int kt = group; kt < n_kt; kt += G) {
         const int k0 = kt * FN;
-        sync_group();     // previous tile's Ks/Vs/Ps fully consumed
-        load_tile<TIn, D, FN, GT>(Ks, K, k0, min(FN, S - k0), a.rope_mode, a.rope, a.vec, tid);
-        load_tile<TIn, D, FN, GT>(Vs, V, k0, min(FN, S - k0), GRL_ROPE_NONE, nullptr, a.vec, tid);
-        sync_group();
+        if (kt != group) {
+            sync_group();     // previous tile's Ks/Vs/Ps fully consumed
+            load_kv(kt);
+            tile_wait();
+            sync_group();
+        }
 
         float2 s2[4][CK];       // even and odd elements of d
 #pragma unroll
