@@ -8,7 +8,10 @@
 // (mma.sync m16n8k16, the group's query heads padded to the 16-row operand, q split into
 // bf16 hi+lo so that its fp32 precision survives), with a private fp32 online softmax in the
 // exp2 domain.  K and V cross HBM -> SM exactly once; the four warps' partials are merged in
-// shared memory and leave the CTA as (O un-normalised, m, l), the layout lse_merge_kernel reads.
+// shared memory and leave the CTA as (O un-normalised, m, l), the layout lse_merge_kernel reads.  Splits of one head that fit a
+// thread-block cluster merge through its shared memory instead, and a launch sets up its ring and barriers under the kernel before
+// it.  Append + decode step: 1 sequence x 8 kv heads x 1001 tokens 19.4 us before, 9.9 now (latency); 32 x 8 x 4096 93 and 85 us
+// (HBM); 1 x 8 x 131072 quantised 107 and 79 us (the conversion's integer instructions).
 //
 // The same kernel, instantiated for the quantised cache (GRL_FP8_INT4: FP8-E4M3 keys, INT4 values, one float16 scale
 // per 32 key elements, cpp/src/ops/kv_cache.cpp:272-399 and :500-577), streams 12.5 KiB per (page, kv head) instead
@@ -37,7 +40,6 @@ template <bool QUANT, int HD> struct Ring {
 };
 constexpr int QK_BYTES = P * D;          // 8 KiB of key bytes per 64 tokens of a kv head
 constexpr int QV_BYTES = P * D / 2;      // 4 KiB of packed value nibbles
-constexpr int QS_BYTES = P * (D / 32) * 2;   // 512 B of float16 scales
 template <> struct Ring<true, 128> {
     static constexpr int SLAB = 0;
     static constexpr int NST = 6;

@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(1024) kv_append_kernel(AppendArgs a) {
 // thread moves 8 elements of a row (two 16-byte loads, one 16-byte store of bf16), two heads of keys and values in flight.
 // It owns four rotation pairs of ONE token and walks that token's heads: the double-precision angle reduction, once per
 // (token, head, pair) in the element-wise kernel above and most of its time, runs once per (token, pair).  Measured (4 x 2048
-// tokens x 8 kv heads x 128, bf16, RoPE; 100 MB): 61 us before.
+// tokens x 8 kv heads x 128, bf16, RoPE; 100 MB): 61 us before, 20 us now (5.0 TB/s).
 constexpr int kAppendHeads = 2;
 template <typename T>
 __device__ __forceinline__ void store8(T* row, int o0, int o1, const float (&y)[8]);

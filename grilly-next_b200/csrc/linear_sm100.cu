@@ -67,7 +67,8 @@ __device__ __forceinline__ uint32_t instr_desc(int m, int n) {   // D f32, A and
 // (64 cycles of reads and 64 of TMA writes per 64 cycles of products), which held a one-SM kernel at 1.0 PFLOP/s; a pair
 // reads each half of W's tile once for both SMs.  A CTA stages its 128 rows of x and BN/2 rows of W; the even CTA's thread
 // issues the products for both; the accumulator (128 lanes x BN columns in each SM) is double-buffered, so that one tile's
-// epilogue runs under the next tile's products.
+// epilogue runs under the next tile's products.  4096 x 4096 x 4096: 157 us in 128 x 128 tiles of one SM each, 117 us in pairs
+// (1.17 PFLOP/s), cold L2.
 template <int BN_>
 struct Pair {
     static constexpr int BN = BN_, A_BYTES = 128 * BK * 2, B_BYTES = BN / 2 * BK * 2, STAGE = A_BYTES + B_BYTES;

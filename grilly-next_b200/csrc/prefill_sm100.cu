@@ -21,7 +21,14 @@
 // S is produced in 64-key halves into two TMEM buffers per tile, so that QK^T of step i+1 and i+2
 // runs while the softmax of step i is still busy and P.V of step i does not gate the next scores.
 // TMEM columns of tile t: S halves at t*256 + {0, 64} (P overlays the first 32 columns of its
-// half), O at t*256 + 128.  Every mbarrier wait is bounded; on expiry the CTA records an error, drains
+// half), O at t*256 + 128.
+//
+// Bound: the chain of scores, softmax and products of a tile, and at length the 1000 W power cap.  The products are issued by
+// one elected lane of a converged warp (a warp that diverges for it re-issues its uniform work per lane), and a launch sets up its
+// barriers under the end of the kernel before it: 1 x 32 heads x 333 tokens 15.5 -> 13.2 us; 4 x 32 x 2048 causal with RoPE 229 us
+// before and after, at the power cap.
+//
+// Every mbarrier wait is bounded; on expiry the CTA records an error, drains
 // its copies and returns.
 #include <cuda.h>
 
