@@ -26,7 +26,7 @@
 // Bound: the chain of scores, softmax and products of a tile, and at length the 1000 W power cap.  The products are issued by
 // one elected lane of a converged warp (a warp that diverges for it re-issues its uniform work per lane), and a launch sets up its
 // barriers under the end of the kernel before it: 1 x 32 heads x 333 tokens 15.5 -> 13.2 us; 4 x 32 x 2048 causal with RoPE 229 us
-// before and after, at the power cap.
+// before and after, at the power cap.  Calls of few tiles take the split form (see the kernel).
 //
 // Every mbarrier wait is bounded; on expiry the CTA records an error, drains
 // its copies and returns.
@@ -59,7 +59,9 @@ constexpr int SMEM_Q = 0;
 constexpr int SMEM_K = SMEM_Q + NQ * TILE_BYTES;
 constexpr int SMEM_V = SMEM_K + NSTAGE * TILE_BYTES;
 constexpr int SMEM_BAR = SMEM_V + NSTAGE * TILE_BYTES;
-constexpr int SMEM_TOTAL = SMEM_BAR + 256 + 1024;  // + barrier block + alignment slack
+constexpr int SMEM_TOTAL = SMEM_BAR + 256 + 1024;  // + barrier block + alignment slack: with the system's 1 KiB just below 196 KiB,
+                                                   // which leaves 60 KiB of L1 (one step more costs 1 % at 2048 tokens)
+constexpr int SMEM_ML = SMEM_Q + TILE_BYTES;       // split form: row maxima and sums, in the Q tile that it does not have
 constexpr int kHeadGroup = 32;      // (batch, head) slices scheduled together under a causal mask
 constexpr int BH = 64;              // keys per softmax step: S is computed in 64-key halves, double-buffered
 constexpr uint32_t TMEM_COLS = 512;
@@ -287,7 +289,12 @@ __device__ __forceinline__ void store_row_chunk<__nv_bfloat16>(__nv_bfloat16* ds
     }
 }
 
-template <typename TOut, int HD>
+// SPLIT: a CTA owns ONE 128-row query tile, and the two "tiles" t of everything below are the two halves of its keys: t takes the
+// 64 keys t of every K tile, one step per K tile, with scores, accumulator and row state of its own.  Both leave their maxima and
+// sums in shared memory and each writes half of the output's columns from the two accumulators.  The chain of steps of a query
+// tile, which bounds a call that leaves SMs idle, is half as long, on twice as many SMs.  Measured, us, pairs / split: 32 heads x 333
+// tokens 13.2 / 11.9, 32 x 512 20.5 / 14.6, 8 x 2048 45.1 / 30.9, 4 x 4096 81.7 / 56.9 (causal, RoPE), 16 x 1024 full 27.8 / 19.7.
+template <typename TOut, int HD, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 1)
 flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                        const __grid_constant__ CUtensorMap tmV, const Args a) {
@@ -348,12 +355,13 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     }
     const int b = bh / a.H;
     const int S = a.S;
-    const int q0 = qp * (NQ * BM);
+    constexpr int ROWS = SPLIT ? BM : NQ * BM;
+    const int q0 = qp * ROWS;
     const int len = a.seq_lens ? min(a.seq_lens[b], S) : S;
     TOut* O = reinterpret_cast<TOut*>(a.o) + (size_t)bh * S * HD;
 
     if (q0 >= len) {  // padded query rows are defined as zero
-        const int rows = min(NQ * BM, S - q0);
+        const int rows = min(ROWS, S - q0);
         for (int idx = tid; idx < rows * HD; idx += kThreads) store_from_float<TOut>(O + (size_t)q0 * HD + idx, 0.f);
         return;
     }
@@ -368,15 +376,15 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     for (int t = 0; t < NQ; ++t) {
         const int qt0 = q0 + t * BM;
         const int k_end = a.causal ? min(len, qt0 + BM) : len;
-        n_kt[t] = (qt0 < len) ? (k_end + BN - 1) / BN : 0;
+        n_kt[t] = (qt0 < len && !(SPLIT && t)) ? (k_end + BN - 1) / BN : 0;
     }
     // 64-key softmax steps of tile t (the second half of its last K tile may be wholly invisible)
     int n_half[NQ];
 #pragma unroll
     for (int t = 0; t < NQ; ++t) {
-        const int qt0 = q0 + t * BM;
+        const int qt0 = SPLIT ? q0 : q0 + t * BM;
         const int k_end = a.causal ? min(len, qt0 + BM) : len;
-        n_half[t] = (qt0 < len) ? (k_end + BH - 1) / BH : 0;
+        n_half[t] = (qt0 < len) ? (SPLIT ? (k_end - t * BH + BN - 1) / BN : (k_end + BH - 1) / BH) : 0;
     }
     const int n_total = max(n_kt[0], n_kt[1]);
     const bool use_rope = a.rope_mode != GRL_ROPE_NONE;
@@ -446,36 +454,40 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         const int t = uniform(warp) == WARP_MMA ? 0 : 1;
         if ((t ? n_half[1] : n_half[0]) > 0) {
             bool ok = true;
-            const uint32_t qa = desc_lo(base_addr + SMEM_Q + t * TILE_BYTES, 16);
+            const int qt = SPLIT ? 0 : t;
+            const uint32_t qa = desc_lo(base_addr + SMEM_Q + qt * TILE_BYTES, 16);
             const uint32_t k_lo = desc_lo(base_addr + SMEM_K, 16), v_lo = desc_lo(base_addr + SMEM_V, HALF_BYTES);
-            const int nh = uniform(t ? n_half[1] : n_half[0]), other_tiles = uniform(t ? n_kt[0] : n_kt[1]);
+            const int nh = uniform(t ? n_half[1] : n_half[0]), other_tiles = SPLIT ? uniform(t ? n_half[0] : n_half[1]) : uniform(t ? n_kt[0] : n_kt[1]);
             const uint32_t s_tmem = (uint32_t)uniform((int)tmem_base) + (uint32_t)t * TMEM_TILE, o_tmem = s_tmem + TMEM_O;
             // A K or V tile (two 64-key steps) is released once per reading tile: the K_EMPTY / V_EMPTY barriers
             // count two arrivals, and a tile that reads a K/V tile alone arrives twice.
+            auto tile_of = [&](int i) { return SPLIT ? i : i >> 1; };
+            auto half_of = [&](int i) { return (uint32_t)(SPLIT ? t : i & 1); };
+            auto last_of = [&](int i) { return SPLIT || (i & 1) || i + 1 >= nh; };     // this tile's last step on its K tile
             auto release = [&](int bar_id, int j) {
                 mma_commit(bar(bar_id));
                 if (j >= other_tiles) mma_commit(bar(bar_id));
             };
             // S_t[i & 1] = Q_t K[64 keys of step i]^T
             auto issue_qk = [&](int i) -> bool {
-                const int j = i >> 1, s = j % NSTAGE, it = j / NSTAGE;
+                const int j = tile_of(i), s = j % NSTAGE, it = j / NSTAGE;
                 if (!wait_bar_warp(ctx, (use_rope ? K_READY : K_FULL) + s, it & 1)) return false;
                 tc_fence_after();
                 const uint32_t d_tmem = s_tmem + (uint32_t)(i & 1) * BH;
-                const uint32_t kb = k_lo + (uint32_t)s * (TILE_BYTES >> 4) + (uint32_t)(i & 1) * ((BH * 128) >> 4);  // rows 64.. of each box
+                const uint32_t kb = k_lo + (uint32_t)s * (TILE_BYTES >> 4) + half_of(i) * ((BH * 128) >> 4);  // rows 64.. of each box
 #pragma unroll
                 for (int ks = 0; ks < HD / 16; ++ks) {
                     const uint32_t off = (uint32_t)(((ks >> 2) * HALF_BYTES + (ks & 3) * 32) >> 4);
                     mma_ss2(d_tmem, qa + off, kb + off, IDESC_QK, ks != 0);
                 }
                 mma_commit(bar(S_FULL + 2 * t + (i & 1)));
-                if ((i & 1) || i + 1 >= nh) release(K_EMPTY + s, j);   // last step of this tile on K tile j
+                if (last_of(i)) release(K_EMPTY + s, j);
                 return true;
             };
-            ok = wait_bar_warp(ctx, (use_rope ? Q_READY : Q_FULL) + t, 0);
+            ok = wait_bar_warp(ctx, (use_rope ? Q_READY : Q_FULL) + qt, 0);
             for (int i = 0; i < 2 && i < nh && ok; ++i) ok = issue_qk(i);   // two steps of S ahead of the softmax
             for (int i = 0; i < nh && ok; ++i) {
-                const int j = i >> 1, s = j % NSTAGE, it = j / NSTAGE;
+                const int j = tile_of(i), s = j % NSTAGE, it = j / NSTAGE;
                 ok = wait_bar_warp(ctx, P_READY + 2 * t + (i & 1), (i >> 1) & 1);
                 if (ok) ok = wait_bar_warp(ctx, V_FULL + s, it & 1);
                 if (!ok) break;
@@ -484,13 +496,13 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                 // rows of V = 2 KiB per k-step, MN-major (64-column boxes HALF_BYTES apart = LBO, 8-row groups
                 // 1 KiB apart = SBO).
                 const uint32_t p_tmem = s_tmem + (uint32_t)(i & 1) * BH;
-                const uint32_t vb = v_lo + (uint32_t)s * (TILE_BYTES >> 4) + (uint32_t)(i & 1) * ((BH * 128) >> 4);
+                const uint32_t vb = v_lo + (uint32_t)s * (TILE_BYTES >> 4) + half_of(i) * ((BH * 128) >> 4);
                 mma_ts2(o_tmem, p_tmem, vb, IdescPV<HD>::value, i > 0);
 #pragma unroll
                 for (int ks = 1; ks < BH / 16; ++ks)
                     mma_ts2(o_tmem, p_tmem + ks * 8, vb + (uint32_t)ks * (2048 >> 4), IdescPV<HD>::value, 1u);
                 mma_commit(bar(O_DONE + t));
-                if ((i & 1) || i + 1 >= nh) release(V_EMPTY + s, j);
+                if (last_of(i)) release(V_EMPTY + s, j);
                 if (i + 2 < nh) ok = issue_qk(i + 2);   // reuses buffer i & 1: in order after PV(t, i)
             }
         }
@@ -520,10 +532,9 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         reg_inc<REGS_SOFTMAX>();
         const int t = (warp - WARP_SOFTMAX0) >> 2;  // query tile of this warpgroup
         const int row = tid & 127;                 // TMEM lane == query row of the tile
-        const int qt0 = q0 + t * BM;
+        const int qt0 = SPLIT ? q0 : q0 + t * BM;
         const int row_g = qt0 + row;
-        const int n = n_kt[t];
-        if (n == 0) {
+        if (!SPLIT && n_kt[t] == 0) {
             // every row of this tile is padding: zeros (rows inside the tensor only)
             if (row_g < S) {
                 uint32_t z[32];
@@ -536,7 +547,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
             const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
             const uint32_t s_addr = lane_addr + (uint32_t)t * TMEM_TILE, o_addr = s_addr + TMEM_O;
             bool ok = true;
-            if (use_rope) {   // this warpgroup rotates its own Q tile
+            if (use_rope && !(SPLIT && t)) {   // this warpgroup rotates its own Q tile
                 RopeState st;
                 rope_init<HD>(st, a.rope, S, a.rope_mode, row);
                 const RopeStart start = rope_load_start<HD>(qt0, S, a.rope, a.rope_mode, row);
@@ -556,7 +567,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
             const int nc = min(n_half[0], n_half[1]);
             if (t == 1 && nc > 0) mbar_arrive(bar(EXP_TURN + 0));   // tile 0 goes first
             for (int i = 0; i < nh && ok; ++i) {
-                const int bf = i & 1, k0 = i * BH;
+                const int bf = i & 1, k0 = SPLIT ? i * BN + t * BH : i * BH;
                 ok = wait_bar_warp(ctx, S_FULL + 2 * t + bf, (i >> 1) & 1);
                 if (!ok) break;
                 tc_fence_after();
@@ -636,33 +647,70 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                 tc_fence_before();
                 mbar_arrive(bar(P_READY + 2 * t + bf));
             }
-            const int n = nh;
-            if (ok) ok = wait_bar_warp(ctx, O_DONE + t, (n - 1) & 1);
+            if (ok && (!SPLIT || nh > 0)) ok = wait_bar_warp(ctx, O_DONE + t, (nh - 1) & 1);
+            float2 other = make_float2(0.f, 0.f);     // the other half's row maximum and sum
+            if constexpr (SPLIT) {
+                float2* ml = reinterpret_cast<float2*>(smem + SMEM_ML);
+                ml[t * BM + row] = make_float2(m_ref, l);
+                tc_fence_before();
+                asm volatile("bar.sync 1, 256;" ::: "memory");     // both accumulators are final (or *abort is set)
+                other = ml[(t ^ 1) * BM + row];
+                ok = ok && !*ctx.abort;
+            }
             if (ok) {
                 tc_fence_after();
+                float mine = 1.f, theirs = 0.f;
+                if constexpr (SPLIT) {
+                    const float m = l > 0.f ? (other.y > 0.f ? fmaxf(m_ref, other.x) : m_ref) : other.x;
+                    mine = l > 0.f ? ex2(m_ref - m) : 0.f;
+                    theirs = other.y > 0.f ? ex2(other.x - m) : 0.f;
+                    l = l * mine + other.y * theirs;
+                }
                 const bool zero = (row_g >= len) || !(l > 0.f);
-                const float inv = zero ? 0.f : 1.f / l;
+                const float inv = zero ? 0.f : SPLIT ? mine / l : 1.f / l, inv_other = zero ? 0.f : theirs / l;
+                // 32 columns of the accumulator; in the split form those of both, weighted
+                auto load_o = [&](int col, uint32_t (&orow)[32]) {
+                    if constexpr (SPLIT) {
+                        uint32_t more[32];
+                        const uint32_t o0 = lane_addr + TMEM_O;
+                        const float w0 = t ? inv_other : inv, w1 = t ? inv : inv_other;
+                        tmem_ld_x32_sync(o0 + col, orow);
+                        if (n_half[1] > 0) {
+                            tmem_ld_x32_sync(o0 + TMEM_TILE + col, more);
+#pragma unroll
+                            for (int e = 0; e < 32; ++e)
+                                orow[e] = __float_as_uint(fmaf(__uint_as_float(more[e]), w1, __uint_as_float(orow[e]) * w0));
+                        } else {
+#pragma unroll
+                            for (int e = 0; e < 32; ++e) orow[e] = __float_as_uint(__uint_as_float(orow[e]) * w0);
+                        }
+                    } else {
+                        tmem_ld_x32_sync(o_addr + col, orow);
+                    }
+                };
+                const float f = SPLIT ? 1.f : inv;
                 if constexpr (sizeof(TOut) == 4) {
                     // Each thread holds one 512-byte output row; written directly, a warp store would touch 32
                     // rows.  Transpose through shared memory instead (this tile's Q buffer is dead: all of its
-                    // QK^T have completed): 32 rows x 64 columns per pass, 16-byte chunks XOR-swizzled by row, then
+                    // QK^T have completed; in the split form, where both tiles are final, the K ring): 32 rows x 64 columns per pass, 16-byte chunks XOR-swizzled by row, then
                     // every warp store writes 256 contiguous bytes of one row.
-                    const uint32_t stage = base_addr + SMEM_Q + t * TILE_BYTES + (warp & 3) * 8192;
+                    const uint32_t stage = base_addr + (SPLIT ? SMEM_K : SMEM_Q) + t * TILE_BYTES + (warp & 3) * 8192;
                     const int row_w0 = qt0 + (warp & 3) * 32;
 #pragma unroll
                     for (int pass = 0; pass < HD / 64; ++pass) {
+                        if (SPLIT && pass != t) continue;
 #pragma unroll
                         for (int ch = 0; ch < 2; ++ch) {
                             uint32_t orow[32];
-                            tmem_ld_x32_sync(o_addr + pass * 64 + ch * 32, orow);
+                            load_o(pass * 64 + ch * 32, orow);
 #pragma unroll
                             for (int c = 0; c < 8; ++c) {
                                 const int chunk = ch * 8 + c;
                                 sts128(stage + lane * 256 + ((chunk ^ (lane & 15)) << 4),
-                                       make_uint4(__float_as_uint(__uint_as_float(orow[4 * c]) * inv),
-                                                  __float_as_uint(__uint_as_float(orow[4 * c + 1]) * inv),
-                                                  __float_as_uint(__uint_as_float(orow[4 * c + 2]) * inv),
-                                                  __float_as_uint(__uint_as_float(orow[4 * c + 3]) * inv)));
+                                       make_uint4(__float_as_uint(__uint_as_float(orow[4 * c]) * f),
+                                                  __float_as_uint(__uint_as_float(orow[4 * c + 1]) * f),
+                                                  __float_as_uint(__uint_as_float(orow[4 * c + 2]) * f),
+                                                  __float_as_uint(__uint_as_float(orow[4 * c + 3]) * f)));
                             }
                         }
                         __syncwarp();
@@ -677,9 +725,10 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                 } else {
 #pragma unroll
                     for (int ch = 0; ch < HD / 32; ++ch) {
+                        if (SPLIT && ch / 2 != t) continue;
                         uint32_t orow[32];
-                        tmem_ld_x32_sync(o_addr + ch * 32, orow);   // warp-collective: no divergence here
-                        if (row_g < S) store_row_chunk<TOut>(O + (size_t)row_g * HD + ch * 32, orow, inv);
+                        load_o(ch * 32, orow);   // warp-collective: no divergence here
+                        if (row_g < S) store_row_chunk<TOut>(O + (size_t)row_g * HD + ch * 32, orow, f);
                     }
                 }
             }
@@ -729,20 +778,25 @@ int flash_fwd_sm100(grl_device* dev, const grl_flash_params* p, float scale, con
     a.causal = p->causal; a.rope_mode = p->rope_mode;
     a.scale_log2 = scale * 1.4426950408889634f;
     a.wait_limit = dev->wait_limit_cycles;
-    a.n_qp = (p->seq_len + NQ * BM - 1) / (NQ * BM);
+    const int n_qt = (p->seq_len + BM - 1) / BM;
+    // One tile a CTA while that is one wave: a second wave would cost what the shorter chains save, and every tile of its own
+    // loads and rotates K again.
+    const bool split = (long long)BH * n_qt <= dev->prop.multiProcessorCount;
+    a.n_qp = split ? n_qt : (n_qt + NQ - 1) / NQ;
     dim3 grid((unsigned)BH * a.n_qp);
+    using Kernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, Args);
+    static const Kernel kernels[2][2][2] = {     // [head_dim 128][float32 out][split]
+        {{flash_fwd_sm100_kernel<__nv_bfloat16, 64, false>, flash_fwd_sm100_kernel<__nv_bfloat16, 64, true>},
+         {flash_fwd_sm100_kernel<float, 64, false>, flash_fwd_sm100_kernel<float, 64, true>}},
+        {{flash_fwd_sm100_kernel<__nv_bfloat16, 128, false>, flash_fwd_sm100_kernel<__nv_bfloat16, 128, true>},
+         {flash_fwd_sm100_kernel<float, 128, false>, flash_fwd_sm100_kernel<float, 128, true>}}};
     static bool attr_set[64] = {};
     if (!attr_set[dev->ordinal & 63]) {      // a function attribute belongs to the device that was current
-        GRL_CUDA(cudaFuncSetAttribute(flash_fwd_sm100_kernel<float, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_TOTAL));
-        GRL_CUDA(cudaFuncSetAttribute(flash_fwd_sm100_kernel<__nv_bfloat16, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_TOTAL));
-        GRL_CUDA(cudaFuncSetAttribute(flash_fwd_sm100_kernel<float, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_TOTAL));
-        GRL_CUDA(cudaFuncSetAttribute(flash_fwd_sm100_kernel<__nv_bfloat16, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_TOTAL));
+        for (int i = 0; i < 8; ++i)
+            GRL_CUDA(cudaFuncSetAttribute(kernels[i >> 2][(i >> 1) & 1][i & 1], cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_TOTAL));
         attr_set[dev->ordinal & 63] = true;
     }
-    const bool f32 = p->out_dtype == GRL_F32;
-    auto kernel = HD == 128 ? (f32 ? flash_fwd_sm100_kernel<float, 128> : flash_fwd_sm100_kernel<__nv_bfloat16, 128>)
-                            : (f32 ? flash_fwd_sm100_kernel<float, 64> : flash_fwd_sm100_kernel<__nv_bfloat16, 64>);
-    GRL_CUDA(launch_pdl(kernel, grid, kThreads, SMEM_TOTAL, dev->stream, tq, tk, tv, a));
+    GRL_CUDA(launch_pdl(kernels[HD == 128][p->out_dtype == GRL_F32][split], grid, kThreads, SMEM_TOTAL, dev->stream, tq, tk, tv, a));
     GRL_LAUNCHED("flash_fwd_sm100_kernel");
     return GRL_OK;
 }

@@ -330,3 +330,27 @@ def test_fp32_kernel_tile_edges(gpu, B, H, S, D, causal, rope, lens, kind):
     for b in range(B if lens else 0):
         want[b, :, lens[b]:] = 0.0
     assert np.abs(gpu.flash_attention2(Q, K, V, **kw) - want).max() <= TOL_F32
+
+
+@pytest.mark.parametrize("B,H,S,D,causal,rope,lens", [
+    (1, 2, 1, 128, True, "half", None), (1, 3, 64, 128, False, "interleaved", None), (2, 2, 65, 64, True, "none", None),  # one tile a CTA
+    (1, 2, 129, 128, True, "half", None), (2, 3, 700, 128, False, "interleaved", (65, 700)), (3, 1, 1000, 64, True, "half", (1000, 129, 64)),
+    (1, 37, 512, 128, True, "interleaved", None), (1, 37, 513, 128, True, "half", None),                                 # 148 and 185 tiles
+    (3, 50, 65, 64, False, "none", (65, 64, 1)), (2, 40, 333, 128, True, "half", (333, 129))])                           # pairs of tiles
+def test_tcgen05_kernel_tile_edges(dev, B, H, S, D, causal, rope, lens):
+    from grilly_next import cabi
+    from gpu_helpers import flash_cabi
+    rng = np.random.default_rng(S + D)
+    Q, K, V = (rng.standard_normal((B, H, S, D), dtype=np.float32) for _ in range(3))
+    q, k, mode = Q, K, cabi.ROPE_NONE
+    if rope == "interleaved":
+        q, k, mode = orc.rope_interleaved(Q, np.arange(S)), orc.rope_interleaved(K, np.arange(S)), cabi.ROPE_INTERLEAVED
+    elif rope == "half":
+        q, k = (orc.rope_half(t.transpose(0, 2, 1, 3)).transpose(0, 2, 1, 3) for t in (Q, K))
+        mode = cabi.ROPE_HALF
+    want = orc.attention_4d(q, k, V, mask=orc.causal_length_mask(B, H, S, lens, causal))
+    for b in range(B if lens else 0):
+        want[b, :, lens[b]:] = 0.0
+    kw = dict(causal=causal, seq_lens=None if lens is None else np.array(lens, np.int32), rope_mode=mode, bf16=True, kernel=cabi.KERNEL_TCGEN05)
+    assert np.abs(flash_cabi(dev, Q, K, V, **kw) - want).max() <= TOL_BF16
+    assert np.abs(flash_cabi(dev, Q, K, V, out_bf16=True, **kw) - want).max() <= 3e-2
