@@ -6,6 +6,8 @@
 // softmax backward; grad_Q, grad_K).  The fused kernels are the fast path; these exist so that code written against
 // the separate shaders keeps working, and so that training code has a backward.  Every product is a batched float32
 // product of sgemm.cuh with the sum over the inner index in ascending order, as the shaders' loops run.
+#include <type_traits>
+
 #include "common.cuh"
 #include "sgemm.cuh"
 
@@ -131,18 +133,23 @@ __global__ void __launch_bounds__(SH::THREADS, GradAttn<SH>::MIN_CTAS) grad_attn
 }
 
 // blockIdx.z < batch * H: grad_Q[i][d] = scale sum_j gS[i][j] K[j][d]; the other half: grad_K[j][d] = scale sum_i gS[i][j] Q[i][d].
-template <typename SH>
-__global__ void __launch_bounds__(SH::THREADS, SH::MIN_CTAS) grad_qk_kernel(const float* __restrict__ attn, const float* __restrict__ ga,
-                                                              const float* __restrict__ q, const float* __restrict__ k,
-                                                              const float* __restrict__ parts, int n_parts, float* gq, float* gk, int S,
-                                                              int D, int n_bh, int vec_s, int vec_d, float scale) {
+// SPLIT: the K range over four thread groups (see sgemm::split_tile).
+template <typename SH, bool SPLIT> struct GradQK {
+    static constexpr int THREADS = SPLIT ? sgemm::Split<SH>::THREADS : SH::THREADS;
+    static constexpr int MIN_CTAS = SPLIT ? sgemm::Split<SH>::MIN_CTAS : SH::MIN_CTAS;
+    static constexpr int TILES = SPLIT ? sgemm::Split<SH>::SMEM / 4 : 2 * SH::TILE;      // floats
+};
+template <typename SH, bool SPLIT>
+__global__ void __launch_bounds__(GradQK<SH, SPLIT>::THREADS, GradQK<SH, SPLIT>::MIN_CTAS)
+grad_qk_kernel(const float* __restrict__ attn, const float* __restrict__ ga, const float* __restrict__ q, const float* __restrict__ k,
+               const float* __restrict__ parts, int n_parts, float* gq, float* gk, int S, int D, int n_bh, int vec_s, int vec_d, float scale) {
     extern __shared__ __align__(16) float dyn[];      // two tile stages, then the row sums of this head
-    float* dots = dyn + 2 * SH::TILE;
+    float* dots = dyn + GradQK<SH, SPLIT>::TILES;
     const bool is_q = (int)blockIdx.z < n_bh;
     const int z = is_q ? blockIdx.z : blockIdx.z - n_bh;
     const int m0 = blockIdx.y * SH::BM, n0 = blockIdx.x * SH::BN;
     const int d0 = is_q ? m0 : 0, d1 = is_q ? min(S, m0 + SH::BM) : S;          // rows whose sums this CTA needs
-    for (int i = d0 + threadIdx.x; i < d1; i += SH::THREADS) {
+    for (int i = d0 + threadIdx.x; i < d1; i += GradQK<SH, SPLIT>::THREADS) {
         const float* p = parts + ((size_t)z * S + i) * D;
         float dot = 0.f;
         for (int j = 0; j < n_parts; ++j) dot += __ldg(p + j);
@@ -152,6 +159,12 @@ __global__ void __launch_bounds__(SH::THREADS, SH::MIN_CTAS) grad_qk_kernel(cons
     pdl_trigger();      // the row sums are read: the grad_V product, which overwrites them, may take the idle SMs
     const size_t so = (size_t)z * S * S, to = (size_t)z * S * D;
     const Operand A{ga + so, 0, 0, S, vec_s}, B{(is_q ? k : q) + to, 0, 0, D, vec_d};
+    if constexpr (SPLIT) {
+        float* c = (is_q ? gq : gk) + to;
+        if (is_q) sgemm::split_tile<SH, true, false, true>(dyn, A.base, A, B.base, B, c, D, nullptr, m0, n0, S, D, S, scale, attn + so, dots - m0);
+        else sgemm::split_tile<SH, false, false, true>(dyn, A.base, A, B.base, B, c, D, nullptr, m0, n0, S, D, S, scale, attn + so, dots);
+        return;
+    }
     float2 acc[8][4];
     if (is_q) sgemm::mainloop<SH, true, false, false, true>(acc, dyn, A.base, A, B.base, B, m0, n0, S, D, S, attn + so, dots - m0);
     else sgemm::mainloop<SH, false, false, false, true>(acc, dyn, A.base, A, B.base, B, m0, n0, S, D, S, attn + so, dots);
@@ -168,15 +181,16 @@ static int launch_grad_attn(grl_device* dev, const Operand& go, const Operand& v
     return GRL_OK;
 }
 
-template <typename SH>
+template <typename SH, bool SPLIT>
 static int launch_grad_qk(grl_device* dev, const float* attn, const float* ga, const float* q, const float* k, const float* parts,
                           int n_parts, float* gq, float* gk, int S, int D, int n_bh, float scale) {
-    const size_t smem = (2 * SH::TILE + (size_t)S) * sizeof(float);
-    GRL_CUDA(cudaFuncSetAttribute(grad_qk_kernel<SH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * SH::TILE + kMaxDotRows) * 4));
+    const size_t smem = (GradQK<SH, SPLIT>::TILES + (size_t)S) * sizeof(float);
+    GRL_CUDA(cudaFuncSetAttribute(grad_qk_kernel<SH, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (GradQK<SH, SPLIT>::TILES + kMaxDotRows) * 4));
     const int vec_s = S % 4 == 0 && (uintptr_t)attn % 16 == 0 && (uintptr_t)ga % 16 == 0;
     const int vec_d = D % 4 == 0 && (uintptr_t)q % 16 == 0 && (uintptr_t)k % 16 == 0;
     dim3 grid((D + SH::BN - 1) / SH::BN, (S + SH::BM - 1) / SH::BM, 2 * n_bh);
-    grad_qk_kernel<SH><<<grid, SH::THREADS, smem, dev->stream>>>(attn, ga, q, k, parts, n_parts, gq, gk, S, D, n_bh, vec_s, vec_d, scale);
+    grad_qk_kernel<SH, SPLIT><<<grid, GradQK<SH, SPLIT>::THREADS, smem, dev->stream>>>(attn, ga, q, k, parts, n_parts, gq, gk, S, D, n_bh, vec_s, vec_d, scale);
     GRL_LAUNCHED("grad_qk_kernel");
     return GRL_OK;
 }
@@ -248,13 +262,14 @@ int grl_attention_backward(grl_device* dev, const float* grad_out, const float* 
         rc = wide ? launch_grad_attn<sgemm::Shape<128, 128>>(dev, go_rows, v_rows, g_attn, attn, grad_v, seq_len, head_dim, batch, heads)
                   : launch_grad_attn<sgemm::Shape<64, 64>>(dev, go_rows, v_rows, g_attn, attn, grad_v, seq_len, head_dim, batch, heads);
         if (rc) return rc;
-        auto qk = [&](auto shape) {
-            return launch_grad_qk<decltype(shape)>(dev, attn, scratch, q, k, grad_v, n_parts, grad_q, grad_k, seq_len, head_dim, n_bh, scale);
+        auto qk = [&](auto shape, auto split) {
+            return launch_grad_qk<decltype(shape), decltype(split)::value>(dev, attn, scratch, q, k, grad_v, n_parts, grad_q, grad_k, seq_len, head_dim, n_bh, scale);
         };
         const int tile = sgemm::tile_rows(seq_len, head_dim, 3 * n_bh, 64, sms);    // the grad_V product runs beside these two
-        if (head_dim <= 32) rc = qk(sgemm::Shape<64, 32>());
-        else if (tile == 128) rc = qk(sgemm::Shape<128, 64>());
-        else rc = qk(sgemm::Shape<64, 64>());
+        const bool split = sgemm::split_pays(seq_len);
+        if (head_dim <= 32) rc = split ? qk(sgemm::Shape<64, 32>(), std::true_type()) : qk(sgemm::Shape<64, 32>(), std::false_type());
+        else if (tile == 128) rc = qk(sgemm::Shape<128, 64>(), std::false_type());
+        else rc = split ? qk(sgemm::Shape<64, 64>(), std::true_type()) : qk(sgemm::Shape<64, 64>(), std::false_type());
         if (rc) return rc;
         // grad_V[j][d] = sum_i attn[i][j] gO[i][d]
         return sgemm::launch<false, false, false, true>(dev, operand(attn, ab, ah, S), go_rows, Output{grad_v, qb, qh, D}, nullptr, seq_len,

@@ -221,21 +221,28 @@ __global__ void __launch_bounds__(SH::THREADS, SH::MIN_CTAS) kernel(Operand A, O
 
 // 64 x 64 tiles with the K range cut over four groups of threads, whose partial tiles are added in ascending order.  One group
 // alone is two warps an SM where there is one tile for each: the chain of load, barrier and products of a slice is the time
-// then (128 x 768 x 3072: 64 us), and it is four times shorter this way.
+// then (128 x 768 x 3072: 64 us), and it is four times shorter this way.  Backward, us, whole / split: 1 x 4 heads x 1024 x 64 140 / 86,
+// 2 x 12 x 512 x 64 164 / 102, 1 x 8 x 256 x 64 41 / 25, 1 x 4 x 700 x 32 129 / 47.
 constexpr int kSplit = 4;
-template <typename SH, bool AKC, bool BKC>
-__global__ void __launch_bounds__(SH::THREADS * kSplit) split_kernel(Operand A, Operand B, Output C, const float* bias, int M, int N, int K,
-                                                                     int H, float alpha) {
-    extern __shared__ __align__(16) float dyn[];
-    constexpr int REGION = 2 * SH::TILE;
+template <typename SH> struct Split {
+    static constexpr int REGION = 2 * SH::TILE;         // floats a group has
+    static constexpr int THREADS = SH::THREADS * kSplit, SMEM = kSplit * REGION * (int)sizeof(float);
+    static constexpr int MIN_CTAS = THREADS > 128 ? 1 : 2;      // eight warps an SM with every register they ask for (32 columns at 168
+                                                                // registers spilled: 84 us for 47 of the last figure above)
+};
+// One tile; operands, `pair` and `dots` as in mainloop, all of this batch.
+template <typename SH, bool AKC, bool BKC, bool PAIR>
+__device__ __forceinline__ void split_tile(float* dyn, const float* a0, const Operand& A, const float* b0, const Operand& B, float* c, long long ldc,
+                                           const float* bias, int m0, int n0, int M, int N, int K, float alpha, const float* pair,
+                                           const float* dots) {
+    constexpr int REGION = Split<SH>::REGION;
     static_assert(REGION >= SH::THREADS * 64, "a partial tile reuses its group's stages");
-    const int z = blockIdx.z, b = z / H, h = z % H, g = threadIdx.x / SH::THREADS, tid = threadIdx.x % SH::THREADS;
-    const int m0 = blockIdx.y * SH::BM, n0 = blockIdx.x * SH::BN;
+    const int g = threadIdx.x / SH::THREADS, tid = threadIdx.x % SH::THREADS;
     const int slices = (K + BK - 1) / BK, k0 = g * slices / kSplit * BK, k1 = min(K, (g + 1) * slices / kSplit * BK);
-    const float* a = A.base + b * A.sb + h * A.sh + (AKC ? k0 : k0 * A.ld);
-    const float* bb = B.base + b * B.sb + h * B.sh + (BKC ? k0 : k0 * B.ld);
+    const long long ka = AKC ? k0 : k0 * A.ld;
     float2 acc[8][4];
-    mainloop<SH, AKC, BKC, false, false, kSplit>(acc, dyn + g * REGION, a, A, bb, B, m0, n0, M, N, k1 - k0, nullptr, nullptr);
+    mainloop<SH, AKC, BKC, false, PAIR, kSplit>(acc, dyn + g * REGION, a0 + ka, A, b0 + (BKC ? k0 : k0 * B.ld), B, m0, n0, M, N, k1 - k0,
+                                                PAIR ? pair + ka : nullptr, PAIR && !AKC ? dots + k0 : dots);
     float2* mine = reinterpret_cast<float2*>(dyn + g * REGION) + tid;
 #pragma unroll
     for (int i = 0; i < 8; ++i)
@@ -244,8 +251,7 @@ __global__ void __launch_bounds__(SH::THREADS * kSplit) split_kernel(Operand A, 
     __syncthreads();
     // group g finishes rows 2g and 2g + 1 of every thread's eight
     const Place<SH> at(tid);
-    float* c = C.base + b * C.sb + h * C.sh;
-    const bool vec = ((uintptr_t)c % 16 == 0) && C.ld % 4 == 0;
+    const bool vec = ((uintptr_t)c % 16 == 0) && ldc % 4 == 0;
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
         const int i = 2 * g + q, m = m0 + at.row(i);
@@ -261,9 +267,19 @@ __global__ void __launch_bounds__(SH::THREADS * kSplit) split_kernel(Operand A, 
                 y = __fadd2_rn(y, part[(i * 4 + 2 * hh + 1) * SH::THREADS]);
             }
             const float4 bv = bias ? load4(bias, n, N, (uintptr_t)bias % 16 == 0) : make_float4(0.f, 0.f, 0.f, 0.f);
-            store4(c + (long long)m * C.ld + n, make_float4(x.x * alpha + bv.x, x.y * alpha + bv.y, y.x * alpha + bv.z, y.y * alpha + bv.w), N - n, vec);
+            store4(c + (long long)m * ldc + n, make_float4(x.x * alpha + bv.x, x.y * alpha + bv.y, y.x * alpha + bv.z, y.y * alpha + bv.w), N - n, vec);
         }
     }
+}
+
+template <typename SH, bool AKC, bool BKC, bool EARLY>
+__global__ void __launch_bounds__(Split<SH>::THREADS, Split<SH>::MIN_CTAS)
+split_kernel(Operand A, Operand B, Output C, const float* bias, int M, int N, int K, int H, float alpha) {
+    extern __shared__ __align__(16) float dyn[];
+    const int z = blockIdx.z, b = z / H, h = z % H;
+    split_tile<SH, AKC, BKC, false>(dyn, A.base + b * A.sb + h * A.sh, A, B.base + b * B.sb + h * B.sh, B, C.base + b * C.sb + h * C.sh, C.ld, bias,
+                                    blockIdx.y * SH::BM, blockIdx.x * SH::BN, M, N, K, alpha, nullptr, nullptr);
+    if constexpr (EARLY) pdl_wait();
 }
 
 // Which tile: the widest one whose grid still gives every SM two CTAs; 64 rows otherwise, so that a small product
@@ -273,32 +289,36 @@ inline int tile_rows(int M, int N, int batch, int bn, int sms) {
     return big >= 2LL * sms ? 128 : 64;
 }
 
+// One slice a group suffices: backward of 4 x 12 heads x 128 x 128 53.5 us whole, 41.2 split; 1 x 1 x 64 x 64 22.7 and 17.5.
+inline bool split_pays(int K) { return K >= kSplit * BK; }
+
 // EARLY: the launch starts under the kernel before it on the stream, of which it needs nothing but the end (see launch_pdl).
 template <bool AKC, bool BKC, bool CAUSAL = false, bool EARLY = false>
 int launch(grl_device* dev, const Operand& A, const Operand& B, const Output& C, const float* bias, int M, int N, int K, int batch,
            int H, float alpha, const char* name, int rows_hint = 0) {
+    cudaError_t err = cudaSuccess;
     auto go = [&](auto shape) {
         using SH = decltype(shape);
         dim3 grid((N + SH::BN - 1) / SH::BN, (M + SH::BM - 1) / SH::BM, batch * H);
-        if constexpr (EARLY) launch_pdl(kernel<SH, AKC, BKC, CAUSAL, true>, grid, SH::THREADS, 0, dev->stream, A, B, C, bias, M, N, K, H, alpha);
+        if constexpr (EARLY) err = launch_pdl(kernel<SH, AKC, BKC, CAUSAL, true>, grid, SH::THREADS, 0, dev->stream, A, B, C, bias, M, N, K, H, alpha);
         else kernel<SH, AKC, BKC, CAUSAL, false><<<grid, SH::THREADS, 0, dev->stream>>>(A, B, C, bias, M, N, K, H, alpha);
     };
-    const int sms = dev->prop.multiProcessorCount;
-    if (N <= 32) {
-        go(Shape<64, 32>());
-    } else if (N > 64 && !rows_hint && tile_rows(M, N, batch * H, 128, sms) == 128) {
-        go(Shape<128, 128>());
-    } else if ((rows_hint ? rows_hint : tile_rows(M, N, batch * H, 64, sms)) == 128) {
-        go(Shape<128, 64>());
-    } else if (!CAUSAL && !EARLY && K >= 16 * BK) {
-        using SH = Shape<64, 64>;
-        constexpr int smem = kSplit * 2 * SH::TILE * (int)sizeof(float);
-        GRL_CUDA(cudaFuncSetAttribute(split_kernel<SH, AKC, BKC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    auto go_small = [&](auto shape) {
+        using SH = decltype(shape);
+        if (CAUSAL || !split_pays(K)) return go(shape);
+        auto kern = split_kernel<SH, AKC, BKC, EARLY>;
+        err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Split<SH>::SMEM);
+        if (err) return;
         dim3 grid((N + SH::BN - 1) / SH::BN, (M + SH::BM - 1) / SH::BM, batch * H);
-        split_kernel<SH, AKC, BKC><<<grid, SH::THREADS * kSplit, smem, dev->stream>>>(A, B, C, bias, M, N, K, H, alpha);
-    } else {
-        go(Shape<64, 64>());
-    }
+        if constexpr (EARLY) err = launch_pdl(kern, grid, Split<SH>::THREADS, Split<SH>::SMEM, dev->stream, A, B, C, bias, M, N, K, H, alpha);
+        else kern<<<grid, Split<SH>::THREADS, Split<SH>::SMEM, dev->stream>>>(A, B, C, bias, M, N, K, H, alpha);
+    };
+    const int sms = dev->prop.multiProcessorCount;
+    if (N <= 32) go_small(Shape<64, 32>());
+    else if (N > 64 && !rows_hint && tile_rows(M, N, batch * H, 128, sms) == 128) go(Shape<128, 128>());
+    else if ((rows_hint ? rows_hint : tile_rows(M, N, batch * H, 64, sms)) == 128) go(Shape<128, 64>());
+    else go_small(Shape<64, 64>());
+    GRL_CUDA(err);
     GRL_LAUNCHED(name);
     return GRL_OK;
 }

@@ -109,6 +109,7 @@ def test_argument_errors(gpu):
 
 @pytest.mark.parametrize("B,H,S,D", [
     (1, 1, 1, 8), (1, 2, 65, 32), (3, 8, 129, 64),      # one row; 64-row tiles and their remainders
+    (2, 2, 63, 64), (1, 2, 64, 40), (1, 3, 100, 32),    # around the length from which four groups share the k range
     (1, 3, 70, 33), (1, 1, 600, 8),                     # rows off 16-byte boundaries; more tiles a row than head_dim
     (8, 40, 130, 64), (4, 40, 256, 96)])                # 128-row tiles, two tiles of columns
 def test_backward_tile_edges(gpu, B, H, S, D):

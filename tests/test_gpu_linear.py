@@ -77,7 +77,7 @@ def test_fused_qkv_projection_feeds_attention(gpu):
 
 
 @pytest.mark.parametrize("M,K,N", [(1, 4, 1), (2, 131, 9), (8, 132, 300), (9, 17, 65), (64, 33, 32), (130, 40, 2500), (2100, 70, 1025),
-                                   (200, 300, 3001), (70, 1031, 4500)])     # K cut over four groups of threads
+                                   (200, 300, 3001), (70, 1031, 4500), (2400, 64, 30), (300, 127, 2000)])     # K cut over four groups of threads
 def test_linear_fp32_tile_edges(gpu, M, K, N):
     rng = np.random.default_rng(M + K + N)
     x, w = rng.standard_normal((M, K), dtype=np.float32), rng.standard_normal((N, K), dtype=np.float32)
