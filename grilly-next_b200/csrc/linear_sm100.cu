@@ -206,25 +206,31 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
 #pragma unroll
                     for (int e = 0; e < 32; ++e) r[e] = __float_as_uint(__uint_as_float(r[e]) + __shfl_sync(0xffffffffu, bl, e));
                 }
-                if (a.tma_store) {
-                    // 32 rows x 128 bytes under the 128-byte swizzle, two boxes in turn
-                    const uint32_t box = stage + (uint32_t)(c & 1) * 4096u;
-                    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-                    __syncwarp();
+                // 32 rows x 128 bytes under the 128-byte swizzle, two boxes in turn
+                const uint32_t box = stage + (uint32_t)(c & 1) * 4096u;
+                if (a.tma_store && lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+                __syncwarp();
 #pragma unroll
-                    for (int q = 0; q < 8; ++q)
-                        sts128(box + lane * 128 + ((q ^ (lane & 7)) << 4), make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]));
+                for (int q = 0; q < 8; ++q)
+                    sts128(box + lane * 128 + ((q ^ (lane & 7)) << 4), make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]));
+                if (a.tma_store) {
                     fence_async_smem();
                     __syncwarp();
                     if (lane == 0) {
                         tma_store_2d(&tmY, box, col, row0);
                         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                     }
-                } else if (row0 + lane < a.M) {
-                    float* dst = a.y + (size_t)(row0 + lane) * a.N + col;
-#pragma unroll
-                    for (int e = 0; e < 32; ++e)
-                        if (col + e < a.N) dst[e] = __uint_as_float(r[e]);
+                } else {       // rows of y off 16-byte boundaries: the warp stores 32 consecutive floats of one row at a time
+                    __syncwarp();
+                    const int rows = min(32, a.M - row0);
+                    float* dst = a.y + (size_t)row0 * a.N + col + lane;
+                    if (col + lane < a.N) {
+#pragma unroll 16
+                        for (int rr = 0; rr < 32; ++rr) {
+                            const float v = lds32f(box + rr * 128 + (((lane >> 2) ^ (rr & 7)) << 4) + (lane & 3) * 4);
+                            if (rr < rows) dst[(size_t)rr * a.N] = v;
+                        }
+                    }
                 }
             }
         }

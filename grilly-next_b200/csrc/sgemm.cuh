@@ -289,8 +289,8 @@ inline int tile_rows(int M, int N, int batch, int bn, int sms) {
     return big >= 2LL * sms ? 128 : 64;
 }
 
-// One slice a group suffices: backward of 4 x 12 heads x 128 x 128 53.5 us whole, 41.2 split; 1 x 1 x 64 x 64 22.7 and 17.5.
-inline bool split_pays(int K) { return K >= kSplit * BK; }
+// From two slices on: backward of 4 x 12 heads x 128 x 128 53.5 us whole, 41.2 split; 1 x 1 x 64 x 64 22.7 and 17.5.
+inline bool split_pays(int K) { return K > BK; }
 
 // EARLY: the launch starts under the kernel before it on the stream, of which it needs nothing but the end (see launch_pdl).
 template <bool AKC, bool BKC, bool CAUSAL = false, bool EARLY = false>
