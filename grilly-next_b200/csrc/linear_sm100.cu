@@ -24,6 +24,7 @@ using namespace sm100;
 
 constexpr int BK = 64;             // one 128-byte swizzle row of bf16
 constexpr int kThreads = 256;      // warp 0 TMA, warp 1 MMA, warp 2 TMEM, warp 3 idle, warps 4-7 epilogue (TMEM lanes 0..127)
+constexpr int kPairThreads = 384;  // pair kernel: warps 8-11 are epilogue as well
 constexpr int kSmemMax = 227 * 1024;
 
 struct Args {
@@ -72,13 +73,13 @@ __device__ __forceinline__ uint32_t instr_desc(int m, int n) {   // D f32, A and
 template <int BN_>
 struct Pair {
     static constexpr int BN = BN_, A_BYTES = 128 * BK * 2, B_BYTES = BN / 2 * BK * 2, STAGE = A_BYTES + B_BYTES;
-    static constexpr int OUT_BYTES = 4 * 2 * 4096;                  // a warp's two 32 x 32 float boxes on their way out
+    static constexpr int OUT_BYTES = 8 * 4096;                      // a 32 x 32 float box a warp on its way out
     static constexpr int NST = (kSmemMax - 2048 - OUT_BYTES) / STAGE;      // 6 or 8
     static constexpr int SMEM_OUT = NST * STAGE, SMEM_BAR = SMEM_OUT + OUT_BYTES, SMEM = SMEM_BAR + 256 + 1024;
 };
 
 template <int BN>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 linear_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmY,
                    const Args a) {
     using P = Pair<BN>;
@@ -105,7 +106,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmX)) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmW)) : "memory");
         for (int s = 0; s < NST; ++s) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
-        for (int i = 0; i < 2; ++i) { mbar_init(acc_full(i), 1); mbar_init(acc_empty(i), 8); }     // 4 epilogue warps of 2 CTAs
+        for (int i = 0; i < 2; ++i) { mbar_init(acc_full(i), 1); mbar_init(acc_empty(i), 16); }     // 8 epilogue warps of 2 CTAs
         *abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         fence_async_smem();
@@ -178,8 +179,10 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
         }
     } else if (warp >= 4) {
         // ------------------------------------------------------------------ epilogue: TMEM -> (+ bias) -> global
-        const int w = warp & 3;
-        const uint32_t stage = base + P::SMEM_OUT + (uint32_t)w * 8192u;
+        // Two warps take the same 32 lanes, every other 32 columns each: with one the epilogue, not the products, was the time of a
+        // tile of short K (4096 x 128 x 4097 66 us).
+        const int w = warp & 3, half = (warp - 4) >> 2;
+        const uint32_t box = base + P::SMEM_OUT + (uint32_t)(warp - 4) * 4096u;
         int n = 0;
         for (int t = pair; t < tiles; t += pairs, ++n) {
             const int acc = n & 1;
@@ -191,11 +194,11 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
             const int row0 = tm * 256 + (int)rank * 128 + w * 32;
             const uint32_t t_addr = tmem + (uint32_t)acc * 256u + ((uint32_t)(w * 32) << 16);
 #pragma unroll 1
-            for (int c = 0; c < BN / 32; ++c) {
+            for (int c = half; c < BN / 32; c += 2) {
                 uint32_t r[32];
                 tmem_ld_x32_sync(t_addr + c * 32, r);
                 const int col = tn * BN + c * 32;
-                if (c == BN / 32 - 1) {        // the last read of this accumulator: the next tile's products may overwrite it
+                if (c + 2 >= BN / 32) {        // this warp's last read of this accumulator: the next tile's products may overwrite it
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive_cluster(cluster_map(acc_empty(acc), 0));
@@ -206,9 +209,8 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
 #pragma unroll
                     for (int e = 0; e < 32; ++e) r[e] = __float_as_uint(__uint_as_float(r[e]) + __shfl_sync(0xffffffffu, bl, e));
                 }
-                // 32 rows x 128 bytes under the 128-byte swizzle, two boxes in turn
-                const uint32_t box = stage + (uint32_t)(c & 1) * 4096u;
-                if (a.tma_store && lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+                // 32 rows x 128 bytes under the 128-byte swizzle
+                if (a.tma_store && lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
                 __syncwarp();
 #pragma unroll
                 for (int q = 0; q < 8; ++q)
@@ -464,7 +466,7 @@ static int launch_pair(grl_device* dev, const void* x, const void* w, Args a) {
         attr_set[dev->ordinal & 63] = true;
     }
     const int tiles = (a.M + 255) / 256 * ((a.N + BN - 1) / BN), pairs = dev->prop.multiProcessorCount / 2;
-    GRL_CUDA(launch_pdl(linear_pair_kernel<BN>, 2 * (tiles < pairs ? tiles : pairs), kThreads, P::SMEM, dev->stream, tx, tw, ty, a));
+    GRL_CUDA(launch_pdl(linear_pair_kernel<BN>, 2 * (tiles < pairs ? tiles : pairs), kPairThreads, P::SMEM, dev->stream, tx, tw, ty, a));
     GRL_LAUNCHED("linear_pair_kernel");
     return GRL_OK;
 }
