@@ -90,6 +90,7 @@ def test_linear_fp32_tile_edges(gpu, M, K, N):
     (1, 8, 1), (3, 4096, 300), (17, 520, 128), (250, 1032, 129),     # split over a cluster, and too short to split
     (300, 72, 4000), (512, 2048, 520),                                # several tiles of rows
     (2100, 72, 1025), (4097, 64, 640), (2500, 136, 516), (260, 64, 4744),   # pairs of SMs: odd rows, 256, 192, 128 columns a tile
+    (2500, 264, 517), (300, 328, 3003), (1000, 256, 2047),           # rows of y off 16-byte boundaries
     (9000, 80, 260)])                                                 # more tiles than pairs
 def test_linear_bf16_tiles(gpu, M, K, N):
     from oracle import attention_oracle as orc
