@@ -531,10 +531,13 @@ extern "C" int grl_linear(grl_device* dev, const void* x, const void* w, const f
     // The pair kernel wants more than one of its two 128-row halves and tiles for half the pairs; below that the split kernel
     // has more SMs at work.  It also takes a short K whose rows of y are off 16-byte boundaries: the time is that of the stores
     // then, which its accumulators (lane = column of y) need no transpose for: us, pair / split, 4096 x 64 x 12287 113 / 63, 4096 x 128 x
-    // 4097 41 / 28, 4096 x 256 x 4097 43 / 37, but 4096 x 600 x 2047 25 / 31.
+    // 4097 41 / 28, 4096 x 256 x 4097 43 / 37, but 4096 x 600 x 2047 25 / 31; as long as its tiles are one wave of two CTAs an SM, a K
+    // up to 640 as well: 576 x 640 x 6598 19.0 / 12.2, 2000 x 304 x 2001 13.3 / 11.0, 200 x 400 x 4999 9.2 / 9.6.
     const int pairs = dev->prop.multiProcessorCount / 2;
     auto waves = [&](int bn) { return ((long long)((m + 255) / 256) * ((n + bn - 1) / bn) + pairs - 1) / pairs; };
-    if (m <= 128 || (n % 4 != 0 && k <= 256) || (long long)((m + 255) / 256) * ((n + 127) / 128) < pairs / 2) return lin::launch_split(dev, x, w, a);
+    const bool one_wave = (long long)((m + 127) / 128) * ((n + 127) / 128) <= 4 * pairs;
+    if (m <= 128 || (n % 4 != 0 && (k <= 256 || (k <= 640 && one_wave))) || (long long)((m + 255) / 256) * ((n + 127) / 128) < pairs / 2)
+        return lin::launch_split(dev, x, w, a);
     // the tile whose waves cost least: a wave of 256 / 192 / 128 columns took 29.7 / 26.3 / 22.7 us at K = 4096 (narrower tiles are
     // bound by shared memory)
     const long long c256 = waves(256) * 297, c192 = waves(192) * 263, c128 = waves(128) * 227;
