@@ -73,10 +73,12 @@ struct Args {
     int scores_ld;
     PeerExchange x;         // x.world > 1: the merged rows are exchanged with the peers and merged again
     long long wait_limit;   // cycle budget of every mbarrier wait
+    int alone;              // 1: one CTA an SM, and the next kernel starts after this one (see launch_instance)
     int cluster;            // > 1: CTAs of a thread-block cluster; that many splits of a head merge through its shared memory
     int pps_hint;           // stages per split of a sequence of the longest length: what the first block-table read assumes
 };
 constexpr int kMaxCluster = 16;
+constexpr int kAloneSmem = 116 * 1024;      // dynamic shared memory of which an SM (228 KiB, 1 KiB reserved a CTA) does not hold two
 constexpr int kDoneSlot = grl_device::kCounterSlots;
 constexpr int kMaxFusedSplits = 256;
 
@@ -258,6 +260,7 @@ template <bool QUANT, int HD>
 __global__ void __launch_bounds__(kThreads, 2)
 decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const Args a) {
     static_assert(HD == 128 || (HD == 64 && !QUANT), "head_dim 128, or 64 over the bf16 cache");
+    static_assert(Smem<QUANT, HD>::TOTAL <= kAloneSmem, "the wider allocation holds the ring");
     constexpr int D = HD;
     constexpr int NST = Ring<QUANT, HD>::NST, STAGE = Ring<QUANT, HD>::STAGE, SMEM_BAR = Smem<QUANT, HD>::BAR;
     constexpr int SLAB = Ring<QUANT, HD>::SLAB;
@@ -586,8 +589,10 @@ decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
     // ---- merge the four warps' partials (the ring is idle now: reuse it)
     __syncthreads();
     // The next kernel may launch under the merges.  Not before: its CTAs would take slots beside this kernel's and end up
-    // unevenly placed (two on some SMs, none on others: 196 us instead of 107 for a 131072-token quantised step).
-    pdl_trigger();
+    // unevenly placed (two on some SMs, none on others: 196 us instead of 107 for a 131072-token quantised step).  Where the
+    // CTAs have an SM each the next one's could only wait for this one's shared memory, so it is left to start at the end
+    // (131072 tokens x 2 heads, decode after decode: 84.8 us with an early start, 81.5 without).
+    if (!a.alone) pdl_trigger();
     float* sm_o = reinterpret_cast<float*>(smem);                 // [4 warps][8 heads][128]
     float* sm_m = sm_o + 4 * 8 * D;                               // [4][8]
     float* sm_l = sm_m + 32;
@@ -897,13 +902,13 @@ static int launch_instance(grl_device* dev, const CUtensorMap& tk, const CUtenso
     static bool attr_set[64] = {};
     if (!attr_set[dev->ordinal & 63]) {      // a function attribute belongs to the device that was current
         GRL_CUDA(cudaFuncSetAttribute(decode_mma_kernel<QUANT, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      Smem<QUANT, HD>::TOTAL));
+                                      kAloneSmem));
         GRL_CUDA(cudaFuncSetAttribute(decode_mma_kernel<QUANT, HD>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         attr_set[dev->ordinal & 63] = true;
     }
     // Splits merge in clusters while a split is short, the largest equal share of them whose clusters fit the device at once.
     // Long splits (more than 40 stages) are bound by the stream, and a cluster's CTAs sit two on an SM where one each would
-    // stream faster: 131072 tokens x 8 heads in 18 splits 98 us apart, 111 us in clusters of 9; 4096 tokens in 16 splits 13.8 us
+    // stream faster: 131072 tokens x 8 heads in 18 splits 97 us apart, 111 us in clusters of 9; 4096 tokens in 16 splits 13.8 us
     // in clusters of 16, 16.1 us apart.
     a.cluster = 1;
     if (a.fuse && !a.direct && a.x.world <= 1 && a.pps_hint <= 40)
@@ -911,8 +916,18 @@ static int launch_instance(grl_device* dev, const CUtensorMap& tk, const CUtenso
             if (a.n_splits % c == 0 && (int)(grid.y * grid.z) * (a.n_splits / c) <=
                 max_active_clusters(dev, (const void*)decode_mma_kernel<QUANT, HD>, kThreads, Smem<QUANT, HD>::TOTAL, c))
                 a.cluster = c;
-    GRL_CUDA(launch_pdl_cluster(decode_mma_kernel<QUANT, HD>, grid, kThreads, Smem<QUANT, HD>::TOTAL, dev->stream,
-                                a.cluster, tk, tv, a));
+    // Splits that merge through global memory, at most one CTA for every SM: two of them must not share an SM, which they do when
+    // they are placed while the SMs still hold CTAs of the kernel before (a decode that merges, or the append).  So they ask for
+    // more than half of an SM's shared memory.  Decode after decode / append + decode, us, 131072 tokens, bf16:
+    //   8 heads, 144 CTAs: 102.5 / 97.2 where pairs could form, 93.2 / 97.1 now;  7 heads, 147 CTAs: 92.4 / 94.5 and 84.1 / 87.0;
+    //   4 heads, 148 CTAs: 74.0 / 78.0 and 67.9 / 71.3.  A plain launch: 93.5 / 96.6, 84.4 / 87.3, 67.7 / 70.8 from a graph, but
+    //   append + decode from a stream 99.4, 90.2 and 73.8 for 97.4, 87.2 and 71.6.
+    a.alone = a.fuse && !a.direct && a.cluster == 1 && (int)(grid.x * grid.y * grid.z) <= dev->prop.multiProcessorCount;
+    if (a.alone)
+        GRL_CUDA(launch_pdl(decode_mma_kernel<QUANT, HD>, grid, kThreads, kAloneSmem, dev->stream, tk, tv, a));
+    else
+        GRL_CUDA(launch_pdl_cluster(decode_mma_kernel<QUANT, HD>, grid, kThreads, Smem<QUANT, HD>::TOTAL, dev->stream,
+                                    a.cluster, tk, tv, a));
     GRL_LAUNCHED(QUANT ? "decode_mma_kernel<quantised>" : "decode_mma_kernel");
     return GRL_OK;
 }

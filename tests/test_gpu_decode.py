@@ -385,3 +385,58 @@ def test_every_split_form_agrees(dev, dtype, D, Hq, Hkv, lens):
         part = pc.decode(q, n_splits=ns, partial=True)
         o, l = part[:B * Hq * D].reshape(B, 1, Hq, D), part[B * Hq * (D + 1):].reshape(B, 1, Hq, 1)
         assert np.abs(o / l - want).max() <= 2e-3 * scale, ns
+
+
+def test_long_decode_steps_in_a_row_keep_an_sm_each(dev):
+    """Decode after decode over 131072 tokens, as from a graph: the splits (144 CTAs) have an SM each, so that the steps take
+    less than the same steps with an append between them, which keeps the next decode's CTAs from being placed beside this one's
+    (93 against 97 us; where two CTAs could share an SM, 102 against 97)."""
+    from gpu_helpers import PagedCache
+    from grilly_next import cabi
+    Hq, Hkv, D, T, n = 32, 8, 128, 131072, 20
+    pc = PagedCache(dev, 1, Hkv, D, T, dtype=cabi.BF16)
+    for pool in (pc.k_pages, pc.v_pages):
+        cabi.check(dev.L.grl_memset(dev.h, pool, 0, T * Hkv * D * 2))
+    dev.L.grl_memcpy_h2d(dev.h, pc.seq_lens, np.asarray([T], np.int32).ctypes.data, 4)
+    before = dev.upload(np.asarray([T - 1], np.int32))
+    q, new = (dev.upload(np.zeros((1, 1, h, D), np.float32)) for h in (Hq, Hkv))
+    q_rot, out = (dev.malloc(Hq * D * 4) for _ in range(2))
+    a = cabi.AppendParams()
+    a.kv = pc.layout()
+    a.kv.seq_lens, a.k_new, a.v_new, a.n_new = before, new, new, 1
+    a.q_in, a.q_out, a.num_q_heads = q, q_rot, Hq
+    a.rope_mode, a.rope_theta, a.rope_scaling = cabi.ROPE_INTERLEAVED, 10000.0, 1.0
+    p = cabi.DecodeParams()
+    p.kv, p.q, p.out, p.num_q_heads, p.max_seq_len = pc.layout(), q, out, Hq, T
+    ns, wb = C.c_int(), C.c_size_t()
+    cabi.check(dev.L.grl_decode_pick_splits(dev.h, C.byref(p), C.byref(ns)))
+    cabi.check(dev.L.grl_decode_workspace_bytes(C.byref(p), ns, C.byref(wb)))
+    ws = dev.malloc(wb.value)
+    p.workspace, p.workspace_bytes = ws, wb.value
+
+    def per_step_us(append):
+        g, e0, e1, times = C.c_void_p(), dev.event(), dev.event(), []
+        cabi.check(dev.L.grl_graph_begin(dev.h))
+        for _ in range(n):
+            if append:
+                cabi.check(dev.L.grl_kv_append(dev.h, C.byref(a)))
+            cabi.check(dev.L.grl_gqa_decode(dev.h, C.byref(p)))
+        cabi.check(dev.L.grl_graph_end(dev.h, C.byref(g)))
+        for _ in range(6):
+            dev.record(e0)
+            cabi.check(dev.L.grl_graph_launch(dev.h, g))
+            dev.record(e1)
+            dev.sync()
+            times.append(dev.elapsed_ms(e0, e1) / n * 1e3)
+        dev.L.grl_graph_destroy(g)
+        for e in (e0, e1):
+            dev.L.grl_event_destroy(e)
+        return min(times[1:])
+
+    for f in (a, p):                                # what a first call allocates is not for a capture
+        cabi.check((dev.L.grl_kv_append if f is a else dev.L.grl_gqa_decode)(dev.h, C.byref(f)))
+    dev.sync()
+    alone, with_append = per_step_us(False), per_step_us(True)
+    for x in (pc.k_pages, pc.v_pages, pc.block_table, pc.seq_lens, before, q, new, q_rot, out, ws):
+        dev.free(x)
+    assert alone <= with_append, (alone, with_append)
