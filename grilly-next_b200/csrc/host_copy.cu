@@ -131,7 +131,7 @@ static cudaError_t take_slot(HostStage::Ring& r, int* slot) {
 
 cudaError_t staged_upload(grl_device* dev, void* dst, const void* src, size_t bytes) {
     HostStage& st = dev->stage;
-    std::lock_guard<std::mutex> lock(st.mu);
+    std::lock_guard<std::mutex> lock(st.up.mu);
     cudaError_t rc = open_ring(st.up);
     for (size_t off = 0, n = 0; off < bytes && rc == cudaSuccess; off += n) {
         n = std::min(off == 0 ? HostStage::kShort : HostStage::kPiece, bytes - off);
@@ -150,7 +150,7 @@ cudaError_t staged_upload(grl_device* dev, void* dst, const void* src, size_t by
 cudaError_t staged_download(grl_device* dev, void* dst, const void* src, size_t bytes, const cudaEvent_t* parts, int n_parts,
                             size_t part_bytes) {
     HostStage& st = dev->stage;
-    std::lock_guard<std::mutex> lock(st.mu);
+    std::lock_guard<std::mutex> lock(st.down.mu);
     cudaError_t rc = open_ring(st.down);
     // every slot is free between calls: a download leaves none in flight
     auto piece = [&](size_t off) {

@@ -44,17 +44,18 @@ private:
     bool stream_ = false;
 };
 
-// The page-locked rings of one device handle: allocated on first use, given back when the handle is closed.
+// The page-locked rings of one device handle: allocated on first use, given back when the handle is closed.  Each has a lock of its
+// own, held for a whole copy: a download that waits for the kernels before it does not keep another thread's upload waiting.
 struct HostStage {
     static constexpr size_t kPiece = 2u << 20, kShort = 512u << 10;    // the end of a copy that no transfer hides is short
     static constexpr int kSlots = 4;
     struct Ring {
+        std::mutex mu;
         char* mem = nullptr;
         cudaEvent_t ev[kSlots] = {};
         bool busy[kSlots] = {};
         int next = 0;
     };
-    std::mutex mu;
     Ring up, down;
     ~HostStage();
 };
