@@ -16,6 +16,17 @@ def dev():
         yield d
 
 
+def host(dev, n, pinned, fill=0):
+    """n bytes of host memory and what gives them back."""
+    if not pinned:
+        return np.full(n, fill, np.uint8), lambda: None
+    p = C.c_void_p()
+    assert dev.L.grl_host_alloc(C.c_size_t(n), C.byref(p)) == 0
+    a = np.frombuffer((C.c_uint8 * n).from_address(p.value), np.uint8)
+    a[:] = fill
+    return a, lambda: dev.L.grl_host_free(p)
+
+
 def slow_kernels(dev, buf, n):
     """n products of 2048^3 (a quarter of a millisecond or more each) on the handle's stream; buf holds 3 * 16 MiB."""
     from grilly_next import cabi
@@ -78,3 +89,43 @@ def test_threads_copy_through_one_handle(dev):
         t.join()
     dev.sync()
     assert not wrong
+
+
+@pytest.mark.parametrize("pinned", [False, True])
+@pytest.mark.parametrize("part,parts,short", [
+    (3 << 20, 4, 1 << 20),       # parts longer than a staging piece, the last one short
+    (300_000, 5, 17),            # shorter than a piece, not aligned
+    (1000, 3, 0),                # too small for the ring
+    (1 << 20, 3, 1 << 20)])      # a part with nothing left to copy
+def test_download_in_parts_waits_for_each_part(dev, pinned, part, parts, short):
+    from grilly_next import cabi
+    n = part * parts - short
+    want = np.random.default_rng(part).integers(1, 256, n, dtype=np.uint8)
+    made, src, scratch = dev.upload(want), dev.malloc(n), dev.malloc(48 << 20)
+    cabi.check(dev.L.grl_memset(dev.h, src, 0, n))
+    cabi.check(dev.L.grl_memset(dev.h, scratch, 0, 48 << 20))
+    dev.sync()
+    got, free = host(dev, n, pinned)
+    events = []
+    with cabi.Device(0) as down:
+        for i in range(parts):       # a part is made behind a few slow kernels: one that is copied too early reads zeros
+            off, m = i * part, min(part, max(0, n - i * part))
+            slow_kernels(dev, scratch, 8)
+            if m:
+                cabi.check(dev.L.grl_memcpy_d2d(dev.h, C.c_void_p(src.value + off), C.c_void_p(made.value + off), m))
+            events.append(dev.event())
+            dev.record(events[-1])
+        ev = (C.c_void_p * parts)(*[e.value for e in events])
+        cabi.check(dev.L.grl_memcpy_d2h_parts(down.h, got.ctypes.data, src, n, ev, parts, part))
+        if pinned:
+            down.sync()
+        assert np.array_equal(got, want)
+        dev.sync()
+        bad = (C.c_void_p * 65)(*[events[0].value] * 65)
+        for args in ((ev, 0, part), (bad, 65, part), (ev, parts, part - short // parts - 1), ((C.c_void_p * parts)(), parts, part), (ev, parts, 0)):
+            with pytest.raises(cabi.GrlError):
+                cabi.check(dev.L.grl_memcpy_d2h_parts(down.h, got.ctypes.data, src, n, *args))
+        down.sync()
+    for e in events:
+        dev.L.grl_event_destroy(e)
+    free()
