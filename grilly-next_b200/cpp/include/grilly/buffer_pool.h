@@ -51,11 +51,16 @@ private:
 /// Host arrays of one small call in ONE transfer each way.  A transfer costs some 10 us of driver and link latency whatever its
 /// size, which is most of a small call's time: the inputs are packed into one page-locked block, and the result leaves through
 /// another.  Reused by the next call on the device, so a call waits for its work (CommandBatch::submit) before it ends.
+/// An array of 512 KiB or more is left to the pageable copies (grl_memcpy_h2d / d2h), which take several threads from there on,
+/// where packing takes one.  us a call, packed / apart: 4 x 256 x 64 attention (three inputs of 256 KiB) 100 / 102; linear 256 x 256 x 256
+/// (inputs and result of 256 KiB) 79 / 86, 128 x 128 x 1000 (two arrays of 500 KiB) 92 / 95; but with one array of 512 KiB to 1 MiB
+/// 100 x 256 x 512 82 / 72, 8 x 256 x 900 81 / 66, 256 x 128 x 512 82 / 74, 256 x 200 x 1000 185 / 106.
 class SmallCall {
 public:
-    static constexpr size_t kMaxBytes = 1u << 20;      // inputs together, and the result
+    static constexpr size_t kMaxBytes = 1u << 20;      // inputs together
+    static constexpr size_t kMaxArray = 512u << 10;    // each of them, and the result: below this
     static constexpr int kInSlot = 6, kOutSlot = 7;    // GrillyDevice::pinnedStaging
-    static bool fits(size_t inputBytes, size_t outputBytes) { return inputBytes <= kMaxBytes && outputBytes <= kMaxBytes; }
+    static bool fits(size_t inputBytes, size_t largestArray) { return inputBytes <= kMaxBytes && largestArray < kMaxArray; }
     explicit SmallCall(BufferPool& pool);
     ~SmallCall();
     SmallCall(const SmallCall&) = delete;

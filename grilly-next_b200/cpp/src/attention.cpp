@@ -89,7 +89,7 @@ void flashAttention2Ex(CommandBatch& batch, BufferPool& pool, PipelineCache& cac
     size_t mElems = 0;          // of the mask array
     if (mask)
         mElems = opt.maskRank == 2 ? size_t(B) * S : (opt.maskRank == 3 || opt.maskBroadcastHeads) ? size_t(B) * S * S : size_t(B) * H * S * S;
-    const bool small = SmallCall::fits((3 * n + mElems + B) * 4, n * 4);
+    const bool small = SmallCall::fits((3 * n + mElems + B) * 4, std::max(n, mElems) * 4);
     GrillyBuffer q32, k32, v32, out = pool.acquire(n * 4);
     // share of a chunk that the host threads round to bf16 themselves (the rest is cast on the device)
     size_t hostPct = kPipelineHostCastPct;

@@ -23,7 +23,7 @@ void linearEx(CommandBatch& batch, BufferPool& pool, PipelineCache& cache, const
     grl_device* dev = pool.device().handle();
     cache.getOrCreate(std::string(bf16 ? "fnn-linear-tcgen05/" : "fnn-linear/") + std::to_string(p.inputDim));
     const size_t nx = size_t(p.batchSeq) * p.inputDim, nw = size_t(p.outputDim) * p.inputDim, ny = size_t(p.batchSeq) * p.outputDim;
-    const bool small = SmallCall::fits((nx + nw + p.outputDim) * 4, ny * 4);
+    const bool small = SmallCall::fits((nx + nw + p.outputDim) * 4, std::max({nx, nw, ny}) * 4);
     GrillyBuffer xb, wb, yb = pool.acquire(ny * 4), bb, x16, w16;
     std::vector<grl_event*> events;
     auto releaseAll = [&]() {

@@ -299,11 +299,11 @@ void SmallCall::send() {
 }
 
 void SmallCall::fetch(const void* device, size_t bytes) {
-    check(grl_memcpy_d2h(pool_.device().handle(), pool_.device().pinnedStaging(kOutSlot, kMaxBytes), device, bytes), "SmallCall: download");
+    check(grl_memcpy_d2h(pool_.device().handle(), pool_.device().pinnedStaging(kOutSlot, kMaxArray), device, bytes), "SmallCall: download");
 }
 
 void SmallCall::deliver(void* host, size_t bytes) const {
-    std::memcpy(host, pool_.device().pinnedStaging(kOutSlot, kMaxBytes), bytes);
+    std::memcpy(host, pool_.device().pinnedStaging(kOutSlot, kMaxArray), bytes);
 }
 
 // ---------------------------------------------------------------- PipelineCache

@@ -111,3 +111,20 @@ def test_linear_in_pieces(gpu, M, K, N, dtype):
     r = orc.round_bf16 if dtype == "bf16" else (lambda t: t)
     want = r(x).astype(np.float64) @ r(w).astype(np.float64).T
     assert np.abs(gpu.linear(x, w, dtype=dtype) - want).max() <= 2e-5 * K + 1e-4
+
+
+@pytest.mark.parametrize("M,K,N,packed", [
+    (100, 128, 1023, True), (100, 128, 1024, False),      # w below 512 KiB and at it
+    (1023, 128, 100, True), (1024, 128, 100, False),      # x
+    (256, 64, 511, True), (256, 64, 512, False),          # the result
+    (300, 436, 300, True), (300, 437, 300, False)])       # x and w; 1 MiB of inputs together
+def test_small_calls_pack_arrays_below_half_a_mebibyte(M, K, N, packed):
+    import grilly_core as core
+    ctx = core.Device()
+    rng = np.random.default_rng(M + K + N)
+    x, w = rng.standard_normal((M, K), dtype=np.float32), rng.standard_normal((N, K), dtype=np.float32)
+    before = ctx.pool_stats()["total_acquired"]
+    got = core.linear(ctx, x, w)
+    # the packed block and the result, or x, w and the result
+    assert ctx.pool_stats()["total_acquired"] - before == (2 if packed else 3)
+    assert np.abs(got - x.astype(np.float64) @ w.astype(np.float64).T).max() <= 1e-4 * np.sqrt(K / 64)
