@@ -11,7 +11,10 @@ namespace grilly {
 namespace ops {
 
 namespace {
-constexpr size_t kPieceBytes = 2u << 20, kPieceRows = 64;     // results from 2 MiB up, in pieces of whole 64-row tiles
+// Results from 2.5 MiB up leave in four pieces of whole 64-row tiles.  us a call in one piece / four (K = 768): result of 2 MiB 235 / 260,
+// 2.5 MiB 288 / 286, 3.5 MiB 336 / 318, 6 MiB 486 / 453, 16 MiB 935 / 835.  Two pieces: 477 and 870 for the last two; eight: 532 and 820,
+// and from 32 to 64 MiB within 3 % of four.
+constexpr size_t kPieceBytes = 5u << 19, kPieceRows = 64;
 }
 
 void linearEx(CommandBatch& batch, BufferPool& pool, PipelineCache& cache, const float* x, const float* weights,

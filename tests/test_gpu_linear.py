@@ -128,3 +128,21 @@ def test_small_calls_pack_arrays_below_half_a_mebibyte(M, K, N, packed):
     # the packed block and the result, or x, w and the result
     assert ctx.pool_stats()["total_acquired"] - before == (2 if packed else 3)
     assert np.abs(got - x.astype(np.float64) @ w.astype(np.float64).T).max() <= 1e-4 * np.sqrt(K / 64)
+
+
+@pytest.mark.parametrize("M,N,pieces", [(512, 1024, 1), (512, 1279, 1), (512, 1280, 4), (255, 2600, 1), (257, 2600, 5)])
+def test_results_from_two_and_a_half_mebibytes_leave_in_pieces(gpu, M, N, pieces):
+    import grilly_core as core
+    ctx = core.Device()
+    rng = np.random.default_rng(M + N)
+    x, w = rng.standard_normal((M, 64), dtype=np.float32), rng.standard_normal((N, 64), dtype=np.float32)
+    core.linear(ctx, x, w)
+    before = launches()
+    got = core.linear(ctx, x, w)
+    assert launches() - before == pieces            # a product each
+    assert np.abs(got - x.astype(np.float64) @ w.astype(np.float64).T).max() <= 1e-4
+
+
+def launches():
+    from grilly_next import cabi
+    return cabi.lib().grl_launch_count()
