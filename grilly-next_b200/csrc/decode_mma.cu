@@ -11,7 +11,7 @@
 // shared memory and leave the CTA as (O un-normalised, m, l), the layout lse_merge_kernel reads.  Splits of one head that fit a
 // thread-block cluster merge through its shared memory instead, and a launch sets up its ring and barriers under the kernel before
 // it.  Append + decode step: 1 sequence x 8 kv heads x 1001 tokens 19.4 us before, 9.9 now (latency); 32 x 8 x 4096 93 and 85 us
-// (HBM); 1 x 8 x 131072 quantised 107 and 79 us (the conversion's integer instructions).
+// (HBM); 1 x 8 x 131072 104 and 97 us (HBM; the decode alone 93), quantised 107 and 78 us (the conversion's integer instructions).
 //
 // The same kernel, instantiated for the quantised cache (GRL_FP8_INT4: FP8-E4M3 keys, INT4 values, one float16 scale
 // per 32 key elements, cpp/src/ops/kv_cache.cpp:272-399 and :500-577), streams 12.5 KiB per (page, kv head) instead

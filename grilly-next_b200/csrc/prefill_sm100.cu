@@ -780,7 +780,10 @@ int flash_fwd_sm100(grl_device* dev, const grl_flash_params* p, float scale, con
     a.wait_limit = dev->wait_limit_cycles;
     const int n_qt = (p->seq_len + BM - 1) / BM;
     // One tile a CTA while that is one wave: a second wave would cost what the shorter chains save, and every tile of its own
-    // loads and rotates K again.
+    // loads and rotates K again.  us, pair / one tile, causal with RoPE: 49 heads x 333 (147 tiles) 24.5 / 22.9, 7 x 2560 (140) 63 / 48; past one
+    // wave 62 x 333 (186) 24.4 / 28.2, 44 x 640 (220) 29.1 / 36.6; not causal 18 x 1280 (180) 41 / 54, 7 x 4096 (224) 94 / 128.  Causal tiles of long
+    // sequences differ in length, and up to some 290 of them would still be faster one a CTA, which this line does not take: 18 x 1280
+    // (180) 44 / 34, 11 x 2560 (220) 63 / 50, 9 x 4096 (288) 91 / 77; 16 x 2560 (320) 65 / 69.
     const bool split = (long long)BH * n_qt <= dev->prop.multiProcessorCount;
     a.n_qp = split ? n_qt : (n_qt + NQ - 1) / NQ;
     dim3 grid((unsigned)BH * a.n_qp);

@@ -11,11 +11,17 @@
  * Conventions
  *  - All data pointers are DEVICE pointers unless a parameter says "host".
  *  - All launches and copies are asynchronous on the device's stream (grl_device_use_stream
- *    adopts a caller's stream); grl_sync waits for it.
+ *    adopts a caller's stream); grl_sync waits for it.  Copies from and to pageable host memory go through page-locked
+ *    rings of the device handle: an upload returns when the source may be reused, a download when the destination is
+ *    complete.  One upload and one download at a time use a handle's rings; an upload does not wait for a download.
  *  - Callers own every buffer (grl_malloc / grl_free); kernels never allocate.  The library
  *    itself caches only per-device RoPE cos/sin tables (one per (head_dim, theta, scaling), sized to the
  *    longest sequence seen, rounded up to a power of two) that it frees in grl_device_close, and
  *    the encoded tensor maps of recent launches (host memory).
+ *  - The low bits of a result depend on the size of the call: attention, decode and the projections choose the split of
+ *    their sums (and with it what a 16-bit probability is scaled by) by how much of the GPU a call fills, so a sequence
+ *    alone and the same sequence in a batch agree to rounding, not bit for bit (grl_decode_params.n_splits fixes the number
+ *    of splits of a decode, GRL_KERNEL_SIMT_F32_WIDE the form of the float32 attention).
  */
 #ifndef GRILLY_CUDA_H
 #define GRILLY_CUDA_H
