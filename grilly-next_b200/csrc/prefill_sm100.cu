@@ -26,7 +26,10 @@
 // Bound: the chain of scores, softmax and products of a tile, and at length the 1000 W power cap.  The products are issued by
 // one elected lane of a converged warp (a warp that diverges for it re-issues its uniform work per lane), and a launch sets up its
 // barriers under the end of the kernel before it: 1 x 32 heads x 333 tokens 15.5 -> 13.2 us; 4 x 32 x 2048 causal with RoPE 229 us
-// before and after, at the power cap.  Calls of few tiles take the split form (see the kernel).
+// before and after, at the power cap.  A wait whose barrier has long completed still costs some 190 cycles beside the exponentials, of
+// 2000 a step: V is looked at ahead of P, the softmax looks at P.V of the step before only where it scales the accumulator, and the two
+// tiles' exponentials take no turns (4 x 32 x 2048 230 -> 223 us, 8 ragged sequences of 4096 828 -> 801, 8 x 32 x 1024 152 -> 143, 32 x 333 x 8
+// 57 -> 54).  Calls of few tiles take the split form (see the kernel).
 //
 // Every mbarrier wait is bounded; on expiry the CTA records an error, drains
 // its copies and returns.
@@ -71,8 +74,8 @@ constexpr uint32_t TMEM_TILE = 256, TMEM_O = 128;
 
 enum Bar { Q_FULL = 0, Q_READY = Q_FULL + NQ, K_FULL = Q_READY + NQ, K_READY = K_FULL + NSTAGE,
            K_EMPTY = K_READY + NSTAGE, V_FULL = K_EMPTY + NSTAGE, V_EMPTY = V_FULL + NSTAGE,
-           S_FULL = V_EMPTY + NSTAGE, P_READY = S_FULL + 2 * NQ, O_DONE = P_READY + 2 * NQ, EXP_TURN = O_DONE + NQ,
-           NUM_BARS = EXP_TURN + NQ };
+           S_FULL = V_EMPTY + NSTAGE, P_READY = S_FULL + 2 * NQ, O_DONE = P_READY + 2 * NQ, O_PREV = O_DONE + NQ,
+           NUM_BARS = O_PREV + NQ };
 // S_FULL / P_READY are indexed [t * 2 + buffer]: a barrier per S half-buffer, so that a waiter can
 // never fall two phases behind (the next use of a buffer needs this waiter's own arrival first).
 static_assert(NUM_BARS * 8 + 16 <= 256, "barrier block");
@@ -320,7 +323,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                 mbar_init(bar(P_READY + 2 * t + bf), 128);
             }
             mbar_init(bar(O_DONE + t), 1);
-            mbar_init(bar(EXP_TURN + t), 128);
+            mbar_init(bar(O_PREV + t), 1);
         }
         for (int s = 0; s < NSTAGE; ++s) {
             mbar_init(bar(K_FULL + s), 1);
@@ -488,8 +491,8 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
             for (int i = 0; i < 2 && i < nh && ok; ++i) ok = issue_qk(i);   // two steps of S ahead of the softmax
             for (int i = 0; i < nh && ok; ++i) {
                 const int j = tile_of(i), s = j % NSTAGE, it = j / NSTAGE;
-                ok = wait_bar_warp(ctx, P_READY + 2 * t + (i & 1), (i >> 1) & 1);
-                if (ok) ok = wait_bar_warp(ctx, V_FULL + s, it & 1);
+                ok = wait_bar_warp(ctx, V_FULL + s, it & 1);     // there already, as a rule: looked at ahead of P
+                if (ok) ok = wait_bar_warp(ctx, P_READY + 2 * t + (i & 1), (i >> 1) & 1);
                 if (!ok) break;
                 tc_fence_after();
                 // O_t += P_t[step i] V[64 keys]: A = P in TMEM (16 keys = 8 packed columns per k-step), B = 16 key
@@ -501,7 +504,7 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
 #pragma unroll
                 for (int ks = 1; ks < BH / 16; ++ks)
                     mma_ts2(o_tmem, p_tmem + ks * 8, vb + (uint32_t)ks * (2048 >> 4), IdescPV<HD>::value, 1u);
-                mma_commit(bar(O_DONE + t));
+                if (i + 2 >= nh) mma_commit(bar((i + 2 == nh ? O_PREV : O_DONE) + t));
                 if (last_of(i)) release(V_EMPTY + s, j);
                 if (i + 2 < nh) ok = issue_qk(i + 2);   // reuses buffer i & 1: in order after PV(t, i)
             }
@@ -560,12 +563,6 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
             }
             float m_ref = -INFINITY, l = 0.f;
             const int nh = n_half[t];
-            // The two softmax warpgroups take turns in the exponential phase (it saturates the MUFU unit they
-            // share): a warpgroup starts its exponentials when the other has finished its own, and spends its
-            // loads, maxima, stores and barrier hops while the other one exponentiates.  Only for the steps that
-            // both tiles have.
-            const int nc = min(n_half[0], n_half[1]);
-            if (t == 1 && nc > 0) mbar_arrive(bar(EXP_TURN + 0));   // tile 0 goes first
             for (int i = 0; i < nh && ok; ++i) {
                 const int bf = i & 1, k0 = SPLIT ? i * BN + t * BH : i * BH;
                 ok = wait_bar_warp(ctx, S_FULL + 2 * t + bf, (i >> 1) & 1);
@@ -589,15 +586,15 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                 }
                 const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
                 const float m_new = fmaxf(m_ref, mx * a.scale_log2);
-                bool o_waited = false;
                 if (i == 0) {
                     m_ref = (m_new == -INFINITY) ? 0.f : m_new;
                 } else {
                     const bool need = m_new > m_ref + 8.f;
                     if (__any_sync(0xffffffffu, need)) {
-                        ok = wait_bar_warp(ctx, O_DONE + t, (i - 1) & 1);   // PV(t, i-1) has written O
+                        // PV(t, i-1) must be in O: it is once S(t, i+1) is there, whose product is issued after it; ahead of the
+                        // last step it has a barrier of its own.
+                        ok = i + 1 < nh ? wait_bar_warp(ctx, S_FULL + 2 * t + (bf ^ 1), ((i + 1) >> 1) & 1) : wait_bar_warp(ctx, O_PREV + t, 0);
                         if (!ok) break;
-                        o_waited = true;
                         tc_fence_after();
                         const float f = need ? ex2(m_ref - m_new) : 1.f;
                         if (need) m_ref = m_new;
@@ -612,10 +609,6 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                         }
                         tmem_st_wait();
                     }
-                }
-                if (i < nc) {
-                    ok = wait_bar_warp(ctx, EXP_TURN + t, i & 1);
-                    if (!ok) break;
                 }
                 // p = exp2(s * scale_log2 - m_ref): packed two-wide FMA and add, scalar ex2 (MUFU)
                 const float2 sc2 = make_float2(a.scale_log2, a.scale_log2), nm2 = make_float2(-m_ref, -m_ref);
@@ -634,20 +627,12 @@ flash_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                     }
                     tmem_st_x16(s_addr + bf * BH + ch * 16, pk);
                 }
-                if (t == 0 ? (i < nc) : (i + 1 < nc)) mbar_arrive(bar(EXP_TURN + (t ^ 1)));   // the other tile's turn
                 l += ((rs4[0].x + rs4[0].y) + (rs4[1].x + rs4[1].y)) + ((rs4[2].x + rs4[2].y) + (rs4[3].x + rs4[3].y));
                 tmem_st_wait();
-                // Consume the phase of PV(t, i-1) BEFORE arriving: after the arrival PV(t, i) may complete too,
-                // and a waiter that then looks for the parity of phase i-1 would find the barrier two phases
-                // ahead and never return.  PV(t, i-1) was issued a whole softmax step ago: no stall here.
-                if (i >= 1 && !o_waited) {
-                    ok = wait_bar_warp(ctx, O_DONE + t, (i - 1) & 1);
-                    if (!ok) break;
-                }
                 tc_fence_before();
                 mbar_arrive(bar(P_READY + 2 * t + bf));
             }
-            if (ok && (!SPLIT || nh > 0)) ok = wait_bar_warp(ctx, O_DONE + t, (nh - 1) & 1);
+            if (ok && (!SPLIT || nh > 0)) ok = wait_bar_warp(ctx, O_DONE + t, 0);
             float2 other = make_float2(0.f, 0.f);     // the other half's row maximum and sum
             if constexpr (SPLIT) {
                 float2* ml = reinterpret_cast<float2*>(smem + SMEM_ML);

@@ -354,3 +354,28 @@ def test_tcgen05_kernel_tile_edges(dev, B, H, S, D, causal, rope, lens):
     kw = dict(causal=causal, seq_lens=None if lens is None else np.array(lens, np.int32), rope_mode=mode, bf16=True, kernel=cabi.KERNEL_TCGEN05)
     assert np.abs(flash_cabi(dev, Q, K, V, **kw) - want).max() <= TOL_BF16
     assert np.abs(flash_cabi(dev, Q, K, V, out_bf16=True, **kw) - want).max() <= 3e-2
+
+
+@pytest.mark.parametrize("heads", [2, 40])                      # one query tile a CTA; pairs of tiles
+@pytest.mark.parametrize("S,jump", [(640, 64), (640, 128), (640, 512), (640, 576), (600, 576), (577, 576), (129, 128), (128, 64), (640, 0)])
+@pytest.mark.parametrize("causal", [False, True])
+def test_tcgen05_kernel_rescales_at_any_step(dev, heads, S, jump, causal):
+    """Scores that rise by 2^12 at one 64-key step (jump = its first key; 0: at every step): the accumulator is scaled when the
+    product of the step before is in it, ahead of the last step and elsewhere.  Left unscaled, the keys before the jump would
+    weigh 4096 times too much.  Tolerance: probabilities and inputs in bf16, as for the other cases."""
+    from grilly_next import cabi
+    from gpu_helpers import flash_cabi
+    rng = np.random.default_rng(S + jump)
+    D = 128
+    u = np.ones(D, np.float32)
+    rise = 12 * np.log(2) / np.sqrt(D)                           # per unit of u.u / sqrt(D), in natural logarithms
+    k0 = np.arange(S)
+    level = (k0 // 64 if jump == 0 else (k0 >= jump)) * np.float32(rise)
+    Q = np.broadcast_to(u, (1, heads, S, D)).astype(np.float32)
+    K = (rng.standard_normal((1, heads, S, D), dtype=np.float32) * 0.05 + level[:, None] * u).astype(np.float32)
+    V = rng.standard_normal((1, heads, S, D), dtype=np.float32)
+    out = flash_cabi(dev, Q, K, V, causal=causal, bf16=True, kernel=cabi.KERNEL_TCGEN05)
+    want = orc.attention_4d(orc.round_bf16(Q[:, :2]), orc.round_bf16(K[:, :2]), V[:, :2], mask=orc.causal_length_mask(1, 2, S, None, causal))
+    assert np.abs(out[:, :2] - want).max() <= TOL_BF16
+    want = orc.attention_4d(orc.round_bf16(Q[:, -1:]), orc.round_bf16(K[:, -1:]), V[:, -1:], mask=orc.causal_length_mask(1, 1, S, None, causal))
+    assert np.abs(out[:, -1:] - want).max() <= TOL_BF16
