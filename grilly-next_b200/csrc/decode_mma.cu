@@ -11,7 +11,7 @@
 // shared memory and leave the CTA as (O un-normalised, m, l), the layout lse_merge_kernel reads.  Splits of one head that fit a
 // thread-block cluster merge through its shared memory instead, and a launch sets up its ring and barriers under the kernel before
 // it.  Append + decode step: 1 sequence x 8 kv heads x 1001 tokens 19.4 us before, 9.9 now (latency); 32 x 8 x 4096 93 and 85 us
-// (HBM); 1 x 8 x 131072 104 and 97 us (HBM; the decode alone 93), quantised 107 and 78 us (the conversion's integer instructions).
+// (HBM); 1 x 8 x 131072 104 and 94 us (HBM; the decode alone 90), quantised 107 and 71 us (instructions: some 450 a 16-token slice).
 //
 // The same kernel, instantiated for the quantised cache (GRL_FP8_INT4: FP8-E4M3 keys, INT4 values, one float16 scale
 // per 32 key elements, cpp/src/ops/kv_cache.cpp:272-399 and :500-577), streams 12.5 KiB per (page, kv head) instead
@@ -23,6 +23,8 @@
 #include <cuda.h>
 #include <cuda_fp16.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace grl {
@@ -30,24 +32,36 @@ namespace dmma {
 
 constexpr int P = 64;               // tokens per ring stage: one 64-token page, or two / four smaller ones side by side
 constexpr int D = 128;              // head_dim of the quantised instance (the bf16 instances carry theirs as HD)
-constexpr int kThreads = 160;       // 4 compute warps + 1 producer warp
-// The shared-memory ring of the two instances.  After the ring: 128 bytes of barriers and flags, 128 of block table, 1 KiB of per-warp
-// scratch for the quantised instance (1/scale of a warp's 16 tokens x 4 groups), 1 KiB of slack for the 1024-byte alignment of the ring.
-template <bool QUANT, int HD> struct Ring {
+// FORM of an instance: over the bf16 cache, over the quantised cache, and that with one CTA an SM.
+enum Form { BF16 = 0, QUANT_PAIR = 1, QUANT_WIDE = 2 };
+// Compute warps, in groups of four that take the ring's stages in turn (16 tokens of one a warp), and the producer warps behind
+// them (stages in turn, too).  A producer's serial chain of waits and copies is some 1300 cycles a stage beside busy compute
+// warps, so the quantised stages, which are small, have several (131072 tokens x 8 heads, decode alone: 15 compute warps and one
+// producer 79 us, 14 and 2 64, 12 and 4 64; with the shorter conversion 12 and 1 61, 12 and 4 59; four compute warps and 1 / 2
+// producers, two CTAs an SM, 66 / 65).
+template <int FORM> struct Warps {
+    static constexpr int COMPUTE = FORM == QUANT_WIDE ? 12 : 4, PROD = FORM == QUANT_WIDE ? 4 : FORM == QUANT_PAIR ? 2 : 1;
+    static constexpr int THREADS = 32 * (COMPUTE + PROD), CTAS = FORM == QUANT_WIDE ? 1 : 2;
+};
+// The shared-memory ring of an instance.  After the ring: 256 bytes of barriers and flags, 128 of block table a producer, 256 a compute
+// warp over the quantised cache (1/scale of its 16 tokens x 4 groups), 1 KiB of slack for the 1024-byte alignment of the ring.
+template <int FORM, int HD> struct Ring {
     static constexpr int SLAB = P * HD * 2;             // 64 tokens of K (or V) for one kv head: 16 KiB at head_dim 128
     static constexpr int STAGE = 2 * SLAB;              // K then V
     static constexpr int NST = 3 * 128 / HD;            // ring stages: 96 KiB in flight per CTA
 };
 constexpr int QK_BYTES = P * D;          // 8 KiB of key bytes per 64 tokens of a kv head
 constexpr int QV_BYTES = P * D / 2;      // 4 KiB of packed value nibbles
-template <> struct Ring<true, 128> {
+template <int NST_> struct QuantRing {
     static constexpr int SLAB = 0;
-    static constexpr int NST = 6;
+    static constexpr int NST = NST_;
     static constexpr int STAGE = 13 * 1024;  // keys at 0, values at 8 KiB, scales at 12 KiB
 };
-template <bool QUANT, int HD> struct Smem {
-    static constexpr int BAR = Ring<QUANT, HD>::NST * Ring<QUANT, HD>::STAGE;
-    static constexpr int TOTAL = BAR + 128 + 128 + (QUANT ? 1024 : 0) + 1024;
+template <> struct Ring<QUANT_PAIR, 128> : QuantRing<6> {};
+template <> struct Ring<QUANT_WIDE, 128> : QuantRing<14> {};
+template <int FORM, int HD> struct Smem {
+    static constexpr int BAR = Ring<FORM, HD>::NST * Ring<FORM, HD>::STAGE;
+    static constexpr int TOTAL = BAR + 256 + 128 * Warps<FORM>::PROD + (FORM != BF16 ? 256 * Warps<FORM>::COMPUTE : 0) + 1024;
 };
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kEmpty = -1e30f;
@@ -209,10 +223,11 @@ __device__ __forceinline__ uint32_t nib_hi(uint32_t w) {
 // 1/scale from the stored float16 bit pattern, as the reference's decode forms it (kv_cache.cpp:517-533): bits moved
 // into a float32, not converted; a scale that is not positive gives 1.
 __device__ __forceinline__ float inv_scale_bits(uint32_t h) {
-    const uint32_t e = (h >> 10) & 0x1Fu, m = h & 0x03FFu;
-    const float sc = e == 0 ? (float)m * 5.9604644775390625e-08f
-                            : __uint_as_float(((h & 0x8000u) << 16) | ((e + 112u) << 23) | (m << 13));
-    return sc > 0.f ? __fdividef(1.0f, sc) : 1.0f;     // within an ulp of the reference's quotient
+    // exponent and mantissa under the float32 exponent field are the value times 2^-112, subnormal scales included
+    const float sc = __uint_as_float((h & 0x7FFFu) << 13) * 5.192296858534828e+33f;
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(sc));     // within an ulp of the reference's quotient
+    return (h - 1u) < 0x7FFFu ? r : 1.0f;
 }
 __device__ __forceinline__ float ex2(float x) {
     float y;
@@ -256,14 +271,17 @@ __device__ __forceinline__ uint32_t slab_off(int row, int d) {
     return (uint32_t)((d >> 6) * (P * 128) + row * 128 + ((((d & 63) >> 3) ^ (row & 7)) << 4));
 }
 
-template <bool QUANT, int HD>
-__global__ void __launch_bounds__(kThreads, 2)
+template <int FORM, int HD>
+__global__ void __launch_bounds__(Warps<FORM>::THREADS, Warps<FORM>::CTAS)
 decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const Args a) {
+    constexpr bool QUANT = FORM != BF16;
     static_assert(HD == 128 || (HD == 64 && !QUANT), "head_dim 128, or 64 over the bf16 cache");
-    static_assert(Smem<QUANT, HD>::TOTAL <= kAloneSmem, "the wider allocation holds the ring");
+    static_assert(FORM == QUANT_WIDE || Smem<FORM, HD>::TOTAL <= kAloneSmem, "the wider allocation holds the ring");
     constexpr int D = HD;
-    constexpr int NST = Ring<QUANT, HD>::NST, STAGE = Ring<QUANT, HD>::STAGE, SMEM_BAR = Smem<QUANT, HD>::BAR;
-    constexpr int SLAB = Ring<QUANT, HD>::SLAB;
+    constexpr int NST = Ring<FORM, HD>::NST, STAGE = Ring<FORM, HD>::STAGE, SMEM_BAR = Smem<FORM, HD>::BAR;
+    constexpr int SLAB = Ring<FORM, HD>::SLAB;
+    constexpr int COMPUTE = Warps<FORM>::COMPUTE, PROD = Warps<FORM>::PROD, kThreads = Warps<FORM>::THREADS;
+    static_assert(2 * NST * 8 + 16 <= 256 && NST <= 32, "barrier block; a lane a stage in the first fill");
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw_addr = smem_u32(smem_raw);
     const uint32_t base = (raw_addr + 1023u) & ~1023u;
@@ -291,8 +309,8 @@ decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
     const int32_t raw_len = a.seq_lens[b];
     // the split's first block-table entries, read beside the length on the guess that this sequence is the longest
     const int bt_guess = split * a.pps_hint * a.ppt;
-    int32_t* bt_s = reinterpret_cast<int32_t*>(smem + SMEM_BAR + 128);      // 32 entries (per-warp scratch of the compute warps starts behind)
-    if (warp == 4) bt_s[lane] = bt[min(bt_guess + lane, a.max_pages - 1)];
+    int32_t* bt_s = reinterpret_cast<int32_t*>(smem + SMEM_BAR + 256 + 128 * (warp >= COMPUTE ? warp - COMPUTE : 0));      // 32 entries a producer
+    if (warp >= COMPUTE) bt_s[lane] = bt[min(bt_guess + lane, a.max_pages - 1)];
     const int len = max(0, min(raw_len, a.max_pages * a.page));   // never past the block table
     const int n_pages = (len + P - 1) / P;        // 64-token stages ("pages" below)
     const int pps = (n_pages + a.n_splits - 1) / a.n_splits;
@@ -304,45 +322,84 @@ decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
 #pragma unroll
     for (int i = 0; i < D / 8; ++i) { o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f; }
 
-    if (warp == 4) {
-        // ------------------------------------------------------------------ producer
+    if (warp >= COMPUTE) {
+        // ------------------------------------------------------------------ producers
         __syncwarp();
-        if (lane == 0) {
-            auto page_of = [&](int i) { return (unsigned)(i - bt_guess) < 32u ? bt_s[i - bt_guess] : bt[i]; };
-            int issued = 0;
-            for (int p = p_begin; p < p_end; ++p) {
-                const int i = p - p_begin, s = i % NST, it = i / NST;
-                if (it > 0 && !wait_bar(ctx, NST + s, (it - 1) & 1, true)) break;
-                // the pages of this stage that hold tokens of the sequence (all of them but in the last stage); rows of
-                // the stage that no copy fills keep what they held: their tokens are past the length and masked
-                const int np = min(a.ppt, (len - p * P + a.page - 1) / a.page);
-                const uint32_t dst = base + (uint32_t)s * STAGE;
-                if constexpr (QUANT) {
-                    mbar_expect_tx(full(s), (uint32_t)np * a.page * (D + D / 2 + D / 16));
-                    for (int j = 0; j < np; ++j) {
-                        const int blk = page_of(p * a.ppt + j) * a.Hkv + kvh;
-                        // rows of 128 key bytes under the 128-byte swizzle; a page's value and scale blocks are contiguous
-                        tma_load_2d(dst + j * a.page * 128, &tmK, 0, blk * a.page, full(s));
-                        bulk_load(dst + QK_BYTES + j * a.page * (D / 2), a.v_q + (size_t)blk * a.page * (D / 2), a.page * (D / 2), full(s));
-                        bulk_load(dst + QK_BYTES + QV_BYTES + j * a.page * (D / 16), a.scales + (size_t)blk * a.page * (D / 32),
-                                  a.page * (D / 16), full(s));
-                    }
-                } else {
-                    mbar_expect_tx(full(s), (uint32_t)np * a.page * D * 4);
-                    for (int j = 0; j < np; ++j) {
-                        const int row0 = (page_of(p * a.ppt + j) * a.Hkv + kvh) * a.page;
+        int issued = 0;
+        const int pr = warp - COMPUTE;
+        auto issue = [&](uint32_t dst, int page, int j, int s) {
+            const int blk = page * a.Hkv + kvh;
+            if constexpr (QUANT) {
+                // rows of 128 key bytes under the 128-byte swizzle; a page's value and scale blocks are contiguous
+                tma_load_2d(dst + j * a.page * 128, &tmK, 0, blk * a.page, full(s));
+                bulk_load(dst + QK_BYTES + j * a.page * (D / 2), a.v_q + (size_t)blk * a.page * (D / 2), a.page * (D / 2), full(s));
+                bulk_load(dst + QK_BYTES + QV_BYTES + j * a.page * (D / 16), a.scales + (size_t)blk * a.page * (D / 32),
+                          a.page * (D / 16), full(s));
+            } else {
 #pragma unroll
-                        for (int c0 = 0; c0 < D; c0 += 64) {        // 64-column boxes (128 bytes: the swizzle span)
-                            tma_load_2d(dst + (c0 / 64) * (P * 128) + j * a.page * 128, &tmK, c0, row0, full(s));
-                            tma_load_2d(dst + SLAB + (c0 / 64) * (P * 128) + j * a.page * 128, &tmV, c0, row0, full(s));
-                        }
-                    }
+                for (int c0 = 0; c0 < D; c0 += 64) {        // 64-column boxes (128 bytes: the swizzle span)
+                    tma_load_2d(dst + (c0 / 64) * (P * 128) + j * a.page * 128, &tmK, c0, blk * a.page, full(s));
+                    tma_load_2d(dst + SLAB + (c0 / 64) * (P * 128) + j * a.page * 128, &tmV, c0, blk * a.page, full(s));
                 }
+            }
+        };
+        constexpr uint32_t TOKEN_BYTES = QUANT ? D + D / 2 + D / 16 : D * 4;
+        bool ok = true;
+        // the pages of stage p that hold tokens of the sequence (all of them but in the last stage); rows of the stage that no copy
+        // fills keep what they held: their tokens are past the length and masked
+        auto pages_of = [&](int p) { return min(a.ppt, (len - p * P + a.page - 1) / a.page); };
+        if (a.ppt <= 2) {
+            // One or two pages a stage: lane 0 alone, in a shorter loop for one page a stage where that chain bounds the stream of
+            // a CTA alone on its SM (131072 tokens x 8 heads, append + decode 97.8 -> 94.2 us; two CTAs an SM, 32 x 8 x 4096, 85.0 -> 85.6).
+            auto page_of = [&](int i) { return (unsigned)(i - bt_guess) < 32u ? bt_s[i - bt_guess] : bt[i]; };
+            auto walk = [&](auto one) {
+                for (int p = p_begin + pr; p < p_end; p += PROD) {
+                    const int i = p - p_begin, s = i % NST, it = i / NST;
+                    if (it > 0 && !wait_bar(ctx, NST + s, (it - 1) & 1, true)) break;
+                    if constexpr (decltype(one)::value) {
+                        mbar_expect_tx(full(s), P * TOKEN_BYTES);
+                        issue(base + (uint32_t)s * STAGE, page_of(p), 0, s);
+                    } else {
+                        const int np = pages_of(p);
+                        mbar_expect_tx(full(s), (uint32_t)np * a.page * TOKEN_BYTES);
+                        for (int j = 0; j < np; ++j) issue(base + (uint32_t)s * STAGE, page_of(p * a.ppt + j), j, s);
+                    }
+                    issued = i + 1;
+                }
+            };
+            if (lane == 0) {
+                if (a.ppt == 1 && (a.alone || FORM == QUANT_WIDE)) walk(std::true_type{});
+                else walk(std::false_type{});
+            }
+        } else {
+            // Four pages a stage: lane l holds the block-table entry of page first + l and issues that page's copies; the next 32
+            // entries are read while these are used up (16-token pages, 131072 tokens x 8 heads: 143 -> 115 us, append + decode).
+            int first = p_begin * a.ppt;
+            int entry = first == bt_guess ? bt_s[lane] : bt[min(first + lane, a.max_pages - 1)];
+            int entry_next = bt[min(first + 32 + lane, a.max_pages - 1)];
+            for (int p = p_begin + pr; p < p_end; p += PROD) {
+                const int i = p - p_begin, s = i % NST, it = i / NST;
+                if (p * a.ppt - first >= 32) {
+                    first += 32;
+                    entry = entry_next;
+                    entry_next = bt[min(first + 32 + lane, a.max_pages - 1)];
+                }
+                ok = lane != 0 || it == 0 || wait_bar(ctx, NST + s, (it - 1) & 1, true);
+                if (!__all_sync(0xffffffffu, ok)) break;
+                const int np = pages_of(p);
+                if (lane == 0) mbar_expect_tx(full(s), (uint32_t)np * a.page * TOKEN_BYTES);
+                __syncwarp();
+                const int j = lane - (p * a.ppt - first);
+                if (j >= 0 && j < np) issue(base + (uint32_t)s * STAGE, entry, j, s);
+                __syncwarp();
                 issued = i + 1;
             }
+        }
+        if (lane == 0) {
             if (*ctx.abort) {   // copies already issued must land before the shared memory is released
                 const long long t0 = clock64();
                 for (int i = max(0, issued - NST); i < issued; ++i)
+                    if (i % PROD == pr)
                     while (!mbar_try_wait(full(i % NST), (i / NST) & 1) && clock64() - t0 < ctx.limit) {}
             }
         }
@@ -368,38 +425,44 @@ decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
                 qf[ks][1] = pack_f16(v.y * sc, v.w * sc);      // bytes 1 and 3
             }
         }
-        float* inv_w = reinterpret_cast<float*>(smem + SMEM_BAR + 256) + warp * 64;   // [16 tokens][4 groups]
+        float* inv_w = reinterpret_cast<float*>(smem + SMEM_BAR + 256 + 128 * PROD) + warp * 64;   // [16 tokens][4 groups]
         bool ok = true;
-        for (int p = p_begin; p < p_end && ok; ++p) {
-            const int i = p - p_begin, s = i % NST, it = i / NST;
-            ok = __all_sync(0xffffffffu, wait_bar(ctx, s, it & 1));
+        constexpr int GROUPS = COMPUTE / 4;
+        const int slice = warp & 3;             // which 16 tokens of a stage
+        int s = (warp >> 2) - GROUPS;           // ring slot; the parity of its phase
+        uint32_t parity = 0;
+        for (int p = p_begin + (warp >> 2); p < p_end; p += GROUPS) {
+            s += GROUPS;
+            if (s >= NST) { s -= NST; parity ^= 1u; }
+            ok = __all_sync(0xffffffffu, wait_bar(ctx, s, parity));
             if (!ok) break;
             const uint8_t* kst = smem + s * STAGE;
             const uint8_t* vst = kst + QK_BYTES;
             const uint8_t* sst = vst + QV_BYTES;
-            const int tok0 = p * P + 16 * warp;
+            const int tok0 = p * P + 16 * slice;
             if (tok0 < len) {
                 {   // 1/scale of this warp's tokens: lane -> token lane/2, groups 2*(lane&1) and the next; 0 past the end
                     const int tl = lane >> 1, g2 = (lane & 1) * 2;
-                    const uint32_t hh = *reinterpret_cast<const uint32_t*>(sst + ((16 * warp + tl) * 4 + g2) * 2);
+                    const uint32_t hh = *reinterpret_cast<const uint32_t*>(sst + ((16 * slice + tl) * 4 + g2) * 2);
                     const bool live_t = tok0 + tl < len;
-                    *reinterpret_cast<float2*>(inv_w + tl * 4 + g2) =
-                        make_float2(live_t ? inv_scale_bits(hh & 0xFFFFu) : 0.f, live_t ? inv_scale_bits(hh >> 16) : 0.f);
+                    // token 4 q + 2 e + nt goes to [q][group][2 nt + e]
+                    float* dst = inv_w + (tl >> 2) * 16 + g2 * 4 + (tl & 1) * 2 + ((tl >> 1) & 1);
+                    dst[0] = live_t ? inv_scale_bits(hh & 0xFFFFu) : 0.f;
+                    dst[4] = live_t ? inv_scale_bits(hh >> 16) : 0.f;
                 }
                 __syncwarp();
-                float inv[2][2][4];
+                float2 inv[2][4];           // [nt][group], of the lane's two tokens of tile nt
 #pragma unroll
-                for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        const float4 v = *reinterpret_cast<const float4*>(inv_w + (4 * t4 + 2 * e + nt) * 4);
-                        inv[nt][e][0] = v.x; inv[nt][e][1] = v.y; inv[nt][e][2] = v.z; inv[nt][e][3] = v.w;
-                    }
+                for (int grp = 0; grp < 4; ++grp) {
+                    const float4 v = *reinterpret_cast<const float4*>(inv_w + t4 * 16 + grp * 4);
+                    inv[0][grp] = make_float2(v.x, v.y);
+                    inv[1][grp] = make_float2(v.z, v.w);
+                }
                 // ---- S = q K^T for 16 tokens, one accumulator per scale group, combined with 1/scale
-                float sacc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+                float2 sc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
                 for (int nt = 0; nt < 2; ++nt) {
-                    const int row = 16 * warp + 2 * g + nt;     // column n of tile nt is token 2 n + nt of the slice
+                    const int row = 16 * slice + 2 * g + nt;     // column n of tile nt is token 2 n + nt of the slice
 #pragma unroll
                     for (int grp = 0; grp < 4; ++grp) {
                         const int chunk = (2 * grp + (t4 >> 1)) ^ (row & 7);
@@ -407,10 +470,10 @@ decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
                         float c[4];
                         mma_f16_first(c, qf[2 * grp][0], qf[2 * grp][1], e4m3_pair02_f16x2(kb.x), e4m3_pair13_f16x2(kb.x));
                         mma_f16(c, qf[2 * grp + 1][0], qf[2 * grp + 1][1], e4m3_pair02_f16x2(kb.y), e4m3_pair13_f16x2(kb.y));
-                        sacc[nt][0] = fmaf(c[0], inv[nt][0][grp], sacc[nt][0]);
-                        sacc[nt][1] = fmaf(c[1], inv[nt][1][grp], sacc[nt][1]);
+                        sc[nt] = __ffma2_rn(make_float2(c[0], c[1]), inv[nt][grp], sc[nt]);
                     }
                 }
+                float sacc[2][2] = {{sc[0].x, sc[0].y}, {sc[1].x, sc[1].y}};
                 // ---- online softmax for head row g.  Only the last tile of a sequence has tokens past its end: they
                 // get the "empty" score there, so the common path carries no per-token predicate
                 if (tok0 + 16 > len) {
@@ -429,39 +492,37 @@ decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
                             if (tok0 + 4 * t4 + 2 * e + nt < len) srow[2 * e + nt] = sacc[nt][e] * 0.6931471805599453f;
                 }
                 float mx = fmaxf(fmaxf(sacc[0][0], sacc[0][1]), fmaxf(sacc[1][0], sacc[1][1]));
-                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-                const float m_new = fmaxf(m_run, mx);
-                const float corr = ex2(m_run - m_new);
-                float pv[2][2];
-#pragma unroll
-                for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) pv[nt][e] = ex2(sacc[nt][e] - m_new);    // 0 for an "empty" score
-                const float ps = (pv[0][0] + pv[0][1]) + (pv[1][0] + pv[1][1]);
-                l_run = l_run * corr + ps;
-                m_run = m_new;
-                if (__any_sync(0xffffffffu, corr != 1.f)) {
+                if (__any_sync(0xffffffffu, mx > m_run)) {      // a new maximum: seldom, after the first few tiles
+                    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+                    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+                    const float m_new = fmaxf(m_run, mx);
+                    const float corr = ex2(m_run - m_new);
+                    l_run *= corr;
+                    m_run = m_new;
                     // the accumulator columns of this lane are heads 2 t4 and 2 t4 + 1: their factors live in other lanes
                     const float ca = __shfl_sync(0xffffffffu, corr, 8 * t4), cb = __shfl_sync(0xffffffffu, corr, 8 * t4 + 4);
 #pragma unroll
                     for (int n = 0; n < 8; ++n) { o[n][0] *= ca; o[n][2] *= ca; o[n][1] *= cb; o[n][3] *= cb; }
                 }
+                float2 pv[2];
+#pragma unroll
+                for (int nt = 0; nt < 2; ++nt) pv[nt] = make_float2(ex2(sacc[nt][0] - m_run), ex2(sacc[nt][1] - m_run));    // 0 for an "empty" score
+                l_run += (pv[0].x + pv[0].y) + (pv[1].x + pv[1].y);
                 // ---- O^T += V^T (P / scale)^T: rows are head_dim elements, columns heads, so all sixteen rows of the
                 // product work and P is used as it comes out of S (pairs of tokens per head).  The two token pairs of
                 // this lane, 16 value bytes (all four groups) each
                 // (this lane's tokens 4 t4 .. 4 t4 + 3 of the slice: pairs 2 t4 and 2 t4 + 1; the 16-byte pieces of a
                 // pair are stored XOR-swizzled by the pair index, which keeps the eight lanes of a quarter-warp on
                 // different banks)
-                const int pr = 8 * warp + 2 * t4;
+                const int pr = 8 * slice + 2 * t4;
                 const uint4 va = *reinterpret_cast<const uint4*>(vst + pr * 128 + ((g ^ (pr & 7)) << 4));
                 const uint4 vb = *reinterpret_cast<const uint4*>(vst + (pr + 1) * 128 + ((g ^ ((pr + 1) & 7)) << 4));
                 const uint32_t xa[4] = {va.x, va.y, va.z, va.w}, xb[4] = {vb.x, vb.y, vb.z, vb.w};
 #pragma unroll
                 for (int grp = 0; grp < 4; ++grp) {
                     // B of the value product: k pairs are (even, odd) tokens of a pair = (tile 0, tile 1) of a column
-                    const uint32_t pa0 = pack_f16(pv[0][0] * inv[0][0][grp], pv[1][0] * inv[1][0][grp]);
-                    const uint32_t pa2 = pack_f16(pv[0][1] * inv[0][1][grp], pv[1][1] * inv[1][1][grp]);
+                    const float2 w0 = __fmul2_rn(pv[0], inv[0][grp]), w1 = __fmul2_rn(pv[1], inv[1][grp]);
+                    const uint32_t pa0 = pack_f16(w0.x, w1.x), pa2 = pack_f16(w0.y, w1.y);
                     const uint32_t x = xa[grp], y = xb[grp], xs = x >> 8, ys = y >> 8;
                     // nibble n of the even | odd token of a pair as f16x2: 1024 + n (low nibble) or 64 + n (high
                     // nibble) by one logic operation, then n - 8 exactly by one subtraction
@@ -593,10 +654,10 @@ decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
     // CTAs have an SM each the next one's could only wait for this one's shared memory, so it is left to start at the end
     // (131072 tokens x 2 heads, decode after decode: 84.8 us with an early start, 81.5 without).
     if (!a.alone) pdl_trigger();
-    float* sm_o = reinterpret_cast<float*>(smem);                 // [4 warps][8 heads][128]
-    float* sm_m = sm_o + 4 * 8 * D;                               // [4][8]
-    float* sm_l = sm_m + 32;
-    if (warp < 4) {
+    float* sm_o = reinterpret_cast<float*>(smem);                 // [warps][8 heads][128]
+    float* sm_m = sm_o + COMPUTE * 8 * D;                         // [warps][8]
+    float* sm_l = sm_m + COMPUTE * 8;
+    if (warp < COMPUTE) {
         if constexpr (QUANT) {
             // tile (grp, j): columns are heads 2 t4 | 2 t4 + 1, rows elements 32 grp + 4 g + 2 j | + 1
 #pragma unroll
@@ -614,20 +675,23 @@ decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
     }
     __syncthreads();
     const int rows = a.B * a.Hq;
-    float* cl_o = sm_l + 32;                                      // cluster form: this split's rows [8][D], then m [8], l [8]
+    const int used = COMPUTE == 4 ? 4 : min(COMPUTE, 4 * (p_end - p_begin));         // warps that had a slice
+    float* cl_o = sm_l + COMPUTE * 8;                                      // cluster form: this split's rows [8][D], then m [8], l [8]
     float* cl_ml = cl_o + 8 * D;
     for (int idx = tid; idx < a.group * D; idx += kThreads) {
         const int h = idx / D, d = idx % D;
         float mt = kEmpty;
 #pragma unroll
-        for (int w = 0; w < 4; ++w) mt = fmaxf(mt, sm_m[w * 8 + h]);
+        for (int w = 0; w < COMPUTE; ++w)
+            if (w < used) mt = fmaxf(mt, sm_m[w * 8 + h]);
         float ov = 0.f, lt = 0.f;
 #pragma unroll
-        for (int w = 0; w < 4; ++w) {
-            const float wgt = ex2(sm_m[w * 8 + h] - mt);
-            ov = fmaf(wgt, sm_o[(w * 8 + h) * D + d], ov);
-            lt = fmaf(wgt, sm_l[w * 8 + h], lt);
-        }
+        for (int w = 0; w < COMPUTE; ++w)
+            if (w < used) {
+                const float wgt = ex2(sm_m[w * 8 + h] - mt);
+                ov = fmaf(wgt, sm_o[(w * 8 + h) * D + d], ov);
+                lt = fmaf(wgt, sm_l[w * 8 + h], lt);
+            }
         const int row = b * a.Hq + kvh * a.group + h;
         if (a.direct) {
             a.out[(size_t)row * D + d] = lt > 0.f ? ov / lt : 0.f;
@@ -896,14 +960,19 @@ bool decode_mma_supported(const grl_decode_params* p) {
     return kv.cache_dtype == GRL_BF16 && geometry && (kv.head_dim == 128 || kv.head_dim == 64) && ((uintptr_t)p->q % 8 == 0);
 }
 
-template <bool QUANT, int HD>
+// The quantised cache's one-CTA-an-SM form: where the CTAs are no more than the SMs and each streams at least 12 stages (see
+// grl_decode_pick_splits).  us, decode alone, pair / wide: 1 x 8 x 131072 tokens 65 / 59, x 65536 43 / 34, x 16384 24 / 18.7, 1 x 2 x
+// 131072 52 / 27, 64 x 2 x 2048 20.7 / 18.9; shorter splits or more CTAs: 1 x 8 x 4096 11.5 / 13.2, 64 x 8 x 500 21 / 29, 32 x 8 x 4096 60 / 65.
+bool decode_mma_wide(const grl_device* dev, int ctas, int stages) { return ctas <= dev->prop.multiProcessorCount && stages >= 12; }
+
+template <int FORM, int HD>
 static int launch_instance(grl_device* dev, const CUtensorMap& tk, const CUtensorMap& tv, dmma::Args a, dim3 grid) {
     using namespace dmma;
+    constexpr int kAlone = FORM == QUANT_WIDE ? Smem<FORM, HD>::TOTAL : kAloneSmem;
     static bool attr_set[64] = {};
     if (!attr_set[dev->ordinal & 63]) {      // a function attribute belongs to the device that was current
-        GRL_CUDA(cudaFuncSetAttribute(decode_mma_kernel<QUANT, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      kAloneSmem));
-        GRL_CUDA(cudaFuncSetAttribute(decode_mma_kernel<QUANT, HD>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        GRL_CUDA(cudaFuncSetAttribute(decode_mma_kernel<FORM, HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAlone));
+        GRL_CUDA(cudaFuncSetAttribute(decode_mma_kernel<FORM, HD>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         attr_set[dev->ordinal & 63] = true;
     }
     // Splits merge in clusters while a split is short, the largest equal share of them whose clusters fit the device at once.
@@ -914,7 +983,7 @@ static int launch_instance(grl_device* dev, const CUtensorMap& tk, const CUtenso
     if (a.fuse && !a.direct && a.x.world <= 1 && a.pps_hint <= 40)
         for (int c = kMaxCluster; c > 1 && a.cluster == 1; --c)
             if (a.n_splits % c == 0 && (int)(grid.y * grid.z) * (a.n_splits / c) <=
-                max_active_clusters(dev, (const void*)decode_mma_kernel<QUANT, HD>, kThreads, Smem<QUANT, HD>::TOTAL, c))
+                max_active_clusters(dev, (const void*)decode_mma_kernel<FORM, HD>, Warps<FORM>::THREADS, Smem<FORM, HD>::TOTAL, c))
                 a.cluster = c;
     // Splits that merge through global memory, at most one CTA for every SM: two of them must not share an SM, which they do when
     // they are placed while the SMs still hold CTAs of the kernel before (a decode that merges, or the append).  So they ask for
@@ -924,11 +993,11 @@ static int launch_instance(grl_device* dev, const CUtensorMap& tk, const CUtenso
     //   append + decode from a stream 99.4, 90.2 and 73.8 for 97.4, 87.2 and 71.6.
     a.alone = a.fuse && !a.direct && a.cluster == 1 && (int)(grid.x * grid.y * grid.z) <= dev->prop.multiProcessorCount;
     if (a.alone)
-        GRL_CUDA(launch_pdl(decode_mma_kernel<QUANT, HD>, grid, kThreads, kAloneSmem, dev->stream, tk, tv, a));
+        GRL_CUDA(launch_pdl(decode_mma_kernel<FORM, HD>, grid, Warps<FORM>::THREADS, kAlone, dev->stream, tk, tv, a));
     else
-        GRL_CUDA(launch_pdl_cluster(decode_mma_kernel<QUANT, HD>, grid, kThreads, Smem<QUANT, HD>::TOTAL, dev->stream,
+        GRL_CUDA(launch_pdl_cluster(decode_mma_kernel<FORM, HD>, grid, Warps<FORM>::THREADS, Smem<FORM, HD>::TOTAL, dev->stream,
                                     a.cluster, tk, tv, a));
-    GRL_LAUNCHED(QUANT ? "decode_mma_kernel<quantised>" : "decode_mma_kernel");
+    GRL_LAUNCHED(FORM == BF16 ? "decode_mma_kernel" : "decode_mma_kernel<quantised>");
     return GRL_OK;
 }
 
@@ -983,8 +1052,10 @@ int decode_mma_launch(grl_device* dev, const grl_decode_params* p, int n_splits,
     }
     dev->status_dirty = true;
     dim3 grid(n_splits, kv.num_kv_heads, kv.batch);
-    if (quant) return launch_instance<true, 128>(dev, tk, tv, a, grid);
-    return kv.head_dim == 64 ? launch_instance<false, 64>(dev, tk, tv, a, grid) : launch_instance<false, 128>(dev, tk, tv, a, grid);
+    if (quant)
+        return decode_mma_wide(dev, kv.batch * kv.num_kv_heads * n_splits, a.pps_hint) ? launch_instance<QUANT_WIDE, 128>(dev, tk, tv, a, grid)
+                                                                                       : launch_instance<QUANT_PAIR, 128>(dev, tk, tv, a, grid);
+    return kv.head_dim == 64 ? launch_instance<BF16, 64>(dev, tk, tv, a, grid) : launch_instance<BF16, 128>(dev, tk, tv, a, grid);
 }
 
 }  // namespace grl

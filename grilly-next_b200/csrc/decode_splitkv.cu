@@ -353,22 +353,23 @@ int grl_decode_pick_splits(grl_device* dev, const grl_decode_params* p, int* n_s
         // Two CTAs an SM (twice the bytes in flight, or twice the warps that dequantise) while the splits of a head are one
         // cluster: a power of two up to 16, which packs into the GPCs (16 sequences x 8 heads x 4096 tokens: 63 us unsplit, 51 us
         // in 2 splits; 4 x 8 x 2048: 15.0 us in 8 splits, 19.1 in 9).  Few heads: one CTA an SM over the bf16 cache (131072 tokens
-        // x 8 heads, append + decode: 97 us with 18 splits, 97 with 36; decode alone 93 and 94), two over the quantised one (104 us with
-        // 18, 78 with 37), in whole clusters of 16 of at least 8 stages a split while splits are short enough to merge in clusters (see
-        // launch_instance).
+        // x 8 heads, append + decode: 97 us with 18 splits, 97 with 36; decode alone 93 and 94) and over the quantised one where each
+        // CTA then has 12 stages or more (decode_mma_wide: twelve compute warps a CTA); below that two over the quantised one, in whole
+        // clusters of 16 of at least 8 stages a split while splits are short enough to merge in clusters (see launch_instance).
         // More (sequence, head) pairs than SMs: unsplit (us, unsplit / 2 splits, decode alone: 19 x 8 x 8192 tokens 114 / 142, 25 x 8 x
-        // 4096 67 / 82, 32 x 8 x 4096 81 / 92, 37 x 8 x 2048 52 / 62; quantised 25 x 8 x 4096 66 / 73, 32 x 8 x 4096 66 / 78; lengths from 4096 to
-        // 8192 24 x 8 106 / 114).  Just past one CTA an SM two splits would be the better ones where lengths differ or the cache is
-        // quantised (20 x 8, 4096 to 8192 tokens: 95 / 90, quantised 108 / 77; quantised 19 x 8 x 8192 131 / 116): not distinguished here.
-        const int twice = 2 * sms / base_ctas;
+        // 4096 67 / 82, 32 x 8 x 4096 81 / 92, 37 x 8 x 2048 52 / 62; quantised, before its present form, 25 x 8 x 4096 66 / 73, 32 x 8 x 4096
+        // 66 / 78; lengths from 4096 to 8192 24 x 8 106 / 114).  Just past one CTA an SM two splits would be the better ones where lengths
+        // differ or the cache is quantised (20 x 8, 4096 to 8192 tokens: 95 / 90): not distinguished here.
+        const bool quant = kv.cache_dtype == GRL_FP8_INT4;
+        const bool one = quant && base_ctas <= sms && (long long)pages * base_ctas >= 12LL * sms;
+        const int most = (one ? 1 : 2) * sms / base_ctas, wide = (quant && !one ? 2 : 1) * sms / base_ctas;
         if (base_ctas > sms) s = 1;
-        else if (twice < 32) {
+        else if (most < 32) {
             s = 1;
-            while (2 * s <= twice) s *= 2;
-            const int wide = kv.cache_dtype == GRL_FP8_INT4 ? twice : sms / base_ctas;
+            while (2 * s <= most) s *= 2;
             if (s == 16 && pages > 32 * wide) s = wide;
         } else {
-            s = kv.cache_dtype == GRL_FP8_INT4 ? twice : sms / base_ctas;
+            s = wide;
             if (pages <= 32 * s) {
                 if (s > pages / 8) s = pages / 8;
                 s = s < 32 ? 16 : s / 16 * 16;

@@ -127,6 +127,42 @@ def test_tensor_core_decode_over_the_quantised_cache(Hq, Hkv, lens, P):
         dev.close()
 
 
+@pytest.mark.parametrize("Hq,Hkv,lens,P,splits", [
+    (8, 2, (768,), 64, 1), (8, 2, (767,), 64, 1), (4, 1, (897, 12), 32, 1), (16, 2, (2000, 1, 1985), 64, 1),       # 12 stages; the ring's 14
+    (8, 8, (5000,), 16, 1), (32, 8, (9000, 8999), 64, 5), (3, 1, (16400,), 16, 17), (8, 2, (40000,), 64, 48)])     # clusters; splits apart
+def test_one_cta_an_sm_decode_over_the_quantised_cache(Hq, Hkv, lens, P, splits):
+    """Splits of 12 stages and more, no more CTAs than SMs: twelve compute and four producer warps a CTA.  Against the oracle on the
+    same quantised cache and against the form of short splits, tolerance as for the other tensor-core cases."""
+    from grilly_next import cabi
+    from gpu_helpers import PagedCache
+    from oracle import attention_oracle as orc
+    dev = cabi.Device(0)
+    try:
+        rng = np.random.default_rng(sum(lens) + P)
+        B, D, T = len(lens), 128, max(lens)
+        k = rng.standard_normal((B, T, Hkv, D), dtype=np.float32) * rng.uniform(0.2, 3.0, (B, T, Hkv, 1)).astype(np.float32)
+        v = rng.standard_normal((B, T, Hkv, D), dtype=np.float32)
+        q = rng.standard_normal((B, 1, Hq, D), dtype=np.float32)
+        pc = PagedCache(dev, B, Hkv, D, T + 64, page_tokens=P, dtype=cabi.FP8_INT4, shuffle_pages=True, seed=6)
+        pc.append(k, v)
+        cut = np.array(lens, np.int32)
+        dev.L.grl_memcpy_h2d(dev.h, pc.seq_lens, cut.ctypes.data_as(C.c_void_p), cut.nbytes)
+        dev.sync()
+        pc.lens[:] = cut
+        kd, vd = _dequantised(k, v)
+        want = np.concatenate([orc.gqa_decode_attention(q[b:b + 1], kd[b:b + 1, :lens[b]], vd[b:b + 1, :lens[b]], Hq, Hkv, D)
+                               for b in range(B)])
+        tol = 1e-3 * np.abs(want).max()
+        got = pc.decode(q, n_splits=splits)
+        assert np.abs(got - want).max() <= tol
+        part = pc.decode(q, n_splits=max(2, splits), partial=True)
+        o, l = part[:B * Hq * D].reshape(B, 1, Hq, D), part[B * Hq * (D + 1):].reshape(B, 1, Hq, 1)
+        assert np.abs(o / l - want).max() <= tol
+        assert np.abs(pc.decode(q, n_splits=min(256, (T + 63) // 64 // 4)) - want).max() <= tol        # short splits
+    finally:
+        dev.close()
+
+
 def test_quantised_append_with_rope_and_queries():
     """RoPE of the new keys happens before the quantiser; the step's queries are rotated alongside."""
     from grilly_next import cabi
