@@ -316,9 +316,32 @@ __device__ __forceinline__ float fp8_decode(uint8_t c) {                    // k
     return s ? -v : v;
 }
 
-// grid (ceil(n_new*Hkv*G / warps per CTA), B), G = D/32 groups per head.  With one CTA per sequence (a decode step) the
-// kernel also rotates the step's queries (q_in != NULL) and advances the length (update_lens): one launch per step.
-__global__ void __launch_bounds__(1024) kv_append_quant_kernel(const __grid_constant__ AppendArgs a) {
+// One group of 32 elements of one token and kv head, an element a lane: scales, key byte, value nibble.
+__device__ __forceinline__ void quantise_group(const AppendArgs& a, float kx, float vx, int page, int h, int slot, int g, int lane) {
+    const int G = a.D / 32, half = a.D / 2, d = g * 32 + lane;
+    uint8_t* kp = reinterpret_cast<uint8_t*>(a.k_pages);
+    uint8_t* vp = reinterpret_cast<uint8_t*>(a.v_pages);
+    float kmax = fabsf(kx), vmax = fabsf(vx);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        kmax = fmaxf(kmax, __shfl_xor_sync(0xffffffffu, kmax, o));
+        vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
+    }
+    const float kscale = kmax > 0.f ? __fdiv_rn(448.0f, kmax) : 1.0f;
+    const float vscale = vmax > 0.f ? __fdiv_rn(7.0f, vmax) : 1.0f;
+    const size_t row = ((size_t)page * a.Hkv + h) * a.P + slot;
+    kp[row * a.D + d] = fp8_encode(__fmul_rn(kx, kscale));
+    int q = (int)roundf(__fmul_rn(vx, vscale)) + 8;                       // kv_cache.cpp:363-366
+    q = max(0, min(15, q));
+    const int q_hi = __shfl_down_sync(0xffffffffu, q, 1);
+    if ((lane & 1) == 0)
+        vp[((size_t)page * a.Hkv + h) * a.P * half + quant_v_off(slot, d >> 1, a.D)] =
+            (uint8_t)((q & 0x0F) | ((q_hi & 0x0F) << 4));
+    if (lane == 0) a.scales[row * G + g] = scale_to_half_bits(kscale);   // the value scale is dropped (:393-398)
+}
+
+// Bulk: grid (ceil(n_new*Hkv*G / warps per CTA), B), G = D/32 groups per head.
+__global__ void __launch_bounds__(256) kv_append_quant_kernel(const __grid_constant__ AppendArgs a) {
     const int b = blockIdx.y, lane = threadIdx.x & 31;
     const int G = a.D / 32;
     pdl_wait();
@@ -336,8 +359,6 @@ __global__ void __launch_bounds__(1024) kv_append_quant_kernel(const __grid_cons
     // an item is one group of one token for a run of heads: the angles of its elements are the same for all of them
     const int half = a.D / 2, per = a.heads_per_item, runs = (a.Hkv + per - 1) / per;
     const int items = a.n_new * runs * G;
-    uint8_t* kp = reinterpret_cast<uint8_t*>(a.k_pages);
-    uint8_t* vp = reinterpret_cast<uint8_t*>(a.v_pages);
     for (int item = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); item < items; item += gridDim.x * (blockDim.x >> 5)) {
         const int g = item % G, h0 = ((item / G) % runs) * per, i = item / (G * runs);
         const int d = g * 32 + lane;
@@ -360,43 +381,91 @@ __global__ void __launch_bounds__(1024) kv_append_quant_kernel(const __grid_cons
                 kx = first ? kx * c - other * s : other * s + kx * c;
             }
             const float vx = a.v_new[src + d];
-            float kmax = fabsf(kx), vmax = fabsf(vx);
+            quantise_group(a, kx, vx, page, h, slot_pos % a.P, g, lane);
+        }
+    }
+}
+
+// A decode step, or as few tokens: one CTA a sequence, a warp a (token, kv head, group of 32), and the step's queries and its length
+// with them.  Latency: what does not depend on the length is read beside it, and an angle is formed once, in shared memory, for all
+// heads (forming it per key element and per query pair took most of the kernel: 1 sequence x 8 kv heads, append before decode
+// 8.0 -> 4.3 us of the step).
+constexpr int kStepWarps = 32;
+__global__ void __launch_bounds__(32 * kStepWarps) kv_append_quant_step_kernel(const __grid_constant__ AppendArgs a) {
+    __shared__ float2 cs[kStepWarps * 16];           // (cos, sin) [token][pair]: n_new * D / 2 <= 32 * 32 / 2
+    const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+    const int G = a.D / 32, half = a.D / 2, angles = a.n_new * half;
+    const bool rope = a.rope_mode != GRL_ROPE_NONE;
+    const double freq = rope && tid < angles ? a.freq.inv_freq[tid % half] : 0.0;
+    const int item = tid >> 5, g = item % G, h = (item / G) % a.Hkv, i = item / (G * a.Hkv), d = g * 32 + lane;
+    const bool live = item < a.n_new * a.Hkv * G;
+    int j = 0, d_other = d;
+    bool first = true;
+    if (a.rope_mode == GRL_ROPE_INTERLEAVED) { j = d >> 1; first = (d & 1) == 0; d_other = d ^ 1; }
+    else if (rope) { j = d % half; first = d < half; d_other = first ? d + half : d - half; }
+    pdl_wait();
+    pdl_trigger();      // the decode that follows sets itself up meanwhile
+    const int len0 = a.seq_lens[b], pos_off = a.pos_offsets ? a.pos_offsets[b] : 0;
+    const size_t src = (((size_t)b * a.n_new + i) * a.Hkv + h) * a.D;
+    float kx = 0.f, other = 0.f, vx = 0.f;
+    if (live) { kx = a.k_new[src + d]; other = a.k_new[src + d_other]; vx = a.v_new[src + d]; }
+    // this thread's first query pairs
+    constexpr int kAhead = 2;
+    const int qitems = a.q_in ? a.n_new * a.Hq * half : 0;
+    float q0[kAhead], q1[kAhead];
+    auto q_place = [&](int idx, int* d0, int* d1) -> size_t {
+        const int jq = idx % half;
+        *d0 = a.rope_mode == GRL_ROPE_HALF ? jq : 2 * jq;
+        *d1 = a.rope_mode == GRL_ROPE_HALF ? jq + half : 2 * jq + 1;
+        return ((size_t)b * a.n_new * a.Hq + idx / half) * a.D;
+    };
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                kmax = fmaxf(kmax, __shfl_xor_sync(0xffffffffu, kmax, o));
-                vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
-            }
-            const float kscale = kmax > 0.f ? __fdiv_rn(448.0f, kmax) : 1.0f;
-            const float vscale = vmax > 0.f ? __fdiv_rn(7.0f, vmax) : 1.0f;
-            const size_t row = ((size_t)page * a.Hkv + h) * a.P + slot_pos % a.P;
-            kp[row * a.D + d] = fp8_encode(__fmul_rn(kx, kscale));
-            int q = (int)roundf(__fmul_rn(vx, vscale)) + 8;                       // kv_cache.cpp:363-366
-            q = max(0, min(15, q));
-            const int q_hi = __shfl_down_sync(0xffffffffu, q, 1);
-            if ((lane & 1) == 0)
-                vp[((size_t)page * a.Hkv + h) * a.P * half + quant_v_off(slot_pos % a.P, d >> 1, a.D)] =
-                    (uint8_t)((q & 0x0F) | ((q_hi & 0x0F) << 4));
-            if (lane == 0) a.scales[row * G + g] = scale_to_half_bits(kscale);   // the value scale is dropped (:393-398)
+    for (int e = 0; e < kAhead; ++e) {
+        const int idx = tid + e * 32 * kStepWarps;
+        int d0, d1;
+        q0[e] = q1[e] = 0.f;
+        if (idx < qitems) { const size_t qo = q_place(idx, &d0, &d1); q0[e] = a.q_in[qo + d0]; q1[e] = a.q_in[qo + d1]; }
+    }
+    if (len0 < 0 || len0 + a.n_new > a.max_pages * a.P) {
+        if (tid == 0 && a.status && atomicCAS(a.status, 0, GRL_ERR_INVALID) == 0) {
+            a.status[1] = 4 << 28;
+            a.status[2] = b;
+            a.status[3] = len0;
         }
+        return;
     }
-    if (a.q_in) {           // the queries of the new positions, rotated like the keys (float32 in, float32 out)
-        const int qitems = a.n_new * a.Hq * half;
-        for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < qitems; idx += gridDim.x * blockDim.x) {
-            const int j = idx % half, h = (idx / half) % a.Hq, i = idx / (half * a.Hq);
-            int d0 = 2 * j, d1 = 2 * j + 1;
-            if (a.rope_mode == GRL_ROPE_HALF) { d0 = j; d1 = j + half; }
-            float c = 1.f, s = 0.f;
-            if (a.rope_mode != GRL_ROPE_NONE) rope_sincos(a.pos_base + pos_off + len0 + i, a.freq.inv_freq[j], &c, &s);
-            const size_t qo = (((size_t)b * a.n_new + i) * a.Hq + h) * a.D;
-            const float q0 = a.q_in[qo + d0], q1 = a.q_in[qo + d1];
-            a.q_out[qo + d0] = q0 * c - q1 * s;
-            a.q_out[qo + d1] = q0 * s + q1 * c;
+    const int slot_pos = len0 + i;
+    const int page = live ? a.block_table[(size_t)b * a.max_pages + slot_pos / a.P] : 0;
+    if (rope && tid < angles) {
+        float c, s;
+        rope_sincos(a.pos_base + pos_off + len0 + tid / half, freq, &c, &s);
+        cs[tid] = make_float2(c, s);
+    }
+    __syncthreads();
+    if (live) {
+        if (rope) {
+            const float c = cs[i * half + j].x, s = cs[i * half + j].y;
+            kx = first ? kx * c - other * s : other * s + kx * c;
         }
+        quantise_group(a, kx, vx, page, h, slot_pos % a.P, g, lane);
     }
-    if (a.update_lens) {    // gridDim.x == 1 here: every warp has read len0
-        __syncthreads();
-        if (threadIdx.x == 0) a.seq_lens[b] = len0 + a.n_new;
+    auto rotate_q = [&](int idx, float x0, float x1) {
+        int d0, d1;
+        const size_t qo = q_place(idx, &d0, &d1);
+        float c = 1.f, s = 0.f;
+        if (rope) { const float2 v = cs[idx / (half * a.Hq) * half + idx % half]; c = v.x; s = v.y; }
+        a.q_out[qo + d0] = x0 * c - x1 * s;
+        a.q_out[qo + d1] = x0 * s + x1 * c;
+    };
+#pragma unroll
+    for (int e = 0; e < kAhead; ++e)
+        if (tid + e * 32 * kStepWarps < qitems) rotate_q(tid + e * 32 * kStepWarps, q0[e], q1[e]);
+    for (int idx = tid + kAhead * 32 * kStepWarps; idx < qitems; idx += 32 * kStepWarps) {
+        int d0, d1;
+        const size_t qo = q_place(idx, &d0, &d1);
+        rotate_q(idx, a.q_in[qo + d0], a.q_in[qo + d1]);
     }
+    if (a.update_lens && tid == 0) a.seq_lens[b] = len0 + a.n_new;      // every warp has read len0: the barrier above
 }
 
 // Dequantise sequence b as token-major float32 (T, Hkv, D): kv_cache.cpp:500-577.  One thread per element.
@@ -518,11 +587,10 @@ int grl_kv_append(grl_device* dev, const grl_append_params* p) {
     if (kv.cache_dtype == GRL_FP8_INT4) {
         // K and V: one warp per (token, kv head, group of 32); the queries, if any, through the plain kernel
         const long long warps = (long long)p->n_new * kv.num_kv_heads * (kv.head_dim / 32);
-        if (warps <= 32) {      // a decode step: one wide CTA per sequence does keys, values, queries and the length
+        if (warps <= kStepWarps) {      // a decode step: one wide CTA per sequence does keys, values, queries and the length
             a.update_lens = p->update_lens ? 1 : 0;
-            a.heads_per_item = 1;
-            GRL_CUDA(launch_pdl(kv_append_quant_kernel, dim3(1, kv.batch), 1024, 0, dev->stream, a));
-            GRL_LAUNCHED("kv_append_quant_kernel");
+            GRL_CUDA(launch_pdl(kv_append_quant_step_kernel, dim3(kv.batch), 32 * kStepWarps, 0, dev->stream, a));
+            GRL_LAUNCHED("kv_append_quant_step_kernel");
             return GRL_OK;
         }
         // eight heads a warp once there are enough tokens to fill the SMs (64 warps each) all the same

@@ -190,6 +190,39 @@ def test_quantised_append_with_rope_and_queries():
         dev.close()
 
 
+@pytest.mark.parametrize("D,Hq,Hkv,n", [(128, 32, 8, 1), (128, 4, 1, 8), (128, 3, 3, 2), (64, 70, 2, 7), (32, 5, 5, 6), (32, 2, 1, 32), (256, 8, 4, 1)])
+@pytest.mark.parametrize("mode", ["none", "interleaved", "half"])
+def test_quantised_append_in_steps_stores_what_a_bulk_append_does(D, Hq, Hkv, n, mode):
+    """A step of at most 32 (token, kv head, group) warps has a kernel of its own: the same bytes as one call with
+    all the tokens, and its rotated queries to the last bit but the order of one rounding, at positions that start anywhere, and the lengths advance."""
+    from grilly_next import cabi
+    from gpu_helpers import PagedCache
+    assert n * Hkv * (D // 32) <= 32
+    dev = cabi.Device(0)
+    try:
+        rng = np.random.default_rng(D + n)
+        B, T = 2, 3 * n + 40
+        k, v = (rng.standard_normal((B, T, Hkv, D), dtype=np.float32) for _ in range(2))
+        q = rng.standard_normal((B, T, Hq, D), dtype=np.float32)
+        kw = {"rope_mode": {"none": cabi.ROPE_NONE, "interleaved": cabi.ROPE_INTERLEAVED, "half": cabi.ROPE_HALF}[mode]}
+        off = dev.upload(np.asarray([3, 70000], np.int32))
+        whole, steps = (PagedCache(dev, B, Hkv, D, T, page_tokens=16, dtype=cabi.FP8_INT4, shuffle_pages=True, seed=8) for _ in range(2))
+        want_q = whole.append(k, v, q=q, pos_base=5, pos_offsets=off, **kw)
+        steps.append(k[:, :40], v[:, :40], pos_base=5, pos_offsets=off, **kw)
+        got_q = [steps.append(k[:, t:t + n], v[:, t:t + n], q=q[:, t:t + n], pos_base=5, pos_offsets=off, **kw) for t in range(40, T, n)]
+        # x0 c - x1 s with one product fused into the subtraction, which of them is the compiler's choice in each kernel: each result is
+        # within half an ulp of the unfused product and of the result, 2^-24 (|x| + |y|) <= 2^-23 (|x0| + |x1|) of the exact value
+        q = np.abs(q[:, 40:])
+        pair = q + {"none": 0 * q, "half": np.roll(q, D // 2, -1), "interleaved": q.reshape(*q.shape[:-1], D // 2, 2)[..., ::-1].reshape(q.shape)}[mode]
+        assert (np.abs(np.concatenate(got_q, 1) - want_q[:, 40:]) <= 2.0 ** -22 * pair).all()
+        for b in range(B):
+            for got, want in zip(_stored(dev, steps, b, T), _stored(dev, whole, b, T)):
+                assert np.array_equal(got, want)
+        assert (dev.download(steps.seq_lens, (B,), np.int32) == T).all()
+    finally:
+        dev.close()
+
+
 def test_python_ops_on_a_quantised_cache():
     """create_kv_cache(use_asymmetric_quant=True): append, kv_cache_decode (dequantised, bit for bit) and decode."""
     import grilly_core
