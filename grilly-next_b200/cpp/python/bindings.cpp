@@ -283,8 +283,14 @@ PYBIND11_MODULE(grilly_core, m) {
             if (seqLens.has_value()) {
                 if (seqLens->ndim() != 1 || seqLens->shape(0) != B) throw std::runtime_error("seq_lens must be (batch,)");
                 lens = ctx->pool.acquire(size_t(B) * 4);
-                ctx->pool.upload(lens, seqLens->data(), size_t(B) * 4);
-                check(grl_sync(ctx->device.handle(), 0), "flash_attention2: seq_lens upload");
+                // The lengths leave the caller's array at the call.  A copy had to be waited for, and with it all the work before it
+                // (2 x 8 heads x 68 tokens 28.9 -> 8.9 us a call, 8 x 32 heads of up to 4096 tokens 801 -> 773).
+                if (size_t(B) * 4 <= GRL_PUT_BYTES) {
+                    check(grl_put(ctx->device.handle(), lens.dptr, seqLens->data(), size_t(B) * 4), "flash_attention2: seq_lens upload");
+                } else {
+                    ctx->pool.upload(lens, seqLens->data(), size_t(B) * 4);
+                    check(grl_sync(ctx->device.handle(), 0), "flash_attention2: seq_lens upload");
+                }
             }
             const ops::RopeMode mode = ropeTheta != 0.0f ? parseRopeMode(ropeMode, false) : ops::RopeMode::None;
             try {

@@ -172,6 +172,15 @@ __global__ void cast_kernel(const S* __restrict__ src, D* __restrict__ dst, size
     for (; i < n; i += stride) store_from_float<D>(dst + i, load_as_float<S>(src + i));
 }
 
+struct PutArgs {
+    uint32_t word[GRL_PUT_BYTES / 4];
+};
+__global__ void __launch_bounds__(GRL_PUT_BYTES / 4) put_kernel(uint32_t* dst, int n, const __grid_constant__ PutArgs a) {
+    pdl_wait();
+    pdl_trigger();
+    if ((int)threadIdx.x < n) dst[threadIdx.x] = a.word[threadIdx.x];
+}
+
 // 8 elements per thread with 16/32-byte accesses; n8 = n / 8.
 __global__ void cast_f32_bf16_vec8(const float4* __restrict__ src, uint4* __restrict__ dst, size_t n8) {
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -365,6 +374,21 @@ int grl_memcpy_h2d(grl_device* dev, void* dst, const void* src_host, size_t byte
         return GRL_OK;
     }
     GRL_CUDA(cudaMemcpyAsync(dst, src_host, bytes, cudaMemcpyHostToDevice, dev->stream));
+    return GRL_OK;
+}
+
+int grl_put(grl_device* dev, void* dst, const void* src_host, size_t bytes) {
+    GRL_REQUIRE(dev && dst && src_host, "NULL argument");
+    GRL_REQUIRE(bytes > 0 && bytes <= GRL_PUT_BYTES && bytes % 4 == 0 && (uintptr_t)dst % 4 == 0,
+                "grl_put takes up to %d bytes in whole words (got %zu)", GRL_PUT_BYTES, bytes);
+    DeviceGuard g(dev->ordinal);
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    GRL_CUDA(cudaStreamIsCapturing(dev->stream, &cap));
+    GRL_REQUIRE(cap == cudaStreamCaptureStatusNone, "grl_put is not for a stream capture: its bytes are those of the call");
+    PutArgs a;
+    memcpy(a.word, src_host, bytes);
+    GRL_CUDA(launch_pdl(put_kernel, dim3(1), dim3(GRL_PUT_BYTES / 4), 0, dev->stream, (uint32_t*)dst, (int)(bytes / 4), a));
+    GRL_LAUNCHED("put_kernel");
     return GRL_OK;
 }
 

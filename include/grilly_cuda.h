@@ -96,6 +96,10 @@ int grl_free(grl_device* dev, void* ptr);
 int grl_host_alloc(size_t bytes, void** out); /* pinned host memory for staging */
 int grl_host_free(void* ptr);
 int grl_memcpy_h2d(grl_device* dev, void* dst, const void* src_host, size_t bytes);
+/* At most GRL_PUT_BYTES (a multiple of 4) from host memory of any kind, as an argument of a kernel: the bytes are taken at the call, which
+   returns at once, and no copy engine is involved.  Not in a stream capture. */
+#define GRL_PUT_BYTES 960
+int grl_put(grl_device* dev, void* dst, const void* src_host, size_t bytes);
 int grl_memcpy_d2h(grl_device* dev, void* dst_host, const void* src, size_t bytes);
 /* The same in up to 64 parts: bytes [i*part_bytes, (i+1)*part_bytes) are copied once parts[i] has completed, so that the copy of
  * one part of a result runs beside the kernel that makes the next. */

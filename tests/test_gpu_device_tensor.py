@@ -61,6 +61,53 @@ def test_flash_on_device_tensors_equals_host_path(core, ctx, dtype):
         core.flash_attention2(ctx, tq, tk, core.DeviceTensor.empty(ctx, (B, H, S, 64), dtype))
 
 
+def test_ragged_calls_in_a_row_take_their_lengths_at_the_call(core, ctx):
+    """Nothing is waited for between ragged calls: the lengths are those of the call, whatever becomes of the array, also where
+    there are more of them than travel as a kernel argument (240), and the pooled buffer they go to is the same each time."""
+    rng = np.random.default_rng(6)
+    for B, S in ((3, 300), (240, 17), (241, 17)):
+        Q, K, V = (core.DeviceTensor.from_numpy(ctx, rng.standard_normal((B, 2, S, 64), dtype=np.float32), dtype="bf16") for _ in range(3))
+        all_lens = [rng.integers(1, S + 1, B).astype(np.int32) for _ in range(4)]
+        want = []
+        for lens in all_lens:
+            o = core.flash_attention2(ctx, Q, K, V, causal=True, seq_lens=lens)
+            want.append(o.to_numpy())
+        outs, lens = [], np.empty(B, np.int32)
+        for l in all_lens:
+            lens[:] = l
+            outs.append(core.flash_attention2(ctx, Q, K, V, causal=True, seq_lens=lens))
+            lens[:] = 1
+        for o, w, l in zip(outs, want, all_lens):
+            got = o.to_numpy()
+            assert np.array_equal(got, w)
+            assert all((got[b, :, l[b]:] == 0).all() and (got[b, :, l[b] - 1] != 0).any() for b in range(B))
+
+
+def test_put_sizes_and_refusals():
+    import ctypes as C
+    from grilly_next import cabi
+    dev = cabi.Device(0)
+    try:
+        src = np.arange(1, 242, dtype=np.uint32)
+        for n in (1, 31, 240):
+            d = dev.upload(np.zeros(241, np.uint32))
+            cabi.check(dev.L.grl_put(dev.h, d, src.ctypes.data, 4 * n))
+            got = dev.download(d, (241,), np.uint32)
+            assert np.array_equal(got[:n], src[:n]) and not got[n:].any()
+            dev.free(d)
+        d = dev.malloc(1024)
+        for n in (0, 6, 964):
+            assert dev.L.grl_put(dev.h, d, src.ctypes.data, n) == -1
+        cabi.check(dev.L.grl_graph_begin(dev.h))
+        assert dev.L.grl_put(dev.h, d, src.ctypes.data, 4) == -1 and b"capture" in dev.L.grl_last_error()
+        g = C.c_void_p()
+        cabi.check(dev.L.grl_graph_end(dev.h, C.byref(g)))
+        dev.L.grl_graph_destroy(g)
+        dev.free(d)
+    finally:
+        dev.close()
+
+
 def test_decode_on_device_tensors_equals_host_path(core, ctx):
     rng = np.random.default_rng(3)
     B, Hq, Hkv, D, T = 2, 8, 2, 128, 150
