@@ -11,7 +11,7 @@
 // shared memory and leave the CTA as (O un-normalised, m, l), the layout lse_merge_kernel reads.  Splits of one head that fit a
 // thread-block cluster merge through its shared memory instead, and a launch sets up its ring and barriers under the kernel before
 // it.  Append + decode step: 1 sequence x 8 kv heads x 1001 tokens 19.4 us before, 9.9 now (latency); 32 x 8 x 4096 93 and 85 us
-// (HBM); 1 x 8 x 131072 104 and 94 us (HBM; the decode alone 90), quantised 107 and 71 us (instructions: some 450 a 16-token slice).
+// (HBM); 1 x 8 x 131072 104 and 94 us (HBM; the decode alone 90), quantised 107 and 60 us (instructions: 444 a 16-token slice).
 //
 // The same kernel, instantiated for the quantised cache (GRL_FP8_INT4: FP8-E4M3 keys, INT4 values, one float16 scale
 // per 32 key elements, cpp/src/ops/kv_cache.cpp:272-399 and :500-577), streams 12.5 KiB per (page, kv head) instead
@@ -170,14 +170,6 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(dst), "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(bar) : "memory");
 }
-// f16 form of the same product.  Rows 8..15 of the accumulator (d[2], d[3]) multiply the zero half of A: they stay
-// whatever they were and are never read, but they stay in place -- the instruction wants four consecutive registers,
-// and carving two live ones out of the quad costs a move and a clear around every product.
-__device__ __forceinline__ void mma_f16(float (&d)[4], uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%5}, {%7,%8}, {%0,%1,%2,%3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a0), "r"(0u), "r"(a2), "r"(b0), "r"(b1));
-}
 // All sixteen rows of A live (the transposed value product: rows are head_dim elements, columns query heads).
 __device__ __forceinline__ void mma_f16_full(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                              uint32_t b1) {
@@ -185,11 +177,11 @@ __device__ __forceinline__ void mma_f16_full(float (&d)[4], uint32_t a0, uint32_
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-// The first product of a chain: C is zero (no register needs clearing for it).
-__device__ __forceinline__ void mma_f16_first(float (&d)[4], uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%5}, {%7,%8}, {%9,%9,%9,%9};"
+// The same with C zero.
+__device__ __forceinline__ void mma_f16_zero(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
         : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-        : "r"(a0), "r"(0u), "r"(a2), "r"(b0), "r"(b1), "f"(0.f));
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
 }
 __device__ __forceinline__ uint32_t pack_f16(float lo, float hi) {
     __half2 v = __floats2half2_rn(lo, hi);
@@ -209,14 +201,20 @@ __device__ __forceinline__ uint32_t prmt(uint32_t w, uint32_t selector) {   // a
 __device__ __forceinline__ uint32_t e4m3_pair02_f16x2(uint32_t w) { return (prmt(w, 0xA280u) << 7) & 0xBF80BF80u; }
 __device__ __forceinline__ uint32_t e4m3_pair13_f16x2(uint32_t w) { return (prmt(w, 0xB391u) << 7) & 0xBF80BF80u; }
 // Value codes to f16x2 (low half: even token of the pair, high half: odd token): the nibble is placed in the mantissa of
-// 1024 (bits 0-3) or of 64 (bits 4-7), and the offset plus the code's bias of 8 is subtracted, which is exact in f16.
+// 1024 (bits 0-3) or of 64 (bits 4-7) by one three-input operation (mask and literal: the compiler makes two of it), and the
+// offset plus the code's bias of 8 is subtracted, which is exact in f16.
+__device__ __forceinline__ uint32_t and_or(uint32_t w, uint32_t mask, uint32_t bits) {
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(w), "r"(mask), "r"(bits));
+    return r;
+}
 __device__ __forceinline__ uint32_t nib_lo(uint32_t w) {
-    const uint32_t v = (w & 0x000F000Fu) | 0x64006400u, off = 0x64086408u;    // 1032, 1032
+    const uint32_t v = and_or(w, 0x000F000Fu, 0x64006400u), off = 0x64086408u;    // 1032, 1032
     __half2 r = __hsub2(*reinterpret_cast<const __half2*>(&v), *reinterpret_cast<const __half2*>(&off));
     return *reinterpret_cast<uint32_t*>(&r);
 }
 __device__ __forceinline__ uint32_t nib_hi(uint32_t w) {
-    const uint32_t v = (w & 0x00F000F0u) | 0x54005400u, off = 0x54805480u;    // 72, 72
+    const uint32_t v = and_or(w, 0x00F000F0u, 0x54005400u), off = 0x54805480u;    // 72, 72
     __half2 r = __hsub2(*reinterpret_cast<const __half2*>(&v), *reinterpret_cast<const __half2*>(&off));
     return *reinterpret_cast<uint32_t*>(&r);
 }
@@ -412,7 +410,11 @@ decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         // Tokens: column n of score tile nt is token 2 n + nt of the warp's 16 (so that a half-warp's key loads hit
         // all banks once), and a lane's four scores are the four consecutive tokens 4 t4 .. 4 t4 + 3.
         const int qh0 = kvh * a.group;
-        uint32_t qf[8][2];
+        // A of a group's two k-steps is one operand: rows 0..7 the query heads of step w = 0, rows 8..15 those of w = 1.  A product's
+        // other half goes unused, as the rows beyond the heads did before, and no operand needs a zero register moved in beside the
+        // two live ones: with the nibbles' three-input operation 505 -> 444 instructions a slice, append + decode of 131072 tokens x
+        // 8 heads 64.4 -> 59.6 us, 32 sequences x 4096 67.5 -> 61.8.
+        uint32_t qf[4][4];
         {
             const float sc = a.scale * kLog2e * 256.f;      // the key registers hold code / 256
             const float* qrow = a.q + ((size_t)b * a.Hq + qh0 + g) * D;
@@ -421,8 +423,8 @@ decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
             for (int ks = 0; ks < 8; ++ks) {
                 float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (live) v = *reinterpret_cast<const float4*>(qrow + 32 * (ks >> 1) + 8 * t4 + 4 * (ks & 1));
-                qf[ks][0] = pack_f16(v.x * sc, v.z * sc);      // with the key codes of bytes 0 and 2 of the word
-                qf[ks][1] = pack_f16(v.y * sc, v.w * sc);      // bytes 1 and 3
+                qf[ks >> 1][ks & 1] = pack_f16(v.x * sc, v.z * sc);            // with the key codes of bytes 0 and 2 of the word
+                qf[ks >> 1][2 + (ks & 1)] = pack_f16(v.y * sc, v.w * sc);      // bytes 1 and 3
             }
         }
         float* inv_w = reinterpret_cast<float*>(smem + SMEM_BAR + 256 + 128 * PROD) + warp * 64;   // [16 tokens][4 groups]
@@ -434,7 +436,9 @@ decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         for (int p = p_begin + (warp >> 2); p < p_end; p += GROUPS) {
             s += GROUPS;
             if (s >= NST) { s -= NST; parity ^= 1u; }
-            ok = __all_sync(0xffffffffu, wait_bar(ctx, s, parity));
+            // one try first: the bounded wait's clock and branches only where the slot is not there yet
+            if (!__all_sync(0xffffffffu, mbar_try_wait(ctx.bars + s * 8, parity)))
+                ok = __all_sync(0xffffffffu, wait_bar(ctx, s, parity));
             if (!ok) break;
             const uint8_t* kst = smem + s * STAGE;
             const uint8_t* vst = kst + QK_BYTES;
@@ -467,10 +471,11 @@ decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
                     for (int grp = 0; grp < 4; ++grp) {
                         const int chunk = (2 * grp + (t4 >> 1)) ^ (row & 7);
                         const uint2 kb = *reinterpret_cast<const uint2*>(kst + row * 128 + chunk * 16 + (t4 & 1) * 8);
-                        float c[4];
-                        mma_f16_first(c, qf[2 * grp][0], qf[2 * grp][1], e4m3_pair02_f16x2(kb.x), e4m3_pair13_f16x2(kb.x));
-                        mma_f16(c, qf[2 * grp + 1][0], qf[2 * grp + 1][1], e4m3_pair02_f16x2(kb.y), e4m3_pair13_f16x2(kb.y));
-                        sc[nt] = __ffma2_rn(make_float2(c[0], c[1]), inv[nt][grp], sc[nt]);
+                        float c0[4], c1[4];
+                        mma_f16_zero(c0, qf[grp], e4m3_pair02_f16x2(kb.x), e4m3_pair13_f16x2(kb.x));
+                        mma_f16_zero(c1, qf[grp], e4m3_pair02_f16x2(kb.y), e4m3_pair13_f16x2(kb.y));
+                        sc[nt] = __ffma2_rn(make_float2(c0[0], c0[1]), inv[nt][grp], sc[nt]);
+                        sc[nt] = __ffma2_rn(make_float2(c1[2], c1[3]), inv[nt][grp], sc[nt]);
                     }
                 }
                 float sacc[2][2] = {{sc[0].x, sc[0].y}, {sc[1].x, sc[1].y}};
