@@ -11,7 +11,7 @@
 // shared memory and leave the CTA as (O un-normalised, m, l), the layout lse_merge_kernel reads.  Splits of one head that fit a
 // thread-block cluster merge through its shared memory instead, and a launch sets up its ring and barriers under the kernel before
 // it.  Append + decode step: 1 sequence x 8 kv heads x 1001 tokens 19.4 us before, 9.9 now (latency); 32 x 8 x 4096 93 and 85 us
-// (HBM); 1 x 8 x 131072 104 and 94 us (HBM; the decode alone 90), quantised 107 and 60 us (instructions: 444 a 16-token slice).
+// (HBM); 1 x 8 x 131072 104 and 94 us (HBM; the decode alone 90), quantised 107 and 59 us (instructions: 444 a 16-token slice).
 //
 // The same kernel, instantiated for the quantised cache (GRL_FP8_INT4: FP8-E4M3 keys, INT4 values, one float16 scale
 // per 32 key elements, cpp/src/ops/kv_cache.cpp:272-399 and :500-577), streams 12.5 KiB per (page, kv head) instead
@@ -462,6 +462,12 @@ decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
                     inv[0][grp] = make_float2(v.x, v.y);
                     inv[1][grp] = make_float2(v.z, v.w);
                 }
+                // The two token pairs of this lane, 16 value bytes (all four groups) each (its tokens 4 t4 .. 4 t4 + 3 of the slice:
+                // pairs 2 t4 and 2 t4 + 1; the 16-byte pieces of a pair are stored XOR-swizzled by the pair index, which keeps the
+                // eight lanes of a quarter-warp on different banks), read ahead of the scores (131072 tokens x 8 heads 59.5 -> 58.9 us)
+                const int pr = 8 * slice + 2 * t4;
+                const uint4 va = *reinterpret_cast<const uint4*>(vst + pr * 128 + ((g ^ (pr & 7)) << 4));
+                const uint4 vb = *reinterpret_cast<const uint4*>(vst + (pr + 1) * 128 + ((g ^ ((pr + 1) & 7)) << 4));
                 // ---- S = q K^T for 16 tokens, one accumulator per scale group, combined with 1/scale
                 float2 sc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
@@ -514,14 +520,7 @@ decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
                 for (int nt = 0; nt < 2; ++nt) pv[nt] = make_float2(ex2(sacc[nt][0] - m_run), ex2(sacc[nt][1] - m_run));    // 0 for an "empty" score
                 l_run += (pv[0].x + pv[0].y) + (pv[1].x + pv[1].y);
                 // ---- O^T += V^T (P / scale)^T: rows are head_dim elements, columns heads, so all sixteen rows of the
-                // product work and P is used as it comes out of S (pairs of tokens per head).  The two token pairs of
-                // this lane, 16 value bytes (all four groups) each
-                // (this lane's tokens 4 t4 .. 4 t4 + 3 of the slice: pairs 2 t4 and 2 t4 + 1; the 16-byte pieces of a
-                // pair are stored XOR-swizzled by the pair index, which keeps the eight lanes of a quarter-warp on
-                // different banks)
-                const int pr = 8 * slice + 2 * t4;
-                const uint4 va = *reinterpret_cast<const uint4*>(vst + pr * 128 + ((g ^ (pr & 7)) << 4));
-                const uint4 vb = *reinterpret_cast<const uint4*>(vst + (pr + 1) * 128 + ((g ^ ((pr + 1) & 7)) << 4));
+                // product work and P is used as it comes out of S (pairs of tokens per head)
                 const uint32_t xa[4] = {va.x, va.y, va.z, va.w}, xb[4] = {vb.x, vb.y, vb.z, vb.w};
 #pragma unroll
                 for (int grp = 0; grp < 4; ++grp) {
