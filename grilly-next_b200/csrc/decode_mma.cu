@@ -970,7 +970,7 @@ bool decode_mma_supported(const grl_decode_params* p) {
 bool decode_mma_wide(const grl_device* dev, int ctas, int stages) { return ctas <= dev->prop.multiProcessorCount && stages >= 12; }
 
 template <int FORM, int HD>
-static int launch_instance(grl_device* dev, const CUtensorMap& tk, const CUtensorMap& tv, dmma::Args a, dim3 grid) {
+static int set_attributes(grl_device* dev) {
     using namespace dmma;
     constexpr int kAlone = FORM == QUANT_WIDE ? Smem<FORM, HD>::TOTAL : kAloneSmem;
     static bool attr_set[64] = {};
@@ -979,12 +979,38 @@ static int launch_instance(grl_device* dev, const CUtensorMap& tk, const CUtenso
         GRL_CUDA(cudaFuncSetAttribute(decode_mma_kernel<FORM, HD>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         attr_set[dev->ordinal & 63] = true;
     }
+    return GRL_OK;
+}
+
+// Quantised, (sequence, head) pairs just past one CTA an SM: most SMs hold one CTA, whose four compute warps take as long as the two
+// that others hold (19 to 36 sequences x 8 heads x 4096 tokens are all 61 us).  In thirds they are two rounds of half-length clusters
+// instead, while two rounds hold them; a cluster is the whole head, so nothing is left in the workspace and nobody counts arrivals.
+// us, append + decode, whole / thirds: 19 x 8 x 8192 110.1 / 86.3, x 4096 61.1 / 54.1, x 2600 42.0 / 39.5, 20 x 8 x 4096 ragged 56.3 / 46.1,
+// 22 x 8 x 6000 84.0 / 70.7, 38 x 4 x 3000 45.3 / 42.5, 75 x 2 x 30000 366 / 258; shorter: 19 x 8 x 2000 34.2 / 34.5.  Fifths of the first
+// two: 87, 57.5.  The rounds (93 clusters of three each) may not be full: they start while the append still holds SMs, and what is placed late
+// is a third round.  4096 tokens, 178 / 180 / 182 / 184 heads: 55.9 / 58.5 / 62.3 / 69.0 for 59.6 whole; hence a twentieth of slack.
+bool decode_mma_thirds(grl_device* dev, int heads, int stages) {
+    using namespace dmma;
+    if (heads <= dev->prop.multiProcessorCount || heads > 2 * dev->prop.multiProcessorCount || stages < 40) return false;
+    DeviceGuard g(dev->ordinal);
+    return set_attributes<QUANT_PAIR, 128>(dev) == GRL_OK &&
+           heads + heads / 20 <= 2 * max_active_clusters(dev, (const void*)decode_mma_kernel<QUANT_PAIR, 128>, Warps<QUANT_PAIR>::THREADS,
+                                                             Smem<QUANT_PAIR, 128>::TOTAL, 3);
+}
+
+template <int FORM, int HD>
+static int launch_instance(grl_device* dev, const CUtensorMap& tk, const CUtensorMap& tv, dmma::Args a, dim3 grid, int stages) {
+    using namespace dmma;
+    constexpr int kAlone = FORM == QUANT_WIDE ? Smem<FORM, HD>::TOTAL : kAloneSmem;
+    const int rc = set_attributes<FORM, HD>(dev);
+    if (rc) return rc;
     // Splits merge in clusters while a split is short, the largest equal share of them whose clusters fit the device at once.
     // Long splits (more than 40 stages) are bound by the stream, and a cluster's CTAs sit two on an SM where one each would
     // stream faster: 131072 tokens x 8 heads in 18 splits 97 us apart, 111 us in clusters of 9; 4096 tokens in 16 splits 13.8 us
     // in clusters of 16, 16.1 us apart.
     a.cluster = 1;
-    if (a.fuse && !a.direct && a.x.world <= 1 && a.pps_hint <= 40)
+    if (FORM == QUANT_PAIR && a.fuse && a.n_splits == 3 && a.x.world <= 1 && decode_mma_thirds(dev, (int)(grid.y * grid.z), stages)) a.cluster = 3;
+    else if (a.fuse && !a.direct && a.x.world <= 1 && a.pps_hint <= 40)
         for (int c = kMaxCluster; c > 1 && a.cluster == 1; --c)
             if (a.n_splits % c == 0 && (int)(grid.y * grid.z) * (a.n_splits / c) <=
                 max_active_clusters(dev, (const void*)decode_mma_kernel<FORM, HD>, Warps<FORM>::THREADS, Smem<FORM, HD>::TOTAL, c))
@@ -1041,7 +1067,8 @@ int decode_mma_launch(grl_device* dev, const grl_decode_params* p, int n_splits,
     a.x.world = 1;
     a.wait_limit = dev->wait_limit_cycles;
     const int bound = p->max_seq_len > 0 ? p->max_seq_len : kv.max_pages * kv.page_tokens;
-    a.pps_hint = ((bound + P - 1) / P + n_splits - 1) / n_splits;
+    const int stages = (bound + P - 1) / P;
+    a.pps_hint = (stages + n_splits - 1) / n_splits;
     if (p->exchange) {
         GRL_REQUIRE(fuse && !direct, "the fused cross-GPU merge needs the split-KV path");
         rc = fill_peer_exchange(dev, p->exchange, &a.x);
@@ -1057,9 +1084,9 @@ int decode_mma_launch(grl_device* dev, const grl_decode_params* p, int n_splits,
     dev->status_dirty = true;
     dim3 grid(n_splits, kv.num_kv_heads, kv.batch);
     if (quant)
-        return decode_mma_wide(dev, kv.batch * kv.num_kv_heads * n_splits, a.pps_hint) ? launch_instance<QUANT_WIDE, 128>(dev, tk, tv, a, grid)
-                                                                                       : launch_instance<QUANT_PAIR, 128>(dev, tk, tv, a, grid);
-    return kv.head_dim == 64 ? launch_instance<BF16, 64>(dev, tk, tv, a, grid) : launch_instance<BF16, 128>(dev, tk, tv, a, grid);
+        return decode_mma_wide(dev, kv.batch * kv.num_kv_heads * n_splits, a.pps_hint) ? launch_instance<QUANT_WIDE, 128>(dev, tk, tv, a, grid, stages)
+                                                                                       : launch_instance<QUANT_PAIR, 128>(dev, tk, tv, a, grid, stages);
+    return kv.head_dim == 64 ? launch_instance<BF16, 64>(dev, tk, tv, a, grid, stages) : launch_instance<BF16, 128>(dev, tk, tv, a, grid, stages);
 }
 
 }  // namespace grl

@@ -7,6 +7,7 @@
 namespace grl {
 
 bool decode_mma_supported(const grl_decode_params* p);
+bool decode_mma_thirds(grl_device* dev, int heads, int stages);
 int decode_mma_launch(grl_device* dev, const grl_decode_params* p, int n_splits, float scale, bool direct, bool fuse);
 
 constexpr float kEmptyMax = -1e30f;  // running max of a part that saw no token (finite on purpose)
@@ -358,12 +359,12 @@ int grl_decode_pick_splits(grl_device* dev, const grl_decode_params* p, int* n_s
         // clusters of 16 of at least 8 stages a split while splits are short enough to merge in clusters (see launch_instance).
         // More (sequence, head) pairs than SMs: unsplit (us, unsplit / 2 splits, decode alone: 19 x 8 x 8192 tokens 114 / 142, 25 x 8 x
         // 4096 67 / 82, 32 x 8 x 4096 81 / 92, 37 x 8 x 2048 52 / 62; quantised, before its present form, 25 x 8 x 4096 66 / 73, 32 x 8 x 4096
-        // 66 / 78; lengths from 4096 to 8192 24 x 8 106 / 114).  Just past one CTA an SM two splits would be the better ones where lengths
-        // differ or the cache is quantised (20 x 8, 4096 to 8192 tokens: 95 / 90): not distinguished here.
+        // 66 / 78; lengths from 4096 to 8192 24 x 8 106 / 114), but just past one CTA an SM over the quantised cache in three
+        // (decode_mma_thirds); two splits of ragged lengths over the bf16 cache (20 x 8, 4096 to 8192 tokens: 95 / 90) are not distinguished.
         const bool quant = kv.cache_dtype == GRL_FP8_INT4;
         const bool one = quant && base_ctas <= sms && (long long)pages * base_ctas >= 12LL * sms;
         const int most = (one ? 1 : 2) * sms / base_ctas, wide = (quant && !one ? 2 : 1) * sms / base_ctas;
-        if (base_ctas > sms) s = 1;
+        if (base_ctas > sms) s = quant && decode_mma_thirds(dev, base_ctas, pages) ? 3 : 1;
         else if (most < 32) {
             s = 1;
             while (2 * s <= most) s *= 2;
@@ -412,9 +413,12 @@ int grl_gqa_decode(grl_device* dev, const grl_decode_params* p) {
     const grl_kv_layout& kv = p->kv;
     const int D = kv.head_dim;
     const bool direct = (n_splits == 1) && !p->partial_out && !p->exchange;
+    // the kernel's own choice of thirds merges inside clusters: it asks for the workspace of an unsplit launch, which it does not use
+    const bool thirds = p->n_splits <= 0 && n_splits == 3 && decode_mma_supported(p) && !p->force_simt &&
+                        kv.batch * kv.num_kv_heads > dev->prop.multiProcessorCount;
     size_t need = 0;
-    grl_decode_workspace_bytes(p, n_splits, &need);
-    if (!direct)
+    if (!(thirds && !p->partial_out)) grl_decode_workspace_bytes(p, thirds ? 1 : n_splits, &need);
+    if (need && !direct)
         GRL_REQUIRE(p->workspace && p->workspace_bytes >= need, "decode workspace too small: %zu < %zu",
                     p->workspace_bytes, need);
     DeviceGuard g(dev->ordinal);

@@ -163,6 +163,51 @@ def test_one_cta_an_sm_decode_over_the_quantised_cache(Hq, Hkv, lens, P, splits)
         dev.close()
 
 
+@pytest.mark.parametrize("B,Hkv,group,T,P,splits", [
+    (75, 2, 4, 2560, 64, 3), (50, 3, 8, 2700, 16, 3), (75, 2, 1, 2496, 64, 1), (100, 3, 2, 2600, 64, 1)])    # 40 stages; 39; too many heads
+def test_heads_just_past_the_sms_decode_in_thirds(B, Hkv, group, T, P, splits):
+    """More quantised (sequence, head) pairs than SMs, two rounds of clusters of three: ragged lengths (some shorter than a third of
+    the longest, one of 1), with no workspace at all where an unsplit call needs none.  Three sequences against the oracle on the same
+    quantised cache, all of them against unsplit launches, tolerance as for the other tensor-core cases."""
+    from grilly_next import cabi
+    from gpu_helpers import PagedCache
+    from oracle import attention_oracle as orc
+    dev = cabi.Device(0)
+    try:
+        rng = np.random.default_rng(B + T)
+        D, Hq = 128, Hkv * group
+        k, v = rng.standard_normal((B, T, Hkv, D), dtype=np.float32), rng.standard_normal((B, T, Hkv, D), dtype=np.float32)
+        q = rng.standard_normal((B, 1, Hq, D), dtype=np.float32)
+        pc = PagedCache(dev, B, Hkv, D, T + 64, page_tokens=P, dtype=cabi.FP8_INT4, shuffle_pages=True, seed=7)
+        pc.append(k, v)
+        cut = rng.integers(1, T + 1, B).astype(np.int32)
+        cut[0], cut[1], cut[2] = T, 1, T // 3
+        dev.L.grl_memcpy_h2d(dev.h, pc.seq_lens, cut.ctypes.data_as(C.c_void_p), cut.nbytes)
+        dev.sync()
+        pc.lens[:] = cut
+        kd, vd = _dequantised(k[:3], v[:3])
+        want = np.concatenate([orc.gqa_decode_attention(q[b:b + 1], kd[b:b + 1, :cut[b]], vd[b:b + 1, :cut[b]], Hq, Hkv, D) for b in range(3)])
+        whole = pc.decode(q, n_splits=1)
+        got = pc.decode(q)
+        assert pc.last_splits == splits
+        tol = 1e-3 * np.abs(want).max()
+        assert np.abs(got[:3] - want).max() <= tol and np.abs(whole[:3] - want).max() <= tol
+        assert np.abs(got - whole).max() <= 2 * tol * max(1.0, np.abs(whole).max() / np.abs(want).max())       # tol of each side's own scale
+        part = pc.decode(q, partial=True)
+        o, l = part[:B * Hq * D].reshape(B, 1, Hq, D), part[B * Hq * (D + 1):].reshape(B, 1, Hq, 1)
+        np.testing.assert_allclose(o / l, got, rtol=1e-5, atol=1e-6)          # the same merge; the division is fp32 on both sides
+        qd, od = dev.upload(q), dev.malloc(q.nbytes)
+        p = cabi.DecodeParams()
+        p.kv = pc.layout()
+        p.q, p.out, p.num_q_heads, p.max_seq_len = qd, od, Hq, T
+        cabi.check(dev.L.grl_gqa_decode(dev.h, C.byref(p)))
+        np.testing.assert_array_equal(dev.download(od, q.shape, np.float32), got)
+        dev.free(qd)
+        dev.free(od)
+    finally:
+        dev.close()
+
+
 def test_quantised_append_with_rope_and_queries():
     """RoPE of the new keys happens before the quantiser; the step's queries are rotated alongside."""
     from grilly_next import cabi
