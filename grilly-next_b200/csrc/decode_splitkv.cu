@@ -412,10 +412,20 @@ int grl_gqa_decode(grl_device* dev, const grl_decode_params* p) {
     if (rc) return rc;
     const grl_kv_layout& kv = p->kv;
     const int D = kv.head_dim;
+    // A workspace sized at a longer max_seq_len: over the quantised cache fewer splits are chosen there (one CTA an SM) than for some
+    // shorter lengths.  Where it holds that choice but not this one, the call takes that one.
+    const int heads = kv.batch * kv.num_kv_heads, sms = dev->prop.multiProcessorCount;
+    if (p->n_splits <= 0 && kv.cache_dtype == GRL_FP8_INT4 && heads <= sms && p->workspace && !p->exchange && !p->force_simt && decode_mma_supported(p)) {
+        int fewer = sms / heads >= 32 ? sms / heads / 16 * 16 : 1;
+        while (fewer < 32 && 2 * fewer <= sms / heads) fewer *= 2;
+        size_t bytes = 0, least = 0;
+        grl_decode_workspace_bytes(p, n_splits, &bytes);
+        grl_decode_workspace_bytes(p, fewer, &least);
+        if (fewer < n_splits && p->workspace_bytes < bytes && p->workspace_bytes >= least) n_splits = fewer;
+    }
     const bool direct = (n_splits == 1) && !p->partial_out && !p->exchange;
     // the kernel's own choice of thirds merges inside clusters: it asks for the workspace of an unsplit launch, which it does not use
-    const bool thirds = p->n_splits <= 0 && n_splits == 3 && decode_mma_supported(p) && !p->force_simt &&
-                        kv.batch * kv.num_kv_heads > dev->prop.multiProcessorCount;
+    const bool thirds = p->n_splits <= 0 && n_splits == 3 && decode_mma_supported(p) && !p->force_simt && heads > sms;
     size_t need = 0;
     if (!(thirds && !p->partial_out)) grl_decode_workspace_bytes(p, thirds ? 1 : n_splits, &need);
     if (need && !direct)

@@ -208,6 +208,41 @@ def test_heads_just_past_the_sms_decode_in_thirds(B, Hkv, group, T, P, splits):
         dev.close()
 
 
+@pytest.mark.parametrize("B,Hkv,T,longest", [(2, 8, 1500, 131072), (1, 2, 50000, 131072), (20, 5, 700, 4096)])
+def test_workspace_sized_at_the_longest_length_serves_shorter_ones(B, Hkv, T, longest):
+    """Fewer splits are chosen at the longest length than at this one: the call takes what the workspace holds."""
+    from grilly_next import cabi
+    from gpu_helpers import PagedCache
+    dev = cabi.Device(0)
+    try:
+        rng = np.random.default_rng(T)
+        k, v = (rng.standard_normal((B, T, Hkv, 128), dtype=np.float32) for _ in range(2))
+        q = rng.standard_normal((B, 1, Hkv, 128), dtype=np.float32)
+        pc = PagedCache(dev, B, Hkv, 128, T + 64, page_tokens=64, dtype=cabi.FP8_INT4, seed=8)
+        pc.append(k, v)
+        want = pc.decode(q)
+        splits, size, one = C.c_int(), C.c_size_t(), C.c_size_t()
+        p = cabi.DecodeParams()
+        p.kv = pc.layout()
+        qd, od = dev.upload(q), dev.malloc(q.nbytes)
+        p.q, p.out, p.num_q_heads, p.max_seq_len = qd, od, Hkv, longest
+        cabi.check(dev.L.grl_decode_pick_splits(dev.h, C.byref(p), C.byref(splits)))
+        assert splits.value < pc.last_splits
+        cabi.check(dev.L.grl_decode_workspace_bytes(C.byref(p), splits.value, C.byref(size)))
+        cabi.check(dev.L.grl_decode_workspace_bytes(C.byref(p), 1, C.byref(one)))
+        ws = dev.malloc(size.value)
+        p.max_seq_len, p.workspace, p.workspace_bytes = T, ws, size.value
+        cabi.check(dev.L.grl_gqa_decode(dev.h, C.byref(p)))
+        got = dev.download(od, q.shape, np.float32)
+        assert np.abs(got - want).max() <= 1e-3 * np.abs(want).max()
+        p.workspace_bytes = one.value - 4                     # less than any count needs: refused as before
+        assert dev.L.grl_gqa_decode(dev.h, C.byref(p)) != 0
+        for x in (qd, od, ws):
+            dev.free(x)
+    finally:
+        dev.close()
+
+
 def test_quantised_append_with_rope_and_queries():
     """RoPE of the new keys happens before the quantiser; the step's queries are rotated alongside."""
     from grilly_next import cabi
