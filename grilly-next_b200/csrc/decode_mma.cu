@@ -26,6 +26,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "decode_plan.h"
 
 namespace grl {
 namespace dmma {
@@ -87,14 +88,12 @@ struct Args {
     int scores_ld;
     PeerExchange x;         // x.world > 1: the merged rows are exchanged with the peers and merged again
     long long wait_limit;   // cycle budget of every mbarrier wait
-    int alone;              // 1: one CTA an SM, and the next kernel starts after this one (see launch_instance)
+    int alone;              // 1: one CTA an SM, and the next kernel starts after this one (decode_plan)
     int cluster;            // > 1: CTAs of a thread-block cluster; that many splits of a head merge through its shared memory
     int pps_hint;           // stages per split of a sequence of the longest length: what the first block-table read assumes
 };
-constexpr int kMaxCluster = 16;
 constexpr int kAloneSmem = 116 * 1024;      // dynamic shared memory of which an SM (228 KiB, 1 KiB reserved a CTA) does not hold two
 constexpr int kDoneSlot = grl_device::kCounterSlots;
-constexpr int kMaxFusedSplits = 256;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
@@ -964,11 +963,6 @@ bool decode_mma_supported(const grl_decode_params* p) {
     return kv.cache_dtype == GRL_BF16 && geometry && (kv.head_dim == 128 || kv.head_dim == 64) && ((uintptr_t)p->q % 8 == 0);
 }
 
-// The quantised cache's one-CTA-an-SM form: where the CTAs are no more than the SMs and each streams at least 12 stages (see
-// grl_decode_pick_splits).  us, decode alone, pair / wide: 1 x 8 x 131072 tokens 65 / 59, x 65536 43 / 34, x 16384 24 / 18.7, 1 x 2 x
-// 131072 52 / 27, 64 x 2 x 2048 20.7 / 18.9; shorter splits or more CTAs: 1 x 8 x 4096 11.5 / 13.2, 64 x 8 x 500 21 / 29, 32 x 8 x 4096 60 / 65.
-bool decode_mma_wide(const grl_device* dev, int ctas, int stages) { return ctas <= dev->prop.multiProcessorCount && stages >= 12; }
-
 template <int FORM, int HD>
 static int set_attributes(grl_device* dev) {
     using namespace dmma;
@@ -982,46 +976,27 @@ static int set_attributes(grl_device* dev) {
     return GRL_OK;
 }
 
-// Quantised, (sequence, head) pairs just past one CTA an SM: most SMs hold one CTA, whose four compute warps take as long as the two
-// that others hold (19 to 36 sequences x 8 heads x 4096 tokens are all 61 us).  In thirds they are two rounds of half-length clusters
-// instead, while two rounds hold them; a cluster is the whole head, so nothing is left in the workspace and nobody counts arrivals.
-// us, append + decode, whole / thirds: 19 x 8 x 8192 110.1 / 86.3, x 4096 61.1 / 54.1, x 2600 42.0 / 39.5, 20 x 8 x 4096 ragged 56.3 / 46.1,
-// 22 x 8 x 6000 84.0 / 70.7, 38 x 4 x 3000 45.3 / 42.5, 75 x 2 x 30000 366 / 258; shorter: 19 x 8 x 2000 34.2 / 34.5.  Fifths of the first
-// two: 87, 57.5.  The rounds (93 clusters of three each) may not be full: they start while the append still holds SMs, and what is placed late
-// is a third round.  4096 tokens, 178 / 180 / 182 / 184 heads: 55.9 / 58.5 / 62.3 / 69.0 for 59.6 whole; hence a twentieth of slack.
-bool decode_mma_thirds(grl_device* dev, int heads, int stages) {
+template <int FORM, int HD>
+static int instance_clusters(grl_device* dev, int size) {
     using namespace dmma;
-    if (heads <= dev->prop.multiProcessorCount || heads > 2 * dev->prop.multiProcessorCount || stages < 40) return false;
+    return set_attributes<FORM, HD>(dev) != GRL_OK ? 0
+        : max_active_clusters(dev, (const void*)decode_mma_kernel<FORM, HD>, Warps<FORM>::THREADS, Smem<FORM, HD>::TOTAL, size);
+}
+
+// Clusters of `size` CTAs of the kernel that serves this call that the device holds at once.
+int decode_mma_clusters(grl_device* dev, const grl_decode_params* p, bool wide, int size) {
+    using namespace dmma;
     DeviceGuard g(dev->ordinal);
-    return set_attributes<QUANT_PAIR, 128>(dev) == GRL_OK &&
-           heads + heads / 20 <= 2 * max_active_clusters(dev, (const void*)decode_mma_kernel<QUANT_PAIR, 128>, Warps<QUANT_PAIR>::THREADS,
-                                                             Smem<QUANT_PAIR, 128>::TOTAL, 3);
+    if (p->kv.cache_dtype == GRL_FP8_INT4) return wide ? instance_clusters<QUANT_WIDE, 128>(dev, size) : instance_clusters<QUANT_PAIR, 128>(dev, size);
+    return p->kv.head_dim == 64 ? instance_clusters<BF16, 64>(dev, size) : instance_clusters<BF16, 128>(dev, size);
 }
 
 template <int FORM, int HD>
-static int launch_instance(grl_device* dev, const CUtensorMap& tk, const CUtensorMap& tv, dmma::Args a, dim3 grid, int stages) {
+static int launch_instance(grl_device* dev, const CUtensorMap& tk, const CUtensorMap& tv, const dmma::Args& a, dim3 grid) {
     using namespace dmma;
     constexpr int kAlone = FORM == QUANT_WIDE ? Smem<FORM, HD>::TOTAL : kAloneSmem;
     const int rc = set_attributes<FORM, HD>(dev);
     if (rc) return rc;
-    // Splits merge in clusters while a split is short, the largest equal share of them whose clusters fit the device at once.
-    // Long splits (more than 40 stages) are bound by the stream, and a cluster's CTAs sit two on an SM where one each would
-    // stream faster: 131072 tokens x 8 heads in 18 splits 97 us apart, 111 us in clusters of 9; 4096 tokens in 16 splits 13.8 us
-    // in clusters of 16, 16.1 us apart.
-    a.cluster = 1;
-    if (FORM == QUANT_PAIR && a.fuse && a.n_splits == 3 && a.x.world <= 1 && decode_mma_thirds(dev, (int)(grid.y * grid.z), stages)) a.cluster = 3;
-    else if (a.fuse && !a.direct && a.x.world <= 1 && a.pps_hint <= 40)
-        for (int c = kMaxCluster; c > 1 && a.cluster == 1; --c)
-            if (a.n_splits % c == 0 && (int)(grid.y * grid.z) * (a.n_splits / c) <=
-                max_active_clusters(dev, (const void*)decode_mma_kernel<FORM, HD>, Warps<FORM>::THREADS, Smem<FORM, HD>::TOTAL, c))
-                a.cluster = c;
-    // Splits that merge through global memory, at most one CTA for every SM: two of them must not share an SM, which they do when
-    // they are placed while the SMs still hold CTAs of the kernel before (a decode that merges, or the append).  So they ask for
-    // more than half of an SM's shared memory.  Decode after decode / append + decode, us, 131072 tokens, bf16:
-    //   8 heads, 144 CTAs: 102.5 / 97.2 where pairs could form, 93.2 / 97.1 now;  7 heads, 147 CTAs: 92.4 / 94.5 and 84.1 / 87.0;
-    //   4 heads, 148 CTAs: 74.0 / 78.0 and 67.9 / 71.3.  A plain launch: 93.5 / 96.6, 84.4 / 87.3, 67.7 / 70.8 from a graph, but
-    //   append + decode from a stream 99.4, 90.2 and 73.8 for 97.4, 87.2 and 71.6.
-    a.alone = a.fuse && !a.direct && a.cluster == 1 && (int)(grid.x * grid.y * grid.z) <= dev->prop.multiProcessorCount;
     if (a.alone)
         GRL_CUDA(launch_pdl(decode_mma_kernel<FORM, HD>, grid, Warps<FORM>::THREADS, kAlone, dev->stream, tk, tv, a));
     else
@@ -1031,8 +1006,9 @@ static int launch_instance(grl_device* dev, const CUtensorMap& tk, const CUtenso
     return GRL_OK;
 }
 
-int decode_mma_launch(grl_device* dev, const grl_decode_params* p, int n_splits, float scale, bool direct, bool fuse) {
+int decode_mma_launch(grl_device* dev, const grl_decode_params* p, const DecodePlan& plan, float scale) {
     using namespace dmma;
+    const int n_splits = plan.n_splits;
     const grl_kv_layout& kv = p->kv;
     const uint64_t pages = kv.num_pages > 0 ? (uint64_t)kv.num_pages : (uint64_t)kv.batch * kv.max_pages;
     const uint64_t rows = pages * kv.num_kv_heads * kv.page_tokens;
@@ -1061,8 +1037,8 @@ int decode_mma_launch(grl_device* dev, const grl_decode_params* p, int n_splits,
     a.B = kv.batch; a.Hq = p->num_q_heads; a.Hkv = kv.num_kv_heads; a.max_pages = kv.max_pages;
     a.page = kv.page_tokens; a.ppt = P / kv.page_tokens;
     a.n_splits = n_splits; a.group = p->num_q_heads / kv.num_kv_heads;
-    a.scale = scale; a.direct = direct ? 1 : 0;
-    a.fuse = fuse ? 1 : 0; a.counters = dev->d_counters; a.partial_out = p->partial_out;
+    a.scale = scale; a.direct = plan.direct ? 1 : 0; a.cluster = plan.cluster; a.alone = plan.alone ? 1 : 0;
+    a.fuse = plan.fused ? 1 : 0; a.counters = dev->d_counters; a.partial_out = p->partial_out;
     a.scores_out = p->scores_out; a.scores_ld = p->scores_ld;
     a.x.world = 1;
     a.wait_limit = dev->wait_limit_cycles;
@@ -1070,7 +1046,7 @@ int decode_mma_launch(grl_device* dev, const grl_decode_params* p, int n_splits,
     const int stages = (bound + P - 1) / P;
     a.pps_hint = (stages + n_splits - 1) / n_splits;
     if (p->exchange) {
-        GRL_REQUIRE(fuse && !direct, "the fused cross-GPU merge needs the split-KV path");
+        GRL_REQUIRE(plan.fused, "the fused cross-GPU merge needs the split-KV path");
         rc = fill_peer_exchange(dev, p->exchange, &a.x);
         if (rc) return rc;
         const int heads = kv.batch * kv.num_kv_heads;
@@ -1083,10 +1059,8 @@ int decode_mma_launch(grl_device* dev, const grl_decode_params* p, int n_splits,
     }
     dev->status_dirty = true;
     dim3 grid(n_splits, kv.num_kv_heads, kv.batch);
-    if (quant)
-        return decode_mma_wide(dev, kv.batch * kv.num_kv_heads * n_splits, a.pps_hint) ? launch_instance<QUANT_WIDE, 128>(dev, tk, tv, a, grid, stages)
-                                                                                       : launch_instance<QUANT_PAIR, 128>(dev, tk, tv, a, grid, stages);
-    return kv.head_dim == 64 ? launch_instance<BF16, 64>(dev, tk, tv, a, grid, stages) : launch_instance<BF16, 128>(dev, tk, tv, a, grid, stages);
+    if (quant) return plan.wide ? launch_instance<QUANT_WIDE, 128>(dev, tk, tv, a, grid) : launch_instance<QUANT_PAIR, 128>(dev, tk, tv, a, grid);
+    return kv.head_dim == 64 ? launch_instance<BF16, 64>(dev, tk, tv, a, grid) : launch_instance<BF16, 128>(dev, tk, tv, a, grid);
 }
 
 }  // namespace grl

@@ -3,12 +3,13 @@
 // three global-memory phases with a (B,Hq,T) scratch) by a single streaming pass: every K and V
 // row is read once with 16-byte loads and shared by all query heads of its KV group.
 #include "common.cuh"
+#include "decode_plan.h"
 
 namespace grl {
 
 bool decode_mma_supported(const grl_decode_params* p);
-bool decode_mma_thirds(grl_device* dev, int heads, int stages);
-int decode_mma_launch(grl_device* dev, const grl_decode_params* p, int n_splits, float scale, bool direct, bool fuse);
+int decode_mma_clusters(grl_device* dev, const grl_decode_params* p, bool wide, int size);
+int decode_mma_launch(grl_device* dev, const grl_decode_params* p, const DecodePlan& plan, float scale);
 
 constexpr float kEmptyMax = -1e30f;  // running max of a part that saw no token (finite on purpose)
 constexpr int kDecodeThreads = 128;
@@ -325,6 +326,22 @@ static int check_decode(const grl_decode_params* p, bool need_tensors = true) {
     return GRL_OK;
 }
 
+static DecodeShape decode_shape(const grl_device* dev, const grl_decode_params* p) {
+    const grl_kv_layout& kv = p->kv;
+    DecodeShape d;
+    d.mma = decode_mma_supported(p) && !p->force_simt;
+    // the tensor-core kernel walks 64-token stages whatever the page size
+    const int max_len = p->max_seq_len > 0 ? p->max_seq_len : kv.max_pages * kv.page_tokens, unit = d.mma ? 64 : kv.page_tokens;
+    d.heads = kv.batch * kv.num_kv_heads;
+    d.stages = (max_len + unit - 1) / unit;
+    d.sms = dev->prop.multiProcessorCount;
+    d.counter_slots = grl_device::kCounterSlots;
+    d.quant = kv.cache_dtype == GRL_FP8_INT4;
+    d.exchange = p->exchange != nullptr;
+    d.partial = p->partial_out != nullptr;
+    return d;
+}
+
 }  // namespace grl
 
 using namespace grl;
@@ -339,48 +356,7 @@ int grl_decode_pick_splits(grl_device* dev, const grl_decode_params* p, int* n_s
         *n_splits = p->n_splits;
         return GRL_OK;
     }
-    const grl_kv_layout& kv = p->kv;
-    const int max_len = p->max_seq_len > 0 ? p->max_seq_len : kv.max_pages * kv.page_tokens;
-    const bool generic = !decode_mma_supported(p) || p->force_simt;
-    // the tensor-core kernel walks 64-token stages whatever the page size
-    const int unit = generic ? kv.page_tokens : 64;
-    const int pages = (max_len + unit - 1) / unit;
-    const int base_ctas = kv.batch * kv.num_kv_heads;
-    const int sms = dev->prop.multiProcessorCount;
-    // The generic kernel (128-thread CTAs, no shared-memory ring) wants several CTAs per SM to hide its loads and,
-    // over a quantised cache, its dequantising arithmetic: aim at eight per SM.
-    int s = generic ? (8 * sms + base_ctas - 1) / base_ctas : sms / base_ctas;
-    if (!generic && !p->exchange) {
-        // Two CTAs an SM (twice the bytes in flight, or twice the warps that dequantise) while the splits of a head are one
-        // cluster: a power of two up to 16, which packs into the GPCs (16 sequences x 8 heads x 4096 tokens: 63 us unsplit, 51 us
-        // in 2 splits; 4 x 8 x 2048: 15.0 us in 8 splits, 19.1 in 9).  Few heads: one CTA an SM over the bf16 cache (131072 tokens
-        // x 8 heads, append + decode: 97 us with 18 splits, 97 with 36; decode alone 93 and 94) and over the quantised one where each
-        // CTA then has 12 stages or more (decode_mma_wide: twelve compute warps a CTA); below that two over the quantised one, in whole
-        // clusters of 16 of at least 8 stages a split while splits are short enough to merge in clusters (see launch_instance).
-        // More (sequence, head) pairs than SMs: unsplit (us, unsplit / 2 splits, decode alone: 19 x 8 x 8192 tokens 114 / 142, 25 x 8 x
-        // 4096 67 / 82, 32 x 8 x 4096 81 / 92, 37 x 8 x 2048 52 / 62; quantised, before its present form, 25 x 8 x 4096 66 / 73, 32 x 8 x 4096
-        // 66 / 78; lengths from 4096 to 8192 24 x 8 106 / 114), but just past one CTA an SM over the quantised cache in three
-        // (decode_mma_thirds); two splits of ragged lengths over the bf16 cache (20 x 8, 4096 to 8192 tokens: 95 / 90) are not distinguished.
-        const bool quant = kv.cache_dtype == GRL_FP8_INT4;
-        const bool one = quant && base_ctas <= sms && (long long)pages * base_ctas >= 12LL * sms;
-        const int most = (one ? 1 : 2) * sms / base_ctas, wide = (quant && !one ? 2 : 1) * sms / base_ctas;
-        if (base_ctas > sms) s = quant && decode_mma_thirds(dev, base_ctas, pages) ? 3 : 1;
-        else if (most < 32) {
-            s = 1;
-            while (2 * s <= most) s *= 2;
-            if (s == 16 && pages > 32 * wide) s = wide;
-        } else {
-            s = wide;
-            if (pages <= 32 * s) {
-                if (s > pages / 8) s = pages / 8;
-                s = s < 32 ? 16 : s / 16 * 16;
-            }
-        }
-    }
-    if (s > pages / 2) s = pages / 2;          // every split keeps at least 2 pages
-    if (s > 256) s = 256;
-    if (s < 1) s = 1;
-    *n_splits = s;
+    *n_splits = decode_splits(decode_shape(dev, p), [&](bool wide, int c) { return decode_mma_clusters(dev, p, wide, c); });
     return GRL_OK;
 }
 
@@ -407,28 +383,18 @@ int grl_gqa_decode(grl_device* dev, const grl_decode_params* p) {
     GRL_REQUIRE(dev, "dev is NULL");
     int rc = check_decode(p);
     if (rc) return rc;
-    int n_splits = 0;
-    rc = grl_decode_pick_splits(dev, p, &n_splits);
-    if (rc) return rc;
     const grl_kv_layout& kv = p->kv;
     const int D = kv.head_dim;
-    // A workspace sized at a longer max_seq_len: over the quantised cache fewer splits are chosen there (one CTA an SM) than for some
-    // shorter lengths.  Where it holds that choice but not this one, the call takes that one.
-    const int heads = kv.batch * kv.num_kv_heads, sms = dev->prop.multiProcessorCount;
-    if (p->n_splits <= 0 && kv.cache_dtype == GRL_FP8_INT4 && heads <= sms && p->workspace && !p->exchange && !p->force_simt && decode_mma_supported(p)) {
-        int fewer = sms / heads >= 32 ? sms / heads / 16 * 16 : 1;
-        while (fewer < 32 && 2 * fewer <= sms / heads) fewer *= 2;
-        size_t bytes = 0, least = 0;
-        grl_decode_workspace_bytes(p, n_splits, &bytes);
-        grl_decode_workspace_bytes(p, fewer, &least);
-        if (fewer < n_splits && p->workspace_bytes < bytes && p->workspace_bytes >= least) n_splits = fewer;
-    }
-    const bool direct = (n_splits == 1) && !p->partial_out && !p->exchange;
-    // the kernel's own choice of thirds merges inside clusters: it asks for the workspace of an unsplit launch, which it does not use
-    const bool thirds = p->n_splits <= 0 && n_splits == 3 && decode_mma_supported(p) && !p->force_simt && heads > sms;
-    size_t need = 0;
-    if (!(thirds && !p->partial_out)) grl_decode_workspace_bytes(p, thirds ? 1 : n_splits, &need);
-    if (need && !direct)
+    size_t part_bytes = 0;
+    rc = grl_decode_workspace_bytes(p, 1, &part_bytes);
+    if (rc) return rc;
+    DecodeShape shape = decode_shape(dev, p);
+    if (p->exchange) shape.world = p->exchange->world;
+    const DecodePlan plan = decode_plan(shape, p->n_splits, part_bytes, p->workspace != nullptr, p->workspace_bytes,
+                                        [&](bool wide, int c) { return decode_mma_clusters(dev, p, wide, c); });
+    const int n_splits = plan.n_splits;
+    const size_t need = plan.parts * part_bytes;
+    if (need)
         GRL_REQUIRE(p->workspace && p->workspace_bytes >= need, "decode workspace too small: %zu < %zu",
                     p->workspace_bytes, need);
     DeviceGuard g(dev->ordinal);
@@ -439,21 +405,18 @@ int grl_gqa_decode(grl_device* dev, const grl_decode_params* p) {
     a.B = kv.batch; a.Hq = p->num_q_heads; a.Hkv = kv.num_kv_heads; a.P = kv.page_tokens;
     a.max_pages = kv.max_pages; a.n_splits = n_splits; a.group = p->num_q_heads / kv.num_kv_heads;
     a.scale = p->scale == 0.f ? 1.f / sqrtf((float)D) : p->scale;
-    a.direct = direct ? 1 : 0;
-    const bool mma = decode_mma_supported(p) && !p->force_simt;
-    // the tensor-core kernel merges its own splits (last CTA of a head to arrive) when its counters can hold the heads
-    const bool fused = mma && !direct && n_splits <= 256 && kv.batch * kv.num_kv_heads <= grl_device::kCounterSlots;
-    GRL_REQUIRE(!p->exchange || fused,
+    a.direct = plan.direct ? 1 : 0;
+    GRL_REQUIRE(!p->exchange || plan.fused,
                 "the cross-GPU merge inside the decode needs the tensor-core geometry (bf16 cache at head_dim 128 / 64 or "
                 "the quantised cache at 128, pages of 64 / 32 / 16 tokens, at most 8 query heads per kv head) and a split "
                 "launch; use partial_out and grl_exchange_merge instead");
-    if (mma)
-        rc = decode_mma_launch(dev, p, n_splits, a.scale, direct, fused);
+    if (shape.mma)
+        rc = decode_mma_launch(dev, p, plan, a.scale);
     else
         rc = kv.cache_dtype == GRL_BF16       ? dispatch_decode_d<__nv_bfloat16>(dev, a, D)
              : kv.cache_dtype == GRL_FP8_INT4 ? dispatch_decode_d<QuantKV>(dev, a, D)
                                               : dispatch_decode_d<float>(dev, a, D);
-    if (rc || direct || fused) return rc;
+    if (rc || plan.direct || plan.fused) return rc;
     const int rows = kv.batch * p->num_q_heads;
     const size_t stride = (size_t)rows * (D + 2);
     if (p->partial_out)
