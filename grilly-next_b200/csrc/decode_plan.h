@@ -78,7 +78,10 @@ int decode_splits(const DecodeShape& d, Fits&& fits) {
         else if (most < 32) {
             s = 1;
             while (2 * s <= most) s *= 2;
-            if (s == 16 && d.stages > 32 * wide) s = wide;
+            // Splits too long for clusters (kClusterStages) need no power of two: as many as there are SMs for.  us, append + decode over the
+            // quantised cache, power of two / all: 10 heads, 8 / 14 splits of 41 stages 27.8 / 23.4, of 100 50.2 / 35.7, of 256 107 / 69; 40
+            // heads, 2 / 3 splits 28.9 / 22.2, 51.4 / 39.6, 108 / 77.9; 24 heads, 4 / 6 29.3 / 26.7, 52.1 / 40.9; 16 heads, 8 / 9 29.5 / 28.7, 52.8 / 49.
+            if ((s == 16 && d.stages > 32 * wide) || (one && d.stages > kClusterStages * s)) s = wide;
         } else {
             s = wide;
             if (d.stages <= 32 * s) {

@@ -111,3 +111,16 @@ def test_a_workspace_sized_at_a_longer_length_serves_this_one(rules):
                 p = rules.of(heads, stages, 1, held=100 * sized)
                 assert p["parts"] <= sized and p["n_splits"] <= want, (heads, stages, longest, p)
             assert rules.of(heads, stages, 1, held=99)["n_splits"] == want          # less than any count needs: refused by its size
+
+
+def test_long_splits_of_the_quantised_cache_leave_no_sm_idle_that_a_whole_split_fills(rules):
+    """One CTA an SM and splits of more than 40 stages at a power of two: no clusters, so nothing asks for one."""
+    for heads in range(5, SMS + 1):
+        power = 1
+        while 2 * power <= SMS // heads:
+            power *= 2
+        for per_split in (41, 60, 100, 1000):
+            assert rules.splits(heads, per_split * power, 1, 0) == SMS // heads, (heads, per_split)
+        if SMS // heads < 16 and 40 * power * heads >= 12 * SMS:
+            assert rules.splits(heads, 40 * power, 1, 0) == power       # 40 stages a split: clusters
+    assert rules.splits(10, 2048, 1, 0) == 14 and rules.splits(40, 512, 1, 0) == 3

@@ -208,6 +208,34 @@ def test_heads_just_past_the_sms_decode_in_thirds(B, Hkv, group, T, P, splits):
         dev.close()
 
 
+@pytest.mark.parametrize("B,Hkv,T,P,splits", [(2, 5, 41 * 8 * 64, 64, 14), (5, 8, 41 * 2 * 64 - 63, 32, 3), (2, 5, 40 * 8 * 64, 64, 8)])
+def test_long_splits_that_are_no_power_of_two(B, Hkv, T, P, splits):
+    """As many splits as the SMs hold where a power of two of them would be too long for clusters: ragged lengths, one of a single token
+    (its other splits are empty), against the oracle on the same quantised cache, tolerance as for the other tensor-core cases."""
+    from grilly_next import cabi
+    from gpu_helpers import PagedCache
+    from oracle import attention_oracle as orc
+    dev = cabi.Device(0)
+    try:
+        rng = np.random.default_rng(B + T)
+        D, Hq = 128, 2 * Hkv
+        k, v = (rng.standard_normal((B, T, Hkv, D), dtype=np.float32) for _ in range(2))
+        q = rng.standard_normal((B, 1, Hq, D), dtype=np.float32)
+        pc = PagedCache(dev, B, Hkv, D, T + 64, page_tokens=P, dtype=cabi.FP8_INT4, shuffle_pages=True, seed=9)
+        pc.append(k, v)
+        cut = np.array([T, 1, T // 3, T - 7, 700][:B], np.int32)
+        dev.L.grl_memcpy_h2d(dev.h, pc.seq_lens, cut.ctypes.data_as(C.c_void_p), cut.nbytes)
+        dev.sync()
+        pc.lens[:] = cut
+        kd, vd = _dequantised(k, v)
+        want = np.concatenate([orc.gqa_decode_attention(q[b:b + 1], kd[b:b + 1, :cut[b]], vd[b:b + 1, :cut[b]], Hq, Hkv, D) for b in range(B)])
+        got = pc.decode(q)
+        assert pc.last_splits == splits
+        assert np.abs(got - want).max() <= 1e-3 * np.abs(want).max()
+    finally:
+        dev.close()
+
+
 @pytest.mark.parametrize("B,Hkv,T,longest", [(2, 8, 1500, 131072), (1, 2, 50000, 131072), (20, 5, 700, 4096)])
 def test_workspace_sized_at_the_longest_length_serves_shorter_ones(B, Hkv, T, longest):
     """Fewer splits are chosen at the longest length than at this one: the call takes what the workspace holds."""
