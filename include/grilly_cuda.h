@@ -350,6 +350,9 @@ typedef struct {
                              * other GPUs are merged in over NVLink inside the decode kernel; `out` then holds
                              * the attention over ALL ranks' shards.  NULL: single-GPU decode. */
 } grl_decode_params;
+/* The count for this max_seq_len.  Over the quantised cache it may be smaller for a longer one: grl_gqa_decode with
+ * n_splits = 0 takes that smaller count where the workspace holds no more, so a workspace sized at the longest length
+ * (none, where the count there is 1 and partial_out and exchange are NULL) serves all shorter ones. */
 int grl_decode_pick_splits(grl_device* dev, const grl_decode_params* p, int* n_splits);
 int grl_decode_workspace_bytes(const grl_decode_params* p, int n_splits, size_t* bytes);
 int grl_gqa_decode(grl_device* dev, const grl_decode_params* p);

@@ -124,3 +124,20 @@ def test_long_splits_of_the_quantised_cache_leave_no_sm_idle_that_a_whole_split_
         if SMS // heads < 16 and 40 * power * heads >= 12 * SMS:
             assert rules.splits(heads, 40 * power, 1, 0) == power       # 40 stages a split: clusters
     assert rules.splits(10, 2048, 1, 0) == 14 and rules.splits(40, 512, 1, 0) == 3
+
+
+def test_a_call_without_a_workspace_where_the_longest_length_needs_none(rules):
+    """A program that asks at its longest length, is told 1 and passes no workspace must be served at every shorter length."""
+    served = 0
+    for heads in range(1, 300):
+        for longest in STAGES:
+            if not rules.of(heads, longest, 1)["direct"]:
+                continue
+            for stages in STAGES:
+                if stages <= longest:
+                    p = rules.of(heads, stages, 1)
+                    assert p["parts"] == 0 and p["direct"], (heads, stages, longest, p)
+                    served += rules.splits(heads, stages, 1, 0) > 1
+    assert served > 0
+    for heads in (75, 148):
+        assert rules.of(heads, 11, 1, partial=1)["parts"] > 0 and rules.of(heads, 11, 0)["parts"] > 0      # these were and are refused

@@ -271,6 +271,40 @@ def test_workspace_sized_at_the_longest_length_serves_shorter_ones(B, Hkv, T, lo
         dev.close()
 
 
+def test_no_workspace_at_any_length_where_the_longest_needs_none():
+    """100 heads: unsplit at the longest length, two splits at this one.  Without a workspace the call is unsplit here too; rows that
+    leave un-normalised still need one."""
+    from grilly_next import cabi
+    from gpu_helpers import PagedCache
+    dev = cabi.Device(0)
+    try:
+        rng = np.random.default_rng(15)
+        B, Hkv, T = 20, 5, 700
+        k, v = (rng.standard_normal((B, T, Hkv, 128), dtype=np.float32) for _ in range(2))
+        q = rng.standard_normal((B, 1, Hkv, 128), dtype=np.float32)
+        pc = PagedCache(dev, B, Hkv, 128, T + 64, page_tokens=64, dtype=cabi.FP8_INT4, seed=8)
+        pc.append(k, v)
+        pc.decode(q)
+        assert pc.last_splits == 2
+        want = pc.decode(q, n_splits=1)
+        splits = C.c_int()
+        p = cabi.DecodeParams()
+        p.kv = pc.layout()
+        qd, od, pd = dev.upload(q), dev.malloc(q.nbytes), dev.malloc(B * Hkv * 130 * 4)
+        p.q, p.out, p.num_q_heads, p.max_seq_len = qd, od, Hkv, 4096
+        cabi.check(dev.L.grl_decode_pick_splits(dev.h, C.byref(p), C.byref(splits)))
+        assert splits.value == 1
+        p.max_seq_len = T
+        cabi.check(dev.L.grl_gqa_decode(dev.h, C.byref(p)))
+        np.testing.assert_array_equal(dev.download(od, q.shape, np.float32), want)
+        p.partial_out = pd
+        assert dev.L.grl_gqa_decode(dev.h, C.byref(p)) != 0 and b"workspace" in dev.L.grl_last_error()
+        for x in (qd, od, pd):
+            dev.free(x)
+    finally:
+        dev.close()
+
+
 def test_quantised_append_with_rope_and_queries():
     """RoPE of the new keys happens before the quantiser; the step's queries are rotated alongside."""
     from grilly_next import cabi
