@@ -44,6 +44,17 @@ struct GrillyCoreContext {
 
 using ContextPtr = std::shared_ptr<GrillyCoreContext>;
 
+/// A pooled buffer that goes back to its pool on every way out.  Stream order protects one that is handed out again; the pool
+/// waits before it frees one.
+struct Pooled {
+    BufferPool& pool;
+    GrillyBuffer buf;
+    Pooled(BufferPool& p, size_t bytes) : pool(p), buf(p.acquire(bytes)) {}
+    ~Pooled() { pool.release(buf); }
+    Pooled(const Pooled&) = delete;
+    Pooled& operator=(const Pooled&) = delete;
+};
+
 /// HBM-resident tensor (float32 or bf16) owned by a Device's buffer pool.  Ops that take DeviceTensors
 /// run asynchronously on the device's stream: no host copy, no wait (Device.synchronize() waits).
 struct DeviceTensor {
@@ -203,11 +214,10 @@ PYBIND11_MODULE(grilly_core, m) {
                     check(grl_memcpy_h2d(dev, t->buf.dptr, a.data(), n * 4), "DeviceTensor.from_numpy");
                     check(grl_sync(dev, 0), "DeviceTensor.from_numpy");     // the source array may go away
                 } else {
-                    GrillyBuffer tmp = ctx->pool.acquire(std::max<size_t>(n * 4, 16));
-                    check(grl_memcpy_h2d(dev, tmp.dptr, a.data(), n * 4), "DeviceTensor.from_numpy");
-                    check(grl_cast(dev, tmp.dptr, GRL_F32, t->buf.dptr, GRL_BF16, n), "DeviceTensor.from_numpy");
+                    Pooled tmp(ctx->pool, std::max<size_t>(n * 4, 16));
+                    check(grl_memcpy_h2d(dev, tmp.buf.dptr, a.data(), n * 4), "DeviceTensor.from_numpy");
+                    check(grl_cast(dev, tmp.buf.dptr, GRL_F32, t->buf.dptr, GRL_BF16, n), "DeviceTensor.from_numpy");
                     check(grl_sync(dev, 0), "DeviceTensor.from_numpy");
-                    ctx->pool.release(tmp);
                 }
                 return t;
             },
@@ -238,11 +248,10 @@ PYBIND11_MODULE(grilly_core, m) {
                     check(grl_memcpy_d2h(dev, dst, t.buf.dptr, n * 4), "DeviceTensor.to_numpy");
                     check(grl_sync(dev, 0), "DeviceTensor.to_numpy");
                 } else {
-                    GrillyBuffer tmp = t.ctx->pool.acquire(std::max<size_t>(n * 4, 16));
-                    check(grl_cast(dev, t.buf.dptr, GRL_BF16, tmp.dptr, GRL_F32, n), "DeviceTensor.to_numpy");
-                    check(grl_memcpy_d2h(dev, dst, tmp.dptr, n * 4), "DeviceTensor.to_numpy");
+                    Pooled tmp(t.ctx->pool, std::max<size_t>(n * 4, 16));
+                    check(grl_cast(dev, t.buf.dptr, GRL_BF16, tmp.buf.dptr, GRL_F32, n), "DeviceTensor.to_numpy");
+                    check(grl_memcpy_d2h(dev, dst, tmp.buf.dptr, n * 4), "DeviceTensor.to_numpy");
                     check(grl_sync(dev, 0), "DeviceTensor.to_numpy");
-                    t.ctx->pool.release(tmp);
                 }
                 return out;
             },
@@ -279,30 +288,23 @@ PYBIND11_MODULE(grilly_core, m) {
                            D = uint32_t(Q->shape[3]);
             TensorPtr o = out.has_value() ? *out : std::make_shared<DeviceTensor>(ctx, Q->shape, GRL_F32);
             if (o->shape != Q->shape || o->ctx.get() != ctx.get()) throw std::runtime_error("out must have Q's shape and Device");
-            GrillyBuffer lens;
+            std::optional<Pooled> lens;
             if (seqLens.has_value()) {
                 if (seqLens->ndim() != 1 || seqLens->shape(0) != B) throw std::runtime_error("seq_lens must be (batch,)");
-                lens = ctx->pool.acquire(size_t(B) * 4);
+                lens.emplace(ctx->pool, size_t(B) * 4);
                 // The lengths leave the caller's array at the call.  A copy had to be waited for, and with it all the work before it
                 // (2 x 8 heads x 68 tokens 28.9 -> 8.9 us a call, 8 x 32 heads of up to 4096 tokens 801 -> 773).
                 if (size_t(B) * 4 <= GRL_PUT_BYTES) {
-                    check(grl_put(ctx->device.handle(), lens.dptr, seqLens->data(), size_t(B) * 4), "flash_attention2: seq_lens upload");
+                    check(grl_put(ctx->device.handle(), lens->buf.dptr, seqLens->data(), size_t(B) * 4), "flash_attention2: seq_lens upload");
                 } else {
-                    ctx->pool.upload(lens, seqLens->data(), size_t(B) * 4);
+                    ctx->pool.upload(lens->buf, seqLens->data(), size_t(B) * 4);
                     check(grl_sync(ctx->device.handle(), 0), "flash_attention2: seq_lens upload");
                 }
             }
             const ops::RopeMode mode = ropeTheta != 0.0f ? parseRopeMode(ropeMode, false) : ops::RopeMode::None;
-            try {
-                ops::flashAttention2Device(ctx->batch, ctx->cache, Q->buf, K->buf, V->buf, o->buf, Q->dtype, o->dtype, B, S,
-                                           H, D, scale, causal, lens.valid() ? &lens : nullptr, mode,
-                                           ropeTheta != 0.0f ? ropeTheta : 10000.0f, ropeScaling);
-            } catch (...) {
-                ctx->pool.release(lens);
-                throw;
-            }
-            // stream order protects a pooled buffer that is handed out again; the pool waits before it frees one
-            ctx->pool.release(lens);
+            ops::flashAttention2Device(ctx->batch, ctx->cache, Q->buf, K->buf, V->buf, o->buf, Q->dtype, o->dtype, B, S, H, D,
+                                       scale, causal, lens ? &lens->buf : nullptr, mode,
+                                       ropeTheta != 0.0f ? ropeTheta : 10000.0f, ropeScaling);
             return o;
         },
         py::arg("device"), py::arg("Q"), py::arg("K"), py::arg("V"), py::arg("mask") = py::none(),

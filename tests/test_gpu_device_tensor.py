@@ -108,6 +108,16 @@ def test_put_sizes_and_refusals():
         dev.close()
 
 
+def test_a_refused_ragged_call_gives_its_lengths_back_to_the_pool(core, ctx):
+    q = core.DeviceTensor.empty(ctx, (2, 1, 64, 64), "fp32")
+    out = lambda s: s["total_acquired"] - s["total_released"]
+    before = out(ctx.pool_stats())
+    for _ in range(2):
+        with pytest.raises(RuntimeError, match="rope_mode"):
+            core.flash_attention2(ctx, q, q, q, out=q, seq_lens=np.array([64, 3], np.int32), rope_theta=10000.0, rope_mode="sideways")
+    assert out(ctx.pool_stats()) == before
+
+
 def test_decode_on_device_tensors_equals_host_path(core, ctx):
     rng = np.random.default_rng(3)
     B, Hq, Hkv, D, T = 2, 8, 2, 128, 150
