@@ -26,7 +26,7 @@ CUDA_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", 
 
 CU_SOURCES = ["device.cu", "host_copy.cu", "flash.cu", "prefill_fp32.cu", "prefill_sm100.cu", "decode_splitkv.cu", "decode_mma.cu", "p2p_merge.cu", "kv_evict.cu",
               "kv_cache.cu", "rope_mask.cu", "nccl_group.cu", "linear_sm100.cu", "attention_unfused.cu"]
-HEADERS = ["common.cuh", "decode_plan.h", "host_copy.cuh", "sgemm.cuh", "tmem_ops.cuh", "sm100_ptx.cuh", os.path.join(ROOT, "include", "grilly_cuda.h")]
+HEADERS = ["common.cuh", "decode_plan.h", "decode_ring.h", "host_copy.cuh", "sgemm.cuh", "tmem_ops.cuh", "sm100_ptx.cuh", os.path.join(ROOT, "include", "grilly_cuda.h")]
 
 
 def _newer(target, deps):

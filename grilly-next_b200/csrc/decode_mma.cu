@@ -27,41 +27,29 @@
 
 #include "common.cuh"
 #include "decode_plan.h"
+#include "decode_ring.h"
 
 namespace grl {
 namespace dmma {
 
 constexpr int P = 64;               // tokens per ring stage: one 64-token page, or two / four smaller ones side by side
 constexpr int D = 128;              // head_dim of the quantised instance (the bf16 instances carry theirs as HD)
-// FORM of an instance: over the bf16 cache, over the quantised cache, and that with one CTA an SM.
-enum Form { BF16 = 0, QUANT_PAIR = 1, QUANT_WIDE = 2 };
-// Compute warps, in groups of four that take the ring's stages in turn (16 tokens of one a warp), and the producer warps behind
-// them (stages in turn, too).  A producer's serial chain of waits and copies is some 1300 cycles a stage beside busy compute
-// warps, so the quantised stages, which are small, have several (131072 tokens x 8 heads, decode alone: 15 compute warps and one
-// producer 79 us, 14 and 2 64, 12 and 4 64; with the shorter conversion 12 and 1 61, 12 and 4 59; four compute warps and 1 / 2
-// producers, two CTAs an SM, 66 / 65).
-template <int FORM> struct Warps {
-    static constexpr int COMPUTE = FORM == QUANT_WIDE ? 12 : 4, PROD = FORM == QUANT_WIDE ? 4 : FORM == QUANT_PAIR ? 2 : 1;
-    static constexpr int THREADS = 32 * (COMPUTE + PROD), CTAS = FORM == QUANT_WIDE ? 1 : 2;
-};
 // The shared-memory ring of an instance.  After the ring: 256 bytes of barriers and flags, 128 of block table a producer, 256 a compute
 // warp over the quantised cache (1/scale of its 16 tokens x 4 groups), 1 KiB of slack for the 1024-byte alignment of the ring.
 template <int FORM, int HD> struct Ring {
     static constexpr int SLAB = P * HD * 2;             // 64 tokens of K (or V) for one kv head: 16 KiB at head_dim 128
     static constexpr int STAGE = 2 * SLAB;              // K then V
-    static constexpr int NST = 3 * 128 / HD;            // ring stages: 96 KiB in flight per CTA
 };
 constexpr int QK_BYTES = P * D;          // 8 KiB of key bytes per 64 tokens of a kv head
 constexpr int QV_BYTES = P * D / 2;      // 4 KiB of packed value nibbles
-template <int NST_> struct QuantRing {
+struct QuantRing {
     static constexpr int SLAB = 0;
-    static constexpr int NST = NST_;
     static constexpr int STAGE = 13 * 1024;  // keys at 0, values at 8 KiB, scales at 12 KiB
 };
-template <> struct Ring<QUANT_PAIR, 128> : QuantRing<6> {};
-template <> struct Ring<QUANT_WIDE, 128> : QuantRing<14> {};
+template <> struct Ring<QUANT_PAIR, 128> : QuantRing {};
+template <> struct Ring<QUANT_WIDE, 128> : QuantRing {};
 template <int FORM, int HD> struct Smem {
-    static constexpr int BAR = Ring<FORM, HD>::NST * Ring<FORM, HD>::STAGE;
+    static constexpr int BAR = Stages<FORM, HD>::NST * Ring<FORM, HD>::STAGE;
     static constexpr int TOTAL = BAR + 256 + 128 * Warps<FORM>::PROD + (FORM != BF16 ? 256 * Warps<FORM>::COMPUTE : 0) + 1024;
 };
 constexpr float kLog2e = 1.4426950408889634f;
@@ -275,10 +263,10 @@ decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
     static_assert(HD == 128 || (HD == 64 && !QUANT), "head_dim 128, or 64 over the bf16 cache");
     static_assert(FORM == QUANT_WIDE || Smem<FORM, HD>::TOTAL <= kAloneSmem, "the wider allocation holds the ring");
     constexpr int D = HD;
-    constexpr int NST = Ring<FORM, HD>::NST, STAGE = Ring<FORM, HD>::STAGE, SMEM_BAR = Smem<FORM, HD>::BAR;
+    constexpr int NST = Stages<FORM, HD>::NST, STAGE = Ring<FORM, HD>::STAGE, SMEM_BAR = Smem<FORM, HD>::BAR;
     constexpr int SLAB = Ring<FORM, HD>::SLAB;
     constexpr int COMPUTE = Warps<FORM>::COMPUTE, PROD = Warps<FORM>::PROD, kThreads = Warps<FORM>::THREADS;
-    static_assert(2 * NST * 8 + 16 <= 256 && NST <= 32, "barrier block; a lane a stage in the first fill");
+    static_assert(2 * NST * 8 + 16 <= 256, "barrier block");
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw_addr = smem_u32(smem_raw);
     const uint32_t base = (raw_addr + 1023u) & ~1023u;
@@ -428,7 +416,7 @@ decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         }
         float* inv_w = reinterpret_cast<float*>(smem + SMEM_BAR + 256 + 128 * PROD) + warp * 64;   // [16 tokens][4 groups]
         bool ok = true;
-        constexpr int GROUPS = COMPUTE / 4;
+        constexpr int GROUPS = Warps<FORM>::GROUPS;
         const int slice = warp & 3;             // which 16 tokens of a stage
         int s = (warp >> 2) - GROUPS;           // ring slot; the parity of its phase
         uint32_t parity = 0;
