@@ -380,14 +380,7 @@ decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
                 issued = i + 1;
             }
         }
-        if (lane == 0) {
-            if (*ctx.abort) {   // copies already issued must land before the shared memory is released
-                const long long t0 = clock64();
-                for (int i = max(0, issued - NST); i < issued; ++i)
-                    if (i % PROD == pr)
-                    while (!mbar_try_wait(full(i % NST), (i / NST) & 1) && clock64() - t0 < ctx.limit) {}
-            }
-        }
+        if (lane == 0) bt_s[0] = issued;
     } else if constexpr (QUANT) {
         // ------------------------------------------------------------------ compute over the quantised cache
         // Element permutation of the two products.  QK^T: k-step (grp, w) of lane (g, t4) covers elements
@@ -638,8 +631,19 @@ decode_mma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant
         l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
     }
 
-    // ---- merge the four warps' partials (the ring is idle now: reuse it)
     __syncthreads();
+    if (*ctx.abort) {
+        // A wait ran out: what has been issued must land before the shared memory is used again and released.  A producer that stops cannot
+        // tell which of its stages another group has left unread, nor whether a slot is someone else's by now, so each slot waits for
+        // the last stage that any of them issued there; for local copies, whatever budget the caller has set for the waits.
+        if (tid < NST) {
+            const int i = last_in_slot<NST, PROD>(reinterpret_cast<const int*>(smem + SMEM_BAR + 256), 32, tid);
+            const long long t0 = clock64();
+            while (i >= 0 && !mbar_try_wait(full(tid), (i / NST) & 1) && clock64() - t0 < kDefaultWaitLimitCycles) {}
+        }
+        __syncthreads();
+    }
+    // ---- merge the warps' partials (the ring is idle now: reuse it)
     // The next kernel may launch under the merges.  Not before: its CTAs would take slots beside this kernel's and end up
     // unevenly placed (two on some SMs, none on others: 196 us instead of 107 for a 131072-token quantised step).  Where the
     // CTAs have an SM each the next one's could only wait for this one's shared memory, so it is left to start at the end

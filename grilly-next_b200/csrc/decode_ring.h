@@ -2,6 +2,12 @@
 // Constants only, so that the order of its waits can be checked without a GPU.
 #pragma once
 
+#ifdef __CUDACC__
+#define GRL_RING_FN __host__ __device__
+#else
+#define GRL_RING_FN
+#endif
+
 namespace grl {
 namespace dmma {
 
@@ -30,6 +36,16 @@ template <int FORM, int HD> struct Stages {
     static constexpr int NST = FORM == QUANT_WIDE ? 15 : FORM == QUANT_PAIR ? 6 : 3 * 128 / HD;
     static_assert(NST % Warps<FORM>::GROUPS == 0 && Warps<FORM>::PROD * Warps<FORM>::GROUPS <= NST, "phases of a slot in order");
 };
+
+// The last stage that was issued into slot s, or -1.  issued[stride * p] is one past the last stage that producer p has issued.  After a
+// wait that ran out, these stages are the only ones whose copies may still be in flight, and each is the phase its barrier is in.
+template <int NST, int PROD> GRL_RING_FN int last_in_slot(const int* issued, int stride, int s) {
+    int last = -1;
+    for (int p = 0; p < PROD; ++p)
+        for (int j = issued[stride * p] - 1, n = 0; j > last && n < NST; j -= PROD, ++n)
+            if (j % NST == s) last = j;
+    return last;
+}
 
 }  // namespace dmma
 }  // namespace grl
