@@ -585,7 +585,6 @@ int grl_kv_append(grl_device* dev, const grl_append_params* p) {
     dev->status_dirty = true;
     if (p->rope_mode != GRL_ROPE_NONE) a.freq = cached_rope_freq(dev, kv.head_dim, p->rope_theta, p->rope_scaling);
     if (kv.cache_dtype == GRL_FP8_INT4) {
-        // K and V: one warp per (token, kv head, group of 32); the queries, if any, through the plain kernel
         const long long warps = (long long)p->n_new * kv.num_kv_heads * (kv.head_dim / 32);
         if (warps <= kStepWarps) {      // a decode step: one wide CTA per sequence does keys, values, queries and the length
             a.update_lens = p->update_lens ? 1 : 0;
@@ -593,18 +592,15 @@ int grl_kv_append(grl_device* dev, const grl_append_params* p) {
             GRL_LAUNCHED("kv_append_quant_step_kernel");
             return GRL_OK;
         }
-        // eight heads a warp once there are enough tokens to fill the SMs (64 warps each) all the same
+        // Bulk: K and V by a warp per (token, kv head, group of 32), then the queries, if any, by the float32 cache's kernels.
+        // Eight heads a warp once there are enough tokens to fill the SMs (64 warps each) all the same
         a.heads_per_item = warps * kv.batch / 8 >= 64LL * dev->prop.multiProcessorCount ? 8 : 1;
         int ctas = (int)((warps / a.heads_per_item + 7) / 8);
         if (ctas > 1024) ctas = 1024;
-        a.q_in = nullptr;       // bulk append: the queries go through the plain kernel below
-        a.update_lens = 0;
         GRL_CUDA(launch_pdl(kv_append_quant_kernel, dim3(ctas, kv.batch), 256, 0, dev->stream, a));
         GRL_LAUNCHED("kv_append_quant_kernel");
-        a.q_in = p->q_in;
         if (p->q_in) {
             a.skip_kv = 1;
-            a.update_lens = 0;
             if (append_rows_fit(a)) {
                 GRL_CUDA(launch_pdl(kv_append_rows_kernel<float>, append_rows_grid(dev, a), 256, 0, dev->stream, a));
             } else {
