@@ -1,20 +1,22 @@
 // GQA decode over the paged bf16 cache, head_dim 128 or 64, pages of 64, 32 or 16 tokens: the fast path.
 //
 // Replaces shaders/gqa-attention.glsl:34-130 like decode_splitkv.cu, for the geometry of the
-// benchmark configurations.  One CTA owns (split, kv head, sequence); a producer warp streams
+// benchmark configurations.  One CTA owns (split, kv head, sequence); producer warps (one over the bf16 cache) stream
 // whole (page, kv head) slabs -- 16 KiB of K and 16 KiB of V, each contiguous in HBM -- into a
-// 3-stage shared-memory ring with TMA (128-byte swizzle, mbarrier complete_tx); four compute
-// warps each take 16 of the page's 64 tokens and run QK^T and PV on tensor cores
+// shared-memory ring with TMA (128-byte swizzle, mbarrier complete_tx); compute
+// warps in groups of four (one group over the bf16 cache) each take 16 of a stage's 64 tokens and run QK^T and PV on tensor cores
 // (mma.sync m16n8k16, the group's query heads padded to the 16-row operand, q split into
 // bf16 hi+lo so that its fp32 precision survives), with a private fp32 online softmax in the
-// exp2 domain.  K and V cross HBM -> SM exactly once; the four warps' partials are merged in
-// shared memory and leave the CTA as (O un-normalised, m, l), the layout lse_merge_kernel reads.  Splits of one head that fit a
+// exp2 domain.  K and V cross HBM -> SM exactly once; the compute warps' partials are merged in
+// shared memory and leave the CTA as (O un-normalised, m, l), the layout lse_merge_kernel reads.  Warps, ring stages and the order of
+// their waits in each of the three forms: decode_ring.h.  Splits of one head that fit a
 // thread-block cluster merge through its shared memory instead, and a launch sets up its ring and barriers under the kernel before
 // it.  Append + decode step: 1 sequence x 8 kv heads x 1001 tokens 19.4 us before, 9.9 now (latency); 32 x 8 x 4096 93 and 85 us
 // (HBM); 1 x 8 x 131072 104 and 94 us (HBM; the decode alone 90), quantised 107 and 59 us (instructions: 444 a 16-token slice).
 //
-// The same kernel, instantiated for the quantised cache (GRL_FP8_INT4: FP8-E4M3 keys, INT4 values, one float16 scale
-// per 32 key elements, cpp/src/ops/kv_cache.cpp:272-399 and :500-577), streams 12.5 KiB per (page, kv head) instead
+// The same kernel, in two forms for the quantised cache (GRL_FP8_INT4: FP8-E4M3 keys, INT4 values, one float16 scale
+// per 32 key elements, cpp/src/ops/kv_cache.cpp:272-399 and :500-577): four compute and two producer warps, two CTAs an SM, or twelve
+// and four, one CTA an SM.  It streams 12.5 KiB per (page, kv head) instead
 // of 32 and dequantises in registers: key bytes become f16 by three integer operations per pair (every code is an
 // exact f16 once divided by 256), the four scale groups of a head accumulate separately and are combined with 1/scale per
 // token; value nibbles become f16 by one logic operation and one subtraction per pair (1024 + n or 64 + n in the
