@@ -118,6 +118,52 @@ def test_fused_decode_exchange_times_out_in_a_replayed_graph():
         dev.close()
 
 
+@pytest.mark.parametrize("form,B,Hkv,T", [("quantised, one CTA an SM", 1, 2, 131072), ("quantised, thirds", 19, 8, 4096),
+                                          ("quantised, unsplit", 23, 8, 2400), ("bf16", 1, 2, 131072)])
+def test_ring_waits_that_run_out_are_reported_and_the_next_decode_is_right(form, B, Hkv, T):
+    """A budget of one cycle for the waits on the ring.  A CTA that gives up waits for its copies in flight before it reuses their memory.
+
+    A wait that the hardware ends within its first try does not run out, so a launch may come through: its result is then the right one.
+    """
+    from grilly_next import cabi
+    from gpu_helpers import PagedCache
+    from oracle import attention_oracle as orc
+    dev = cabi.Device(0)
+    try:
+        rng = np.random.default_rng(8)
+        group, D = 4, 128
+        Hq = group * Hkv
+        pc = PagedCache(dev, B, Hkv, D, T, dtype=cabi.BF16 if form == "bf16" else cabi.FP8_INT4)
+        for t0 in range(0, T, 16384):
+            n = min(16384, T - t0)
+            pc.append(rng.standard_normal((B, n, Hkv, D), dtype=np.float32), rng.standard_normal((B, n, Hkv, D), dtype=np.float32))
+        q = rng.standard_normal((B, 1, Hq, D), dtype=np.float32)
+        want = pc.decode(q)
+        qd, out = dev.upload(q), dev.malloc(B * Hq * D * 4)
+        p = cabi.DecodeParams()
+        p.kv, p.q, p.out, p.num_q_heads, p.max_seq_len = pc.layout(), qd, out, Hq, T
+        splits, wb = C.c_int(), C.c_size_t()
+        cabi.check(dev.L.grl_decode_pick_splits(dev.h, C.byref(p), C.byref(splits)))
+        cabi.check(dev.L.grl_decode_workspace_bytes(C.byref(p), splits, C.byref(wb)))
+        p.workspace, p.workspace_bytes = dev.malloc(wb.value), wb.value
+        cabi.check(dev.L.grl_device_set_wait_limits(dev.h, 1, 0))
+        for _ in range(100):
+            cabi.check(dev.L.grl_gqa_decode(dev.h, C.byref(p)))
+            rc = dev.L.grl_sync(dev.h, 0)
+            if rc != 0:
+                break
+            assert np.array_equal(dev.download(out, q.shape, np.float32), want)
+        assert rc == cabi.ERR_TIMEOUT, (rc, dev.L.grl_last_error())
+        cabi.check(dev.L.grl_device_set_wait_limits(dev.h, 0, 0))
+        assert np.array_equal(pc.decode(q), want)        # nothing of the abandoned step is left in counters, workspace or status
+        kg, vg = zip(*(pc.gather(b) for b in range(min(B, 2))))
+        oracle = orc.gqa_decode_attention(q[:2], np.stack(kg), np.stack(vg), Hq, Hkv, D)
+        assert np.abs(want[:2] - oracle).max() <= 5e-3
+        _ordinary_decode_passes(dev, cabi)
+    finally:
+        dev.close()
+
+
 def test_wait_limits_setter_and_defaults():
     from grilly_next import cabi
     dev = cabi.Device(0)
