@@ -391,6 +391,13 @@ __global__ void __launch_bounds__(256) kv_append_quant_kernel(const __grid_const
 // heads (forming it per key element and per query pair took most of the kernel: 1 sequence x 8 kv heads, append before decode
 // 8.0 -> 4.3 us of the step).
 constexpr int kStepWarps = 32;
+// Dynamic shared memory that the kernel does not use: it keeps the decode's CTAs (82 KiB and more) off an append's SM while there are no
+// more sequences than SMs.  Beside one, half of an SM's two decode CTAs would start under the append and the other half after it, and
+// a decode that needs nearly every slot took longer than behind the kernel before this one.  Append + decode, us, that kernel / sharing an SM /
+// alone on it: 9 sequences x 8 kv heads x 700 tokens 21.2 / 21.8 / 18.3, 36 x 8 x 300 16.2 / 16.6 / 13.0, 18 x 8 x 300 16.8 / 17.2 / 13.7, 64 x 2 x 500 13.9
+// / 13.5 / 12.7; 8 x 8 x 700 16.5 / 13.8 / 13.8, 25 x 8 x 2000 42.4 / 34.7 / 34.5, 32 x 8 x 4096 75.0 / 61.8 / 62.0.  More sequences than SMs need two
+// appends an SM: 200 x 1 x 700 21.1 / 17.1.
+constexpr int kStepAloneSmem = 150 * 1024;
 __global__ void __launch_bounds__(32 * kStepWarps) kv_append_quant_step_kernel(const __grid_constant__ AppendArgs a) {
     __shared__ float2 cs[kStepWarps * 16];           // (cos, sin) [token][pair]: n_new * D / 2 <= 32 * 32 / 2
     const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
@@ -588,7 +595,13 @@ int grl_kv_append(grl_device* dev, const grl_append_params* p) {
         const long long warps = (long long)p->n_new * kv.num_kv_heads * (kv.head_dim / 32);
         if (warps <= kStepWarps) {      // a decode step: one wide CTA per sequence does keys, values, queries and the length
             a.update_lens = p->update_lens ? 1 : 0;
-            GRL_CUDA(launch_pdl(kv_append_quant_step_kernel, dim3(kv.batch), 32 * kStepWarps, 0, dev->stream, a));
+            const int smem = kv.batch <= dev->prop.multiProcessorCount ? kStepAloneSmem : 0;
+            static bool attr_set[64] = {};
+            if (!attr_set[dev->ordinal & 63]) {
+                GRL_CUDA(cudaFuncSetAttribute(kv_append_quant_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStepAloneSmem));
+                attr_set[dev->ordinal & 63] = true;
+            }
+            GRL_CUDA(launch_pdl(kv_append_quant_step_kernel, dim3(kv.batch), 32 * kStepWarps, smem, dev->stream, a));
             GRL_LAUNCHED("kv_append_quant_step_kernel");
             return GRL_OK;
         }
